@@ -100,6 +100,9 @@ struct rsg_solver {
     double* dinv = nullptr;
     SplitFactors<double> s64;
     SplitFactors<float> s32;
+    RingFactors<double> r64;     // the thread-block sweeps' records where they run on the ring (rsg_ring.cu)
+    RingFactors<float> r32;
+    RingDev ring[2];             // steps for FP64 and FP32 sweep vectors
     bool cta = false;
     bool splitCpr = false;       // CPR on the thread-block path: V-cycle grid-wide (PrecDev::split)
     bool escalated = false;      // precision form: failed systems re-solved with FP64 sweep vectors (until the next set-up)
@@ -145,6 +148,7 @@ struct rsg_solver {
         int split = -1;              // CPR form on the thread-block path: -1 as planned (splitCpr), 0 one kernel, 1 split
         int vform = 3;
         int cpr2Threads = 256;
+        int ring = 1;                // BILU0 stage on the ring where it fits (0: the thread count's own kernel)
         std::string desc = "defaults";
     } tune;
     unsigned long long patHash = 0;   // FNV-1a of the plan's pattern (0: not computed)
@@ -177,6 +181,7 @@ void free_plan(rsg_solver* h) {
     h->dp = DevPlan{};
     h->val = nullptr; h->lu = nullptr; h->luf = nullptr; h->work = nullptr; h->dinv = nullptr;
     h->s64 = SplitFactors<double>{}; h->s32 = SplitFactors<float>{}; h->cta = false;
+    h->r64 = RingFactors<double>{}; h->r32 = RingFactors<float>{}; h->ring[0] = h->ring[1] = RingDev{};
     h->amg = DevAmg{}; h->haveAmg = false; h->amgLevels = 0; h->d_nfb = nullptr;
     h->V = BicgVecs{};
     h->b = h->xout = h->tmp = nullptr;
@@ -242,6 +247,16 @@ int alloc_plan(rsg_solver* h) {
     // GPU's loads in flight); a single system keeps the one-kernel form (one launch per application instead of a
     // launch per pass). Both give the same results bit for bit, so a system's result does not depend on its batch.
     h->splitCpr = h->cta && (h->opt.sweep == 3 || (h->opt.sweep == 0 && P.nsys > 1));
+    for (int v32 = 0; v32 < 2 && h->cta; ++v32) {
+        RingHost H;
+        ring_steps(P, v32 != 0, H);
+        if (H.ok) {
+            RingDev& R = h->ring[v32];
+            if ((rc = upload(M, &R.desc, H.desc, st)) || (rc = upload(M, &R.stepOff, H.stepOff, st))) return rc;
+            R.maxSteps = H.maxSteps; R.maxRows = H.maxRows; R.maxWidth = H.maxWidth;
+            R.maxStage32 = H.maxStage32; R.maxStage64 = H.maxStage64;
+        }
+    }
     const size_t N = size_t(P.n) * NB, E = size_t(P.nnzb) * NB2;
     if ((rc = dalloc(M, &h->val, E)) || (rc = dalloc(M, &h->val0, E)) || (rc = dalloc(M, &h->b, N)) || (rc = dalloc(M, &h->xout, N)) ||
         (rc = dalloc(M, &h->tmp, N)))
@@ -297,6 +312,21 @@ int precond_launches(const PrecDev& M) {
     return M.cpr || M.cta || M.kind == 2 ? 1 : 2;
 }
 
+// whether the thread-block BILU0 stage of this factor kind (0 FP64, 1 FP32 factors with FP64 vectors, 3 all FP32) runs on
+// the ring: its vector and steps fit one SM, and the launch shape is not fixed by the options (the one-kernel CPR
+// application and a BILU0 stage of a given thread count read the component-major records)
+bool ring_on(const rsg_solver* h, int kind) {
+    if (!h->cta || kind == 2 || h->opt.cpr2_threads != 0 || !h->tune.ring) return false;
+    if (h->opt.precond == RSG_PREC_CPR && h->opt.sweep == 1) return false;
+    return ring_fits(h->ring[kind == 3 ? 1 : 0], kind != 0, kind == 3);
+}
+int prec_kind(const rsg_solver* h) {
+    if (h->opt.precond == RSG_PREC_JACOBI) return 2;
+    if (h->opt.precision == RSG_MIXED) return 1;
+    if (h->opt.precision == RSG_MIXED_F32) return h->escalated ? 1 : 3;
+    return 0;
+}
+
 PrecDev prec_dev(rsg_solver* h) {
     PrecDev M;
     if (h->opt.precond == RSG_PREC_JACOBI) { M.kind = 2; M.dinv = h->dinv; }
@@ -304,6 +334,7 @@ PrecDev prec_dev(rsg_solver* h) {
     else if (h->opt.precision == RSG_MIXED_F32) { M.kind = h->escalated ? 1 : 3; M.luf = h->luf; }
     else { M.kind = 0; M.lu = h->lu; }
     M.val = h->val;
+    M.err = h->d_err;
     M.y32 = h->V.y32;
     M.yt = h->V.yt;
     if (h->opt.precond == RSG_PREC_CPR && h->haveAmg) { M.cpr = true; M.amg = &h->amg; }
@@ -313,6 +344,9 @@ PrecDev prec_dev(rsg_solver* h) {
         M.cta = true;
         M.s64 = h->s64;
         M.s32 = h->s32;
+        M.r64 = h->r64;
+        M.r32 = h->r32;
+        if (ring_on(h, M.kind)) M.ring = h->ring;
         M.split = M.cpr && (h->tune.split >= 0 ? h->tune.split != 0 : h->splitCpr);
         M.vform = h->tune.vform;
         M.cpr2Threads = h->tune.cpr2Threads;
@@ -546,6 +580,38 @@ int alloc_split(rsg_solver* h, SplitFactors<T>& F) {
     return RSG_OK;
 }
 
+template <class T>
+int alloc_ring(rsg_solver* h, RingFactors<T>& F) {
+    const size_t ow = ring_ov_words(sizeof(T) == 4);
+    int rc;
+    if ((rc = dalloc(h->pmem, &F.L, size_t(h->dp.n) * LREC)) || (rc = dalloc(h->pmem, &F.UD, size_t(h->dp.n) * UREC)) ||
+        (rc = dalloc(h->pmem, &F.Lov, size_t(h->dp.nLov) * ow)) || (rc = dalloc(h->pmem, &F.Uov, size_t(h->dp.nUov) * ow)))
+        return rc;
+    return RSG_OK;
+}
+// the thread-block sweeps' records of the current factors, in the layout of the sweeps that will read them
+int pack_factors(rsg_solver* h) {
+    const int kind = prec_kind(h);
+    int rc;
+    if (kind == 0) {
+        if (ring_on(h, kind)) {
+            if (!h->r64.L && (rc = alloc_ring(h, h->r64))) return rc;
+            launch_ring_pack(h->dp, h->lu, h->r64, h->stream);
+        } else {
+            if (!h->s64.L && (rc = alloc_split(h, h->s64))) return rc;
+            launch_pack_f64(h->dp, h->lu, h->s64, h->stream);
+        }
+    } else if (ring_on(h, kind)) {
+        if (!h->r32.L && (rc = alloc_ring(h, h->r32))) return rc;
+        launch_ring_pack(h->dp, h->luf, h->r32, h->stream);
+    } else {
+        if (!h->s32.L && (rc = alloc_split(h, h->s32))) return rc;
+        launch_pack_f32(h->dp, h->luf, h->s32, h->stream);
+    }
+    h->launches += 1;
+    return RSG_OK;
+}
+
 int ensure_precond_storage(rsg_solver* h) {
     const size_t E = size_t(h->plan.nnzb) * NB2;
     int rc;
@@ -560,10 +626,8 @@ int ensure_precond_storage(rsg_solver* h) {
             if ((rc = dalloc(h->pmem, &h->V.yt, size_t(h->plan.n) * NB))) return rc;
             RSG_CUDA(cudaMemsetAsync(h->V.yt, 0, size_t(h->plan.n) * NB * sizeof(unsigned long long), h->stream));
         }
-        if (h->cta && !h->s32.L && (rc = alloc_split(h, h->s32))) return rc;
     } else {
         if (!h->lu && (rc = dalloc(h->pmem, &h->lu, E))) return rc;
-        if (h->cta && !h->s64.L && (rc = alloc_split(h, h->s64))) return rc;
     }
     return RSG_OK;
 }
@@ -856,8 +920,8 @@ int build_dev_amg(rsg_solver* h, const std::vector<SysAmg>& H) {
     if ((rc = dalloc(M, &G.val, size_t(ents) + OV_CHUNK - 1)) || (rc = dalloc(M, &G.valf, size_t(ents) + OV_CHUNK - 1)) || (rc = dalloc(M, &G.apVal, size_t(std::max(aps, 1)))) ||
         (rc = dalloc(M, &G.lu, size_t(std::max(lus, 1)))) || (rc = dalloc(M, &G.luf, size_t(std::max(lus, 1)))) ||
         (rc = dalloc(M, &G.invf, size_t(std::max(lus, 1)))) ||
-        (rc = dalloc(M, &G.piv, size_t(std::max(lurows, 1)))) || (rc = dalloc(M, &G.x, size_t(rows))) || (rc = dalloc(M, &G.b, size_t(rows))) ||
-        (rc = dalloc(M, &G.r, size_t(rows))) || (rc = dalloc(M, &G.xf, size_t(rows))) || (rc = dalloc(M, &G.bf, size_t(rows))) ||
+        (rc = dalloc(M, &G.piv, size_t(std::max(lurows, 1)))) || (rc = dalloc(M, &G.x, size_t(rows) + 2)) || (rc = dalloc(M, &G.b, size_t(rows))) ||
+        (rc = dalloc(M, &G.r, size_t(rows))) || (rc = dalloc(M, &G.xf, size_t(rows) + 4)) || (rc = dalloc(M, &G.bf, size_t(rows))) ||
         (rc = dalloc(M, &G.rf, size_t(rows))))
         return rc;
     // the fused V-cycle's phase table and barrier counter (the split CPR form)
@@ -1001,30 +1065,41 @@ int tune_shapes(rsg_solver* h) {
     const bool cprCta = h->opt.precond == RSG_PREC_CPR && h->cta && h->haveAmg;
     // a single system under the automatic sweep choice: the one-kernel application (one launch, one SM) and the split
     // form (the V-cycle's passes grid-wide) are both candidates; they give the same results bit for bit
-    const bool free_split = cprCta && h->opt.sweep == 0 && h->plan.nsys == 1;
-    const bool split = cprCta && (h->splitCpr || free_split);
-    t.split = h->splitCpr ? 1 : 0;
+    // (with the BILU0 stage on the ring only the split form: 1,600-13,000 rows alone, it is faster at every size)
+    int packed = h->tune.ring;                       // the layout the set-up packed the factors in
+    h->tune = t;
+    const bool ring = cprCta && ring_on(h, prec_kind(h));
+    const bool free_split = cprCta && h->opt.sweep == 0 && h->plan.nsys == 1 && !ring;
+    const bool split = cprCta && (h->splitCpr || free_split || ring);
+    t.split = h->splitCpr || ring ? 1 : 0;
     t.vform = h->opt.vcycle_form ? h->opt.vcycle_form : 3;
     if (t.vform == 1 && h->amg.nPhases == 0) t.vform = 2;                  // no phase table for this hierarchy
     t.cpr2Threads = h->opt.cpr2_threads ? h->opt.cpr2_threads : 256;
     const bool free_form = h->opt.vcycle_form == 0, free_thr = h->opt.cpr2_threads == 0;
-    auto describe = [](const rsg_solver::Tune& c) {
+    auto describe = [ring](const rsg_solver::Tune& c) {
         if (c.split == 0) return std::string("cpr_form=one-kernel");
-        return std::string("vcycle_form=") + std::to_string(c.vform) + " cpr2_threads=" + std::to_string(c.cpr2Threads);
+        return std::string("vcycle_form=") + std::to_string(c.vform) +
+               (ring && c.ring ? std::string(" bilu0=ring") : " cpr2_threads=" + std::to_string(c.cpr2Threads));
+    };
+    // a shape is taken: the records its BILU0 stage reads are packed if they are not yet
+    auto take = [&](const rsg_solver::Tune& c) {
+        const bool repack = ring && c.ring != packed;
+        packed = c.ring;
+        h->tune = c;
+        return repack ? pack_factors(h) : RSG_OK;
     };
     if (!split) { t.desc = "no split CPR: fixed shapes"; h->tune = t; return RSG_OK; }
     if (!h->opt.autotune || (!free_form && !free_thr && !free_split)) {
         t.desc = describe(t) + (h->opt.autotune ? " source=options" : " source=defaults");
-        h->tune = t;
-        return RSG_OK;
+        return take(t);
     }
-    const int key2 = h->opt.precision * 1000 + h->opt.vcycle_form * 10000 + h->opt.cpr2_threads + h->device * 100000 +
+    const int key2 = (ring ? 2000000 : 0) + h->opt.sweep * 10000000 + h->opt.precision * 1000 + h->opt.vcycle_form * 10000 + h->opt.cpr2_threads + h->device * 100000 +
                      (free_split ? 1000000 : 0);
     const auto key = std::make_pair(pattern_hash(h), key2);
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tune_cache.find(key);
-        if (it != g_tune_cache.end()) { h->tune = it->second; return RSG_OK; }
+        if (it != g_tune_cache.end()) return take(it->second);
     }
     const size_t N = size_t(h->plan.n) * NB;
     RSG_CUDA(cudaMemsetAsync(h->tmp, 0, N * sizeof(double), h->stream));
@@ -1041,6 +1116,13 @@ int tune_shapes(rsg_solver* h) {
             if (f == 1 && h->amg.nPhases == 0) continue;
             rsg_solver::Tune c;
             c.split = 1;
+            c.ring = ring ? 1 : 0;
+            if (ring && thr == 256) {                                  // the ring's own shape follows from the level widths
+                c.vform = f;
+                cand.push_back(c);
+            }
+            if (ring && h->opt.sweep == 0) continue;                   // (faster than the others at every size measured)
+            c.ring = 0;
             c.vform = f;
             c.cpr2Threads = thr;
             cand.push_back(c);
@@ -1052,9 +1134,8 @@ int tune_shapes(rsg_solver* h) {
     std::string timings;
     for (const auto& c : cand) {
         if (c.vform == 1 && !fusedOk) continue;
-        h->tune = c;
-        int rc = precond_apply_dev(h, h->tmp, h->xout);        // warm-up (first launch of the shape)
-        if (rc) return rc;
+        int rc = take(c);
+        if (rc || (rc = precond_apply_dev(h, h->tmp, h->xout))) return rc;   // warm-up (first launch of the shape)
         if (c.vform == 1 && !fused_capturable(h, h->tmp, h->xout)) { fusedOk = false; continue; }
         RSG_CUDA(cudaEventRecord(h->ev0, h->stream));
         for (int k = 0; k < 3; ++k)
@@ -1066,6 +1147,7 @@ int tune_shapes(rsg_solver* h) {
         ms /= 3;
         char buf[96];
         if (c.split == 0) std::snprintf(buf, sizeof(buf), "%sone-kernel %.3f ms", timings.empty() ? "" : ", ", ms);
+        else if (ring && c.ring) std::snprintf(buf, sizeof(buf), "%sform%d/ring %.3f ms", timings.empty() ? "" : ", ", c.vform, ms);
         else std::snprintf(buf, sizeof(buf), "%sform%d/%d %.3f ms", timings.empty() ? "" : ", ", c.vform, c.cpr2Threads, ms);
         timings += buf;
         if (ms < best) { best = ms; pick = c; }
@@ -1073,7 +1155,8 @@ int tune_shapes(rsg_solver* h) {
     const int rce = check_device_errors(h);
     if (rce) return rce;
     pick.desc = describe(pick) + " source=tuned (CPR application: " + timings + (fusedOk ? "" : "; fused kernel not capturable here") + ")";
-    h->tune = pick;
+    const int rct = take(pick);
+    if (rct) return rct;
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tune_cache[key] = pick;
     return RSG_OK;
@@ -1107,10 +1190,10 @@ int do_setup(rsg_solver* h, const double* acc) {
         if (h->opt.precision == RSG_MIXED || h->opt.precision == RSG_MIXED_F32) {
             if (h->cta && h->opt.precision == RSG_MIXED_F32) launch_factor_cta_f32(h->dp, h->val, h->luf, h->d_nreg, h->stream);
             else launch_factor_lean(h->dp, h->val, h->luf, h->work, h->S, h->epoch, h->d_nreg, h->d_err, h->stream);
-            if (h->cta) { launch_pack_f32(h->dp, h->luf, h->s32, h->stream); h->launches += 1; }
+            if (h->cta && (rc = pack_factors(h))) return rc;
         } else {
             launch_factor_f64(h->dp, h->val, h->lu, h->S, h->epoch, h->d_nreg, h->d_err, h->stream);
-            if (h->cta) { launch_pack_f64(h->dp, h->lu, h->s64, h->stream); h->launches += 1; }
+            if (h->cta && (rc = pack_factors(h))) return rc;
         }
     }
     RSG_CUDA(cudaGetLastError());
@@ -1130,7 +1213,7 @@ int do_setup(rsg_solver* h, const double* acc) {
 int graph_kind(const PrecDev& M) {
     // distinct fields: kind 0-3, the three form flags, V-cycle form 0-3, BILU0-stage thread count (256 / 512 / 128)
     return (M.kind & 3) | (M.cpr ? 4 : 0) | (M.cta ? 8 : 0) | (M.split ? 16 : 0) | ((M.vform & 3) << 5) |
-           ((M.cpr2Threads >= 512 ? 1 : M.cpr2Threads <= 128 ? 2 : 0) << 7);
+           ((M.cpr2Threads >= 512 ? 1 : M.cpr2Threads <= 128 ? 2 : 0) << 7) | (M.ring ? 512 : 0);
 }
 
 int launch_iterations(rsg_solver* h, int k) {
@@ -1275,8 +1358,10 @@ int escalate(rsg_solver* h, double tol, int maxIt, bool gmres = false) {
     if (h->cta) {
         ++h->epoch;
         launch_factor_lean(h->dp, h->val, h->luf, h->work, h->S, h->epoch, h->d_nreg, h->d_err, h->stream);
-        launch_pack_f32(h->dp, h->luf, h->s32, h->stream);
-        h->launches += 2;
+        h->launches += 1;
+        h->escalated = true;                       // the FP32 factors with FP64 sweep vectors
+        const int rc = pack_factors(h);
+        if (rc) return rc;
         RSG_CUDA(cudaGetLastError());
     }
     h->escalated = true;

@@ -119,6 +119,20 @@ __device__ __forceinline__ void load9_ro(const double* p, double* a) {
     for (int e = 0; e < 9; ++e) a[e] = __ldg(p + e);
 }
 
+// one row of a 3x3 block (factor type TF) times a 3-vector of type TV, accumulated from zero left to right
+__device__ __forceinline__ double rdot(const double* a, const double* x) { return da(da(dm(a[0], x[0]), dm(a[1], x[1])), dm(a[2], x[2])); }
+__device__ __forceinline__ double rdot(const float* a, const double* x) {
+    return da(da(dm(double(a[0]), x[0]), dm(double(a[1]), x[1])), dm(double(a[2]), x[2]));
+}
+__device__ __forceinline__ float rdot(const float* a, const float* x) {
+    float s = 0.f;
+    s += a[0] * x[0];
+    s += a[1] * x[1];
+    s += a[2] * x[2];
+    return s;
+}
+__device__ __forceinline__ double vsub(double a, double b) { return ds(a, b); }
+__device__ __forceinline__ float vsub(float a, float b) { return a - b; }
 
 }  // namespace
 }  // namespace rsg

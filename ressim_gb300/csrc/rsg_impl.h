@@ -357,6 +357,28 @@ struct SplitFactors {
     T *L = nullptr, *UD = nullptr, *Lov = nullptr, *Uov = nullptr;
 };
 
+// Row-major factor records of the ring sweeps (rsg_ring.cu): L = n x LREC, UD = n x UREC, overflow entries of
+// ring_ov_words values {block, column, pad}.
+template <class T>
+struct RingFactors {
+    T *L = nullptr, *UD = nullptr, *Lov = nullptr, *Uov = nullptr;
+};
+// The steps of the ring sweeps: per system its forward levels, then the same levels in reverse (a wide level is several
+// steps), as {first row, rows | overflow entries << 16, first overflow entry, 0}.
+struct RingHost {
+    std::vector<int4> desc;
+    std::vector<int> stepOff;
+    int maxSteps = 0, maxRows = 0, maxWidth = 0;
+    size_t maxStage32 = 0, maxStage64 = 0;      // largest step in the ring (bytes), by factor type
+    bool ok = false;
+};
+struct RingDev {
+    int4* desc = nullptr;
+    int* stepOff = nullptr;
+    int maxSteps = 0, maxRows = 0, maxWidth = 0;
+    size_t maxStage32 = 0, maxStage64 = 0;
+};
+
 struct SweepState {                   // sync-free sweep flags and claim counters
     int *flagF = nullptr, *flagB = nullptr, *flagL = nullptr;
     unsigned *ctr = nullptr;          // [0] forward, [1] backward, [2] factorisation, [3] spare
@@ -429,7 +451,22 @@ struct PrecDev {
                                       // levels one thread block per system
     int cpr2Threads = 256;            // split CPR: threads per block of the BILU0 stage (128, 256 or 512; same results)
     const DevAmg* amg = nullptr;
+    const RingDev* ring = nullptr;    // ring sweeps on r64 / r32, steps for FP64 [0] and FP32 [1] vectors (null: they do not
+                                      // fit this plan or this kind)
+    RingFactors<double> r64;
+    RingFactors<float> r32;
+    int* err = nullptr;               // device error bits
 };
+// ---- ring sweeps (rsg_ring.cu)
+void ring_steps(const HostPlan& P, bool vec32, RingHost& H);
+bool ring_fits(const RingDev& R, bool factors32, bool vec32);
+size_t ring_ov_words(bool factors32);
+void launch_ring_pack(const DevPlan& P, const double* lu, RingFactors<double>& F, cudaStream_t st);
+void launch_ring_pack(const DevPlan& P, const float* luf, RingFactors<float>& F, cudaStream_t st);
+void launch_ring_ilu(const DevPlan& P, const PrecDev& M, int mode, const double* r, double* pv, const double* v, double* z, const KScal* ks,
+                     int* err, cudaStream_t st);
+void launch_ring_cpr2(const DevPlan& P, const PrecDev& M, const DevAmg& G, const void* T, double* z, const KScal* ks, int* err,
+                      cudaStream_t st);
 // all-FP32 factorisation (FP32 elimination, FP64 pivot inversion), one thread block per system
 void launch_factor_cta_f32(const DevPlan& P, const double* val, float* luf, int* nreg, cudaStream_t st);
 // gather the factors (original block layout) into the level-ordered split layout

@@ -37,21 +37,6 @@ template <class TF, class TV>
 __host__ __device__ constexpr int cta_threads() { return 256; }
 constexpr int kAhead = 4;                  // levels prefetched into L2 ahead of the sweep front
 
-// one row of a 3x3 block (factor type TF) times a 3-vector of type TV, accumulated from zero left to right
-__device__ __forceinline__ double rdot(const double* a, const double* x) { return da(da(dm(a[0], x[0]), dm(a[1], x[1])), dm(a[2], x[2])); }
-__device__ __forceinline__ double rdot(const float* a, const double* x) {
-    return da(da(dm(double(a[0]), x[0]), dm(double(a[1]), x[1])), dm(double(a[2]), x[2]));
-}
-__device__ __forceinline__ float rdot(const float* a, const float* x) {
-    float s = 0.f;
-    s += a[0] * x[0];
-    s += a[1] * x[1];
-    s += a[2] * x[2];
-    return s;
-}
-__device__ __forceinline__ double vsub(double a, double b) { return ds(a, b); }
-__device__ __forceinline__ float vsub(float a, float b) { return a - b; }
-
 enum { IN_PLAIN = 0, IN_PUPDATE = 1, IN_SUPDATE = 2 };
 
 // L2 prefetch of bytes [b, e) of base by the bulk-copy unit. The bulk unit wants a 16-byte aligned address and
@@ -1357,7 +1342,8 @@ void launch_cta(const DevPlan& P, const SplitFactors<TF>& S, size_t smem, const 
 template <int MODE>
 void dispatch(const DevPlan& P, const PrecDev& M, const double* r, double* pv, const double* v, double* z, const KScal* ks,
               cudaStream_t st) {
-    if (M.kind == 0) launch_cta<double, double, MODE>(P, M.s64, M.smem, r, pv, v, z, z, ks, st);
+    if (M.ring) launch_ring_ilu(P, M, MODE, r, pv, v, z, ks, M.err, st);
+    else if (M.kind == 0) launch_cta<double, double, MODE>(P, M.s64, M.smem, r, pv, v, z, z, ks, st);
     else if (M.kind == 1) launch_cta<float, double, MODE>(P, M.s32, M.smem, r, pv, v, z, z, ks, st);
     else launch_cta<float, float, MODE>(P, M.s32, M.smem, r, pv, v, z, M.y32, ks, st);
 }
@@ -2126,6 +2112,10 @@ void launch_cpr2_nt(const DevPlan& P, const PrecDev& M, const DevAmg& G, const C
 template <class TA, class TT>
 void launch_cpr2(const DevPlan& P, const PrecDev& M, const DevAmg& G, const CprArgs<TA>& C, TT* Tsplit, double* z, const KScal* ks,
                  cudaStream_t st) {
+    if (M.ring) {
+        launch_ring_cpr2(P, M, G, Tsplit, z, ks, M.err, st);
+        return;
+    }
     const int nt = M.cpr2Threads;
     if constexpr (sizeof(TA) == 8) {
         if (nt >= 512) launch_cpr2_nt<double, double, TA, 512>(P, M, G, C, Tsplit, z, z, ks, st);

@@ -1,0 +1,87 @@
+"""The ring-fed block sweeps (rsg_ring.cu) at the shapes where they can go wrong: levels of one row and levels wider than a
+step, a step's remainder, rows with long overflow lists, systems at and beyond what one SM's shared memory holds, and
+batches of uneven systems. FP64 and mixed sweeps against the oracle bit for bit; the all-FP32 sweeps bit for bit those of
+the fixed-thread-count kernels (the same arithmetic in the same order) and within float rounding of the oracle's."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def system(n, pairs, seed):
+    """A structurally symmetric, diagonally dominant 3 x 3 block system with the given off-diagonal pairs."""
+    from ressim_gb300.bsr import BSR
+    rng = np.random.default_rng(seed)
+    pairs = np.asarray(sorted(set(map(tuple, pairs))), dtype=np.int64).reshape(-1, 2)
+    rows = np.concatenate([np.arange(n), pairs[:, 0], pairs[:, 1]])
+    cols = np.concatenate([np.arange(n), pairs[:, 1], pairs[:, 0]])
+    order = np.lexsort((cols, rows))
+    rows, cols = rows[order], cols[order]
+    val = 0.2 * rng.standard_normal((rows.size, 3, 3))
+    deg = np.bincount(rows, minlength=n)
+    val[rows == cols] += (2.0 + deg)[:, None, None] * np.eye(3)
+    return BSR(n, 3, np.concatenate([[0], np.cumsum(deg)]).astype(np.int32), cols.astype(np.int32), val.reshape(-1))
+
+
+def box(nx, ny, nz):
+    i = np.arange(nx * ny * nz).reshape(nz, ny, nx)
+    return [p for a, b in ((i[:, :, :-1], i[:, :, 1:]), (i[:, :-1], i[:, 1:]), (i[:-1], i[1:])) for p in zip(a.ravel(), b.ravel())]
+
+
+SHAPES = {
+    "one_row": (1, []),
+    "chain": (301, [(k, k + 1) for k in range(300)]),                      # 301 levels of one row
+    "diagonal": (1003, []),                                                # one level: several steps and a remainder
+    "star": (400, [(0, k) for k in range(1, 400)]),                        # an overflow list of 396 entries
+    "arrow": (200, [(k, 199) for k in range(199)]),                        # the same in the forward sweep
+    "two_colours": (1200, [(k, 600 + (7 * k + j) % 600) for k in range(600) for j in range(5)]),   # every row overflows
+    "box": (9 * 7 * 5, box(9, 7, 5)),
+    "slab": (70 * 61 * 2, box(70, 61, 2)),
+    "box_13k": (33 * 40 * 10, box(33, 40, 10)),                            # FP32: the vector fills most of the SM
+    "box_20k": (40 * 50 * 10, box(40, 50, 10)),                            # no vector fits
+}
+
+
+@pytest.mark.parametrize("name", SHAPES)
+def test_sweeps_match_the_oracle(name, oracle):
+    from ressim_gb300.solver import DeviceSolver
+    n, pairs = SHAPES[name]
+    A = system(n, pairs, seed=len(name))
+    r = np.random.default_rng(1).standard_normal(3 * n)
+    lu, _ = oracle.bilu0_factor(A)
+    luf, _ = oracle.bilu0_factor_lean(A)
+    f32, _ = oracle.bilu0_factor_f32(A)
+    z = {}
+    for precision, threads in (("fp64", 0), ("mixed", 0), ("mixed_f32", 0), ("mixed_f32", 256)):
+        with DeviceSolver(precond="bilu0", precision=precision, sweep="cta", cpr2_threads=threads) as d:
+            d.set_matrix(A)
+            d.setup()
+            z[precision, threads] = d.precond_apply(r)
+            if not threads:
+                x, res = d.solve(r, tol=1e-8, maxit=100)                   # the input fused with the Krylov updates
+                assert res.converged
+    assert np.array_equal(z["fp64", 0], oracle.bilu0_apply(A, lu, r))
+    assert np.array_equal(z["mixed", 0], oracle.bilu0_apply_fd(A, luf, r))
+    assert np.array_equal(z["mixed_f32", 0], z["mixed_f32", 256])
+    ref = oracle.bilu0_apply_ff(A, f32, r)
+    assert np.linalg.norm(z["mixed_f32", 0] - ref) <= 1e-5 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed_f32"])
+def test_batch_of_uneven_systems(precision):
+    """A batch gives every system the result it has alone, whatever its place in the concatenated arrays (the input's
+    16-byte alignment differs from system to system)."""
+    from ressim_gb300.solver import DeviceSolver
+    mats = [system(n, pairs, seed=3) for n, pairs in (SHAPES[k] for k in ("chain", "one_row", "box", "two_colours", "star"))]
+    r = np.random.default_rng(2).standard_normal(sum(3 * A.n for A in mats))
+    alone, off = [], 0
+    for A in mats:
+        with DeviceSolver(precond="bilu0", precision=precision) as d:
+            d.set_matrix(A)
+            d.setup()
+            alone.append(d.precond_apply(r[off:off + 3 * A.n]))
+        off += 3 * A.n
+    with DeviceSolver(precond="bilu0", precision=precision) as d:
+        d.set_batch(mats)
+        d.setup()
+        assert np.array_equal(d.precond_apply(r), np.concatenate(alone))
