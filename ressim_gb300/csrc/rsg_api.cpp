@@ -238,6 +238,7 @@ int alloc_plan(rsg_solver* h) {
     {
         int maxLv = 1;
         for (int s = 0; s < P.nsys; ++s) maxLv = std::max(maxLv, P.sysLvl0[size_t(s) + 1] - P.sysLvl0[size_t(s)] - 1);
+        D.avgLevelRows = double(P.n) / double(std::max(1, P.nlevF));
         D.sweepBlocks = sweep_blocks_for(double(P.n) / double(maxLv), h->opt.sweep_inflight);
     }
     h->cta = h->opt.sweep != 2 && cta_sweep_supported(D, P);
@@ -1188,7 +1189,7 @@ int do_setup(rsg_solver* h, const double* acc) {
     } else {
         ++h->epoch;
         if (h->opt.precision == RSG_MIXED || h->opt.precision == RSG_MIXED_F32) {
-            if (h->cta && h->opt.precision == RSG_MIXED_F32) launch_factor_cta_f32(h->dp, h->val, h->luf, h->d_nreg, h->stream);
+            if (h->cta && h->opt.precision == RSG_MIXED_F32) launch_factor_f32(h->dp, h->val, h->luf, h->S, h->epoch, h->d_nreg, h->d_err, h->stream);
             else launch_factor_lean(h->dp, h->val, h->luf, h->work, h->S, h->epoch, h->d_nreg, h->d_err, h->stream);
             if (h->cta && (rc = pack_factors(h))) return rc;
         } else {

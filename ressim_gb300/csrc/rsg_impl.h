@@ -344,6 +344,7 @@ struct DevPlan {
     int* Dsrc = nullptr;
     int2* rowLevel = nullptr;         // level-space row -> (first row of its forward level, rows of that level)
     int nLov = 0, nUov = 0, maxSysRows = 0;
+    double avgLevelRows = 0;          // rows of a forward level of the whole batch, on average
     int sweepBlocks = 0;              // persistent grid of the sync-free sweeps (0: sized from n)
     bool spmvFma = true;              // SpMV with fused multiply-adds (else the reference's rounding, bitwise)
 };
@@ -400,6 +401,8 @@ void launch_factor_f64(const DevPlan& P, const double* val, double* lu, SweepSta
                        cudaStream_t st);
 void launch_factor_lean(const DevPlan& P, const double* val, float* luf, double* work, SweepState& S, int epoch, int* nreg,
                         int* err, cudaStream_t st);
+// all-FP32 factorisation (FP32 elimination, FP64 pivot inversion)
+void launch_factor_f32(const DevPlan& P, const double* val, float* luf, SweepState& S, int epoch, int* nreg, int* err, cudaStream_t st);
 // z = U^-1 L^-1 r (FP64 factors, FP64 vectors) or with FP32 factors / FP32 vectors and accumulation.
 void launch_ilu_apply_f64(const DevPlan& P, const double* lu, const double* r, double* z, SweepState& S, int* err,
                           cudaStream_t st);
@@ -467,8 +470,6 @@ void launch_ring_ilu(const DevPlan& P, const PrecDev& M, int mode, const double*
                      int* err, cudaStream_t st);
 void launch_ring_cpr2(const DevPlan& P, const PrecDev& M, const DevAmg& G, const void* T, double* z, const KScal* ks, int* err,
                       cudaStream_t st);
-// all-FP32 factorisation (FP32 elimination, FP64 pivot inversion), one thread block per system
-void launch_factor_cta_f32(const DevPlan& P, const double* val, float* luf, int* nreg, cudaStream_t st);
 // gather the factors (original block layout) into the level-ordered split layout
 void launch_pack_f64(const DevPlan& P, const double* lu, SplitFactors<double>& F, cudaStream_t st);
 void launch_pack_f32(const DevPlan& P, const float* luf, SplitFactors<float>& F, cudaStream_t st);

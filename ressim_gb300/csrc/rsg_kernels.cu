@@ -29,93 +29,203 @@ namespace {
 constexpr int kSweepThreads = 128;
 
 // ------------------------------------------------------------------ BILU0 factorisation (sync-free, level order)
-// engine/src/bsr.cpp:183-215 row by row; rows of a system claimed in forward level order.
-__global__ void __launch_bounds__(kSweepThreads) k_factor_f64(int n, const int* __restrict__ rowPtr, const int* __restrict__ col,
-                                                             const int* __restrict__ diag, const int* __restrict__ ford,
-                                                             const int* __restrict__ elimPtr, const int* __restrict__ elimT,
-                                                             const int* __restrict__ elimQ, double* lu, int* flagL, int epoch,
-                                                             unsigned* ctr, int* nreg, int* err) {
-    const int lane = threadIdx.x & 31;
-    for (;;) {
-        __syncwarp();
-        const int base = warp_claim(ctr);
-        if (base >= n) break;
-        const int idx = base + lane;
-        if (idx < n) {
-            const int i = __ldg(ford + idx);
-            const int r0 = __ldg(rowPtr + i), d = __ldg(diag + i);
-            wait_cols(flagL, col, r0, d, epoch, err);
-            for (int p = r0; p < d; ++p) {
-                const int k = __ldg(col + p);
-                double a[9], u[9], L[9];
-                load9(lu + size_t(p) * 9, a);
-                load9(lu + size_t(__ldg(diag + k)) * 9, u);
-                gemm3(a, u, L);                                   // L_ik = A_ik U_kk^-1
-                store9(lu + size_t(p) * 9, L);
-                for (int e = __ldg(elimPtr + p); e < __ldg(elimPtr + p + 1); ++e) {
-                    const int t = __ldg(elimT + e), q = __ldg(elimQ + e);
-                    double U[9], Cb[9];
-                    load9(lu + size_t(q) * 9, U);
-                    load9(lu + size_t(t) * 9, Cb);
-                    gemm3_sub(L, U, Cb);                          // A_ij -= L_ik U_kj
-                    store9(lu + size_t(t) * 9, Cb);
-                }
+// engine/src/bsr.cpp:183-215 row by row; rows of a system claimed in forward level order. W: arithmetic of the
+// elimination, F: storage of the factors. (double, double) is the reference's FP64 factorisation; (double, float) the
+// lean one (engine/src/bsr.cpp:219-263: the row, rounded to float, eliminated in double against the float factors of
+// earlier rows, then rounded); (float, float) the precision form's FP32 elimination. The pivot block is inverted in FP64.
+//
+// A warp takes one row. What bounds the factorisation is its chain of dependent rows -- a level of the stencil, or a well
+// clique of 30-40 rows that each eliminate against all the earlier ones -- so the work of one row is spread over the
+// lanes: the row lives in shared memory, nine lanes form the block L_ik, 27 lanes update three target blocks at a time
+// (one element each, the reference's operations in its order), six lanes hold the columns of [D | I] in the inversion, and
+// the blocks of the next entry are on their way while one is eliminated. A thread per row paid every block's loads and
+// arithmetic one after another: 180,000 rows with four 30-layer wells 28 ms, 277,000 rows with five 42-layer wells (lean)
+// 115 ms, 1,600 rows 1.16 ms.
+constexpr int kFacRow = 40;                  // blocks of a row in shared memory; longer rows work in global memory
+__device__ __forceinline__ double fmul(double a, double b) { return dm(a, b); }
+__device__ __forceinline__ double fadd(double a, double b) { return da(a, b); }
+__device__ __forceinline__ double fsub(double a, double b) { return ds(a, b); }
+__device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
+
+// Inversion of a pivot block by a warp: lane j < 6 holds column j of [D | I]; invert3's operations in its order
+// (rsg_block3.cuh), so the same bits. The result of D^-1 element (i, j) is in out[i] of lane 3 + j. False (every lane): a
+// singular or non-finite block.
+template <class W>
+__device__ __forceinline__ bool warp_invert3(const W* D, int lane, double (&out)[3]) {
+    double m[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) m[i] = lane < 3 ? double(D[3 * i + lane]) : (lane == 3 + i ? 1.0 : 0.0);
+    double sc = lane < 3 ? fmax(fmax(fmax(0.0, fabs(m[0])), fabs(m[1])), fabs(m[2])) : 0.0;
+    sc = fmax(fmax(__shfl_sync(0xffffffffu, sc, 0), __shfl_sync(0xffffffffu, sc, 1)), __shfl_sync(0xffffffffu, sc, 2));
+    if (!(sc > 0) || !isfinite(sc)) return false;
+    const double thr = dm(1e-14, sc);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        double c[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) c[i] = __shfl_sync(0xffffffffu, m[i], k);
+        int pr = k;
+        double big = fabs(c[k]), cp = c[k];
+#pragma unroll
+        for (int i = k + 1; i < 3; ++i)
+            if (fabs(c[i]) > big) { pr = i; big = fabs(c[i]); cp = c[i]; }
+        if (big <= thr) return false;
+#pragma unroll
+        for (int i = k + 1; i < 3; ++i)
+            if (pr == i) {
+                const double t = m[k], u = c[k];
+                m[k] = m[i]; m[i] = t;
+                c[k] = c[i]; c[i] = u;
             }
-            double D[9];
-            load9(lu + size_t(d) * 9, D);
-            if (invert_pivot3(D)) atomicAdd(nreg, 1);
-            store9(lu + size_t(d) * 9, D);
-            st_release(flagL + i, epoch);
-        }
+        m[k] = dm(m[k], __ddiv_rn(1.0, cp));
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            if (i != k && c[i] != 0.0) m[i] = ds(m[i], dm(c[i], m[k]));
     }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) out[i] = m[i];
+    return true;
 }
 
-// C45 lean factorisation (engine/src/bsr.cpp:219-263): the row is eliminated in double (work) against the float
-// factors of earlier rows, the pivot inverted in double, and the row stored rounded to float.
-__global__ void __launch_bounds__(kSweepThreads) k_factor_lean(int n, const int* __restrict__ rowPtr, const int* __restrict__ col,
-                                                              const int* __restrict__ diag, const int* __restrict__ ford,
-                                                              const int* __restrict__ elimPtr, const int* __restrict__ elimT,
-                                                              const int* __restrict__ elimQ, const double* __restrict__ val,
-                                                              float* F, double* work, int* flagL, int epoch, unsigned* ctr,
-                                                              int* nreg, int* err) {
+template <class W, class F>
+__global__ void __launch_bounds__(kSweepThreads) k_factor(int n, int chunk, const int* __restrict__ rowPtr, const int* __restrict__ col,
+                                                          const int* __restrict__ diag, const int* __restrict__ ford,
+                                                          const int* __restrict__ elimPtr, const int* __restrict__ elimT,
+                                                          const int* __restrict__ elimQ, const double* __restrict__ val, F* lu, W* work,
+                                                          int* flagL, int epoch, unsigned* ctr, int* nreg, int* err) {
+    __shared__ W rows[kSweepThreads / 32][kFacRow * 9];
     const int lane = threadIdx.x & 31;
+    const unsigned all = 0xffffffffu;
+    const int g = lane / 9, el = lane % 9, er = el / 3, ec = el % 3;   // this lane's target of three, and element
+    int at = 0, end = 0;
     for (;;) {
-        __syncwarp();
-        const int base = warp_claim(ctr);
-        if (base >= n) break;
-        const int idx = base + lane;
-        if (idx < n) {
-            const int i = __ldg(ford + idx);
-            const int r0 = __ldg(rowPtr + i), r1 = __ldg(rowPtr + i + 1), d = __ldg(diag + i);
-            for (int p = r0; p < r1; ++p)
-                for (int e = 0; e < 9; ++e) work[size_t(p) * 9 + e] = double(float(__ldg(val + size_t(p) * 9 + e)));
-            wait_cols(flagL, col, r0, d, epoch, err);
-            for (int p = r0; p < d; ++p) {
-                const int k = __ldg(col + p);
-                double a[9], u[9], L[9];
-                load9(work + size_t(p) * 9, a);
-                const float* fk = F + size_t(__ldg(diag + k)) * 9;
-                for (int e = 0; e < 9; ++e) u[e] = double(fk[e]);
-                gemm3(a, u, L);
-                store9(work + size_t(p) * 9, L);
-                for (int e = __ldg(elimPtr + p); e < __ldg(elimPtr + p + 1); ++e) {
-                    const int t = __ldg(elimT + e), q = __ldg(elimQ + e);
-                    double U[9], Cb[9];
-                    const float* fq = F + size_t(q) * 9;
-                    for (int j = 0; j < 9; ++j) U[j] = double(fq[j]);
-                    load9(work + size_t(t) * 9, Cb);
-                    gemm3_sub(L, U, Cb);
-                    store9(work + size_t(t) * 9, Cb);
+        if (at >= end) {                                      // the next `chunk` rows of the claim order
+            unsigned got = 0;
+            if (lane == 0) got = atomicAdd(ctr, unsigned(chunk));
+            at = int(__shfl_sync(all, got, 0));
+            end = min(n, at + chunk);
+            if (at >= n) break;
+        }
+        const int i = __ldg(ford + at++);
+        const int r0 = __ldg(rowPtr + i), r1 = __ldg(rowPtr + i + 1), d = __ldg(diag + i);
+        W* row = (r1 - r0) <= kFacRow ? rows[threadIdx.x >> 5] : work + size_t(r0) * 9;
+        for (int e = lane; e < 9 * (r1 - r0); e += 32) row[e] = W(F(__ldg(val + size_t(r0) * 9 + e)));
+        for (int c0 = r0; c0 < d; c0 += 32) {                 // the entries before the diagonal, 32 at a time
+            const int cn = min(32, d - c0);
+            int k = 0, dk = 0, q0 = 0, q1 = 0;                // this lane's entry: column, its pivot block, its eliminations
+            if (lane < cn) {
+                k = __ldg(col + c0 + lane);
+                dk = __ldg(diag + k);
+                q0 = __ldg(elimPtr + c0 + lane);
+                q1 = __ldg(elimPtr + c0 + lane + 1);
+            }
+            {                                                 // wait for the rows of the chunk (bounded)
+                bool pending = lane < cn;
+                unsigned ns = 0;
+                for (unsigned it = 0;; ++it) {
+                    if (pending && ld_relaxed(flagL + k) == epoch) pending = false;
+                    if (!__any_sync(all, pending)) break;
+                    if (it >= 64) {
+                        __nanosleep(ns);
+                        ns = ns < 32 ? 32 : (ns < 256 ? 2 * ns : 256);
+                        if (it >= 64 + kSpinLimit) { if (pending) atomicOr(err, ERR_TIMEOUT); break; }
+                        if ((it & 255u) == 255u && *(volatile int*)err != 0) break;
+                    }
                 }
             }
-            double D[9];
-            load9(work + size_t(d) * 9, D);
-            if (invert_pivot3(D)) atomicAdd(nreg, 1);
-            store9(work + size_t(d) * 9, D);
-            for (int p = r0; p < r1; ++p)
-                for (int e = 0; e < 9; ++e) F[size_t(p) * 9 + e] = float(work[size_t(p) * 9 + e]);
-            st_release(flagL + i, epoch);
+            fence_acquire();
+            __syncwarp();
+            // blocks of an entry: column ec of U_kk (lanes 0-8) and of the first three targets' U_kq (27 lanes)
+            W u[3], U[3];
+            int t = -1;
+            auto fetch = [&](int p, W (&pu)[3], W (&pU)[3], int& pt) {
+                const int pd = __shfl_sync(all, dk, p), a0 = __shfl_sync(all, q0, p), a1 = __shfl_sync(all, q1, p);
+                pt = -1;
+                if (lane < 27 && a0 + g < a1) {
+                    pt = __ldg(elimT + a0 + g) - r0;
+                    const F* f = lu + size_t(__ldg(elimQ + a0 + g)) * 9 + ec;
+#pragma unroll
+                    for (int m = 0; m < 3; ++m) pU[m] = W(f[3 * m]);
+                }
+                if (lane < 9) {
+                    const F* f = lu + size_t(pd) * 9 + ec;
+#pragma unroll
+                    for (int m = 0; m < 3; ++m) pu[m] = W(f[3 * m]);
+                }
+            };
+            fetch(0, u, U, t);
+            for (int p = 0; p < cn; ++p) {
+                W un[3], Un[3];
+                int tn = -1;
+                if (p + 1 < cn) fetch(p + 1, un, Un, tn);     // the next entry's blocks (final rows: nothing here changes them)
+                const int a0 = __shfl_sync(all, q0, p), a1 = __shfl_sync(all, q1, p);
+                W* L = row + size_t(c0 - r0 + p) * 9;
+                W l = W(0);                                   // L_ik = A_ik U_kk^-1
+                if (lane < 9) {
+#pragma unroll
+                    for (int m = 0; m < 3; ++m) l = fadd(l, fmul(L[3 * er + m], u[m]));
+                }
+                __syncwarp();
+                if (lane < 9) L[el] = l;
+                __syncwarp();
+                W Lr[3];
+#pragma unroll
+                for (int m = 0; m < 3; ++m) Lr[m] = L[3 * er + m];
+                auto elim = [&](int tt, const W (&uu)[3]) {    // A_it -= L_ik U_kq, one element
+                    W s = W(0);
+#pragma unroll
+                    for (int m = 0; m < 3; ++m) s = fadd(s, fmul(Lr[m], uu[m]));
+                    row[size_t(tt) * 9 + el] = fsub(row[size_t(tt) * 9 + el], s);
+                };
+                if (t >= 0) elim(t, U);
+                for (int q = a0 + 3 + g; q - g < a1; q += 12) {   // further targets: the loads of twelve at once
+                    W V[4][3];
+                    int tt[4];
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) {
+                        tt[v] = -1;
+                        if (lane < 27 && q + 3 * v < a1) {
+                            tt[v] = __ldg(elimT + q + 3 * v) - r0;
+                            const F* f = lu + size_t(__ldg(elimQ + q + 3 * v)) * 9 + ec;
+#pragma unroll
+                            for (int m = 0; m < 3; ++m) V[v][m] = W(f[3 * m]);
+                        }
+                    }
+#pragma unroll
+                    for (int v = 0; v < 4; ++v)
+                        if (tt[v] >= 0) elim(tt[v], V[v]);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int m = 0; m < 3; ++m) { u[m] = un[m]; U[m] = Un[m]; }
+                t = tn;
+            }
         }
+        __syncwarp();
+        W* D = row + size_t(d - r0) * 9;
+        double inv[3];
+        if (warp_invert3(D, lane, inv)) {
+            __syncwarp();
+            if (lane >= 3 && lane < 6)
+#pragma unroll
+                for (int m = 0; m < 3; ++m) D[3 * m + lane - 3] = W(inv[m]);
+        } else {                                              // the reference's regularised inverse
+            __syncwarp();
+            if (lane == 0) {
+                double B[9];
+#pragma unroll
+                for (int e = 0; e < 9; ++e) B[e] = double(D[e]);
+                if (invert_pivot3(B)) atomicAdd(nreg, 1);
+#pragma unroll
+                for (int e = 0; e < 9; ++e) D[e] = W(B[e]);
+            }
+        }
+        __syncwarp();
+        for (int e = lane; e < 9 * (r1 - r0); e += 32) lu[size_t(r0) * 9 + e] = F(row[e]);
+        __syncwarp();                                         // (orders the lanes' stores before the release)
+        if (lane == 0) st_release(flagL + i, epoch);
     }
 }
 
@@ -720,19 +830,27 @@ void launch_scatter_vec(const DevPlan& P, const double* lev, double* orig, cudaS
     k_scatter_vec<<<stream_grid(size_t(P.n) * 3), 256, 0, st>>>(P.n, P.perm, lev, orig);
 }
 
+// a row per warp in a persistent grid; several rows per claim only where a level (of the whole batch) has more rows than the
+// grid has warps
+template <class W, class F>
+static void launch_factor_t(const DevPlan& P, const double* val, F* lu, W* work, SweepState& S, int epoch, int* nreg, int* err,
+                            cudaStream_t st) {
+    cudaMemsetAsync(S.ctr + 2, 0, sizeof(unsigned), st);
+    const int blocks = std::max(1, std::min(8 * device_sm_count(), (P.n + 3) / 4));
+    const int chunk = std::max(1, std::min(8, int(P.avgLevelRows / double(blocks * (kSweepThreads / 32)))));
+    k_factor<W, F><<<blocks, kSweepThreads, 0, st>>>(P.n, chunk, P.rowPtr, P.col, P.diag, P.ford, P.elimPtr, P.elimT, P.elimQ, val, lu, work,
+                                                    S.flagL, epoch, S.ctr + 2, nreg, err);
+}
 void launch_factor_f64(const DevPlan& P, const double* val, double* lu, SweepState& S, int epoch, int* nreg, int* err,
                        cudaStream_t st) {
-    cudaMemcpyAsync(lu, val, size_t(P.nnzb) * 9 * sizeof(double), cudaMemcpyDeviceToDevice, st);
-    cudaMemsetAsync(S.ctr + 2, 0, sizeof(unsigned), st);
-    k_factor_f64<<<sweep_blocks(P), kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, P.elimPtr, P.elimT, P.elimQ, lu,
-                                                           S.flagL, epoch, S.ctr + 2, nreg, err);
+    launch_factor_t<double, double>(P, val, lu, lu, S, epoch, nreg, err, st);
 }
-
 void launch_factor_lean(const DevPlan& P, const double* val, float* luf, double* work, SweepState& S, int epoch, int* nreg,
                         int* err, cudaStream_t st) {
-    cudaMemsetAsync(S.ctr + 2, 0, sizeof(unsigned), st);
-    k_factor_lean<<<sweep_blocks(P), kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, P.elimPtr, P.elimT, P.elimQ,
-                                                            val, luf, work, S.flagL, epoch, S.ctr + 2, nreg, err);
+    launch_factor_t<double, float>(P, val, luf, work, S, epoch, nreg, err, st);
+}
+void launch_factor_f32(const DevPlan& P, const double* val, float* luf, SweepState& S, int epoch, int* nreg, int* err, cudaStream_t st) {
+    launch_factor_t<float, float>(P, val, luf, luf, S, epoch, nreg, err, st);
 }
 
 void launch_ilu_apply_f64(const DevPlan& P, const double* lu, const double* r, double* z, SweepState& S, int* err,

@@ -30,7 +30,6 @@ namespace rsg {
 
 namespace {
 
-constexpr int kCtaThreads = 256;
 // threads per block of a sweep / CPR kernel (a template parameter of the kernels). 512 threads for the all-FP32
 // forms measured slower on the 64-system ensemble (the V-cycle phases spill at 128 registers), so all forms use 256.
 template <class TF, class TV>
@@ -1182,109 +1181,6 @@ __global__ void __launch_bounds__(NT) k_cpr_cta(IluArgs<TF> F, CprArgs<TA> C, co
     }
 }
 
-// ------------------------------------------------------------------ all-FP32 BILU0 factorisation
-// The precision form's factorisation: FP32 elimination and storage, the pivot block inverted in FP64
-// (invert_pivot3: the reference's pivoting and singular-block shift, engine/src/bsr.cpp:67-87, 204-212) and rounded.
-// One thread block per system walks the forward levels; a thread eliminates whole rows (row algorithm of
-// engine/src/bsr.cpp:183-215 with the plan's elimination lists, every float operation rounded on its own).
-__device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float fa(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float fs(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ void gemm3f(const float* a, const float* b, float* c) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        float r0 = 0.f, r1 = 0.f, r2 = 0.f;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float f = a[i * 3 + k];
-            r0 = fa(r0, fm(f, b[k * 3 + 0]));
-            r1 = fa(r1, fm(f, b[k * 3 + 1]));
-            r2 = fa(r2, fm(f, b[k * 3 + 2]));
-        }
-        c[i * 3 + 0] = r0; c[i * 3 + 1] = r1; c[i * 3 + 2] = r2;
-    }
-}
-constexpr int kFacChunk = 4;       // elimination targets of one entry loaded at once
-__device__ __forceinline__ void gemm3f_sub(const float* a, const float* b, float* c) {
-    float t[9];
-    gemm3f(a, b, t);
-#pragma unroll
-    for (int e = 0; e < 9; ++e) c[e] = fs(c[e], t[e]);
-}
-
-__global__ void __launch_bounds__(kCtaThreads) k_factor_cta_f32(const int* __restrict__ sysRow0, const int* __restrict__ sysLvl0,
-                                                               const int* __restrict__ lvlStart, const int* __restrict__ rowPtr,
-                                                               const int* __restrict__ col, const int* __restrict__ diag,
-                                                               const int* __restrict__ elimPtr, const int* __restrict__ elimT,
-                                                               const int* __restrict__ elimQ, const double* __restrict__ val, float* F,
-                                                               int* nreg) {
-    const int s = blockIdx.x, tid = int(threadIdx.x), nt = int(blockDim.x);
-    const int r0 = __ldg(sysRow0 + s), r1 = __ldg(sysRow0 + s + 1);
-    const size_t e0 = size_t(__ldg(rowPtr + r0)) * 9, e1 = size_t(__ldg(rowPtr + r1)) * 9;
-    for (size_t e = e0 + size_t(tid); e < e1; e += size_t(nt)) F[e] = float(__ldg(val + e));
-    __syncthreads();
-    const int l0 = __ldg(sysLvl0 + s), nl = __ldg(sysLvl0 + s + 1) - l0 - 1;
-    __shared__ int lvc[kLvCache];
-    const int* lv = level_starts(lvlStart + l0, nl, lvc);
-    int reg = 0;
-    float Lb[9];
-    for (int L = 0; L < nl; ++L) {
-        const int k1 = lv[L + 1];
-        for (int i = lv[L] + tid; i < k1; i += nt) {
-            const int p0 = __ldg(rowPtr + i), d = __ldg(diag + i);
-            // the indices of entry p (column k, elimination list [q0, q1)) are loaded one entry ahead, so an entry
-            // costs two dependent loads (diag[k] with its first elimination targets, then every block it touches)
-            int k = 0, q0 = 0, q1 = 0;
-            if (p0 < d) { k = __ldg(col + p0); q0 = __ldg(elimPtr + p0); q1 = __ldg(elimPtr + p0 + 1); }
-            for (int p = p0; p < d; ++p) {
-                const int kn = p + 1 < d ? __ldg(col + p + 1) : 0;
-                const int q2 = p + 1 < d ? __ldg(elimPtr + p + 2) : 0;
-                const int dk = __ldg(diag + k);
-                for (int qc = q0; qc == q0 || qc < q1; qc += kFacChunk) {
-                    int t[kFacChunk], uq[kFacChunk];
-#pragma unroll
-                    for (int v = 0; v < kFacChunk; ++v) {
-                        const bool ok = qc + v < q1;
-                        t[v] = ok ? __ldg(elimT + qc + v) : -1;
-                        uq[v] = ok ? __ldg(elimQ + qc + v) : 0;
-                    }
-                    float U[kFacChunk][9], Cb[kFacChunk][9];
-#pragma unroll
-                    for (int v = 0; v < kFacChunk; ++v)
-                        if (t[v] >= 0) {
-#pragma unroll
-                            for (int e = 0; e < 9; ++e) { U[v][e] = F[size_t(uq[v]) * 9 + e]; Cb[v][e] = F[size_t(t[v]) * 9 + e]; }
-                        }
-                    if (qc == q0) {                                   // L_ik = A_ik U_kk^-1, once per entry
-                        float a[9], u[9];
-#pragma unroll
-                        for (int e = 0; e < 9; ++e) { a[e] = F[size_t(p) * 9 + e]; u[e] = F[size_t(dk) * 9 + e]; }
-                        gemm3f(a, u, Lb);
-#pragma unroll
-                        for (int e = 0; e < 9; ++e) F[size_t(p) * 9 + e] = Lb[e];
-                    }
-#pragma unroll
-                    for (int v = 0; v < kFacChunk; ++v)
-                        if (t[v] >= 0) {
-                            gemm3f_sub(Lb, U[v], Cb[v]);                 // A_it -= L_ik U_kq (targets of one entry differ)
-#pragma unroll
-                            for (int e = 0; e < 9; ++e) F[size_t(t[v]) * 9 + e] = Cb[v][e];
-                        }
-                }
-                k = kn; q0 = q1; q1 = q2;
-            }
-            double D[9];
-#pragma unroll
-            for (int e = 0; e < 9; ++e) D[e] = double(F[size_t(d) * 9 + e]);
-            reg += invert_pivot3(D);
-#pragma unroll
-            for (int e = 0; e < 9; ++e) F[size_t(d) * 9 + e] = float(D[e]);
-        }
-        __syncthreads();
-    }
-    if (reg) atomicAdd(nreg, reg);
-}
-
 // factors (level-space CSR block order) -> slot records; overflow blocks
 template <class T>
 __global__ void k_pack(int n, int nLov, int nUov, const int* __restrict__ LslotSrc, const int* __restrict__ UslotSrc,
@@ -1373,11 +1269,6 @@ void launch_pack_f32(const DevPlan& P, const float* luf, SplitFactors<float>& F,
     const int grid = int(std::min<size_t>((total + 255) / 256, size_t(device_sm_count()) * 16));
     k_pack<float><<<grid, 256, 0, st>>>(P.n, P.nLov, P.nUov, P.LslotSrc, P.UslotSrc, P.Dsrc, P.LovSrc, P.UovSrc, P.rowLevel, luf, F.L,
                                         F.UD, F.Lov, F.Uov);
-}
-
-void launch_factor_cta_f32(const DevPlan& P, const double* val, float* luf, int* nreg, cudaStream_t st) {
-    k_factor_cta_f32<<<P.nsys, kCtaThreads, 0, st>>>(P.sysRow0, P.sysLvl0, P.lvlStart, P.rowPtr, P.col, P.diag, P.elimPtr, P.elimT,
-                                                     P.elimQ, val, luf, nreg);
 }
 
 void launch_ilu_cta_apply(const DevPlan& P, const PrecDev& M, const double* r, double* z, cudaStream_t st) {

@@ -1,6 +1,7 @@
-"""The ring-fed block sweeps (rsg_ring.cu) at the shapes where they can go wrong: levels of one row and levels wider than a
+"""The BILU0 factorisation (a warp per row) and the ring-fed block sweeps at the shapes where they can go wrong: rows longer
+than the factorisation keeps on chip, levels of one row and levels wider than a
 step, a step's remainder, rows with long overflow lists, systems at and beyond what one SM's shared memory holds, and
-batches of uneven systems. FP64 and mixed sweeps against the oracle bit for bit; the all-FP32 sweeps bit for bit those of
+batches of uneven systems. The factors of every precision, FP64 and mixed sweeps against the oracle bit for bit; the all-FP32 sweeps bit for bit those of
 the fixed-thread-count kernels (the same arithmetic in the same order) and within float rounding of the oracle's."""
 import numpy as np
 import pytest
@@ -35,6 +36,7 @@ SHAPES = {
     "star": (400, [(0, k) for k in range(1, 400)]),                        # an overflow list of 396 entries
     "arrow": (200, [(k, 199) for k in range(199)]),                        # the same in the forward sweep
     "two_colours": (1200, [(k, 600 + (7 * k + j) % 600) for k in range(600) for j in range(5)]),   # every row overflows
+    "clique": (130, [(k, k + 1) for k in range(129)] + [(a, b) for a in range(20, 67) for b in range(a + 1, 67)]),   # rows of 47+ blocks
     "box": (9 * 7 * 5, box(9, 7, 5)),
     "slab": (70 * 61 * 2, box(70, 61, 2)),
     "box_13k": (33 * 40 * 10, box(33, 40, 10)),                            # FP32: the vector fills most of the SM
@@ -57,6 +59,8 @@ def test_sweeps_match_the_oracle(name, oracle):
             d.set_matrix(A)
             d.setup()
             z[precision, threads] = d.precond_apply(r)
+            if not threads:                                                # the factorisation, a warp per row
+                assert np.array_equal(d.factors(A.nnzb), {"fp64": lu, "mixed": luf, "mixed_f32": f32}[precision])
             if not threads:
                 x, res = d.solve(r, tol=1e-8, maxit=100)                   # the input fused with the Krylov updates
                 assert res.converged
