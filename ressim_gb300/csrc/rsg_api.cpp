@@ -265,11 +265,8 @@ int alloc_plan(rsg_solver* h) {
     double** vecs[] = {&h->V.x, &h->V.r, &h->V.rh, &h->V.p, &h->V.v, &h->V.s, &h->V.t, &h->V.ph, &h->V.sh};
     for (double** v : vecs)
         if ((rc = dalloc(M, v, N))) return rc;
-    if ((rc = dalloc(M, &h->S.flagF, size_t(P.n))) || (rc = dalloc(M, &h->S.flagB, size_t(P.n))) ||
-        (rc = dalloc(M, &h->S.flagL, size_t(P.n))) || (rc = dalloc(M, &h->S.ctr, 4)))
+    if ((rc = dalloc(M, &h->S.flagL, size_t(P.n))) || (rc = dalloc(M, &h->S.ctr, 4)))
         return rc;
-    RSG_CUDA(cudaMemsetAsync(h->S.flagF, 0, sizeof(int) * size_t(P.n), st));
-    RSG_CUDA(cudaMemsetAsync(h->S.flagB, 0, sizeof(int) * size_t(P.n), st));
     RSG_CUDA(cudaMemsetAsync(h->S.flagL, 0, sizeof(int) * size_t(P.n), st));
     RSG_CUDA(cudaMemsetAsync(h->S.ctr, 0, sizeof(unsigned) * 4, st));
     if ((rc = dalloc(M, &h->R.part, size_t(D.ntiles) * MAX_DOTS)) || (rc = dalloc(M, &h->R.done, 1)) ||
@@ -290,13 +287,12 @@ int check_device_errors(rsg_solver* h) {
     if (h->h_pin[1] != 0) {
         const int e = h->h_pin[1];
         cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream);
-        cudaMemsetAsync(h->S.flagF, 0, sizeof(int) * size_t(h->plan.n), h->stream);
-        cudaMemsetAsync(h->S.flagB, 0, sizeof(int) * size_t(h->plan.n), h->stream);
+        if (h->S.yw) cudaMemsetAsync(h->S.yw, 0xff, 2 * size_t(h->plan.n) * NB * sizeof(unsigned long long), h->stream);
         cudaMemsetAsync(h->S.ctr, 0, sizeof(unsigned) * 4, h->stream);
         cudaMemsetAsync(h->R.done, 0, sizeof(unsigned), h->stream);
-        if (h->V.yt) cudaMemsetAsync(h->V.yt, 0, size_t(h->plan.n) * NB * sizeof(unsigned long long), h->stream);
         if (h->amg.gsFlag) {
-            cudaMemsetAsync(h->amg.gsFlag, 0, 2 * size_t(std::max(h->amg.totRows, 1)) * sizeof(int), h->stream);
+            cudaMemsetAsync(h->amg.gsFlag, 0, size_t(std::max(h->amg.totRows, 1)) * sizeof(int), h->stream);
+            cudaMemsetAsync(h->amg.gsWord, 0xff, 2 * size_t(std::max(h->amg.totRows, 1)) * sizeof(unsigned long long), h->stream);
             cudaMemsetAsync(h->amg.gsCtr, 0, 4 * size_t(std::max(h->amg.maxL, 1)) * sizeof(unsigned), h->stream);
         }
         cudaStreamSynchronize(h->stream);
@@ -337,7 +333,6 @@ PrecDev prec_dev(rsg_solver* h) {
     M.val = h->val;
     M.err = h->d_err;
     M.y32 = h->V.y32;
-    M.yt = h->V.yt;
     if (h->opt.precond == RSG_PREC_CPR && h->haveAmg) { M.cpr = true; M.amg = &h->amg; }
     if (h->opt.precond == RSG_PREC_CPR_DEVICE) { M.devcpr = true; M.kind = 4; M.amg = &h->amg; return M; }
     if (M.kind != 2 && h->cta) {
@@ -623,12 +618,13 @@ int ensure_precond_storage(rsg_solver* h) {
         if (!h->luf && (rc = dalloc(h->pmem, &h->luf, E))) return rc;
         if (!h->work && (rc = dalloc(h->pmem, &h->work, E))) return rc;
         if (h->opt.precision == RSG_MIXED_F32 && !h->V.y32 && (rc = dalloc(h->pmem, &h->V.y32, size_t(h->plan.n) * NB))) return rc;
-        if (h->opt.precision == RSG_MIXED_F32 && !h->V.yt) {
-            if ((rc = dalloc(h->pmem, &h->V.yt, size_t(h->plan.n) * NB))) return rc;
-            RSG_CUDA(cudaMemsetAsync(h->V.yt, 0, size_t(h->plan.n) * NB * sizeof(unsigned long long), h->stream));
-        }
     } else {
         if (!h->lu && (rc = dalloc(h->pmem, &h->lu, E))) return rc;
+    }
+    if (h->opt.precond != RSG_PREC_JACOBI && !h->cta && !h->S.yw) {    // grid-wide sweeps: all words empty
+        const size_t words = 2 * size_t(h->plan.n) * NB;
+        if ((rc = dalloc(h->pmem, &h->S.yw, words))) return rc;
+        RSG_CUDA(cudaMemsetAsync(h->S.yw, 0xff, words * sizeof(unsigned long long), h->stream));
     }
     return RSG_OK;
 }
@@ -888,7 +884,8 @@ int build_dev_amg(rsg_solver* h, const std::vector<SysAmg>& H) {
         (rc = upload(M, &G.diagGlob, dgG, st)) || (rc = upload(M, &G.luPerm, luPerm, st)) ||
         (rc = upload(M, &G.slotSrc, slotSrc, st)) || (rc = upload(M, &G.slotCol, slotCol, st)) || (rc = upload(M, &G.gsRows, gsRows, st)) ||
         (rc = upload(M, reinterpret_cast<int**>(&G.rowMeta), meta, st)) || (rc = upload(M, &G.rowLv, rowLv, st)) || (rc = upload(M, &G.cdesc, cdesc, st)) || (rc = upload(M, &G.gci, gci, st)) ||
-        (rc = upload(M, &G.wave, wave, st)) || (rc = dalloc(M, &G.gsFlag, 2 * size_t(std::max(rows, 1)))) ||
+        (rc = upload(M, &G.wave, wave, st)) || (rc = dalloc(M, &G.gsFlag, size_t(std::max(rows, 1)))) ||
+        (rc = dalloc(M, &G.gsWord, 2 * size_t(std::max(rows, 1)))) ||
         (rc = dalloc(M, &G.gsCtr, 4 * size_t(std::max(maxL, 1)))) || (rc = dalloc(M, &G.coarse64, size_t(std::max(nsys, 1)))))
         return rc;
     RSG_CUDA(cudaMemsetAsync(G.coarse64, 0, size_t(std::max(nsys, 1)) * sizeof(int), st));
@@ -906,7 +903,8 @@ int build_dev_amg(rsg_solver* h, const std::vector<SysAmg>& H) {
             (rc = upload(M, &G.dcWorkOff, woff, st)))
             return rc;
     }
-    RSG_CUDA(cudaMemsetAsync(G.gsFlag, 0, 2 * size_t(std::max(rows, 1)) * sizeof(int), st));
+    RSG_CUDA(cudaMemsetAsync(G.gsFlag, 0, size_t(std::max(rows, 1)) * sizeof(int), st));
+    RSG_CUDA(cudaMemsetAsync(G.gsWord, 0xff, 2 * size_t(std::max(rows, 1)) * sizeof(unsigned long long), st));
     RSG_CUDA(cudaMemsetAsync(G.gsCtr, 0, 4 * size_t(std::max(maxL, 1)) * sizeof(unsigned), st));
     {
         const size_t S = size_t(std::max(slots, 1)), R = size_t(std::max(rows, 1)), n = size_t(h->plan.n);
@@ -1017,9 +1015,7 @@ int precond_apply_dev(rsg_solver* h, const double* d_r, double* d_z) {
     else if (M.cpr && M.cta && !M.split) { launch_cpr_cta(h->dp, M, *M.amg, 0, M.kind != 0, d_r, nullptr, nullptr, d_z, nullptr, h->stream); h->launches += 1; }
     else if (M.cpr) h->launches += launch_cpr_grid(h->dp, M, *M.amg, 0, d_r, nullptr, nullptr, d_z, nullptr, h->S, h->d_err, h->stream);
     else if (M.cta) { launch_ilu_cta_apply(h->dp, M, d_r, d_z, h->stream); h->launches += 1; }
-    else if (M.kind == 0) { launch_ilu_apply_f64(h->dp, h->lu, d_r, d_z, h->S, h->d_err, h->stream); h->launches += 2; }
-    else if (M.kind == 1) { launch_ilu_apply_mixed(h->dp, h->luf, d_r, d_z, h->S, h->d_err, h->stream); h->launches += 2; }
-    else if (M.kind == 3) { launch_ilu_apply_f32(h->dp, h->luf, d_r, d_z, h->V.yt, h->S, h->d_err, h->stream); h->launches += 2; }
+    else if (M.kind != 2) { launch_ilu_grid(h->dp, M, 0, d_r, nullptr, nullptr, d_z, nullptr, h->S, h->d_err, h->stream); h->launches += 2; }
     else { launch_block_jacobi_apply(h->dp, h->dinv, d_r, d_z, h->stream); h->launches += 1; }
     RSG_CUDA(cudaGetLastError());
     return RSG_OK;

@@ -338,9 +338,7 @@ void launch_precond_gm(const DevPlan& P, const PrecDev& M, const double* r, doub
     else if (M.cpr && M.cta && !M.split) launch_cpr_cta(P, M, *M.amg, 0, M.kind != 0, r, nullptr, nullptr, z, ks, st);
     else if (M.cpr) launch_cpr_grid(P, M, *M.amg, 0, r, nullptr, nullptr, z, ks, S, err, st);
     else if (M.cta) launch_ilu_cta_apply_ks(P, M, r, z, ks, st);
-    else if (M.kind == 0) launch_ilu_apply_f64(P, M.lu, r, z, S, err, st);
-    else if (M.kind == 1) launch_ilu_apply_mixed(P, M.luf, r, z, S, err, st);
-    else if (M.kind == 3) launch_ilu_apply_f32(P, M.luf, r, z, M.yt, S, err, st);
+    else if (M.kind != 2) launch_ilu_grid(P, M, 0, r, nullptr, nullptr, z, nullptr, S, err, st);
     else launch_block_jacobi_apply(P, M.dinv, r, z, st);
 }
 

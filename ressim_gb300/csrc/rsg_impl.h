@@ -207,8 +207,8 @@ struct DevAmg {
     float *spf = nullptr, *spLovf = nullptr, *spUovf = nullptr;
     // grid-wide V-cycle (systems too large for one SM): per AMG row its (system, level) descriptor index s*maxL+l and
     // its wave (forward GS level, or colour: adjacent rows of an earlier wave are updated before it in a forward
-    // sweep), sync-free sweep flags (phase 0: the smoothing sweeps, phase 1: the GS solve of a coarsest level
-    // without dense LU) and claim counters (per level and phase: forward, backward)
+    // sweep), sync-free sweep words, flags of the small colours' pass and claim counters (per level and phase -- 0: the
+    // smoothing sweeps, 1: the GS solve of a coarsest level without dense LU: forward, backward)
     int* coarse64 = nullptr;           // FP32 forms, per system: 1 = coarsest level solved in FP64 (LU), the FP32 inverse too inexact
     // the GPU-shaped float CPR-AMG (RSG_PREC_CPR_DEVICE): float inverse diagonal of every AMG row, float block-Jacobi
     // inverses (n * 9), per system whether the coarsest inverse exists, the double Gauss-Jordan work matrices
@@ -219,7 +219,8 @@ struct DevAmg {
     size_t* dcWorkOff = nullptr;
     int* rowLv = nullptr;
     int* wave = nullptr;
-    int* gsFlag = nullptr;             // 2 x totRows
+    int* gsFlag = nullptr;             // totRows: the small colours' pass
+    unsigned long long* gsWord = nullptr;   // 2 x totRows: forward and backward values of the sync-free sweeps
     unsigned* gsCtr = nullptr;         // maxL x 4
     std::vector<int> coarseGsLevels;   // host: levels that are some system's coarsest without a dense LU
     // multicolour schedule (FP32 forms), grid-wide: per level the rows of every system that smooths it, colour by
@@ -381,7 +382,8 @@ struct RingDev {
 };
 
 struct SweepState {                   // sync-free sweep flags and claim counters
-    int *flagF = nullptr, *flagB = nullptr, *flagL = nullptr;
+    int* flagL = nullptr;             // factorisation: epoch of every finished row
+    unsigned long long* yw = nullptr; // grid-wide sweeps: word vectors of the forward (3 n) and backward (3 n) results
     unsigned *ctr = nullptr;          // [0] forward, [1] backward, [2] factorisation, [3] spare
 };
 
@@ -403,17 +405,10 @@ void launch_factor_lean(const DevPlan& P, const double* val, float* luf, double*
                         int* err, cudaStream_t st);
 // all-FP32 factorisation (FP32 elimination, FP64 pivot inversion)
 void launch_factor_f32(const DevPlan& P, const double* val, float* luf, SweepState& S, int epoch, int* nreg, int* err, cudaStream_t st);
-// z = U^-1 L^-1 r (FP64 factors, FP64 vectors) or with FP32 factors / FP32 vectors and accumulation.
-void launch_ilu_apply_f64(const DevPlan& P, const double* lu, const double* r, double* z, SweepState& S, int* err,
-                          cudaStream_t st);
-void launch_ilu_apply_f32(const DevPlan& P, const float* luf, const double* r, double* z, unsigned long long* yt, SweepState& S,
-                          int* err, cudaStream_t st);
-// FP32 factors, FP64 vector and accumulation (the reference's float-factor sweeps)
-void launch_ilu_apply_mixed(const DevPlan& P, const float* luf, const double* r, double* z, SweepState& S, int* err,
-                            cudaStream_t st);
-// grid-wide sync-free BILU0 apply z = M^-1 r of the handle's factor kind; systems whose status is not running skip
-void launch_ilu_grid_ks(const DevPlan& P, const PrecDev& M, const double* r, double* z, const KScal* ks, SweepState& S, int* err,
-                        cudaStream_t st);
+// grid-wide sync-free BILU0 sweeps of the handle's factor kind, the input by mode (0 plain, 1 p-update, 2 s-update); systems
+// whose status is not running skip
+void launch_ilu_grid(const DevPlan& P, const PrecDev& M, int mode, const double* r, double* pv, const double* v, double* z, const KScal* ks,
+                     SweepState& S, int* err, cudaStream_t st);
 void launch_spmv_f64(const DevPlan& P, const double* val, const double* x, double* y, cudaStream_t st);
 // x += d over n block rows (3 values each)
 void launch_vec_add(int n, double* x, const double* d, cudaStream_t st);
@@ -427,7 +422,6 @@ void launch_block_jacobi_apply(const DevPlan& P, const double* dinv, const doubl
 struct BicgVecs {
     double *x, *r, *rh, *p, *v, *s, *t, *ph, *sh;
     float* y32;                       // FP32 sweep intermediate of the thread-block sweeps (systems that do not fit on chip)
-    unsigned long long* yt;           // the grid-wide all-FP32 sweeps' vector: tagged words {float, sweep tag}
 };
 void launch_bicg_init(const DevPlan& P, const double* b, BicgVecs& V, KScal* ks, ReduceState& R, double tol, int maxit,
                       int* active, bool guard, bool onlyFailed,
@@ -445,7 +439,6 @@ struct PrecDev {
     SplitFactors<float> s32;
     size_t smem = 0;                  // dynamic shared memory of the CTA sweep (systems whose vector fits keep it there)
     float* y32 = nullptr;             // all-FP32 sweep vector in global memory (systems that do not fit on chip)
-    unsigned long long* yt = nullptr; // grid-wide all-FP32 sweeps: tagged sweep vector
     bool cpr = false;                 // CPR two-stage preconditioner (AMG on the pressure system + BILU0)
     bool devcpr = false;              // the reference's GPU-shaped float CPR-AMG
     bool split = false;               // CPR with cta: V-cycle and second-stage input grid-wide (all systems at once),

@@ -2,8 +2,8 @@
 //
 // * BILU0 factorisation and the forward / backward sweeps are exact natural-order ILU(0): rows are processed in
 //   a level order (a topological order of the L, resp. U, dependencies) by a persistent grid whose warps claim
-//   32 rows at a time from an atomic counter; a row waits for the rows it depends on through per-row flags
-//   (relaxed polls, one acquire fence, a release store when the row is done: rsg_sync.cuh). Claiming in order
+//   rows from an atomic counter; a row waits for the rows it depends on, in the sweeps on their values themselves, in
+//   the factorisation through per-row flags (rsg_sync.cuh). Claiming in order
 //   guarantees that every awaited row belongs to a warp that is already running, so the waits always end; each
 //   wait is additionally bounded and reports RSG_ETIMEOUT.
 // * FP64 block arithmetic uses explicitly rounded multiplies and adds in the reference's loop order
@@ -21,6 +21,7 @@
 #include <cstdio>
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 namespace rsg {
 
@@ -237,149 +238,28 @@ __device__ __forceinline__ bool sys_running(const KScal* ks, const int* rowSys, 
     return ks == nullptr || ks[__ldg(rowSys + i)].status == ST_RUNNING;
 }
 
-// y_i = in_i - sum_{k<i} L_ik y_k   (engine/src/bsr.cpp:568-575)
+// Grid-wide BILU0 sweeps (engine/src/bsr.cpp:568-587). What bounds them is the chain of levels: a row's step is the trip of
+// its neighbours' values through L2 and its own arithmetic. So:
+// * the results travel as words that are their own flags (rsg_sync.cuh): a dependency costs one trip, with no flag, fence
+//   or second load. Two word vectors: yf takes the forward results, yb the backward ones; each sweep clears the other's
+//   words of its rows. Rows of systems that are not running are left out of both;
+// * three lanes take a row, one component each, ten rows per claim: a third of a row's loads and FP64 operations per lane
+//   (a warp of 32 rows kept the FP64 pipe of its SM busy for 0.4 us of every level);
+// * everything that does not depend on a neighbour (factor blocks, the inverted diagonal, the input) is loaded before the
+//   wait.
+// TF: factor storage, TV: vector and arithmetic -- (double, double), (float, double): FP64 explicitly rounded, the
+// reference's sweeps; (float, float): BILU0f (engine/src/bsr.cpp:1100-1121).
 // IN_PUPDATE: in = p = r + beta (p - omega v) (p stored); IN_SUPDATE: in = s = r - alpha v (s stored in pv)
-// factor blocks in FP64 or FP32 storage, read as double (the float-factor sweeps, engine/src/bsr.cpp:500-522)
-__device__ __forceinline__ void ldf9(const double* p, double* a) { load9_ro(p, a); }
-__device__ __forceinline__ void ldf9(const float* p, double* a) {
-#pragma unroll
-    for (int e = 0; e < 9; ++e) a[e] = double(__ldg(p + e));
-}
+constexpr int kSweepRows = 10;               // rows of a warp
 
-// yi -= sum_p B_p y_col(p) over the entries [p0, p1) of a row, in order (FP64 explicitly rounded, the reference's
-// sweep arithmetic). Four blocks at a time: their factor blocks are loaded before the wait (read-only: they need
-// not wait for anything), the four dependency flags are polled together, then one acquire fence and the values.
-template <class TF>
-__device__ __forceinline__ void sub_flagged(double (&yi)[3], const int* __restrict__ col, const TF* __restrict__ lu, int p0, int p1,
-                                            const double* y, const int* flag, int* err) {
-    for (int q = p0; q < p1; q += 4) {
-        const int q1 = q + 4 < p1 ? q + 4 : p1;
-        double a[4][9];
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (q + u < q1) ldf9(lu + size_t(q + u) * 9, a[u]);
-        wait_cols(flag, col, q, q1, 1, err);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            if (q + u >= q1) break;
-            const int k = __ldg(col + q + u);
-            const double yk[3] = {y[size_t(k) * 3 + 0], y[size_t(k) * 3 + 1], y[size_t(k) * 3 + 2]};
-            yi[0] = ds(yi[0], dot3(a[u], yk));
-            yi[1] = ds(yi[1], dot3(a[u] + 3, yk));
-            yi[2] = ds(yi[2], dot3(a[u] + 6, yk));
-        }
-    }
-}
-
-template <class TF, int MODE>
-__global__ void __launch_bounds__(kSweepThreads) k_fwd_f64(int n, const int* __restrict__ rowPtr, const int* __restrict__ col,
-                                                          const int* __restrict__ diag, const int* __restrict__ ford,
-                                                          const TF* __restrict__ lu, const double* r, double* pv,
-                                                          const double* v, double* y, const int* __restrict__ rowSys,
-                                                          const KScal* ks, int* flagF, int* flagB, unsigned* ctr, int* err) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctr[1] = 0u;   // backward claim counter for the next sweep
-    const int lane = threadIdx.x & 31;
-    for (;;) {
-        __syncwarp();
-        const int base = warp_claim(ctr);
-        if (base >= n) break;
-        const int idx = base + lane;
-        if (idx < n) {
-            const int i = __ldg(ford + idx);
-            const bool run = sys_running(ks, rowSys, i);
-            double yi[3];
-            if (MODE == IN_PUPDATE) {
-                const KScal& K = ks[__ldg(rowSys + i)];
-                const double beta = K.beta, omega = K.omega;
-#pragma unroll
-                for (int e = 0; e < 3; ++e) {
-                    const size_t q = size_t(i) * 3 + e;
-                    double pe = pv[q];
-                    if (run) { pe = da(r[q], dm(beta, ds(pe, dm(omega, v[q])))); pv[q] = pe; }
-                    yi[e] = pe;
-                }
-            } else if (MODE == IN_SUPDATE) {
-                const KScal& K = ks[__ldg(rowSys + i)];
-                const double alpha = K.alpha;
-#pragma unroll
-                for (int e = 0; e < 3; ++e) {
-                    const size_t q = size_t(i) * 3 + e;
-                    const double se = ds(r[q], dm(alpha, v[q]));
-                    if (run) pv[q] = se;
-                    yi[e] = se;
-                }
-            } else {
-#pragma unroll
-                for (int e = 0; e < 3; ++e) yi[e] = r[size_t(i) * 3 + e];
-            }
-            if (run) {
-                sub_flagged(yi, col, lu, __ldg(rowPtr + i), __ldg(diag + i), y, flagF, err);
-            }
-            y[size_t(i) * 3 + 0] = yi[0]; y[size_t(i) * 3 + 1] = yi[1]; y[size_t(i) * 3 + 2] = yi[2];
-            flagB[i] = 0;
-            st_release(flagF + i, 1);
-        }
-    }
-}
-
-// z_i = U_ii^-1 (y_i - sum_{j>i} U_ij z_j), in place   (engine/src/bsr.cpp:577-587)
-template <class TF>
-__global__ void __launch_bounds__(kSweepThreads) k_bwd_f64(int n, const int* __restrict__ rowPtr, const int* __restrict__ col,
-                                                          const int* __restrict__ diag, const int* __restrict__ bord,
-                                                          const TF* __restrict__ lu, double* y, const int* __restrict__ rowSys,
-                                                          const KScal* ks, int* flagF, int* flagB, unsigned* ctr, int* err) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctr[0] = 0u;
-    const int lane = threadIdx.x & 31;
-    for (;;) {
-        __syncwarp();
-        const int base = warp_claim(ctr + 1);
-        if (base >= n) break;
-        const int idx = base + lane;
-        if (idx < n) {
-            const int i = __ldg(bord + idx);
-            if (sys_running(ks, rowSys, i)) {
-                double yi[3] = {y[size_t(i) * 3 + 0], y[size_t(i) * 3 + 1], y[size_t(i) * 3 + 2]};
-                const int d = __ldg(diag + i);
-                double D[9];
-                ldf9(lu + size_t(d) * 9, D);
-                sub_flagged(yi, col, lu, d + 1, __ldg(rowPtr + i + 1), y, flagB, err);
-                y[size_t(i) * 3 + 0] = dot3(D, yi);
-                y[size_t(i) * 3 + 1] = dot3(D + 3, yi);
-                y[size_t(i) * 3 + 2] = dot3(D + 6, yi);
-            }
-            flagF[i] = 0;
-            st_release(flagB + i, 1);
-        }
-    }
-}
-
-// FP32 factors, FP32 vectors and accumulation (BILU0f, engine/src/bsr.cpp:1100-1121), the result written to z in
-// double. The sweep vector is a tagged word per component: {float value, sweep tag} in 64 bits (tag 1 once the
-// forward sweep wrote it, 2 once the backward sweep did). A 64-bit access is single-copy atomic, so a poll that
-// sees the tag already holds the value: a dependency costs one round trip, with no flag, no fence and no second
-// load. Every row is written by both sweeps (rows of systems that are not running carry their value along), so
-// the tags alternate and a word never shows the awaited tag before its new value.
-constexpr unsigned kTagF = 1u, kTagB = 2u;
-__device__ __forceinline__ unsigned long long ld_word(const unsigned long long* p) {
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_word(unsigned long long* p, float v, unsigned tag) {
-    const unsigned long long w = (static_cast<unsigned long long>(tag) << 32) | __float_as_uint(v);
-    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
-}
-__device__ __forceinline__ float word_val(unsigned long long w) { return __uint_as_float(unsigned(w & 0xffffffffull)); }
-__device__ __forceinline__ bool word_has(unsigned long long w, unsigned tag) { return unsigned(w >> 32) == tag; }
-// yi -= sum_p B_p y_col(p) over the entries [p0, p1) of a row (in order). The y words of four blocks are awaited
-// together: every poll round re-issues the loads of all words still without the tag (one round trip per round),
-// a short busy phase, then back-off up to 256 ns, bounded (ERR_TIMEOUT).
-__device__ __forceinline__ void sub_tagged(float (&yi)[3], const int* __restrict__ col, const float* __restrict__ lu, int p0, int p1,
-                                           const unsigned long long* y, unsigned tag, int* err) {
+// yi -= sum_p (row e of B_p) . y_col(p) over the entries [p0, p1) of a row, in order, four entries at a time
+template <class TF, class TV>
+__device__ __forceinline__ void sub_polled(TV& yi, const int* __restrict__ col, const TF* __restrict__ lu, int p0, int p1, int e,
+                                           const typename Word<TV>::type* y, int* err) {
     for (int q = p0; q < p1; q += 4) {
         int k[4];
-        unsigned long long w[4][3];
-        float a[4][9];                                            // the factor blocks, loaded before the wait
+        TF a[4][3];
+        TV w[4][3];
         unsigned pending = 0;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -389,128 +269,100 @@ __device__ __forceinline__ void sub_tagged(float (&yi)[3], const int* __restrict
 #pragma unroll
         for (int u = 0; u < 4; ++u)
 #pragma unroll
-            for (int e = 0; e < 9; ++e) a[u][e] = k[u] >= 0 ? __ldg(lu + size_t(q + u) * 9 + e) : 0.f;
+            for (int f = 0; f < 3; ++f) a[u][f] = k[u] >= 0 ? __ldg(lu + size_t(q + u) * 9 + 3 * e + f) : TF(0);
         unsigned ns = 0;
         for (unsigned it = 0; pending; ++it) {
+            typename Word<TV>::type got[4][3];
 #pragma unroll
             for (int u = 0; u < 4; ++u)
 #pragma unroll
-                for (int e = 0; e < 3; ++e)
-                    if ((pending >> (3 * u + e)) & 1u) w[u][e] = ld_word(y + size_t(k[u]) * 3 + e);
+                for (int f = 0; f < 3; ++f)
+                    if ((pending >> (3 * u + f)) & 1u) got[u][f] = ld_word(y + size_t(k[u]) * 3 + f);
 #pragma unroll
             for (int u = 0; u < 4; ++u)
 #pragma unroll
-                for (int e = 0; e < 3; ++e)
-                    if (((pending >> (3 * u + e)) & 1u) && word_has(w[u][e], tag)) pending &= ~(1u << (3 * u + e));
-            if (!pending) break;
-            if (it >= 64) {
-                __nanosleep(ns);
-                ns = ns < 32 ? 32 : (ns < 256 ? 2 * ns : 256);
-                if (it >= 64 + kSpinLimit) { atomicOr(err, ERR_TIMEOUT); break; }
-                if ((it & 255u) == 255u && *(volatile int*)err != 0) break;
-            }
+                for (int f = 0; f < 3; ++f)
+                    if (((pending >> (3 * u + f)) & 1u) && got[u][f] != Word<TV>::empty) {
+                        w[u][f] = Word<TV>::value(got[u][f]);
+                        pending &= ~(1u << (3 * u + f));
+                    }
+            if (!pending || !poll_again(it, ns, err)) break;
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             if (k[u] < 0) break;
-            const float y0 = word_val(w[u][0]), y1 = word_val(w[u][1]), y2 = word_val(w[u][2]);
-#pragma unroll
-            for (int e = 0; e < 3; ++e) {
-                float s = 0.f;
-                s += a[u][e * 3 + 0] * y0;
-                s += a[u][e * 3 + 1] * y1;
-                s += a[u][e * 3 + 2] * y2;
-                yi[e] -= s;
-            }
+            yi = vsub(yi, rdot(a[u], w[u]));
         }
     }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(kSweepThreads) k_fwd_f32(int n, const int* __restrict__ rowPtr, const int* __restrict__ col,
-                                                          const int* __restrict__ diag, const int* __restrict__ ford,
-                                                          const float* __restrict__ lu, const double* r, double* pv,
-                                                          const double* v, unsigned long long* y, const int* __restrict__ rowSys,
-                                                          const KScal* ks, unsigned* ctr, int* err) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctr[1] = 0u;
-    const int lane = threadIdx.x & 31;
+template <class TF, class TV, int MODE>
+__global__ void __launch_bounds__(kSweepThreads) k_fwd(int n, const int* __restrict__ rowPtr, const int* __restrict__ col,
+                                                       const int* __restrict__ diag, const int* __restrict__ ford, const TF* __restrict__ lu,
+                                                       const double* r, double* pv, const double* v, typename Word<TV>::type* yf,
+                                                       typename Word<TV>::type* yb, const int* __restrict__ rowSys, const KScal* ks,
+                                                       unsigned* ctr, int* err) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctr[1] = 0u;   // backward claim counter for the next sweep
+    const int lane = threadIdx.x & 31, rr = lane / 3, e = lane % 3;
     for (;;) {
         __syncwarp();
-        const int base = warp_claim(ctr);
+        const int base = warp_claim(ctr, kSweepRows);
         if (base >= n) break;
-        const int idx = base + lane;
-        if (idx < n) {
-            const int i = __ldg(ford + idx);
-            const bool run = sys_running(ks, rowSys, i);
-            float yi[3];
-            if (MODE == IN_PUPDATE) {
-                const KScal& K = ks[__ldg(rowSys + i)];
-                const double beta = K.beta, omega = K.omega;
-#pragma unroll
-                for (int e = 0; e < 3; ++e) {
-                    const size_t q = size_t(i) * 3 + e;
-                    double pe = pv[q];
-                    if (run) { pe = da(r[q], dm(beta, ds(pe, dm(omega, v[q])))); pv[q] = pe; }
-                    yi[e] = float(pe);
-                }
-            } else if (MODE == IN_SUPDATE) {
-                const KScal& K = ks[__ldg(rowSys + i)];
-                const double alpha = K.alpha;
-#pragma unroll
-                for (int e = 0; e < 3; ++e) {
-                    const size_t q = size_t(i) * 3 + e;
-                    const double se = ds(r[q], dm(alpha, v[q]));
-                    if (run) pv[q] = se;
-                    yi[e] = float(se);
-                }
-            } else {
-#pragma unroll
-                for (int e = 0; e < 3; ++e) yi[e] = float(r[size_t(i) * 3 + e]);
-            }
-            if (run) sub_tagged(yi, col, lu, __ldg(rowPtr + i), __ldg(diag + i), y, kTagF, err);
-#pragma unroll
-            for (int e = 0; e < 3; ++e) st_word(y + size_t(i) * 3 + e, yi[e], kTagF);
+        const int idx = base + rr;
+        if (rr >= kSweepRows || idx >= n) continue;
+        const int i = __ldg(ford + idx);
+        if (!sys_running(ks, rowSys, i)) continue;
+        const size_t q = size_t(i) * 3 + e;
+        double in;
+        if (MODE == IN_PUPDATE) {
+            const KScal& K = ks[__ldg(rowSys + i)];
+            in = da(r[q], dm(K.beta, ds(pv[q], dm(K.omega, v[q]))));
+            pv[q] = in;
+        } else if (MODE == IN_SUPDATE) {
+            const KScal& K = ks[__ldg(rowSys + i)];
+            in = ds(r[q], dm(K.alpha, v[q]));
+            pv[q] = in;
+        } else {
+            in = r[q];
         }
+        TV yi = TV(in);
+        sub_polled<TF, TV>(yi, col, lu, __ldg(rowPtr + i), __ldg(diag + i), e, yf, err);
+        st_word(yf + q, Word<TV>::make(yi));
+        yb[q] = Word<TV>::empty;
     }
 }
 
-__global__ void __launch_bounds__(kSweepThreads) k_bwd_f32(int n, const int* __restrict__ rowPtr, const int* __restrict__ col,
-                                                          const int* __restrict__ diag, const int* __restrict__ bord,
-                                                          const float* __restrict__ lu, unsigned long long* y, double* z,
-                                                          const int* __restrict__ rowSys, const KScal* ks, unsigned* ctr, int* err) {
+// z_i = U_ii^-1 (y_i - sum_{j>i} U_ij z_j)   (engine/src/bsr.cpp:577-587)
+template <class TF, class TV>
+__global__ void __launch_bounds__(kSweepThreads) k_bwd(int n, const int* __restrict__ rowPtr, const int* __restrict__ col,
+                                                       const int* __restrict__ diag, const int* __restrict__ bord, const TF* __restrict__ lu,
+                                                       typename Word<TV>::type* yf, typename Word<TV>::type* yb, double* z,
+                                                       const int* __restrict__ rowSys, const KScal* ks, unsigned* ctr, int* err) {
     if (blockIdx.x == 0 && threadIdx.x == 0) ctr[0] = 0u;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, rr = lane / 3, e = lane % 3;
+    const unsigned mine = 7u << (3 * rr);                    // the row's lanes (a warp's rows may depend on each other)
     for (;;) {
         __syncwarp();
-        const int base = warp_claim(ctr + 1);
+        const int base = warp_claim(ctr + 1, kSweepRows);
         if (base >= n) break;
-        const int idx = base + lane;
-        if (idx < n) {
-            const int i = __ldg(bord + idx);
-            float yi[3] = {word_val(ld_word(y + size_t(i) * 3 + 0)), word_val(ld_word(y + size_t(i) * 3 + 1)),
-                           word_val(ld_word(y + size_t(i) * 3 + 2))};
-            if (sys_running(ks, rowSys, i)) {
-                const int d = __ldg(diag + i);
-                sub_tagged(yi, col, lu, d + 1, __ldg(rowPtr + i + 1), y, kTagB, err);
-                const float* D = lu + size_t(d) * 9;
-                float t[3];
+        const int idx = base + rr;
+        if (rr >= kSweepRows || idx >= n) continue;
+        const int i = __ldg(bord + idx);
+        if (!sys_running(ks, rowSys, i)) continue;
+        const size_t q = size_t(i) * 3 + e;
+        const int d = __ldg(diag + i);
+        TF D[3];
 #pragma unroll
-                for (int e = 0; e < 3; ++e) {
-                    float s = 0.f;
-                    s += __ldg(D + e * 3 + 0) * yi[0];
-                    s += __ldg(D + e * 3 + 1) * yi[1];
-                    s += __ldg(D + e * 3 + 2) * yi[2];
-                    t[e] = s;
-                }
+        for (int f = 0; f < 3; ++f) D[f] = __ldg(lu + size_t(d) * 9 + 3 * e + f);
+        TV yi = Word<TV>::value(yf[q]);
+        yf[q] = Word<TV>::empty;
+        sub_polled<TF, TV>(yi, col, lu, d + 1, __ldg(rowPtr + i + 1), e, yb, err);
+        TV w[3];
 #pragma unroll
-                for (int e = 0; e < 3; ++e) {
-                    yi[e] = t[e];
-                    z[size_t(i) * 3 + e] = double(t[e]);
-                }
-            }
-#pragma unroll
-            for (int e = 0; e < 3; ++e) st_word(y + size_t(i) * 3 + e, yi[e], kTagB);
-        }
+        for (int f = 0; f < 3; ++f) w[f] = __shfl_sync(mine, yi, 3 * rr + f);
+        const TV t = rdot(D, w);
+        st_word(yb + q, Word<TV>::make(t));
+        z[q] = double(t);
     }
 }
 
@@ -853,50 +705,28 @@ void launch_factor_f32(const DevPlan& P, const double* val, float* luf, SweepSta
     launch_factor_t<float, float>(P, val, luf, luf, S, epoch, nreg, err, st);
 }
 
-void launch_ilu_apply_f64(const DevPlan& P, const double* lu, const double* r, double* z, SweepState& S, int* err,
-                          cudaStream_t st) {
-    const int g = sweep_blocks(P);
-    k_fwd_f64<double, IN_PLAIN><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, lu, r, nullptr, nullptr, z, P.rowSys,
-                                                     nullptr, S.flagF, S.flagB, S.ctr, err);
-    k_bwd_f64<double><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.bord, lu, z, P.rowSys, nullptr, S.flagF, S.flagB, S.ctr,
-                                          err);
+// both sweeps, the input by mode
+template <class TF, class TV>
+static void launch_sweeps(const DevPlan& P, const TF* lu, int mode, const double* r, double* pv, const double* v, double* z, const KScal* ks,
+                          SweepState& S, int* err, cudaStream_t st) {
+    using U = typename Word<TV>::type;
+    const int g = std::min(sweep_blocks(P), std::max(1, (P.n + 4 * kSweepRows - 1) / (4 * kSweepRows)));
+    U* yf = reinterpret_cast<U*>(S.yw);
+    U* yb = reinterpret_cast<U*>(S.yw + size_t(P.n) * 3);
+    auto fwd = [&](auto tag) {
+        k_fwd<TF, TV, decltype(tag)::value><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, lu, r, pv, v, yf, yb, P.rowSys, ks,
+                                                                         S.ctr, err);
+    };
+    if (mode == IN_PUPDATE) fwd(std::integral_constant<int, IN_PUPDATE>());
+    else if (mode == IN_SUPDATE) fwd(std::integral_constant<int, IN_SUPDATE>());
+    else fwd(std::integral_constant<int, IN_PLAIN>());
+    k_bwd<TF, TV><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.bord, lu, yf, yb, z, P.rowSys, ks, S.ctr, err);
 }
-
-void launch_ilu_apply_mixed(const DevPlan& P, const float* luf, const double* r, double* z, SweepState& S, int* err,
-                            cudaStream_t st) {
-    const int g = sweep_blocks(P);
-    k_fwd_f64<float, IN_PLAIN><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, luf, r, nullptr, nullptr, z, P.rowSys,
-                                                           nullptr, S.flagF, S.flagB, S.ctr, err);
-    k_bwd_f64<float><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.bord, luf, z, P.rowSys, nullptr, S.flagF, S.flagB, S.ctr,
-                                                 err);
-}
-
-void launch_ilu_apply_f32(const DevPlan& P, const float* luf, const double* r, double* z, unsigned long long* y32, SweepState& S, int* err,
-                          cudaStream_t st) {
-    const int g = sweep_blocks(P);
-    k_fwd_f32<IN_PLAIN><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, luf, r, nullptr, nullptr, y32, P.rowSys,
-                                                     nullptr, S.ctr, err);
-    k_bwd_f32<<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.bord, luf, y32, z, P.rowSys, nullptr, S.ctr, err);
-}
-
-void launch_ilu_grid_ks(const DevPlan& P, const PrecDev& M, const double* r, double* z, const KScal* ks, SweepState& S, int* err,
-                        cudaStream_t st) {
-    const int g = sweep_blocks(P);
-    if (M.kind == 0) {
-        k_fwd_f64<double, IN_PLAIN><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, M.lu, r, nullptr, nullptr, z,
-                                                                 P.rowSys, ks, S.flagF, S.flagB, S.ctr, err);
-        k_bwd_f64<double><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.bord, M.lu, z, P.rowSys, ks, S.flagF, S.flagB,
-                                                       S.ctr, err);
-    } else if (M.kind == 1) {
-        k_fwd_f64<float, IN_PLAIN><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, M.luf, r, nullptr, nullptr, z,
-                                                                P.rowSys, ks, S.flagF, S.flagB, S.ctr, err);
-        k_bwd_f64<float><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.bord, M.luf, z, P.rowSys, ks, S.flagF, S.flagB,
-                                                      S.ctr, err);
-    } else {
-        k_fwd_f32<IN_PLAIN><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, M.luf, r, nullptr, nullptr, M.yt,
-                                                         P.rowSys, ks, S.ctr, err);
-        k_bwd_f32<<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.bord, M.luf, M.yt, z, P.rowSys, ks, S.ctr, err);
-    }
+void launch_ilu_grid(const DevPlan& P, const PrecDev& M, int mode, const double* r, double* pv, const double* v, double* z, const KScal* ks,
+                     SweepState& S, int* err, cudaStream_t st) {
+    if (M.kind == 0) launch_sweeps<double, double>(P, M.lu, mode, r, pv, v, z, ks, S, err, st);
+    else if (M.kind == 1) launch_sweeps<float, double>(P, M.luf, mode, r, pv, v, z, ks, S, err, st);
+    else launch_sweeps<float, float>(P, M.luf, mode, r, pv, v, z, ks, S, err, st);
 }
 
 template <int MODE, bool FMA>
@@ -960,7 +790,6 @@ void launch_bicg_init(const DevPlan& P, const double* b, BicgVecs& V, KScal* ks,
 // (f) t = A sh + <t,t>, <t,s>, <s,s>, (g) x / r update + ||r||, <rh,r>
 void launch_bicg_iteration(const DevPlan& P, const double* val, const PrecDev& M, BicgVecs& V, KScal* ks, ReduceState& R,
                            SweepState& S, int* active, int* err, cudaStream_t st) {
-    const int g = sweep_blocks(P);
     auto prec = [&](bool pupd, double* out) {
         if (M.devcpr) {
             launch_devcpr(P, *M.amg, val, pupd ? 1 : 2, V.r, pupd ? V.p : V.s, V.v, out, ks, st);
@@ -970,32 +799,8 @@ void launch_bicg_iteration(const DevPlan& P, const double* val, const PrecDev& M
             launch_cpr_grid(P, M, *M.amg, pupd ? 1 : 2, V.r, pupd ? V.p : V.s, V.v, out, ks, S, err, st);
         } else if (M.cta && M.kind != 2) {
             launch_ilu_cta_fused(P, M, pupd, V.r, pupd ? V.p : V.s, V.v, out, ks, st);
-        } else if (M.kind == 0) {
-            if (pupd)
-                k_fwd_f64<double, IN_PUPDATE><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, M.lu, V.r, V.p, V.v, out,
-                                                                           P.rowSys, ks, S.flagF, S.flagB, S.ctr, err);
-            else
-                k_fwd_f64<double, IN_SUPDATE><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, M.lu, V.r, V.s, V.v, out,
-                                                                           P.rowSys, ks, S.flagF, S.flagB, S.ctr, err);
-            k_bwd_f64<double><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.bord, M.lu, out, P.rowSys, ks, S.flagF,
-                                                          S.flagB, S.ctr, err);
-        } else if (M.kind == 1) {      // FP32 factors, FP64 sweep vector
-            if (pupd)
-                k_fwd_f64<float, IN_PUPDATE><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, M.luf, V.r, V.p, V.v, out,
-                                                                          P.rowSys, ks, S.flagF, S.flagB, S.ctr, err);
-            else
-                k_fwd_f64<float, IN_SUPDATE><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, M.luf, V.r, V.s, V.v, out,
-                                                                          P.rowSys, ks, S.flagF, S.flagB, S.ctr, err);
-            k_bwd_f64<float><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.bord, M.luf, out, P.rowSys, ks, S.flagF,
-                                                         S.flagB, S.ctr, err);
-        } else if (M.kind == 3) {      // all-FP32 sweep
-            if (pupd)
-                k_fwd_f32<IN_PUPDATE><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, M.luf, V.r, V.p, V.v, V.yt,
-                                                                   P.rowSys, ks, S.ctr, err);
-            else
-                k_fwd_f32<IN_SUPDATE><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, M.luf, V.r, V.s, V.v, V.yt,
-                                                                   P.rowSys, ks, S.ctr, err);
-            k_bwd_f32<<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.bord, M.luf, V.yt, out, P.rowSys, ks, S.ctr, err);
+        } else if (M.kind != 2) {
+            launch_ilu_grid(P, M, pupd ? IN_PUPDATE : IN_SUPDATE, V.r, pupd ? V.p : V.s, V.v, out, ks, S, err, st);
         } else {
             const int gb = (P.n + 127) / 128;
             if (pupd)

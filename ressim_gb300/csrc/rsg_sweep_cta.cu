@@ -1327,7 +1327,7 @@ void launch_cpr_cta(const DevPlan& P, const PrecDev& M, const DevAmg& G, int mod
 // Here every step of BlockCPR::apply runs over the whole batch, one AMG level at a time, with the arithmetic of
 // the thread-block V-cycle:
 // * Gauss-Seidel sweeps are sync-free: a persistent grid claims the level's rows in schedule order (forward levels
-//   of the reference order, or colours) and a row waits, through per-row flags, only for its neighbours of an
+//   of the reference order, or colours) and a row waits, on their values themselves, only for its neighbours of an
 //   earlier wave (the rows a forward sweep updates before it: its lower-numbered neighbours in the reference order,
 //   whose forward level is lower, or those of an earlier colour). Its other neighbours wait for it in turn
 //   (structurally symmetric levels), so their old values are still in place when it reads them. Claiming in
@@ -1382,15 +1382,23 @@ __global__ void __launch_bounds__(256) k_gcpr_in(int n, const int* __restrict__ 
 // one Gauss-Seidel sweep of level l over every system (engine/src/amg.cpp:98-113). Positions [q0, q1) of the
 // level's schedule, claimed forward or backward. phase 0: the smoothing sweeps (systems whose level l is the
 // coarsest skip); phase 1: the symmetric GS solve of a coarsest level without dense LU. ZERO: pre-smoothing from
-// x = 0 (the terms of the neighbours not yet updated vanish and are not read). Flags of skipped rows are set all
-// the same: after every forward sweep of a (level, phase) all its flags are 1, after every backward sweep 0.
+// x = 0 (the terms of the neighbours not yet updated vanish and are not read).
+// The neighbours updated before a row in the sweep are read from the sweep's word vector (values that are their own flags,
+// rsg_sync.cuh: wf forward, wb backward; each sweep clears the other's words of its rows), the others from x: they are
+// updated after this row, which they wait for. The forward and the backward sweep of a (level, phase) alternate.
 template <class TA, bool FWD, bool ZERO, bool POS>
 __device__ __forceinline__ void gs_grid_body(int q0, int q1, int maxL, int phase, const int* __restrict__ rowLv,
                                                           const AmgSysLv* __restrict__ lv, const int* __restrict__ gsRows,
                                                           const int* __restrict__ wave, const int* __restrict__ rp,
                                                           const int* __restrict__ ci, const TA* __restrict__ val,
-                                                          const int* __restrict__ diag, const TA* b, TA* x, int* flag, unsigned* ctr,
-                                                          const KScal* ks, int* err) {
+                                                          const int* __restrict__ diag, const TA* b, TA* x, unsigned long long* words,
+                                                          int totRows, unsigned* ctr, const KScal* ks, int* err) {
+    using U = typename Word<TA>::type;
+    U* wf = reinterpret_cast<U*>(words);
+    U* wb = reinterpret_cast<U*>(words + totRows);
+    const U* in = FWD ? wf : wb;
+    U* out = FWD ? wf : wb;
+    U* clear = FWD ? wb : wf;
     if (blockIdx.x == 0 && threadIdx.x == 0) ctr[FWD ? 1 : 0] = 0u;   // the opposite direction's counter, for its next sweep
     const int n = q1 - q0, lane = int(threadIdx.x & 31);
     for (;;) {
@@ -1398,58 +1406,70 @@ __device__ __forceinline__ void gs_grid_body(int q0, int q1, int maxL, int phase
         const int base = warp_claim(ctr + (FWD ? 0 : 1));
         if (base >= n) break;
         const int idx = base + lane;
-        if (idx < n) {
-            const int g = FWD ? q0 + idx : q1 - 1 - idx;
-            const int sl = __ldg(rowLv + g);
-            const AmgSysLv* A = lv + sl;
-            const int rowOff = __ldg(&A->rowOff), coarse = __ldg(&A->coarse);
-            const int row = rowOff + __ldg(gsRows + g);
-            bool act = phase == 0 ? !coarse : (coarse && !__ldg(&A->dense));
-            if (act && ks) act = ks[sl / maxL].status == ST_RUNNING;
-            if (act) {
-                const int k = row - rowOff, rpOff = __ldg(&A->rpOff), entOff = __ldg(&A->entOff);
-                const int p0 = __ldg(rp + rpOff + k), p1 = __ldg(rp + rpOff + k + 1), pd = __ldg(diag + row);
-                const int* cl = ci + entOff;
-                const TA* vl = val + entOff;
-                const int wi = POS ? 0 : __ldg(wave + row);
-                // the neighbours updated before this row in the sweep: of an earlier wave (forward), a later one
-                // (backward); POS: the entries before (after) the diagonal, which the plan checked to be the same
-                auto dep = [&](int p) {
-                    if (p == pd) return false;
-                    if (POS) return FWD ? p < pd : p > pd;
-                    const int w = __ldg(wave + rowOff + __ldg(cl + p));
-                    return FWD ? w < wi : w > wi;
-                };
-                const int w0 = POS ? (FWD ? p0 : pd + 1) : p0, w1 = POS ? (FWD ? pd : p1) : p1;
-                const int e1 = (FWD && ZERO && POS) ? pd : p1;         // from zero: only the updated neighbours count
-                TA vp[8];                                              // the row's first values and columns, loaded
-                int jp[8];                                             // before the wait (read-only)
+        if (idx >= n) continue;
+        const int g = FWD ? q0 + idx : q1 - 1 - idx;
+        const int sl = __ldg(rowLv + g);
+        const AmgSysLv* A = lv + sl;
+        const int rowOff = __ldg(&A->rowOff), coarse = __ldg(&A->coarse);
+        const int row = rowOff + __ldg(gsRows + g);
+        bool act = phase == 0 ? !coarse : (coarse && !__ldg(&A->dense));
+        if (act && ks) act = ks[sl / maxL].status == ST_RUNNING;
+        if (!act) continue;
+        const int k = row - rowOff, rpOff = __ldg(&A->rpOff), entOff = __ldg(&A->entOff);
+        const int p0 = __ldg(rp + rpOff + k), p1 = __ldg(rp + rpOff + k + 1), pd = __ldg(diag + row);
+        const int* cl = ci + entOff;
+        const TA* vl = val + entOff;
+        const int wi = POS ? 0 : __ldg(wave + row);
+        const TA dv = __ldg(vl + pd);
+        TA s = b[row];
+        const int e1 = (FWD && ZERO && POS) ? pd : p1;                 // from zero: only the updated neighbours count
+        constexpr int CH = 8;                                          // entries at a time: loads, then waits, then the terms in order
+        for (int pc = p0; pc < e1; pc += CH) {
+            int j[CH];
+            TA a[CH], xv[CH];
+            unsigned take = 0, pending = 0;
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    vp[u] = p0 + u < e1 ? __ldg(vl + p0 + u) : TA(0);
-                    jp[u] = p0 + u < e1 ? rowOff + __ldg(cl + p0 + u) : 0;
-                }
-                const TA dv = __ldg(vl + pd);
-                wait_deps(flag, w0, w1, FWD ? 1 : 0, err, [&](int p) { return rowOff + __ldg(cl + p); }, dep);
-                TA s = b[row];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int p = p0 + u;
-                    if (p >= e1) break;
-                    if (p == pd) continue;
-                    if (FWD && ZERO && !POS && __ldg(wave + jp[u]) > wi) continue;   // x_j is still zero: the term vanishes
-                    s = asub(s, amul(vp[u], x[jp[u]]));
-                }
-                for (int p = p0 + 8; p < e1; ++p) {
-                    if (p == pd) continue;
-                    const int j = rowOff + __ldg(cl + p);
-                    if (FWD && ZERO && !POS && __ldg(wave + j) > wi) continue;
-                    s = asub(s, amul(__ldg(vl + p), x[j]));
-                }
-                x[row] = adiv(s, dv);
+            for (int u = 0; u < CH; ++u) {
+                const int p = pc + u;
+                const bool ok = p < e1 && p != pd;
+                j[u] = ok ? rowOff + __ldg(cl + p) : 0;
+                a[u] = ok ? __ldg(vl + p) : TA(0);
+                if (ok) take |= 1u << u;
             }
-            st_release(flag + row, FWD ? 1 : 0);
+#pragma unroll
+            for (int u = 0; u < CH; ++u)
+                if ((take >> u) & 1u) {
+                    // updated before this row in the sweep: of an earlier wave (forward), a later one (backward); POS: the
+                    // entries before (after) the diagonal, which the plan checked to be the same
+                    const int p = pc + u;
+                    const int w = POS ? 0 : __ldg(wave + j[u]);
+                    const bool dep = POS ? (FWD ? p < pd : p > pd) : (FWD ? w < wi : w > wi);
+                    if (dep) pending |= 1u << u;
+                    else if (FWD && ZERO && (POS || w > wi)) take &= ~(1u << u);   // x_j is still zero: the term vanishes
+                    else xv[u] = x[j[u]];
+                }
+            unsigned ns = 0;
+            for (unsigned it = 0; pending; ++it) {
+                U got[CH];
+#pragma unroll
+                for (int u = 0; u < CH; ++u)
+                    if ((pending >> u) & 1u) got[u] = ld_word(in + j[u]);
+#pragma unroll
+                for (int u = 0; u < CH; ++u)
+                    if (((pending >> u) & 1u) && got[u] != Word<TA>::empty) {
+                        xv[u] = Word<TA>::value(got[u]);
+                        pending &= ~(1u << u);
+                    }
+                if (!pending || !poll_again(it, ns, err)) break;
+            }
+#pragma unroll
+            for (int u = 0; u < CH; ++u)
+                if ((take >> u) & 1u) s = asub(s, amul(a[u], xv[u]));
         }
+        const TA xn = adiv(s, dv);
+        st_word(out + row, Word<TA>::make(xn));
+        x[row] = xn;
+        clear[row] = Word<TA>::empty;
     }
 }
 template <class TA, bool FWD, bool ZERO, bool POS>
@@ -1457,9 +1477,9 @@ __global__ void __launch_bounds__(kGridThreads) k_gs_grid(int q0, int q1, int ma
                                                           const AmgSysLv* __restrict__ lv, const int* __restrict__ gsRows,
                                                           const int* __restrict__ wave, const int* __restrict__ rp,
                                                           const int* __restrict__ ci, const TA* __restrict__ val,
-                                                          const int* __restrict__ diag, const TA* b, TA* x, int* flag, unsigned* ctr,
-                                                          const KScal* ks, int* err) {
-    gs_grid_body<TA, FWD, ZERO, POS>(q0, q1, maxL, phase, rowLv, lv, gsRows, wave, rp, ci, val, diag, b, x, flag, ctr, ks, err);
+                                                          const int* __restrict__ diag, const TA* b, TA* x, unsigned long long* words,
+                                                          int totRows, unsigned* ctr, const KScal* ks, int* err) {
+    gs_grid_body<TA, FWD, ZERO, POS>(q0, q1, maxL, phase, rowLv, lv, gsRows, wave, rp, ci, val, diag, b, x, words, totRows, ctr, ks, err);
 }
 
 // Multicolour Gauss-Seidel (FP32 forms) on the colour-major row descriptors {row, first entry, end, diagonal}:
@@ -1851,6 +1871,7 @@ struct VcArgs {
     const int4* cdesc;
     const TA* val;
     int* gsFlag;
+    unsigned long long* gsWord;
     unsigned* gsCtr;
     const int4 *Lslot, *Uslot;
     const int *LovCol, *UovCol;
@@ -1910,17 +1931,17 @@ __global__ void __launch_bounds__(256, 4) k_vcycle(const VPhase* __restrict__ ph
             break;
         }
         case VP_GSGRID: {
-            int* flag = A.gsFlag + size_t(f.d) * size_t(A.totRows);
+            unsigned long long* words = A.gsWord;
             unsigned* ctr = A.gsCtr + 4 * f.c + 2 * f.d;
             if (f.e && f.f)
                 gs_grid_body<TA, true, true, POS>(f.a, f.b, A.maxL, f.d, A.rowLv, A.lv, A.gsRows, A.wave, A.rp, A.ci, A.val, A.diag, A.C.b, A.C.x,
-                                                  flag, ctr, ks, err);
+                                                  words, A.totRows, ctr, ks, err);
             else if (f.e)
                 gs_grid_body<TA, true, false, POS>(f.a, f.b, A.maxL, f.d, A.rowLv, A.lv, A.gsRows, A.wave, A.rp, A.ci, A.val, A.diag, A.C.b,
-                                                   A.C.x, flag, ctr, ks, err);
+                                                   A.C.x, words, A.totRows, ctr, ks, err);
             else
                 gs_grid_body<TA, false, false, POS>(f.a, f.b, A.maxL, f.d, A.rowLv, A.lv, A.gsRows, A.wave, A.rp, A.ci, A.val, A.diag, A.C.b,
-                                                    A.C.x, flag, ctr, ks, err);
+                                                    A.C.x, words, A.totRows, ctr, ks, err);
             break;
         }
         case VP_RESID:
@@ -2059,7 +2080,7 @@ int cpr_grid(const DevPlan& P, const PrecDev& M, const DevAmg& G, const CprArgs<
     if (M.split && M.vform == 1 && G.nPhases > 0) {
         // the whole pass sequence (input .. t) as the phases of one cooperative launch, then the BILU0 stage
         VcArgs<TA, TT> A{C, n, P.nsys, G.maxL, G.totRows, P.rowSys, P.sysRow0, r, v, pv, Tsplit, G.rowLv, G.gsRows, G.wave, G.rp, G.ci,
-                         G.diag, G.gci, G.agg, G.lv, G.cdesc, val, G.gsFlag, G.gsCtr, P.Lslot, P.Uslot, P.LovCol, P.UovCol,
+                         G.diag, G.gci, G.agg, G.lv, G.cdesc, val, G.gsFlag, G.gsWord, G.gsCtr, P.Lslot, P.Uslot, P.LovCol, P.UovCol,
                          G.coarseChunks};
         cudaMemsetAsync(G.vbar, 0, sizeof(unsigned), st);
         if (G.posOrder) launch_vcycle<TA, TT, true>(G, A, mode, ks, err, st);
@@ -2120,20 +2141,19 @@ int cpr_grid(const DevPlan& P, const PrecDev& M, const DevAmg& G, const CprArgs<
             return;
         }
         const int q0 = LB[size_t(l)], q1 = LB[size_t(l) + 1];
-        int* flag = G.gsFlag + size_t(phase) * size_t(G.totRows);
         unsigned* ctr = G.gsCtr + 4 * l + 2 * phase;
         const int g = G.gsBlocks[size_t(l)];
         auto go = [&](auto pos) {
             constexpr bool POS = decltype(pos)::value;
             if (fwd && zero)
                 k_gs_grid<TA, true, true, POS><<<g, kGridThreads, 0, st>>>(q0, q1, G.maxL, phase, G.rowLv, G.lv, G.gsRows, G.wave, G.rp,
-                                                                            G.ci, val, G.diag, C.b, C.x, flag, ctr, ks, err);
+                                                                            G.ci, val, G.diag, C.b, C.x, G.gsWord, G.totRows, ctr, ks, err);
             else if (fwd)
                 k_gs_grid<TA, true, false, POS><<<g, kGridThreads, 0, st>>>(q0, q1, G.maxL, phase, G.rowLv, G.lv, G.gsRows, G.wave, G.rp,
-                                                                             G.ci, val, G.diag, C.b, C.x, flag, ctr, ks, err);
+                                                                             G.ci, val, G.diag, C.b, C.x, G.gsWord, G.totRows, ctr, ks, err);
             else
                 k_gs_grid<TA, false, false, POS><<<g, kGridThreads, 0, st>>>(q0, q1, G.maxL, phase, G.rowLv, G.lv, G.gsRows, G.wave, G.rp,
-                                                                              G.ci, val, G.diag, C.b, C.x, flag, ctr, ks, err);
+                                                                              G.ci, val, G.diag, C.b, C.x, G.gsWord, G.totRows, ctr, ks, err);
         };
         if (G.posOrder) go(std::true_type());
         else go(std::false_type());
@@ -2178,7 +2198,7 @@ int cpr_grid(const DevPlan& P, const PrecDev& M, const DevAmg& G, const CprArgs<
         return launches + 2;
     }
     k_gcpr_t<TA, TT><<<gn, 256, 0, st>>>(n, P.rowSys, P.rowPtr, P.col, M.val, C.x, G.T, ks);
-    launch_ilu_grid_ks(P, M, G.T, z, ks, S, err, st);
+    launch_ilu_grid(P, M, IN_PLAIN, G.T, nullptr, nullptr, z, ks, S, err, st);
     k_gcpr_zp<TA><<<gn, 256, 0, st>>>(n, P.rowSys, C.x, z, ks);
     return launches + 4;
 }
