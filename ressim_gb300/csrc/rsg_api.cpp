@@ -148,7 +148,7 @@ struct rsg_solver {
         int split = -1;              // CPR form on the thread-block path: -1 as planned (splitCpr), 0 one kernel, 1 split
         int vform = 3;
         int cpr2Threads = 256;
-        int ring = 1;                // BILU0 stage on the ring where it fits (0: the thread count's own kernel)
+        int stage = 1;               // BILU0 stage as ilu_stage takes it (0: the thread count's own kernel)
         std::string desc = "defaults";
     } tune;
     unsigned long long patHash = 0;   // FNV-1a of the plan's pattern (0: not computed)
@@ -305,17 +305,30 @@ int check_device_errors(rsg_solver* h) {
 // kernel launches of one preconditioner application
 int precond_launches(const PrecDev& M) {
     if (M.devcpr) return devcpr_launches(*M.amg);
-    if (M.cpr && (!M.cta || M.split)) return cpr_grid_launches(*M.amg, M.split, M.vform);
-    return M.cpr || M.cta || M.kind == 2 ? 1 : 2;
+    if (M.cpr && (!M.cta || M.split)) return cpr_grid_launches(*M.amg, M.split, M.vform) + (M.gridIlu ? 1 : 0);
+    return (M.cpr || M.cta || M.kind == 2) && !M.gridIlu ? 1 : 2;
 }
 
-// whether the thread-block BILU0 stage of this factor kind (0 FP64, 1 FP32 factors with FP64 vectors, 3 all FP32) runs on
-// the ring: its vector and steps fit one SM, and the launch shape is not fixed by the options (the one-kernel CPR
-// application and a BILU0 stage of a given thread count read the component-major records)
-bool ring_on(const rsg_solver* h, int kind) {
-    if (!h->cta || kind == 2 || h->opt.cpr2_threads != 0 || !h->tune.ring) return false;
-    if (h->opt.precond == RSG_PREC_CPR && h->opt.sweep == 1) return false;
-    return ring_fits(h->ring[kind == 3 ? 1 : 0], kind != 0, kind == 3);
+// How the BILU0 stage of a factor kind (0 FP64, 1 FP32 factors with FP64 vectors, 3 all FP32) runs on systems with a
+// thread-block plan:
+// * on the ring where its vector and steps fit one SM and the arithmetic does not bind it there: all FP32, and FP64 vectors up
+//   to kRingRows64 rows;
+// * else by the grid-wide sweeps, whatever the size: FP64 vectors on one SM are bound by its FP64 pipe;
+// * by the kernels on the component-major records only where the options fix the launch shape (the one-kernel CPR
+//   application, a BILU0 stage of a given thread count) or the tuner, asked for the split form, found them faster.
+// Measured: both sweeps alone, FP64, ring / grid-wide: 1,600 rows 127 / 157 us, 3,300 rows 320 / 205 us, 9,800 rows
+// 724 (component-major) / 387 us; a CPR application, FP64, component-major / grid-wide: 11,200 rows 1.89 / 1.47 ms, 64 systems
+// of 8,000-14,400 rows 4.45 / 3.87 ms; FP32 factors with FP64 vectors: 1.13 / 0.51 and 1.72 / 1.00 ms; all FP32, 25,000 rows
+// (no ring): 0.56 / 0.45 ms.
+constexpr int kRingRows64 = 2000;
+enum { STAGE_CTA = 0, STAGE_RING = 1, STAGE_GRID = 2 };
+int ilu_stage(const rsg_solver* h, int kind) {
+    if (!h->cta || kind == 2) return STAGE_GRID;
+    if (h->opt.cpr2_threads != 0 || !h->tune.stage) return STAGE_CTA;
+    if (h->opt.precond == RSG_PREC_CPR && h->opt.sweep == 1) return STAGE_CTA;
+    const bool fits = ring_fits(h->ring[kind == 3 ? 1 : 0], kind != 0, kind == 3);
+    if (fits && (kind == 3 || h->plan.maxSysRows <= kRingRows64 || h->opt.sweep == 1)) return STAGE_RING;
+    return h->opt.sweep == 1 ? STAGE_CTA : STAGE_GRID;
 }
 int prec_kind(const rsg_solver* h) {
     if (h->opt.precond == RSG_PREC_JACOBI) return 2;
@@ -342,7 +355,10 @@ PrecDev prec_dev(rsg_solver* h) {
         M.s32 = h->s32;
         M.r64 = h->r64;
         M.r32 = h->r32;
-        if (ring_on(h, M.kind)) M.ring = h->ring;
+        const int stage = ilu_stage(h, M.kind);
+        if (stage == STAGE_RING) M.ring = h->ring;
+        M.gridIlu = stage == STAGE_GRID;
+        M.S = &h->S;
         M.split = M.cpr && (h->tune.split >= 0 ? h->tune.split != 0 : h->splitCpr);
         M.vform = h->tune.vform;
         M.cpr2Threads = h->tune.cpr2Threads;
@@ -587,17 +603,24 @@ int alloc_ring(rsg_solver* h, RingFactors<T>& F) {
 }
 // the thread-block sweeps' records of the current factors, in the layout of the sweeps that will read them
 int pack_factors(rsg_solver* h) {
-    const int kind = prec_kind(h);
+    const int kind = prec_kind(h), stage = ilu_stage(h, kind);
     int rc;
+    if (stage == STAGE_GRID) {                     // the CSR factors themselves; the sweeps' word vectors, all words empty
+        if (h->S.yw) return RSG_OK;
+        const size_t words = 2 * size_t(h->plan.n) * NB;
+        if ((rc = dalloc(h->pmem, &h->S.yw, words))) return rc;
+        RSG_CUDA(cudaMemsetAsync(h->S.yw, 0xff, words * sizeof(unsigned long long), h->stream));
+        return RSG_OK;
+    }
     if (kind == 0) {
-        if (ring_on(h, kind)) {
+        if (stage == STAGE_RING) {
             if (!h->r64.L && (rc = alloc_ring(h, h->r64))) return rc;
             launch_ring_pack(h->dp, h->lu, h->r64, h->stream);
         } else {
             if (!h->s64.L && (rc = alloc_split(h, h->s64))) return rc;
             launch_pack_f64(h->dp, h->lu, h->s64, h->stream);
         }
-    } else if (ring_on(h, kind)) {
+    } else if (stage == STAGE_RING) {
         if (!h->r32.L && (rc = alloc_ring(h, h->r32))) return rc;
         launch_ring_pack(h->dp, h->luf, h->r32, h->stream);
     } else {
@@ -620,11 +643,6 @@ int ensure_precond_storage(rsg_solver* h) {
         if (h->opt.precision == RSG_MIXED_F32 && !h->V.y32 && (rc = dalloc(h->pmem, &h->V.y32, size_t(h->plan.n) * NB))) return rc;
     } else {
         if (!h->lu && (rc = dalloc(h->pmem, &h->lu, E))) return rc;
-    }
-    if (h->opt.precond != RSG_PREC_JACOBI && !h->cta && !h->S.yw) {    // grid-wide sweeps: all words empty
-        const size_t words = 2 * size_t(h->plan.n) * NB;
-        if ((rc = dalloc(h->pmem, &h->S.yw, words))) return rc;
-        RSG_CUDA(cudaMemsetAsync(h->S.yw, 0xff, words * sizeof(unsigned long long), h->stream));
     }
     return RSG_OK;
 }
@@ -1060,38 +1078,36 @@ bool fused_capturable(rsg_solver* h, const double* d_r, double* d_z) {
 int tune_shapes(rsg_solver* h) {
     rsg_solver::Tune t;
     const bool cprCta = h->opt.precond == RSG_PREC_CPR && h->cta && h->haveAmg;
-    // a single system under the automatic sweep choice: the one-kernel application (one launch, one SM) and the split
-    // form (the V-cycle's passes grid-wide) are both candidates; they give the same results bit for bit
-    // (with the BILU0 stage on the ring only the split form: 1,600-13,000 rows alone, it is faster at every size)
-    int packed = h->tune.ring;                       // the layout the set-up packed the factors in
+    // the automatic choice is the split form, for single systems too (the one-kernel application, one SM, was slower at every
+    // size with the BILU0 stage on the ring or grid-wide); every shape gives the same results bit for bit
+    int packed = h->tune.stage;                      // the layout the set-up packed the factors in
     h->tune = t;
-    const bool ring = cprCta && ring_on(h, prec_kind(h));
-    const bool free_split = cprCta && h->opt.sweep == 0 && h->plan.nsys == 1 && !ring;
-    const bool split = cprCta && (h->splitCpr || free_split || ring);
-    t.split = h->splitCpr || ring ? 1 : 0;
+    const int stage = cprCta ? ilu_stage(h, prec_kind(h)) : STAGE_CTA;
+    const bool own = stage != STAGE_CTA;
+    const bool split = cprCta && (h->splitCpr || own || h->opt.sweep == 0);
+    t.split = split ? 1 : 0;
     t.vform = h->opt.vcycle_form ? h->opt.vcycle_form : 3;
     if (t.vform == 1 && h->amg.nPhases == 0) t.vform = 2;                  // no phase table for this hierarchy
     t.cpr2Threads = h->opt.cpr2_threads ? h->opt.cpr2_threads : 256;
     const bool free_form = h->opt.vcycle_form == 0, free_thr = h->opt.cpr2_threads == 0;
-    auto describe = [ring](const rsg_solver::Tune& c) {
-        if (c.split == 0) return std::string("cpr_form=one-kernel");
+    const std::string ownName = stage == STAGE_RING ? "ring" : "grid";
+    auto describe = [&](const rsg_solver::Tune& c) {
         return std::string("vcycle_form=") + std::to_string(c.vform) +
-               (ring && c.ring ? std::string(" bilu0=ring") : " cpr2_threads=" + std::to_string(c.cpr2Threads));
+               (own && c.stage ? " bilu0=" + ownName : " cpr2_threads=" + std::to_string(c.cpr2Threads));
     };
     // a shape is taken: the records its BILU0 stage reads are packed if they are not yet
     auto take = [&](const rsg_solver::Tune& c) {
-        const bool repack = ring && c.ring != packed;
-        packed = c.ring;
+        const bool repack = own && c.stage != packed;
+        packed = c.stage;
         h->tune = c;
         return repack ? pack_factors(h) : RSG_OK;
     };
     if (!split) { t.desc = "no split CPR: fixed shapes"; h->tune = t; return RSG_OK; }
-    if (!h->opt.autotune || (!free_form && !free_thr && !free_split)) {
+    if (!h->opt.autotune || (!free_form && !free_thr)) {
         t.desc = describe(t) + (h->opt.autotune ? " source=options" : " source=defaults");
         return take(t);
     }
-    const int key2 = (ring ? 2000000 : 0) + h->opt.sweep * 10000000 + h->opt.precision * 1000 + h->opt.vcycle_form * 10000 + h->opt.cpr2_threads + h->device * 100000 +
-                     (free_split ? 1000000 : 0);
+    const int key2 = h->opt.sweep * 10000000 + h->opt.precision * 1000 + h->opt.vcycle_form * 10000 + h->opt.cpr2_threads + h->device * 100000;
     const auto key = std::make_pair(pattern_hash(h), key2);
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -1101,11 +1117,6 @@ int tune_shapes(rsg_solver* h) {
     const size_t N = size_t(h->plan.n) * NB;
     RSG_CUDA(cudaMemsetAsync(h->tmp, 0, N * sizeof(double), h->stream));
     std::vector<rsg_solver::Tune> cand;
-    if (free_split) {
-        rsg_solver::Tune c;
-        c.split = 0;
-        cand.push_back(c);
-    }
     for (int f : {3, 2, 1})
         for (int thr : {256, 512, 128}) {
             if (!free_form && f != t.vform) continue;
@@ -1113,13 +1124,13 @@ int tune_shapes(rsg_solver* h) {
             if (f == 1 && h->amg.nPhases == 0) continue;
             rsg_solver::Tune c;
             c.split = 1;
-            c.ring = ring ? 1 : 0;
-            if (ring && thr == 256) {                                  // the ring's own shape follows from the level widths
+            c.stage = own ? 1 : 0;
+            if (own && thr == 256) {                                   // ilu_stage's own choice has no thread count
                 c.vform = f;
                 cand.push_back(c);
             }
-            if (ring && h->opt.sweep == 0) continue;                   // (faster than the others at every size measured)
-            c.ring = 0;
+            if (own && h->opt.sweep == 0) continue;
+            c.stage = 0;
             c.vform = f;
             c.cpr2Threads = thr;
             cand.push_back(c);
@@ -1143,8 +1154,7 @@ int tune_shapes(rsg_solver* h) {
         cudaEventElapsedTime(&ms, h->ev0, h->ev1);
         ms /= 3;
         char buf[96];
-        if (c.split == 0) std::snprintf(buf, sizeof(buf), "%sone-kernel %.3f ms", timings.empty() ? "" : ", ", ms);
-        else if (ring && c.ring) std::snprintf(buf, sizeof(buf), "%sform%d/ring %.3f ms", timings.empty() ? "" : ", ", c.vform, ms);
+        if (own && c.stage) std::snprintf(buf, sizeof(buf), "%sform%d/%s %.3f ms", timings.empty() ? "" : ", ", c.vform, ownName.c_str(), ms);
         else std::snprintf(buf, sizeof(buf), "%sform%d/%d %.3f ms", timings.empty() ? "" : ", ", c.vform, c.cpr2Threads, ms);
         timings += buf;
         if (ms < best) { best = ms; pick = c; }
@@ -1187,10 +1197,10 @@ int do_setup(rsg_solver* h, const double* acc) {
         if (h->opt.precision == RSG_MIXED || h->opt.precision == RSG_MIXED_F32) {
             if (h->cta && h->opt.precision == RSG_MIXED_F32) launch_factor_f32(h->dp, h->val, h->luf, h->S, h->epoch, h->d_nreg, h->d_err, h->stream);
             else launch_factor_lean(h->dp, h->val, h->luf, h->work, h->S, h->epoch, h->d_nreg, h->d_err, h->stream);
-            if (h->cta && (rc = pack_factors(h))) return rc;
+            if ((rc = pack_factors(h))) return rc;
         } else {
             launch_factor_f64(h->dp, h->val, h->lu, h->S, h->epoch, h->d_nreg, h->d_err, h->stream);
-            if (h->cta && (rc = pack_factors(h))) return rc;
+            if ((rc = pack_factors(h))) return rc;
         }
     }
     RSG_CUDA(cudaGetLastError());
@@ -1210,7 +1220,7 @@ int do_setup(rsg_solver* h, const double* acc) {
 int graph_kind(const PrecDev& M) {
     // distinct fields: kind 0-3, the three form flags, V-cycle form 0-3, BILU0-stage thread count (256 / 512 / 128)
     return (M.kind & 3) | (M.cpr ? 4 : 0) | (M.cta ? 8 : 0) | (M.split ? 16 : 0) | ((M.vform & 3) << 5) |
-           ((M.cpr2Threads >= 512 ? 1 : M.cpr2Threads <= 128 ? 2 : 0) << 7) | (M.ring ? 512 : 0);
+           ((M.cpr2Threads >= 512 ? 1 : M.cpr2Threads <= 128 ? 2 : 0) << 7) | (M.ring ? 512 : 0) | (M.gridIlu ? 1024 : 0);
 }
 
 int launch_iterations(rsg_solver* h, int k) {

@@ -277,7 +277,7 @@ inline int cpr_grid_launches(const DevAmg& G, bool split = false, int vform = 2)
         return nc > 0 ? G.colTail[size_t(l)] + (G.colTail[size_t(l)] < nc ? 1 : 0) : 1;
     };
     if (split && vform == 3) return G.maxL > 1 ? 7 + 2 * sweeps(0) : 4;
-    int n = (split ? 4 : 6) + 3 * (G.maxL > 1 ? G.maxL - 1 : 0) + 40 * int(G.coarseGsLevels.size());
+    int n = (split ? 4 : 5) + 3 * (G.maxL > 1 ? G.maxL - 1 : 0) + 40 * int(G.coarseGsLevels.size());
     for (int l = 0; l + 1 < G.maxL; ++l) n += 2 * sweeps(l);      // pre- and post-smoothing
     return n;
 }
@@ -409,6 +409,8 @@ void launch_factor_f32(const DevPlan& P, const double* val, float* luf, SweepSta
 // whose status is not running skip
 void launch_ilu_grid(const DevPlan& P, const PrecDev& M, int mode, const double* r, double* pv, const double* v, double* z, const KScal* ks,
                      SweepState& S, int* err, cudaStream_t st);
+void launch_ilu_grid_cpr(const DevPlan& P, const PrecDev& M, const double* t, const float* tf, const DevAmg& G, double* z, const KScal* ks,
+                         SweepState& S, int* err, cudaStream_t st);
 void launch_spmv_f64(const DevPlan& P, const double* val, const double* x, double* y, cudaStream_t st);
 // x += d over n block rows (3 values each)
 void launch_vec_add(int n, double* x, const double* d, cudaStream_t st);
@@ -451,6 +453,8 @@ struct PrecDev {
                                       // fit this plan or this kind)
     RingFactors<double> r64;
     RingFactors<float> r32;
+    bool gridIlu = false;             // BILU0 stage by the grid-wide sweeps (on the CSR factors) beside a V-cycle of the split form
+    SweepState* S = nullptr;          // their state
     int* err = nullptr;               // device error bits
 };
 // ---- ring sweeps (rsg_ring.cu)

@@ -296,10 +296,10 @@ __device__ __forceinline__ void sub_polled(TV& yi, const int* __restrict__ col, 
     }
 }
 
-template <class TF, class TV, int MODE>
+template <class TF, class TV, class TI, int MODE>
 __global__ void __launch_bounds__(kSweepThreads) k_fwd(int n, const int* __restrict__ rowPtr, const int* __restrict__ col,
                                                        const int* __restrict__ diag, const int* __restrict__ ford, const TF* __restrict__ lu,
-                                                       const double* r, double* pv, const double* v, typename Word<TV>::type* yf,
+                                                       const TI* r, double* pv, const double* v, typename Word<TV>::type* yf,
                                                        typename Word<TV>::type* yb, const int* __restrict__ rowSys, const KScal* ks,
                                                        unsigned* ctr, int* err) {
     if (blockIdx.x == 0 && threadIdx.x == 0) ctr[1] = 0u;   // backward claim counter for the next sweep
@@ -313,31 +313,28 @@ __global__ void __launch_bounds__(kSweepThreads) k_fwd(int n, const int* __restr
         const int i = __ldg(ford + idx);
         if (!sys_running(ks, rowSys, i)) continue;
         const size_t q = size_t(i) * 3 + e;
-        double in;
-        if (MODE == IN_PUPDATE) {
-            const KScal& K = ks[__ldg(rowSys + i)];
-            in = da(r[q], dm(K.beta, ds(pv[q], dm(K.omega, v[q]))));
-            pv[q] = in;
-        } else if (MODE == IN_SUPDATE) {
-            const KScal& K = ks[__ldg(rowSys + i)];
-            in = ds(r[q], dm(K.alpha, v[q]));
-            pv[q] = in;
+        TV yi;
+        if constexpr (MODE == IN_PLAIN) {
+            yi = TV(r[q]);
         } else {
-            in = r[q];
+            const KScal& K = ks[__ldg(rowSys + i)];
+            const double in = MODE == IN_PUPDATE ? da(r[q], dm(K.beta, ds(pv[q], dm(K.omega, v[q])))) : ds(r[q], dm(K.alpha, v[q]));
+            pv[q] = in;
+            yi = TV(in);
         }
-        TV yi = TV(in);
         sub_polled<TF, TV>(yi, col, lu, __ldg(rowPtr + i), __ldg(diag + i), e, yf, err);
         st_word(yf + q, Word<TV>::make(yi));
         yb[q] = Word<TV>::empty;
     }
 }
 
-// z_i = U_ii^-1 (y_i - sum_{j>i} U_ij z_j)   (engine/src/bsr.cpp:577-587)
-template <class TF, class TV>
+// z_i = U_ii^-1 (y_i - sum_{j>i} U_ij z_j)   (engine/src/bsr.cpp:577-587); xp (CPR): z_p += xp as z is written (bsr.cpp:1083)
+template <class TF, class TV, class TX>
 __global__ void __launch_bounds__(kSweepThreads) k_bwd(int n, const int* __restrict__ rowPtr, const int* __restrict__ col,
                                                        const int* __restrict__ diag, const int* __restrict__ bord, const TF* __restrict__ lu,
                                                        typename Word<TV>::type* yf, typename Word<TV>::type* yb, double* z,
-                                                       const int* __restrict__ rowSys, const KScal* ks, unsigned* ctr, int* err) {
+                                                       const TX* __restrict__ xp, const int* __restrict__ rowSys, const KScal* ks,
+                                                       unsigned* ctr, int* err) {
     if (blockIdx.x == 0 && threadIdx.x == 0) ctr[0] = 0u;
     const int lane = threadIdx.x & 31, rr = lane / 3, e = lane % 3;
     const unsigned mine = 7u << (3 * rr);                    // the row's lanes (a warp's rows may depend on each other)
@@ -354,6 +351,7 @@ __global__ void __launch_bounds__(kSweepThreads) k_bwd(int n, const int* __restr
         TF D[3];
 #pragma unroll
         for (int f = 0; f < 3; ++f) D[f] = __ldg(lu + size_t(d) * 9 + 3 * e + f);
+        const double corr = xp && e == 0 ? double(__ldg(xp + i)) : 0.0;
         TV yi = Word<TV>::value(yf[q]);
         yf[q] = Word<TV>::empty;
         sub_polled<TF, TV>(yi, col, lu, d + 1, __ldg(rowPtr + i + 1), e, yb, err);
@@ -362,7 +360,7 @@ __global__ void __launch_bounds__(kSweepThreads) k_bwd(int n, const int* __restr
         for (int f = 0; f < 3; ++f) w[f] = __shfl_sync(mine, yi, 3 * rr + f);
         const TV t = rdot(D, w);
         st_word(yb + q, Word<TV>::make(t));
-        z[q] = double(t);
+        z[q] = xp && e == 0 ? da(double(t), corr) : double(t);
     }
 }
 
@@ -706,27 +704,38 @@ void launch_factor_f32(const DevPlan& P, const double* val, float* luf, SweepSta
 }
 
 // both sweeps, the input by mode
-template <class TF, class TV>
-static void launch_sweeps(const DevPlan& P, const TF* lu, int mode, const double* r, double* pv, const double* v, double* z, const KScal* ks,
-                          SweepState& S, int* err, cudaStream_t st) {
+template <class TF, class TV, class TI, class TX>
+static void launch_sweeps(const DevPlan& P, const TF* lu, int mode, const TI* r, double* pv, const double* v, double* z, const TX* xp,
+                          const KScal* ks, SweepState& S, int* err, cudaStream_t st) {
     using U = typename Word<TV>::type;
     const int g = std::min(sweep_blocks(P), std::max(1, (P.n + 4 * kSweepRows - 1) / (4 * kSweepRows)));
     U* yf = reinterpret_cast<U*>(S.yw);
     U* yb = reinterpret_cast<U*>(S.yw + size_t(P.n) * 3);
     auto fwd = [&](auto tag) {
-        k_fwd<TF, TV, decltype(tag)::value><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, lu, r, pv, v, yf, yb, P.rowSys, ks,
-                                                                         S.ctr, err);
+        k_fwd<TF, TV, TI, decltype(tag)::value><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, lu, r, pv, v, yf, yb, P.rowSys,
+                                                                             ks, S.ctr, err);
     };
-    if (mode == IN_PUPDATE) fwd(std::integral_constant<int, IN_PUPDATE>());
-    else if (mode == IN_SUPDATE) fwd(std::integral_constant<int, IN_SUPDATE>());
-    else fwd(std::integral_constant<int, IN_PLAIN>());
-    k_bwd<TF, TV><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.bord, lu, yf, yb, z, P.rowSys, ks, S.ctr, err);
+    if (mode == IN_PLAIN) fwd(std::integral_constant<int, IN_PLAIN>());
+    else if constexpr (sizeof(TI) == 8) {
+        if (mode == IN_PUPDATE) fwd(std::integral_constant<int, IN_PUPDATE>());
+        else fwd(std::integral_constant<int, IN_SUPDATE>());
+    }
+    k_bwd<TF, TV, TX><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.bord, lu, yf, yb, z, xp, P.rowSys, ks, S.ctr, err);
 }
 void launch_ilu_grid(const DevPlan& P, const PrecDev& M, int mode, const double* r, double* pv, const double* v, double* z, const KScal* ks,
                      SweepState& S, int* err, cudaStream_t st) {
-    if (M.kind == 0) launch_sweeps<double, double>(P, M.lu, mode, r, pv, v, z, ks, S, err, st);
-    else if (M.kind == 1) launch_sweeps<float, double>(P, M.luf, mode, r, pv, v, z, ks, S, err, st);
-    else launch_sweeps<float, float>(P, M.luf, mode, r, pv, v, z, ks, S, err, st);
+    const double* no = nullptr;
+    if (M.kind == 0) launch_sweeps<double, double>(P, M.lu, mode, r, pv, v, z, no, ks, S, err, st);
+    else if (M.kind == 1) launch_sweeps<float, double>(P, M.luf, mode, r, pv, v, z, no, ks, S, err, st);
+    else launch_sweeps<float, float>(P, M.luf, mode, r, pv, v, z, no, ks, S, err, st);
+}
+// second stage of a CPR application: t in FP64, or (split form of the all-FP32 preconditioner) in FP32; z_p += xp
+void launch_ilu_grid_cpr(const DevPlan& P, const PrecDev& M, const double* t, const float* tf, const DevAmg& G, double* z, const KScal* ks,
+                         SweepState& S, int* err, cudaStream_t st) {
+    if (M.kind == 0) launch_sweeps<double, double>(P, M.lu, IN_PLAIN, t, nullptr, nullptr, z, G.x, ks, S, err, st);
+    else if (M.kind == 1) launch_sweeps<float, double>(P, M.luf, IN_PLAIN, t, nullptr, nullptr, z, G.xf, ks, S, err, st);
+    else if (tf) launch_sweeps<float, float>(P, M.luf, IN_PLAIN, tf, nullptr, nullptr, z, G.xf, ks, S, err, st);
+    else launch_sweeps<float, float>(P, M.luf, IN_PLAIN, t, nullptr, nullptr, z, G.xf, ks, S, err, st);
 }
 
 template <int MODE, bool FMA>

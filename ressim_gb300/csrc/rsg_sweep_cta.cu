@@ -1239,6 +1239,7 @@ template <int MODE>
 void dispatch(const DevPlan& P, const PrecDev& M, const double* r, double* pv, const double* v, double* z, const KScal* ks,
               cudaStream_t st) {
     if (M.ring) launch_ring_ilu(P, M, MODE, r, pv, v, z, ks, M.err, st);
+    else if (M.gridIlu) launch_ilu_grid(P, M, MODE, r, pv, v, z, ks, *M.S, M.err, st);
     else if (M.kind == 0) launch_cta<double, double, MODE>(P, M.s64, M.smem, r, pv, v, z, z, ks, st);
     else if (M.kind == 1) launch_cta<float, double, MODE>(P, M.s32, M.smem, r, pv, v, z, z, ks, st);
     else launch_cta<float, float, MODE>(P, M.s32, M.smem, r, pv, v, z, M.y32, ks, st);
@@ -1803,15 +1804,6 @@ __global__ void __launch_bounds__(256) k_gcpr_t(int n, const int* __restrict__ r
     }
 }
 
-// z_p += xp (bsr.cpp:1083)
-template <class TA>
-__global__ void __launch_bounds__(256) k_gcpr_zp(int n, const int* __restrict__ rowSys, const TA* xp, double* z, const KScal* ks) {
-    for (int k = int(blockIdx.x * blockDim.x + threadIdx.x); k < n; k += int(gridDim.x * blockDim.x)) {
-        if (ks && ks[__ldg(rowSys + k)].status != ST_RUNNING) continue;
-        z[size_t(k) * 3] = da(z[size_t(k) * 3], double(xp[k]));
-    }
-}
-
 // split form, second-stage input: t = T - S[:,p] xp in the thread-block kernel's slot order and arithmetic
 // (bsr.cpp:1071-1081), one row per thread over every system; xp = the level-0 V-cycle solution of the row's system
 template <class TA, class TV>
@@ -2028,6 +2020,11 @@ void launch_cpr2(const DevPlan& P, const PrecDev& M, const DevAmg& G, const CprA
         launch_ring_cpr2(P, M, G, Tsplit, z, ks, M.err, st);
         return;
     }
+    if (M.gridIlu) {
+        if constexpr (sizeof(TT) == 8) launch_ilu_grid_cpr(P, M, Tsplit, nullptr, G, z, ks, *M.S, M.err, st);
+        else launch_ilu_grid_cpr(P, M, nullptr, Tsplit, G, z, ks, *M.S, M.err, st);
+        return;
+    }
     const int nt = M.cpr2Threads;
     if constexpr (sizeof(TA) == 8) {
         if (nt >= 512) launch_cpr2_nt<double, double, TA, 512>(P, M, G, C, Tsplit, z, z, ks, st);
@@ -2087,7 +2084,7 @@ int cpr_grid(const DevPlan& P, const PrecDev& M, const DevAmg& G, const CprArgs<
         else launch_vcycle<TA, TT, false>(G, A, mode, ks, err, st);
         launches += 1;
         launch_cpr2<TA, TT>(P, M, G, C, Tsplit, z, ks, st);
-        return launches + 1;
+        return launches + (M.gridIlu ? 2 : 1);
     }
     if (M.split) {
         if (mode == IN_PUPDATE) k_gcpr_in<IN_PUPDATE, TA, TT, TT><<<gn, 256, 0, st>>>(n, P.rowSys, r, pv, v, G.w, Tsplit, C.b, ks);
@@ -2195,12 +2192,11 @@ int cpr_grid(const DevPlan& P, const PrecDev& M, const DevAmg& G, const CprArgs<
         k_gcpr_tsp<TA, TT><<<gn, 256, 0, st>>>(n, P.rowSys, P.sysRow0, G.maxL, G.lv, P.Lslot, P.Uslot, P.LovCol, P.UovCol, C.sp, C.spLov,
                                               C.spUov, C.x, Tsplit, ks);
         launch_cpr2<TA, TT>(P, M, G, C, Tsplit, z, ks, st);
-        return launches + 2;
+        return launches + (M.gridIlu ? 3 : 2);
     }
     k_gcpr_t<TA, TT><<<gn, 256, 0, st>>>(n, P.rowSys, P.rowPtr, P.col, M.val, C.x, G.T, ks);
-    launch_ilu_grid(P, M, IN_PLAIN, G.T, nullptr, nullptr, z, ks, S, err, st);
-    k_gcpr_zp<TA><<<gn, 256, 0, st>>>(n, P.rowSys, C.x, z, ks);
-    return launches + 4;
+    launch_ilu_grid_cpr(P, M, G.T, nullptr, G, z, ks, S, err, st);
+    return launches + 3;
 }
 
 }  // namespace
