@@ -3,6 +3,7 @@
 // reference's summation order, and the dense LU of the coarsest level. All FP64 arithmetic explicitly rounded.
 #include "rsg_impl.h"
 #include "rsg_block3.cuh"
+#include "rsg_dense.cuh"
 
 #include <cuda_runtime.h>
 
@@ -97,172 +98,109 @@ __global__ void k_diag_fix(int beg, int end, const int* __restrict__ diagGlob, d
     }
 }
 
-// dense LU with partial pivoting of every system's coarsest level in its natural numbering
-// (engine/src/amg.cpp:273-295); one thread block per system. T = double (reference arithmetic) or float (the FP32
-// hierarchy of the precision forms: same algorithm, float operations).
-__device__ __forceinline__ double cmul(double a, double b) { return dm(a, b); }
-__device__ __forceinline__ double csub(double a, double b) { return ds(a, b); }
-__device__ __forceinline__ double cdiv(double a, double b) { return __ddiv_rn(a, b); }
-__device__ __forceinline__ float cmul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float csub(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ float cdiv(float a, float b) { return __fdiv_rn(a, b); }
-template <class T> __device__ __forceinline__ T tiny_pivot();
-template <> __device__ __forceinline__ double tiny_pivot<double>() { return 1e-300; }
-template <> __device__ __forceinline__ float tiny_pivot<float>() { return 1.17549435e-38f; }   // smallest normal float
-
-template <class T>
-__global__ void __launch_bounds__(256) k_coarse_lu(int nsys, int maxL, const AmgSysLv* __restrict__ lv, const int* __restrict__ rp,
-                                                   const int* __restrict__ ci, const double* __restrict__ val,
-                                                   const int* __restrict__ luPerm, T* luAll, int* pivAll, int* cinAll,
-                                                   int skipUpTo, const int* only) {
-    const int s = blockIdx.x;
-    if (only && !only[s]) return;                                 // only the systems flagged (FP64 coarse solve)
-    AmgSysLv L;
-    bool found = false;
+// the dense coarsest level of a system; false: none
+__device__ __forceinline__ bool coarse_level(const AmgSysLv* __restrict__ lv, int maxL, int s, AmgSysLv& L) {
     for (int l = 0; l < maxL; ++l) {
         const AmgSysLv c = lv[s * maxL + l];
-        if (c.n > 0 && c.coarse) { L = c; found = true; break; }
+        if (c.n > 0 && c.coarse) { L = c; return c.dense != 0; }
     }
-    if (!found || !L.dense || L.n <= skipUpTo) return;        // skipUpTo: levels inverted in shared memory
+    return false;
+}
+
+// dense LU with partial pivoting of every system's coarsest level in its natural numbering
+// (engine/src/amg.cpp:273-295; rsg_dense.cuh), one thread block per system. T = double (reference arithmetic) or float (the
+// FP32 hierarchy of the precision forms: same algorithm, float operations).
+template <class T>
+__global__ void __launch_bounds__(kDenseThreads) k_coarse_lu(int maxL, const AmgSysLv* __restrict__ lv, const int* __restrict__ rp,
+                                                             const int* __restrict__ ci, const double* __restrict__ val,
+                                                             const int* __restrict__ luPerm, T* luAll, int* pivAll, int* cinAll,
+                                                             int skipUpTo, const int* only, unsigned smemBytes) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int s = blockIdx.x, tid = int(threadIdx.x), nt = int(blockDim.x);
+    if (only && !only[s]) return;                                 // only the systems flagged (FP64 coarse solve)
+    AmgSysLv L;
+    if (!coarse_level(lv, maxL, s, L) || L.n <= skipUpTo) return;   // skipUpTo: levels inverted in shared memory
     const int m = L.n;
     T* lu = luAll + L.luOff;
+    T* a = dense_lu_place<T>(m, smemBytes, smraw, lu);
     int* piv = pivAll + L.luRowOff;
     const int* nat = luPerm + L.luRowOff;
-    for (size_t q = threadIdx.x; q < size_t(m) * m; q += blockDim.x) lu[q] = T(0);
+    for (int q = tid; q < m * m; q += nt) a[q] = T(0);
     __syncthreads();
-    for (int k = threadIdx.x; k < m; k += blockDim.x) {
+    for (int k = tid; k < m; k += nt) {
         const int I = __ldg(nat + k);
         for (int p = __ldg(rp + L.rpOff + k); p < __ldg(rp + L.rpOff + k + 1); ++p)
-            lu[size_t(I) * m + __ldg(nat + __ldg(ci + L.entOff + p))] = T(val[L.entOff + p]);
+            a[size_t(I) * m + __ldg(nat + __ldg(ci + L.entOff + p))] = T(val[L.entOff + p]);
     }
     __syncthreads();
-    __shared__ T smax[256];
-    __shared__ int sidx[256];
-    for (int k = 0; k < m; ++k) {
-        // pivot: first row with the largest |a_ik|, i >= k
-        T best = T(-1);
-        int bi = m;
-        for (int i = k + int(threadIdx.x); i < m; i += blockDim.x) {
-            const T a = fabs(lu[size_t(i) * m + k]);
-            if (a > best || (a == best && i < bi)) { best = a; bi = i; }
-        }
-        smax[threadIdx.x] = best;
-        sidx[threadIdx.x] = bi;
-        __syncthreads();
-        for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-            if (int(threadIdx.x) < o) {
-                const T b2 = smax[threadIdx.x + o];
-                const int i2 = sidx[threadIdx.x + o];
-                if (b2 > smax[threadIdx.x] || (b2 == smax[threadIdx.x] && i2 < sidx[threadIdx.x])) { smax[threadIdx.x] = b2; sidx[threadIdx.x] = i2; }
-            }
-            __syncthreads();
-        }
-        // reference: pr starts at k and moves only on a strictly larger value -> first maximum
-        const int pr = (smax[0] > fabs(lu[size_t(k) * m + k])) ? sidx[0] : k;
-        __syncthreads();
-        if (threadIdx.x == 0) piv[k] = pr;
-        if (pr != k)
-            for (int j = threadIdx.x; j < m; j += blockDim.x) {
-                const T t = lu[size_t(k) * m + j];
-                lu[size_t(k) * m + j] = lu[size_t(pr) * m + j];
-                lu[size_t(pr) * m + j] = t;
-            }
-        __syncthreads();
-        if (threadIdx.x == 0 && fabs(lu[size_t(k) * m + k]) < tiny_pivot<T>()) lu[size_t(k) * m + k] = tiny_pivot<T>();
-        __syncthreads();
-        const T dk = lu[size_t(k) * m + k];
-        for (int i = k + 1 + int(threadIdx.x); i < m; i += blockDim.x) lu[size_t(i) * m + k] = cdiv(lu[size_t(i) * m + k], dk);
-        __syncthreads();
-        const int w = m - k - 1;
-        for (size_t q = threadIdx.x; q < size_t(w) * w; q += blockDim.x) {
-            const int i = k + 1 + int(q / w), j = k + 1 + int(q % w);
-            const T f = lu[size_t(i) * m + k];
-            if (f != T(0)) lu[size_t(i) * m + j] = csub(lu[size_t(i) * m + j], cmul(f, lu[size_t(k) * m + j]));
-        }
-        __syncthreads();
-    }
+    dense_lu(m, a, piv);
+    if (a != lu)
+        for (int q = tid; q < m * m; q += nt) lu[q] = a[q];
     // gather order of the solve: the level-space row whose value lands at position i once the natural-order
     // vector has gone through the row interchanges piv[0], piv[1], ... (engine/src/amg.cpp:306-308)
-    int* cin = cinAll + L.luRowOff;
-    for (int k = threadIdx.x; k < m; k += blockDim.x) cin[__ldg(nat + k)] = k;
+    __shared__ int cin[kDenseMax];
+    for (int k = tid; k < m; k += nt) cin[__ldg(nat + k)] = k;
     __syncthreads();
-    if (threadIdx.x == 0)
+    if (tid == 0)
         for (int k = 0; k < m; ++k) {
             const int pk = piv[k];
             if (pk != k) { const int t = cin[k]; cin[k] = cin[pk]; cin[pk] = t; }
         }
+    __syncthreads();
+    for (int k = tid; k < m; k += nt) cinAll[L.luRowOff + k] = cin[k];
 }
 
-// Explicit inverse of every coarsest level for the FP32 precision forms (the reference's device-shaped CPR keeps an
-// explicit coarse inverse, engine/src/bsr.cpp:1235-1317): column j = LU^-1 e_j of the level-space unit vector,
+// Explicit inverse of the coarsest levels beyond kInvSmemRows rows for the FP32 precision forms (the reference's device-shaped
+// CPR keeps an explicit coarse inverse, engine/src/bsr.cpp:1235-1317): column j = LU^-1 e_j of the level-space unit vector,
 // stored in natural row order: inv[j * m + nat(k)] = (A^-1)_{k j} (k_coarse_perm then moves it to the V-cycle's
-// level-space layout). All m columns are eliminated together by the
-// block, column-oriented, in an m x m shared-memory work matrix (m <= kInvSmemRows), else one column per thread in
-// global memory.
+// level-space layout). A block takes kInvCols columns of a system, a lane per column. Forward the warps share the rows,
+// column by column (a row's terms come in the same ascending order as row by row); backward a row's terms are taken in
+// ascending order too, which starts with the value just found, so one warp runs the chain while the others stage the
+// factors' next row. 277 rows: one thread per column in global memory took 7.2 ms.
 constexpr int kInvSmemRows = 224;
+constexpr int kInvCols = 32;
 __global__ void __launch_bounds__(256) k_coarse_inv(int maxL, const AmgSysLv* __restrict__ lv, const int* __restrict__ cinAll,
-                                                    const float* __restrict__ luAll, float* invAll, int skipUpTo) {
-    extern __shared__ float W[];
-    const int s = blockIdx.x;
+                                                    const float* __restrict__ luAll, float* invAll, int skipUpTo, unsigned smemBytes) {
+    extern __shared__ float W[];                                  // m x kInvCols, then a column or row of the factors (two buffers)
+    const int s = blockIdx.y, tid = int(threadIdx.x), lane = tid & 31, wid = tid >> 5, nw = int(blockDim.x) >> 5;
     AmgSysLv L;
-    bool found = false;
-    for (int l = 0; l < maxL; ++l) {
-        const AmgSysLv c = lv[s * maxL + l];
-        if (c.n > 0 && c.coarse) { L = c; found = true; break; }
-    }
-    if (!found || !L.dense || L.n <= skipUpTo) return;
-    const int m = L.n;
+    if (!coarse_level(lv, maxL, s, L) || L.n <= skipUpTo) return;
+    const int m = L.n, j0 = int(blockIdx.x) * kInvCols;
+    if (j0 >= m || size_t(m) * (kInvCols + 2) * sizeof(float) > smemBytes) return;
     const float* lu = luAll + L.luOff;
     const int* cin = cinAll + L.luRowOff;
     float* inv = invAll + L.luOff;
-    if (m <= kInvSmemRows && m <= int(blockDim.x)) {
-        // thread j owns column j of the work matrix W[i * m + j] (consecutive threads, consecutive banks); column k
-        // of the factors is staged in shared memory for each elimination step and read by all threads
-        float* lc = W + m * m;
-        const int j = threadIdx.x;
-        if (j < m)
-            for (int i = 0; i < m; ++i) W[i * m + j] = __ldg(cin + i) == j ? 1.f : 0.f;   // pivoted e_j
-        for (int k = 0; k + 1 < m; ++k) {                                         // unit lower
-            __syncthreads();
-            for (int i = threadIdx.x; i < m; i += blockDim.x) lc[i] = __ldg(lu + size_t(i) * m + k);
-            __syncthreads();
-            if (j < m) {
-                const float wk = W[k * m + j];
-                if (wk != 0.f)
-                    for (int i = k + 1; i < m; ++i) W[i * m + j] = __fsub_rn(W[i * m + j], __fmul_rn(lc[i], wk));
-            }
-        }
-        for (int k = m - 1; k >= 0; --k) {                                        // upper
-            __syncthreads();
-            for (int i = threadIdx.x; i < m; i += blockDim.x) lc[i] = __ldg(lu + size_t(i) * m + k);
-            __syncthreads();
-            if (j < m) {
-                const float wk = __fdiv_rn(W[k * m + j], lc[k]);
-                W[k * m + j] = wk;
-                if (wk != 0.f)
-                    for (int i = 0; i < k; ++i) W[i * m + j] = __fsub_rn(W[i * m + j], __fmul_rn(lc[i], wk));
-            }
+    float* lc = W + size_t(m) * kInvCols;
+    for (int q = tid; q < m * kInvCols; q += int(blockDim.x)) W[q] = __ldg(cin + q / kInvCols) == j0 + q % kInvCols ? 1.f : 0.f;   // pivoted e_j
+    for (int i = tid; i < m; i += int(blockDim.x)) lc[i] = __ldg(lu + size_t(i) * m);
+    __syncthreads();
+    for (int k = 0; k < m; ++k) {                                 // unit lower
+        const float* c = lc + (k & 1) * m;
+        float* cn = lc + ((k + 1) & 1) * m;
+        if (k + 1 < m)
+            for (int i = tid; i < m; i += int(blockDim.x)) cn[i] = __ldg(lu + size_t(i) * m + k + 1);
+        const float wk = W[k * kInvCols + lane];
+        for (int i = k + 1 + wid; i < m; i += nw) W[i * kInvCols + lane] = __fsub_rn(W[i * kInvCols + lane], __fmul_rn(c[i], wk));
+        __syncthreads();
+    }
+    for (int q = tid; q < m; q += int(blockDim.x)) lc[((m - 1) & 1) * m + q] = __ldg(lu + size_t(m - 1) * m + q);
+    __syncthreads();
+    for (int i = m - 1; i >= 0; --i) {                            // upper
+        const float* c = lc + (i & 1) * m;
+        if (wid > 0 && i > 0)
+            for (int q = tid - 32; q < m; q += int(blockDim.x) - 32) lc[((i - 1) & 1) * m + q] = __ldg(lu + size_t(i - 1) * m + q);
+        if (wid == 0) {
+            float t = W[i * kInvCols + lane];
+#pragma unroll 8
+            for (int k = i + 1; k < m; ++k) t = __fsub_rn(t, __fmul_rn(c[k], W[k * kInvCols + lane]));
+            t = __fdiv_rn(t, c[i]);
+            W[i * kInvCols + lane] = t;
         }
         __syncthreads();
-        for (int q = threadIdx.x; q < m * m; q += blockDim.x) {
-            const int jj = q / m, i = q - jj * m;
-            inv[q] = W[i * m + jj];
-        }
-        return;
     }
-    for (int j = threadIdx.x; j < m; j += blockDim.x) {
-        float* w = inv + size_t(j) * m;
-        for (int i = 0; i < m; ++i) w[i] = __ldg(cin + i) == j ? 1.f : 0.f;
-        for (int i = 1; i < m; ++i) {
-            float t = w[i];
-            for (int k = 0; k < i; ++k) t = __fsub_rn(t, __fmul_rn(__ldg(lu + size_t(i) * m + k), w[k]));
-            w[i] = t;
-        }
-        for (int i = m - 1; i >= 0; --i) {
-            float t = w[i];
-            for (int k = i + 1; k < m; ++k) t = __fsub_rn(t, __fmul_rn(__ldg(lu + size_t(i) * m + k), w[k]));
-            w[i] = __fdiv_rn(t, __ldg(lu + size_t(i) * m + i));
-        }
+    for (int q = tid; q < m * kInvCols; q += int(blockDim.x)) {
+        const int j = q / m, i = q - j * m;
+        if (j0 + j < m) inv[size_t(j0 + j) * m + i] = W[i * kInvCols + j];
     }
 }
 
@@ -284,12 +222,7 @@ __global__ void __launch_bounds__(kGjThreads, 1) k_coarse_gj(int maxL, const Amg
     extern __shared__ float W[];
     const int s = blockIdx.x, tid = int(threadIdx.x), nt = int(blockDim.x), lane = tid & 31, wg = tid >> 5;
     AmgSysLv L;
-    bool found = false;
-    for (int l = 0; l < maxL; ++l) {
-        const AmgSysLv c = lv[s * maxL + l];
-        if (c.n > 0 && c.coarse) { L = c; found = true; break; }
-    }
-    if (!found || !L.dense) return;
+    if (!coarse_level(lv, maxL, s, L)) return;
     const int m = L.n;
     if (m > kInvSmemRows || nt != kGjThreads) return;          // left to the LU path
     __shared__ float colk[2][kGjWarps * kGjRows];               // column k of the current step, then of the next
@@ -513,12 +446,7 @@ __global__ void __launch_bounds__(256) k_coarse_perm(int maxL, const AmgSysLv* _
     extern __shared__ float colbuf[];
     const int s = blockIdx.x;
     AmgSysLv L;
-    bool found = false;
-    for (int l = 0; l < maxL; ++l) {
-        const AmgSysLv c = lv[s * maxL + l];
-        if (c.n > 0 && c.coarse) { L = c; found = true; break; }
-    }
-    if (!found || !L.dense) return;
+    if (!coarse_level(lv, maxL, s, L)) return;
     const int m = L.n;
     const int* nat = luPerm + L.luRowOff;
     float* inv = invAll + L.luOff;
@@ -542,12 +470,7 @@ __global__ void __launch_bounds__(256) k_coarse_check(int maxL, const AmgSysLv* 
                                                       double* bt, int* coarse64) {
     const int s = blockIdx.x;
     AmgSysLv L;
-    bool found = false;
-    for (int l = 0; l < maxL; ++l) {
-        const AmgSysLv c = lv[s * maxL + l];
-        if (c.n > 0 && c.coarse) { L = c; found = true; break; }
-    }
-    if (!found || !L.dense) {
+    if (!coarse_level(lv, maxL, s, L)) {
         if (threadIdx.x == 0) coarse64[s] = 0;
         return;
     }
@@ -595,19 +518,23 @@ void launch_amg_coarse_lu(const DevAmg& G, bool fp32, cudaStream_t st) {
         raise_smem_limit(reinterpret_cast<const void*>(k_coarse_gj), smem);
         k_coarse_gj<<<G.nsys, kGjThreads, smem, st>>>(G.maxL, G.lv, G.rp, G.ci, G.val, G.luPerm, G.invf);
         if (G.maxCoarse > kInvSmemRows) {                        // levels too large for shared memory: LU, then columns
-            raise_smem_limit(reinterpret_cast<const void*>(k_coarse_inv), smem);
-            k_coarse_lu<float><<<G.nsys, 256, 0, st>>>(G.nsys, G.maxL, G.lv, G.rp, G.ci, G.val, G.luPerm, G.luf, G.piv, G.cin,
-                                                       kInvSmemRows, nullptr);
-            k_coarse_inv<<<G.nsys, 256, smem, st>>>(G.maxL, G.lv, G.cin, G.luf, G.invf, kInvSmemRows);
+            const unsigned sl = dense_lu_smem<float>(G.maxCoarse), si = unsigned(size_t(G.maxCoarse) * (kInvCols + 2) * sizeof(float));
+            raise_smem_limit(reinterpret_cast<const void*>(k_coarse_lu<float>), int(sl));
+            raise_smem_limit(reinterpret_cast<const void*>(k_coarse_inv), int(si));
+            k_coarse_lu<float><<<G.nsys, kDenseThreads, sl, st>>>(G.maxL, G.lv, G.rp, G.ci, G.val, G.luPerm, G.luf, G.piv, G.cin, kInvSmemRows,
+                                                                  nullptr, sl);
+            k_coarse_inv<<<dim3(unsigned((G.maxCoarse + kInvCols - 1) / kInvCols), unsigned(G.nsys)), 256, si, st>>>(
+                G.maxL, G.lv, G.cin, G.luf, G.invf, kInvSmemRows, si);
         }
         k_coarse_perm<<<G.nsys, 256, size_t(std::max(G.maxCoarse, 1)) * sizeof(float), st>>>(G.maxL, G.lv, G.luPerm, G.invf);
         // the FP32 inverse checked per system; the FP64 LU (after the FP32 one: pivots and gather order are its own)
         // only for the systems that need it
         k_coarse_check<<<G.nsys, 256, 0, st>>>(G.maxL, G.lv, G.rp, G.ci, G.val, G.luPerm, G.invf, G.x, G.b, G.coarse64);
-        k_coarse_lu<double><<<G.nsys, 256, 0, st>>>(G.nsys, G.maxL, G.lv, G.rp, G.ci, G.val, G.luPerm, G.lu, G.piv, G.cin, 0, G.coarse64);
-    } else {
-        k_coarse_lu<double><<<G.nsys, 256, 0, st>>>(G.nsys, G.maxL, G.lv, G.rp, G.ci, G.val, G.luPerm, G.lu, G.piv, G.cin, 0, nullptr);
     }
+    const unsigned sm = dense_lu_smem<double>(G.maxCoarse);
+    raise_smem_limit(reinterpret_cast<const void*>(k_coarse_lu<double>), int(sm));
+    k_coarse_lu<double><<<G.nsys, kDenseThreads, sm, st>>>(G.maxL, G.lv, G.rp, G.ci, G.val, G.luPerm, G.lu, G.piv, G.cin, 0,
+                                                           fp32 ? G.coarse64 : nullptr, sm);
 }
 void launch_amg_round(const DevAmg& G, cudaStream_t st) {
     k_round<<<grid_for(size_t(G.totEnt)), 256, 0, st>>>(size_t(G.totEnt), G.val, G.valf);

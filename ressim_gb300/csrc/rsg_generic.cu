@@ -15,6 +15,7 @@
 // recomputes every level's values on the device at each set-up from its Galerkin gather lists.
 #include "rsg_generic.h"
 #include "rsg_impl.h"
+#include "rsg_dense.cuh"
 
 #include <cuda_runtime.h>
 
@@ -149,48 +150,82 @@ struct GenWarpSmem {
     double keep[GEN_MAX_NB * GEN_MAX_NB];
 };
 
-__device__ int find_col(const int* __restrict__ ci, int lo, int hi, int j) {
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        const int c = ci[mid];
-        if (c == j) return mid;
-        if (c < j) lo = mid + 1;
-        else hi = mid;
-    }
-    return -1;
-}
+// A warp factors row i. Its own columns sit in the lanes (32 at a time), so the block of the row that an elimination changes is
+// found by a ballot instead of a search in memory, and the next U block is on its way while one is applied: a row is bound by
+// its blocks' arithmetic, not by chains of loads.
+constexpr int kGenPer = (GEN_MAX_NB * GEN_MAX_NB + 31) / 32;   // block elements per lane
 
 __device__ void factor_row(int i, int nb, const int* __restrict__ rp, const int* __restrict__ ci, const int* __restrict__ dg, double* LU,
                            GenWarpSmem& W, int* nreg) {
     const int lane = int(threadIdx.x & 31), b2 = nb * nb;
+    const unsigned all = 0xffffffffu;
     const int r0 = rp[i], r1 = rp[i + 1];
+    // the block of column j in this row, -1 if none (every lane the same)
+    int have0 = r0, mine = r0 + lane < r1 ? ci[r0 + lane] : -1;
+    auto find = [&](int j) {
+        for (int c0 = r0; c0 < r1; c0 += 32) {
+            if (c0 != have0) {
+                mine = c0 + lane < r1 ? ci[c0 + lane] : -1;
+                have0 = c0;
+            }
+            const unsigned m = __ballot_sync(all, mine == j);
+            if (m) return c0 + __ffs(int(m)) - 1;
+        }
+        return -1;
+    };
     for (int p = r0; p < r1; ++p) {
         const int k = ci[p];
         if (k >= i) break;
         // L_ik = A_ik U_kk^-1 (gemm: every element summed over m in order from zero)
-        const double* d = LU + size_t(dg[k]) * b2;
+        const int dk = dg[k], uEnd = rp[k + 1];
+        const double* d = LU + size_t(dk) * b2;
         double* aik = LU + size_t(p) * b2;
+        // the blocks U_kj that change this row, 32 candidates at a time: lane q holds entry c0 + q and its target
+        for (int t = lane; t < b2; t += 32) { W.m[t] = aik[t]; W.keep[t] = d[t]; }
+        __syncwarp();
         for (int t = lane; t < b2; t += 32) {
             const int r = t / nb, c = t % nb;
             double s = 0;
-            for (int q = 0; q < nb; ++q) s = ga(s, gm(aik[r * nb + q], d[q * nb + c]));
+            for (int q = 0; q < nb; ++q) s = ga(s, gm(W.m[r * nb + q], W.keep[q * nb + c]));
             W.tmp[t] = s;
+            aik[t] = s;
         }
         __syncwarp();
-        for (int t = lane; t < b2; t += 32) aik[t] = W.tmp[t];
-        __syncwarp();
-        for (int q = dg[k] + 1; q < rp[k + 1]; ++q) {
-            const int pj = find_col(ci, r0, r1, ci[q]);
-            if (pj < 0) continue;
-            const double* u = LU + size_t(q) * b2;
-            double* tgt = LU + size_t(pj) * b2;
-            for (int t = lane; t < b2; t += 32) {   // gemmSub: c -= sum_m tmp[r][m] u[m][c]
-                const int r = t / nb, c = t % nb;
-                double s = 0;
-                for (int m = 0; m < nb; ++m) s = ga(s, gm(W.tmp[r * nb + m], u[m * nb + c]));
-                tgt[t] = gs(tgt[t], s);
+        for (int c0 = dk + 1; c0 < uEnd; c0 += 32) {
+            const int cn = min(32, uEnd - c0);
+            const int uc = lane < cn ? ci[c0 + lane] : -1;
+            int tgt = -1;
+            for (int q = 0; q < cn; ++q) {
+                const int pj = find(__shfl_sync(all, uc, q));
+                if (lane == q) tgt = pj;
             }
-            __syncwarp();
+            unsigned todo = __ballot_sync(all, tgt >= 0);
+            double un[kGenPer];
+            auto fetch = [&](int q) {
+                const double* u = LU + size_t(c0 + q) * b2;
+#pragma unroll
+                for (int z = 0; z < kGenPer; ++z)
+                    if (lane + 32 * z < b2) un[z] = u[lane + 32 * z];
+            };
+            if (todo) fetch(__ffs(int(todo)) - 1);
+            while (todo) {
+                const int q = __ffs(int(todo)) - 1;
+                todo &= todo - 1;
+#pragma unroll
+                for (int z = 0; z < kGenPer; ++z)
+                    if (lane + 32 * z < b2) W.keep[lane + 32 * z] = un[z];
+                __syncwarp();
+                if (todo) fetch(__ffs(int(todo)) - 1);
+                double* to = LU + size_t(__shfl_sync(all, tgt, q)) * b2;
+                for (int t = lane; t < b2; t += 32) {   // gemmSub: c -= sum_m tmp[r][m] u[m][c]
+                    const int r = t / nb, c = t % nb;
+                    const double old = to[t];
+                    double s = 0;
+                    for (int m = 0; m < nb; ++m) s = ga(s, gm(W.tmp[r * nb + m], W.keep[m * nb + c]));
+                    to[t] = gs(old, s);
+                }
+                __syncwarp();
+            }
         }
     }
     warp_pivot(W.m, LU + size_t(dg[i]) * b2, W.keep, nb, nreg);
@@ -396,68 +431,23 @@ __global__ void k_gen_diag_fix(int n, const int* __restrict__ dg, double* v) {
         if (fabs(v[dg[i]]) < 1e-300) v[dg[i]] = 1.0;
 }
 // dense LU with partial pivoting of the coarsest level in its natural numbering (AMG::factorCoarsest,
-// engine/src/amg.cpp:273-295), one thread block; lu is m x m, perm: level-space row -> natural row
-__global__ void __launch_bounds__(1024) k_gen_coarse_lu(int m, const int* __restrict__ rp, const int* __restrict__ ci,
-                                                        const double* __restrict__ v, const int* __restrict__ perm, double* lu, int* piv) {
-    __shared__ double smx[32];
-    __shared__ int sid[32];
-    __shared__ int spr;
+// engine/src/amg.cpp:273-295), one thread block (rsg_dense.cuh); lu is m x m, perm: level-space row -> natural row
+__global__ void __launch_bounds__(kDenseThreads) k_gen_coarse_lu(int m, const int* __restrict__ rp, const int* __restrict__ ci,
+                                                                 const double* __restrict__ v, const int* __restrict__ perm, double* lu,
+                                                                 int* piv, unsigned smemBytes) {
+    extern __shared__ __align__(16) unsigned char smraw[];
     const int tid = int(threadIdx.x), nt = int(blockDim.x);
-    for (long long q = tid; q < (long long)m * m; q += nt) lu[q] = 0.0;
+    double* a = dense_lu_place<double>(m, smemBytes, smraw, lu);
+    for (int q = tid; q < m * m; q += nt) a[q] = 0.0;
     __syncthreads();
     for (int k = tid; k < m; k += nt) {
         const int I = perm[k];
-        for (int p = rp[k]; p < rp[k + 1]; ++p) lu[size_t(I) * m + perm[ci[p]]] = v[p];
+        for (int p = rp[k]; p < rp[k + 1]; ++p) a[I * m + perm[ci[p]]] = v[p];
     }
     __syncthreads();
-    for (int k = 0; k < m; ++k) {
-        // pivot: the first row i >= k of the largest |lu[i][k]| (strictly greater replaces)
-        double best = -1.0;
-        int bi = m;
-        for (int i = k + tid; i < m; i += nt) {
-            const double a = fabs(lu[size_t(i) * m + k]);
-            if (a > best || (a == best && i < bi)) { best = a; bi = i; }
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-        }
-        if ((tid & 31) == 0) { smx[tid >> 5] = best; sid[tid >> 5] = bi; }
-        __syncthreads();
-        if (tid == 0) {
-            double b = smx[0];
-            int id = sid[0];
-            for (int w = 1; w < (nt + 31) / 32; ++w)
-                if (smx[w] > b || (smx[w] == b && sid[w] < id)) { b = smx[w]; id = sid[w]; }
-            // the reference keeps k unless a later row is strictly larger: the smallest index among equal maxima
-            // is k itself whenever |lu[k][k]| is the maximum
-            spr = (id < m) ? id : k;
-            if (!(fabs(lu[size_t(spr) * m + k]) > fabs(lu[size_t(k) * m + k]))) spr = k;
-            piv[k] = spr;
-        }
-        __syncthreads();
-        const int pr = spr;
-        if (pr != k)
-            for (int j = tid; j < m; j += nt) {
-                const double t = lu[size_t(k) * m + j];
-                lu[size_t(k) * m + j] = lu[size_t(pr) * m + j];
-                lu[size_t(pr) * m + j] = t;
-            }
-        __syncthreads();
-        if (tid == 0 && fabs(lu[size_t(k) * m + k]) < 1e-300) lu[size_t(k) * m + k] = 1e-300;
-        __syncthreads();
-        const double dk = lu[size_t(k) * m + k];
-        for (int i = k + 1 + tid; i < m; i += nt) lu[size_t(i) * m + k] = gd(lu[size_t(i) * m + k], dk);
-        __syncthreads();
-        const int w = m - k - 1;
-        for (long long q = tid; q < (long long)w * w; q += nt) {
-            const int i = k + 1 + int(q / w), j = k + 1 + int(q % w);
-            const double f = lu[size_t(i) * m + k];
-            if (f != 0) lu[size_t(i) * m + j] = gs(lu[size_t(i) * m + j], gm(f, lu[size_t(k) * m + j]));
-        }
-        __syncthreads();
-    }
+    dense_lu(m, a, piv);
+    if (a != lu)
+        for (int q = tid; q < m * m; q += nt) lu[q] = a[q];
 }
 
 // ------------------------------------------------------------------ AMG V-cycle (AMG::cycle, engine/src/amg.cpp:303-337)
@@ -881,7 +871,9 @@ void refresh_amg(GenEngine& g) {
     }
     GenLevel& Lc = g.lv.back();
     if (Lc.dense) {
-        k_gen_coarse_lu<<<1, 1024, 0, g.st>>>(Lc.n, Lc.rp, Lc.ci, Lc.v, Lc.perm, Lc.lu, Lc.piv);
+        const unsigned sm = dense_lu_smem<double>(Lc.n);
+        raise_smem_limit(reinterpret_cast<const void*>(k_gen_coarse_lu), int(sm));
+        k_gen_coarse_lu<<<1, kDenseThreads, sm, g.st>>>(Lc.n, Lc.rp, Lc.ci, Lc.v, Lc.perm, Lc.lu, Lc.piv, sm);
         ++g.launches;
     }
 }
@@ -1171,7 +1163,9 @@ int gen_setup(GenEngine* gp, const rsg_options& o, const double* acc) {
     }
     GEN_CUDA(cudaMemcpyAsync(g.LU, g.S, size_t(g.nnzb) * b2 * sizeof(double), cudaMemcpyDeviceToDevice, g.st));
     const int nlf = int(g.fStart.size()) - 1;
-    if (g.n <= 2048) {                                     // small: every level in one block
+    // levels of a few rows: every level in one block of four warps; wider ones spread their rows over the GPU, a launch each
+    // (960 rows of 8 x 8 blocks in 31 levels: 9.9 ms in one block)
+    if (g.n <= 4 * kWarpsPerBlock * nlf / 2) {
         k_gen_factor_cta<<<1, kWarpsPerBlock * 32, 0, g.st>>>(nlf, g.fLvl, g.fOrd, g.nb, g.rp, g.ci, g.dg, g.LU, g.dCnt);
         ++g.launches;
     } else {
