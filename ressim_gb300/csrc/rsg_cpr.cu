@@ -108,7 +108,7 @@ __device__ __forceinline__ bool coarse_level(const AmgSysLv* __restrict__ lv, in
 }
 
 // dense LU with partial pivoting of every system's coarsest level in its natural numbering
-// (engine/src/amg.cpp:273-295; rsg_dense.cuh), one thread block per system. T = double (reference arithmetic) or float (the
+// (engine/src/amg.cpp:273-295; rsg_dense.cuh), one cluster of blocks per system. T = double (reference arithmetic) or float (the
 // FP32 hierarchy of the precision forms: same algorithm, float operations).
 template <class T>
 __global__ void __launch_bounds__(kDenseThreads) k_coarse_lu(int maxL, const AmgSysLv* __restrict__ lv, const int* __restrict__ rp,
@@ -116,26 +116,20 @@ __global__ void __launch_bounds__(kDenseThreads) k_coarse_lu(int maxL, const Amg
                                                              const int* __restrict__ luPerm, T* luAll, int* pivAll, int* cinAll,
                                                              int skipUpTo, const int* only, unsigned smemBytes) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    const int s = blockIdx.x, tid = int(threadIdx.x), nt = int(blockDim.x);
-    if (only && !only[s]) return;                                 // only the systems flagged (FP64 coarse solve)
+    const int s = int(blockIdx.x) / kDenseCluster, tid = int(threadIdx.x), nt = int(blockDim.x), rank = cluster_rank();
+    if (only && !only[s]) return;                                 // only the systems flagged (FP64 coarse solve); whole clusters
     AmgSysLv L;
     if (!coarse_level(lv, maxL, s, L) || L.n <= skipUpTo) return;   // skipUpTo: levels inverted in shared memory
     const int m = L.n;
     T* lu = luAll + L.luOff;
-    T* a = dense_lu_place<T>(m, smemBytes, smraw, lu);
     int* piv = pivAll + L.luRowOff;
     const int* nat = luPerm + L.luRowOff;
-    for (int q = tid; q < m * m; q += nt) a[q] = T(0);
-    __syncthreads();
-    for (int k = tid; k < m; k += nt) {
-        const int I = __ldg(nat + k);
-        for (int p = __ldg(rp + L.rpOff + k); p < __ldg(rp + L.rpOff + k + 1); ++p)
-            a[size_t(I) * m + __ldg(nat + __ldg(ci + L.entOff + p))] = T(val[L.entOff + p]);
-    }
-    __syncthreads();
-    dense_lu(m, a, piv);
-    if (a != lu)
-        for (int q = tid; q < m * m; q += nt) lu[q] = a[q];
+    const DenseCols<T> D = dense_place(m, rank, smemBytes, smraw, lu);
+    dense_fill(D, rp + L.rpOff, ci + L.entOff, val + L.entOff, nat);
+    dense_lu(D, piv);
+    dense_out(D, lu);
+    if (rank) return;
+    __syncthreads();                                              // (piv: written by this block)
     // gather order of the solve: the level-space row whose value lands at position i once the natural-order
     // vector has gone through the row interchanges piv[0], piv[1], ... (engine/src/amg.cpp:306-308)
     __shared__ int cin[kDenseMax];
@@ -519,10 +513,9 @@ void launch_amg_coarse_lu(const DevAmg& G, bool fp32, cudaStream_t st) {
         k_coarse_gj<<<G.nsys, kGjThreads, smem, st>>>(G.maxL, G.lv, G.rp, G.ci, G.val, G.luPerm, G.invf);
         if (G.maxCoarse > kInvSmemRows) {                        // levels too large for shared memory: LU, then columns
             const unsigned sl = dense_lu_smem<float>(G.maxCoarse), si = unsigned(size_t(G.maxCoarse) * (kInvCols + 2) * sizeof(float));
-            raise_smem_limit(reinterpret_cast<const void*>(k_coarse_lu<float>), int(sl));
             raise_smem_limit(reinterpret_cast<const void*>(k_coarse_inv), int(si));
-            k_coarse_lu<float><<<G.nsys, kDenseThreads, sl, st>>>(G.maxL, G.lv, G.rp, G.ci, G.val, G.luPerm, G.luf, G.piv, G.cin, kInvSmemRows,
-                                                                  nullptr, sl);
+            launch_dense(k_coarse_lu<float>, G.nsys, sl, st, G.maxL, (const AmgSysLv*)G.lv, (const int*)G.rp, (const int*)G.ci,
+                         (const double*)G.val, (const int*)G.luPerm, G.luf, G.piv, G.cin, kInvSmemRows, (const int*)nullptr, sl);
             k_coarse_inv<<<dim3(unsigned((G.maxCoarse + kInvCols - 1) / kInvCols), unsigned(G.nsys)), 256, si, st>>>(
                 G.maxL, G.lv, G.cin, G.luf, G.invf, kInvSmemRows, si);
         }
@@ -532,9 +525,8 @@ void launch_amg_coarse_lu(const DevAmg& G, bool fp32, cudaStream_t st) {
         k_coarse_check<<<G.nsys, 256, 0, st>>>(G.maxL, G.lv, G.rp, G.ci, G.val, G.luPerm, G.invf, G.x, G.b, G.coarse64);
     }
     const unsigned sm = dense_lu_smem<double>(G.maxCoarse);
-    raise_smem_limit(reinterpret_cast<const void*>(k_coarse_lu<double>), int(sm));
-    k_coarse_lu<double><<<G.nsys, kDenseThreads, sm, st>>>(G.maxL, G.lv, G.rp, G.ci, G.val, G.luPerm, G.lu, G.piv, G.cin, 0,
-                                                           fp32 ? G.coarse64 : nullptr, sm);
+    launch_dense(k_coarse_lu<double>, G.nsys, sm, st, G.maxL, (const AmgSysLv*)G.lv, (const int*)G.rp, (const int*)G.ci, (const double*)G.val,
+                 (const int*)G.luPerm, G.lu, G.piv, G.cin, 0, (const int*)(fp32 ? G.coarse64 : nullptr), sm);
 }
 void launch_amg_round(const DevAmg& G, cudaStream_t st) {
     k_round<<<grid_for(size_t(G.totEnt)), 256, 0, st>>>(size_t(G.totEnt), G.val, G.valf);

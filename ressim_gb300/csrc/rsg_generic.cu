@@ -431,23 +431,16 @@ __global__ void k_gen_diag_fix(int n, const int* __restrict__ dg, double* v) {
         if (fabs(v[dg[i]]) < 1e-300) v[dg[i]] = 1.0;
 }
 // dense LU with partial pivoting of the coarsest level in its natural numbering (AMG::factorCoarsest,
-// engine/src/amg.cpp:273-295), one thread block (rsg_dense.cuh); lu is m x m, perm: level-space row -> natural row
+// engine/src/amg.cpp:273-295), one cluster of blocks (rsg_dense.cuh); lu is m x m, perm: level-space row -> natural row
 __global__ void __launch_bounds__(kDenseThreads) k_gen_coarse_lu(int m, const int* __restrict__ rp, const int* __restrict__ ci,
                                                                  const double* __restrict__ v, const int* __restrict__ perm, double* lu,
                                                                  int* piv, unsigned smemBytes) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    const int tid = int(threadIdx.x), nt = int(blockDim.x);
-    double* a = dense_lu_place<double>(m, smemBytes, smraw, lu);
-    for (int q = tid; q < m * m; q += nt) a[q] = 0.0;
-    __syncthreads();
-    for (int k = tid; k < m; k += nt) {
-        const int I = perm[k];
-        for (int p = rp[k]; p < rp[k + 1]; ++p) a[I * m + perm[ci[p]]] = v[p];
-    }
-    __syncthreads();
-    dense_lu(m, a, piv);
-    if (a != lu)
-        for (int q = tid; q < m * m; q += nt) lu[q] = a[q];
+    const int rank = cluster_rank();
+    const DenseCols<double> D = dense_place(m, rank, smemBytes, smraw, lu);
+    dense_fill(D, rp, ci, v, perm);
+    dense_lu(D, piv);
+    dense_out(D, lu);
 }
 
 // ------------------------------------------------------------------ AMG V-cycle (AMG::cycle, engine/src/amg.cpp:303-337)
@@ -872,8 +865,8 @@ void refresh_amg(GenEngine& g) {
     GenLevel& Lc = g.lv.back();
     if (Lc.dense) {
         const unsigned sm = dense_lu_smem<double>(Lc.n);
-        raise_smem_limit(reinterpret_cast<const void*>(k_gen_coarse_lu), int(sm));
-        k_gen_coarse_lu<<<1, kDenseThreads, sm, g.st>>>(Lc.n, Lc.rp, Lc.ci, Lc.v, Lc.perm, Lc.lu, Lc.piv, sm);
+        launch_dense(k_gen_coarse_lu, 1, sm, g.st, Lc.n, (const int*)Lc.rp, (const int*)Lc.ci, (const double*)Lc.v, (const int*)Lc.perm, Lc.lu,
+                     Lc.piv, sm);
         ++g.launches;
     }
 }
