@@ -21,15 +21,26 @@
 // the accumulation of a cell's three rows, adds its connections' fluxes (negated, with the two cells' derivative slots
 // exchanged, on a connection's second cell) and writes the rows once; k_bo_addends finishes the few rows that take
 // well terms.
+//
+// All of it is FP64 arithmetic on a part with two FP64 lanes per SM, so the number of FP64 instructions is what bounds it.
+// Most derivative slots are structural zeros or ones: the water properties do not depend on x, the gas ones not on Sw, the
+// oil PVT on neither Sw nor, in a saturated cell, x. Products with and sums of such slots change no value (x 0 = 0, x 1 = x,
+// x + 0 = x for finite x; (2 t) / 2 = t), so they are left out, here and in the records and fluxes, which hold only the other
+// slots. Where that would not be the engine's result -- a cell in state 2 or with a value that is not finite, a potential
+// difference that is zero or not finite -- the full dual numbers are formed ("general" cells, flagged phases). Derivative slots
+// are kept in the order (p, Sw, x) and put into the engine's order where rows are written. 742,384 cells: 1.82 -> 1.17 ms
+// (FP64 pipe 88 % busy in the first two kernels).
 #include "rsg.h"
 
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <numeric>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 namespace rsg {
@@ -147,6 +158,7 @@ struct Model {
     // live oil: nsat saturated nodes (Rs, 1/Bo, 1/(Bo mu)) at rs, bsat, bmusat; under tables at utab[2 k] (1/Bo
     // ratio) and utab[2 k + 1] (1/(Bo mu) ratio) of the descriptor array
     int nsat, rs, rsk, bsat, bmusat;   // rsk: order keys of the nodes' Rs
+    int plain;                         // every table value, slope and constant is finite
 };
 
 // FluidModel::liveOil (engine/src/fluid.cpp:257-271): interpolation between the saturated nodes bracketing rs of
@@ -223,73 +235,60 @@ __device__ D3 kro3(const double* T, const Model& m, D3 sw, D3 sg) {
 
 // ---------------------------------------------------------------------------------------------------------------
 // Cell properties (Simulator::evalCell, engine/src/simulator.cpp:2133-2276, for this model): record layout
-// P[0..2] mob[3..5] rho[6..8] mobRs[9] acc[10..12], word j of field f of cell c at rec[(4 f + j) na + c].
-__global__ void __launch_bounds__(kThreads) k_bo_props(int na, Model m, const double* __restrict__ T, const Tab* __restrict__ U,
-                                                       const double* __restrict__ pv0, const double* __restrict__ pres,
-                                                       const double* __restrict__ swv, const double* __restrict__ xv,
-                                                       const unsigned char* __restrict__ state, double* __restrict__ rec) {
-    const int c = blockIdx.x * kThreads + threadIdx.x;
-    if (c >= na) return;
-    const D3 P = dvar(__ldg(pres + c), 0);
-    D3 Sw = dconst(m.water && !m.oil ? 1.0 : 0.0), Sg = dconst(0.0), rs = dconst(0.0);
-    if (m.iSw >= 0) Sw = dvar(__ldg(swv + c), m.iSw);
-    const int st = __ldg(state + c);
-    if (m.gas) {
-        if (st == 1) {
-            Sg = dvar(__ldg(xv + c), m.iX);
-            if (m.live) rs = rs_sat(T, m, P);
-        } else if (st == 0) {
-            rs = dvar(__ldg(xv + c), m.iX);
-        } else {
-            Sg = csub(1.0, Sw);
-            if (m.live) rs = rs_sat(T, m, P);
-        }
+// P[0..2] mob[3..5] rho[6..8] mobRs[9] acc[10..12], word j of field f of cell c at rec[(4 f + j) na + c]: value, then the
+// derivatives in p, Sw and x. gen[c] = 1: the cell is general, its record holds all words; else the structural slots are
+// absent (ldfield).
+
+// every dual number in full
+__device__ __noinline__ void props_general(int c, int na, const Model& m, const double* __restrict__ T, const Tab* __restrict__ U, double pv0,
+                                           double p, double swv, double xv, int st, double* __restrict__ rec) {
+    const D3 P = dvar(p, 0), Sw = dvar(swv, 1);
+    D3 Sg = dconst(0.0), rs = dconst(0.0);
+    if (st == 1) {
+        Sg = dvar(xv, 2);
+        rs = rs_sat(T, m, P);
+    } else if (st == 0) {
+        rs = dvar(xv, 2);
+    } else {
+        Sg = csub(1.0, Sw);
+        rs = rs_sat(T, m, P);
     }
-    const D3 So = (m.oil && !(m.gas && st == 2)) ? sub(csub(1.0, Sw), Sg) : dconst(0.0);
+    const D3 So = st != 2 ? sub(csub(1.0, Sw), Sg) : dconst(0.0);
     // pore volume: FluidModel::pvMult (fluid.cpp:199-202) times the reference pore volume
     D3 pv;
     {
         const D3 X = mulc(subc(P, m.rock_ref), m.rock_cr);
-        pv = mulc(add(addc(X, 1.0), mulc(mul(X, X), 0.5)), __ldg(pv0 + c));
+        pv = mulc(add(addc(X, 1.0), mulc(mul(X, X), 0.5)), pv0);
     }
-    D3 Pp[3] = {dconst(0.0), dconst(0.0), dconst(0.0)}, mob[3] = {dconst(0.0), dconst(0.0), dconst(0.0)};
-    D3 rho[3] = {dconst(0.0), dconst(0.0), dconst(0.0)}, acc[3] = {dconst(0.0), dconst(0.0), dconst(0.0)};
-    D3 mobRs = dconst(0.0), bo = dconst(0.0);
-    if (m.water) {
-        Pp[PW] = m.oil ? sub(P, mulc(mulc(tab_ad(T, m.pcow, Sw), 1.0), 1.0)) : P;
+    D3 f[kRec];
+    {
+        f[PW] = sub(P, mulc(mulc(tab_ad(T, m.pcow, Sw), 1.0), 1.0));
         // FluidModel::bw / bwMu (fluid.cpp:191-198)
-        const D3 X = mulc(subc(Pp[PW], m.pw_ref), m.pw_cw);
+        const D3 X = mulc(subc(f[PW], m.pw_ref), m.pw_cw);
         const D3 bw = mulc(add(addc(X, 1.0), mulc(mul(X, X), 0.5)), m.inv_bw);
-        const D3 Y = mulc(subc(Pp[PW], m.pw_ref), m.pw_cwv);
+        const D3 Y = mulc(subc(f[PW], m.pw_ref), m.pw_cwv);
         const D3 bwmu = mulc(add(addc(Y, 1.0), mulc(mul(Y, Y), 0.5)), m.inv_bwvisc);
-        const D3 kr = !m.oil ? dconst(1.0) : tab_ad(T, m.krw, Sw);
-        mob[PW] = mul(bwmu, kr);
-        rho[PW] = mulc(bw, m.rho_water);
-        acc[PW] = mul(mul(pv, bw), Sw);
+        f[3 + PW] = mul(bwmu, tab_ad(T, m.krw, Sw));
+        f[6 + PW] = mulc(bw, m.rho_water);
+        f[10 + PW] = mul(mul(pv, bw), Sw);
     }
-    if (m.oil) {
-        Pp[PO] = P;
-        D3 bomu;
-        if (m.live) live_oil_ad2(T, U, m, P, rs, bo, bomu);
-        else { bo = tab_ad(T, m.deadB, P); bomu = tab_ad(T, m.deadBMu, P); }
-        D3 kr = dconst(1.0);
-        if (m.water || m.gas) kr = kro3(T, m, Sw, Sg);
-        mob[PO] = mul(bomu, kr);
-        rho[PO] = mul(bo, addc(mulc(rs, m.rho_gfac), m.rho_oil));
-        acc[PO] = mul(mul(pv, bo), So);
-        mobRs = mul(mob[PO], rs);
+    D3 bo, bomu;
+    {
+        f[PO] = P;
+        live_oil_ad2(T, U, m, P, rs, bo, bomu);
+        f[3 + PO] = mul(bomu, kro3(T, m, Sw, Sg));
+        f[6 + PO] = mul(bo, addc(mulc(rs, m.rho_gfac), m.rho_oil));
+        f[10 + PO] = mul(mul(pv, bo), So);
+        f[9] = mul(f[3 + PO], rs);
     }
-    if (m.gas) {
-        Pp[PG] = add(P, tab_ad(T, m.pcog, Sg));
-        const D3 krg = tab_ad(T, m.krg, Sg);
-        const D3 bg = tab_ad(T, m.gasB, Pp[PG]);
-        mob[PG] = mul(tab_ad(T, m.gasBMu, Pp[PG]), krg);
-        rho[PG] = mulc(bg, m.rho_gfac);
-        acc[PG] = mul(pv, add(mul(bg, Sg), m.oil ? mul(mul(rs, bo), So) : dconst(0.0)));
+    {
+        f[PG] = add(P, tab_ad(T, m.pcog, Sg));
+        const D3 bg = tab_ad(T, m.gasB, f[PG]);
+        f[3 + PG] = mul(tab_ad(T, m.gasBMu, f[PG]), tab_ad(T, m.krg, Sg));
+        f[6 + PG] = mulc(bg, m.rho_gfac);
+        f[10 + PG] = mul(pv, add(mul(bg, Sg), mul(mul(rs, bo), So)));
     }
-    const D3 f[kRec] = {Pp[0], Pp[1], Pp[2], mob[0], mob[1], mob[2], rho[0], rho[1], rho[2], mobRs, acc[0], acc[1], acc[2]};
     const size_t N = size_t(na);
-#pragma unroll
     for (int k = 0; k < kRec; ++k) {
         rec[(4 * k + 0) * N + c] = f[k].v;
         rec[(4 * k + 1) * N + c] = f[k].d0;
@@ -298,9 +297,168 @@ __global__ void __launch_bounds__(kThreads) k_bo_props(int na, Model m, const do
     }
 }
 
-__device__ __forceinline__ D3 ld3(const double* __restrict__ rec, size_t N, int field, int c) {
-    return D3{__ldg(rec + (4 * field + 0) * N + c), __ldg(rec + (4 * field + 1) * N + c), __ldg(rec + (4 * field + 2) * N + c),
-              __ldg(rec + (4 * field + 3) * N + c)};
+// 1 + X + X^2 / 2 with the engine's rounding; the derivative factor of X' is 1 + X: (2 X' X) / 2 = X' X, so d = X' + X' X
+__device__ __forceinline__ double series(double X) { return __fma_rn(X * X, 0.5, X + 1.0); }   // (halving is exact)
+__device__ __forceinline__ double series_d(double Xd, double X) { return Xd + Xd * X; }
+
+__global__ void __launch_bounds__(kThreads) k_bo_props(int na, Model m, const double* __restrict__ T, const Tab* __restrict__ U,
+                                                       const double* __restrict__ pv0v, const double* __restrict__ pres,
+                                                       const double* __restrict__ swa, const double* __restrict__ xa,
+                                                       const unsigned char* __restrict__ state, double* __restrict__ rec,
+                                                       unsigned char* __restrict__ gen) {
+    const int c = blockIdx.x * kThreads + threadIdx.x;
+    if (c >= na) return;
+    const double p = __ldg(pres + c), sw = __ldg(swa + c), x = __ldg(xa + c), pv0 = __ldg(pv0v + c);
+    const int st = __ldg(state + c);
+    const size_t N = size_t(na);
+    // outside |input| < 2^256 an intermediate value could overflow behind a structural slot
+    auto wide = [](double v) { return (__double2hiint(v) & 0x7fffffff) >= 0x4ff00000; };
+    bool bad = (st != 0 && st != 1) || !m.plain || wide(p) || wide(sw) || wide(x);
+    auto put = [&](int f, int j, double v) {
+        bad = bad || (__double2hiint(v) & 0x7ff00000) == 0x7ff00000;   // infinite or not a number
+        rec[(4 * f + j) * N + c] = v;
+    };
+    if (!bad) {
+        const bool sat = st == 1;                             // free gas: x = Sg, Rs saturated; else x = Rs, no gas
+        double rs = x, rs0 = 0.0;                             // Rs and its p derivative (undersaturated: d/dx = 1)
+        if (sat) {
+            rs = tab_eval(T, m.rsOfP, p, rs0);
+            if (rs < 0) { rs = 0; rs0 = 0; }
+        }
+        const double sg = sat ? x : 0.0;
+        const double so = (-sw + 1.0) - sg;                   // d/dSw = -1, d/dx = -1 with free gas
+        // pore volume
+        const double Xr = (p - m.rock_ref) * m.rock_cr;
+        const double pv = series(Xr) * pv0, pvp = series_d(m.rock_cr, Xr) * pv0;
+        // water: nothing depends on x
+        {
+            double s, ks;
+            const double pw = p - tab_eval(T, m.pcow, sw, s);
+            put(PW, 0, pw);
+            put(PW, 2, -s);
+            const double X = (pw - m.pw_ref) * m.pw_cw, X1 = -s * m.pw_cw;
+            const double bw = series(X) * m.inv_bw, bw0 = series_d(m.pw_cw, X) * m.inv_bw, bw1 = series_d(X1, X) * m.inv_bw;
+            const double Y = (pw - m.pw_ref) * m.pw_cwv, Y1 = -s * m.pw_cwv;
+            const double bm = series(Y) * m.inv_bwvisc, bm0 = series_d(m.pw_cwv, Y) * m.inv_bwvisc, bm1 = series_d(Y1, Y) * m.inv_bwvisc;
+            const double k = tab_eval(T, m.krw, sw, ks);
+            put(3 + PW, 0, bm * k);
+            put(3 + PW, 1, bm0 * k);
+            put(3 + PW, 2, bm1 * k + bm * ks);
+            put(6 + PW, 0, bw * m.rho_water);
+            put(6 + PW, 1, bw0 * m.rho_water);
+            put(6 + PW, 2, bw1 * m.rho_water);
+            const double q = pv * bw, q0 = pvp * bw + pv * bw0, q1 = pv * bw1;
+            put(10 + PW, 0, q * sw);
+            put(10 + PW, 1, q0 * sw);
+            put(10 + PW, 2, q1 * sw + q);
+        }
+        // live oil (FluidModel::liveOilAD): 1/Bo and 1/(Bo mu) with their central differences in p and Rs
+        double bo, bo0, bo2 = 0.0, om, om0, om2 = 0.0;
+        {
+            const LiveSeg g0 = live_seg(T, m, rs);
+            const double hp = 1e-4 * fmax(1.0, fabs(p)), hr = 1e-5 * fmax(1e-2, fabs(rs));
+            double bp, mp, bm, mm;
+            live_pair(T, U, m, g0, p, bo, om);
+            live_pair(T, U, m, g0, p + hp, bp, mp);
+            live_pair(T, U, m, g0, p - hp, bm, mm);
+            bo0 = (bp - bm) / (2 * hp);
+            om0 = (mp - mm) / (2 * hp);
+            live_pair(T, U, m, live_seg(T, m, rs + hr), p, bp, mp);
+            live_pair(T, U, m, live_seg(T, m, rs - hr), p, bm, mm);
+            const double br = (bp - bm) / (2 * hr), mr = (mp - mm) / (2 * hr);
+            if (sat) { bo0 = bo0 + br * rs0; om0 = om0 + mr * rs0; }
+            else { bo2 = br; om2 = mr; }
+        }
+        // oil relative permeability (SatFunctions::kro): k, d/dSw, d/dx (free gas)
+        double k, k1, k2 = 0.0;
+        {
+            const bool on = !(sw - m.swco < 0);
+            const double dw = on ? sw - m.swco : 0.0, eff = sw + sg, den = sg + dw;
+            double ws;
+            const double wv = tab_eval(T, m.krow, eff, ws);
+            if (den < 1e-9) {
+                k = wv;
+                k1 = ws;
+                if (sat) k2 = ws;
+            } else {
+                double num = dw * wv, n1 = on ? wv + dw * ws : 0.0, n2 = 0.0;
+                if (sat) {
+                    double gs;
+                    const double gv = tab_eval(T, m.krog, eff - m.swco, gs), gg = sg * gs;
+                    num = sg * gv + num;
+                    n1 = gg + n1;
+                    n2 = (gv + gg) + dw * ws;
+                }
+                const double inv = 1.0 / den;
+                k = num * inv;
+                k1 = (on ? n1 * den - num : n1 * den) * inv * inv;
+                if (sat) k2 = (n2 * den - num) * inv * inv;
+            }
+        }
+        {
+            put(PO, 0, p);
+            const double mo = om * k, mo0 = om0 * k, mo1 = om * k1, mo2 = sat ? om * k2 : om2 * k;
+            put(3 + PO, 0, mo);
+            put(3 + PO, 1, mo0);
+            put(3 + PO, 2, mo1);
+            put(3 + PO, 3, mo2);
+            const double d = rs * m.rho_gfac + m.rho_oil;
+            put(6 + PO, 0, bo * d);
+            put(6 + PO, 1, sat ? bo0 * d + bo * (rs0 * m.rho_gfac) : bo0 * d);
+            put(6 + PO, 3, sat ? 0.0 : bo2 * d + bo * m.rho_gfac);
+            const double q = pv * bo, q0 = pvp * bo + pv * bo0;
+            put(10 + PO, 0, q * so);
+            put(10 + PO, 1, q0 * so);
+            put(10 + PO, 2, -q);
+            put(10 + PO, 3, sat ? -q : (pv * bo2) * so);
+            put(9, 0, mo * rs);
+            put(9, 1, sat ? mo0 * rs + mo * rs0 : mo0 * rs);
+            put(9, 2, mo1 * rs);
+            put(9, 3, sat ? mo2 * rs : mo2 * rs + mo);
+        }
+        // gas: nothing but the accumulation depends on Sw
+        {
+            double s, ks, bs, ms;
+            const double pg = p + tab_eval(T, m.pcog, sg, s);
+            const double kg = tab_eval(T, m.krg, sg, ks);
+            const double bg = tab_eval(T, m.gasB, pg, bs), gm = tab_eval(T, m.gasBMu, pg, ms);
+            const double pg2 = sat ? s : 0.0, bg2 = sat ? bs * s : 0.0;
+            put(PG, 0, pg);
+            put(PG, 3, pg2);
+            put(3 + PG, 0, gm * kg);
+            put(3 + PG, 1, ms * kg);
+            put(3 + PG, 3, sat ? (ms * s) * kg + gm * ks : 0.0);
+            put(6 + PG, 0, bg * m.rho_gfac);
+            put(6 + PG, 1, bs * m.rho_gfac);
+            put(6 + PG, 3, sat ? bg2 * m.rho_gfac : 0.0);
+            const double rb = rs * bo;                        // dissolved gas per pore volume, times So
+            double w = rb * so, w0, w2;
+            if (sat) {
+                w0 = bs * sg + (rs0 * bo + rs * bo0) * so;
+                w2 = (bg2 * sg + bg) + -rb;
+                w = bg * sg + w;
+            } else {
+                w0 = (rs * bo0) * so;
+                w2 = (bo + rs * bo2) * so;
+            }
+            put(10 + PG, 0, pv * w);
+            put(10 + PG, 1, pvp * w + pv * w0);
+            put(10 + PG, 2, pv * -rb);
+            put(10 + PG, 3, pv * w2);
+        }
+    }
+    gen[c] = bad ? 1 : 0;
+    if (bad) props_general(c, na, m, T, U, pv0, p, sw, x, st, rec);
+}
+
+// field F of cell c: the words the record holds, and the structural slots of a cell that is not general
+template <int F>
+__device__ __forceinline__ D3 ldfield(const double* __restrict__ rec, size_t N, int c, bool gen) {
+    auto w = [&](int j) { return __ldg(rec + (4 * F + j) * N + c); };
+    constexpr bool P = F == 0 || F == 1 || F == 2;                                   // phase pressures: d/dp = 1
+    constexpr bool S = F == 0 || F == 3 || F == 6 || F == 10 || F == 4 || F == 9 || F == 11 || F == 12;   // depends on Sw
+    constexpr bool X = F == 2 || F == 4 || F == 5 || F == 7 || F == 8 || F == 9 || F == 11 || F == 12;    // depends on x
+    return D3{w(0), P && !gen ? 1.0 : w(1), S || gen ? w(2) : 0.0, X || gen ? w(3) : 0.0};
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -308,16 +466,14 @@ __device__ __forceinline__ D3 ld3(const double* __restrict__ rec, size_t N, int 
 // 2567-2620): dphi = P_a - P_b + rho g dD with rho = (rho_a + rho_b) / 2, F = mob_upstream dphi T. The dual numbers
 // carry a's derivatives (fa) and b's (fb); the slots a lifted operand does not have are exact zeros, so their
 // products and sums are left out (x + 0 and 0 * y change no value), and so is the gravity term of a connection
-// without depth difference.
+// without depth difference. Full form: flagged phases and general cells.
 struct Dphi {
     double v, da[3], db[3];
 };
 
-__device__ __forceinline__ Dphi dphi_of(const double* __restrict__ rec, size_t N, int p, int b, const D3& PA, const D3& RA, double gd) {
-    const D3 PB = ld3(rec, N, p, b);
+__device__ __forceinline__ Dphi dphi_of(const D3& PA, const D3& PB, const D3& RA, const D3& RB, double gd) {
     Dphi d{PA.v - PB.v, {PA.d0, PA.d1, PA.d2}, {-PB.d0, -PB.d1, -PB.d2}};
     if (gd != 0.0) {
-        const D3 RB = ld3(rec, N, 6 + p, b);
         d.v = d.v + ((RA.v + RB.v) * 0.5) * gd;
         d.da[0] = d.da[0] + (RA.d0 * 0.5) * gd;
         d.da[1] = d.da[1] + (RA.d1 * 0.5) * gd;
@@ -348,161 +504,248 @@ __device__ __forceinline__ Flux flux_of(const D3& mo, bool upA, const Dphi& d, d
 
 constexpr int kFluxKinds = 4;                 // per connection: water, oil, dissolved gas (with the oil), gas
 constexpr int kFluxWords = kFluxKinds * 7;    // value, the first cell's 3 derivatives, the second's 3
+// slots of a term that are not structural zeros: the water flux has no x, the gas flux no Sw derivative
+__host__ __device__ constexpr bool flux_slot(int kind, int i) { return kind == 0 ? i != 2 : (kind == 3 ? i != 1 : true); }
+
+// x with its sign turned where `neg` has the sign bit (the integer pipe's work, not the FP64 pipe's)
+__device__ __forceinline__ double flip(double x, int neg) { return __hiloint2double(__double2hiint(x) ^ neg, __double2loint(x)); }
+
+// the terms of connection c between plain cells a and b (without gravity half the arithmetic: 742,384 cells of which 29 % of the
+// connections have a depth difference, 360 us with selects, 262 us with two bodies); hg: half the gravity factor. Returns the phases left to the cells
+template <bool grav>
+__device__ __forceinline__ unsigned conn_terms(size_t N, size_t NC, int c, int a, int b, double tr, double hg, const double* __restrict__ rec,
+                                               double* __restrict__ flux) {
+    auto word = [&](int f, int j, int cell) { return __ldg(rec + (4 * f + j) * N + cell); };
+    unsigned fl = 0;
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        double dv = word(p, 0, a) - word(p, 0, b);
+        if (grav) dv = dv + (word(6 + p, 0, a) + word(6 + p, 0, b)) * hg;
+        const long long bits = __double_as_longlong(dv) & 0x7fffffffffffffffLL;
+        if (bits == 0 || bits >= 0x7ff0000000000000LL) { fl |= 1u << p; continue; }
+        const bool upA = __double2hiint(dv) >= 0;
+        const int up = upA ? a : b, dn = upA ? b : a;
+        const int neg = upA ? 0 : int(0x80000000), pos = neg ^ int(0x80000000);
+        // derivatives of dv on the upstream side (u) and the other (w): +-1 in p, +-dP in the phase's saturation, and the
+        // gravity terms of the phase's density
+        const int sat = p == PW ? 1 : 2;                                   // the slot of the phase's capillary pressure
+        double u[3] = {flip(1.0, neg), 0.0, 0.0}, w[3] = {flip(1.0, pos), 0.0, 0.0};
+        bool hu[3] = {true, false, false}, hw[3] = {true, false, false};
+        if (p != PO) {
+            const double pu = word(p, 1 + sat, up), pw = word(p, 1 + sat, dn);
+            u[sat] = flip(pu, neg);
+            w[sat] = flip(pw, pos);
+            hu[sat] = hw[sat] = true;
+        }
+        if (grav) {
+            u[0] = u[0] + word(6 + p, 1, up) * hg;
+            w[0] = w[0] + word(6 + p, 1, dn) * hg;
+            const int q = p == PW ? 1 : 2;                                 // the slot of the phase's density
+            const double ru = word(6 + p, 1 + q, up) * hg, rw = word(6 + p, 1 + q, dn) * hg;
+            u[q] = p == PO ? ru : u[q] + ru;
+            w[q] = p == PO ? rw : w[q] + rw;
+            hu[q] = hw[q] = true;
+        }
+        // F = m dv T: without gravity the p derivative's m (+-1) is m with that sign
+        auto term = [&](auto kind, int f) {
+            constexpr int KIND = decltype(kind)::value;
+            const double mv = word(f, 0, up), md[3] = {word(f, 1, up), flux_slot(KIND, 1) ? word(f, 2, up) : 0.0,
+                                                       flux_slot(KIND, 2) ? word(f, 3, up) : 0.0};
+            flux[(7 * KIND + 0) * NC + c] = (mv * dv) * tr;
+            double* fu = flux + (7 * KIND + (upA ? 1 : 4)) * NC + c;
+            double* fw = flux + (7 * KIND + (upA ? 4 : 1)) * NC + c;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                if (!flux_slot(KIND, i)) continue;
+                const double mu = i == 0 && !grav ? flip(mv, neg) : mv * u[i], mw = i == 0 && !grav ? flip(mv, pos) : mv * w[i];
+                fu[i * NC] = (hu[i] ? md[i] * dv + mu : md[i] * dv) * tr;
+                fw[i * NC] = hw[i] ? mw * tr : 0.0;
+            }
+        };
+        if (p == PW) term(std::integral_constant<int, 0>(), 3 + PW);
+        else if (p == PO) {
+            term(std::integral_constant<int, 1>(), 3 + PO);
+            term(std::integral_constant<int, 2>(), 9);
+        } else {
+            term(std::integral_constant<int, 3>(), 3 + PG);
+        }
+    }
+    return fl;
+}
 
 // The fluxes of every connection, once, in the perspective of its first cell a (conn_a). Seen from its second cell b
 // the engine's flux is the exact negative with the slots exchanged -- -(x) + -(y) = -(x + y) and (-x) y = -(x y) in
 // IEEE arithmetic, and b takes the same cell as upstream -- except where the potential difference is exactly zero
 // (then each side takes itself as upstream) or not a number: those phases are flagged and their two cells form them
-// themselves. Record layout: word j of term k of connection c at flux[(7 k + j) nconn + c].
+// themselves, as do the phases of a general cell's connections and those with an infinite potential difference (see the top of
+// the file). Record layout: word j of term k of connection c at flux[(7 k + j) nconn + c].
 __global__ void __launch_bounds__(kThreads) k_bo_conn(int nconn, int na, Model m, const double* __restrict__ rec,
-                                                      const int* __restrict__ connA, const int* __restrict__ connB,
-                                                      const double* __restrict__ trans, const double* __restrict__ dDepth,
-                                                      double* __restrict__ flux, unsigned char* __restrict__ flag) {
+                                                      const unsigned char* __restrict__ gen, const int* __restrict__ connA,
+                                                      const int* __restrict__ connB, const double* __restrict__ trans,
+                                                      const double* __restrict__ dDepth, double* __restrict__ flux,
+                                                      unsigned char* __restrict__ flag) {
     const int c = blockIdx.x * kThreads + threadIdx.x;
     if (c >= nconn) return;
     const size_t N = size_t(na), NC = size_t(nconn);
     const int a = __ldg(connA + c), b = __ldg(connB + c);
     const double tr = __ldg(trans + c);
-    const double gd = m.gravity * __ldg(dDepth + c);
-    unsigned fl = 0;
-    auto put = [&](int k, const Flux& F) {
-        flux[(7 * k + 0) * NC + c] = F.v;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            flux[(7 * k + 1 + i) * NC + c] = F.fa[i];
-            flux[(7 * k + 4 + i) * NC + c] = F.fb[i];
-        }
-    };
-#pragma unroll
-    for (int p = 0; p < 3; ++p) {
-        const Dphi d = dphi_of(rec, N, p, b, ld3(rec, N, p, a), ld3(rec, N, 6 + p, a), gd);
-        if (!(d.v > 0 || d.v < 0)) { fl |= 1u << p; continue; }
-        const bool upA = d.v >= 0;
-        const int up = upA ? a : b;
-        put(p == PG ? 3 : p, flux_of(ld3(rec, N, 3 + p, up), upA, d, tr));
-        if (p == PO) put(2, flux_of(ld3(rec, N, 9, up), upA, d, tr));
-    }
-    flag[c] = static_cast<unsigned char>(fl);
+    if ((__ldg(gen + a) | __ldg(gen + b)) || (__double2hiint(tr) & 0x7ff00000) == 0x7ff00000) { flag[c] = 7; return; }
+    const double gd = m.gravity * __ldg(dDepth + c), hg = 0.5 * gd;      // (y / 2) gd = y (gd / 2) exactly
+    flag[c] = static_cast<unsigned char>(gd != 0.0 ? conn_terms<true>(N, NC, c, a, b, tr, hg, rec, flux)
+                                                   : conn_terms<false>(N, NC, c, a, b, tr, hg, rec, flux));
 }
 
 // Accumulation and TPFA flux terms of cell a's rows (Simulator::assemble cell loop, engine/src/simulator.cpp:2511-2686,
 // without the features this model leaves out), then the row scaling dt / PV (:3010-3032). The flux terms come from
-// k_bo_conn (negated and exchanged for the connections whose second cell a is), except for flagged phases, which
-// the cell forms itself. Rows that take well terms (cells listed in acell) are written unscaled and finished by
-// k_bo_addends.
-__global__ void __launch_bounds__(kThreads) k_bo_cells(int na, int nv, int nconn, Model m, double dt, const double* __restrict__ rec,
+// k_bo_conn (negated and exchanged for the connections whose second cell a is, by selects and sign bits: a branch would run
+// both sides' FP64 in the warps that hold both), except for flagged phases, which the cell forms itself. Rows that take well
+// terms (cells listed in acell) are written unscaled and finished by k_bo_addends.
+// A block's rows are consecutive words of J: they are formed in shared memory and written out in order, as a thread's own
+// stores (pieces of 24 bytes, 504 bytes from the neighbouring thread's) would each touch 32 sectors; a block with more words
+// than kCellWords (many well columns) writes them directly. 742,384 cells: 432 -> 381 us.
+constexpr int kCellThreads = 64, kCellWords = 64 * 63 + 96;
+__global__ void __launch_bounds__(kCellThreads, 6) k_bo_cells(int na, int nv, int nconn, Model m, double dt, double invDt,
+                                                       const double* __restrict__ rec, const unsigned char* __restrict__ gen,
                                                        const double* __restrict__ flux, const unsigned char* __restrict__ flag,
                                                        const double* __restrict__ accOld, const double* __restrict__ pv0,
                                                        const int* __restrict__ adjStart, const int* __restrict__ adjNbr,
-                                                       const int* __restrict__ adjConn, const int* __restrict__ adjPos,
-                                                       const int* __restrict__ connA, const double* __restrict__ trans,
-                                                       const double* __restrict__ dDepth, const int* __restrict__ blkStart,
-                                                       const int* __restrict__ selfPos, const int* __restrict__ Jrow,
-                                                       const int* __restrict__ acell, int nacell, double* __restrict__ J,
-                                                       double* __restrict__ R) {
-    const int a = blockIdx.x * kThreads + threadIdx.x;
-    if (a >= na) return;
-    const size_t N = size_t(na), NC = size_t(nconn);
-    const double invDt = 1.0 / dt;
-    // Accumulators per phase balance (the equation row of phase p is m.eq[p]): the cell's own block and residual.
-    // The model has all three phases and dissolved gas (checked at creation), so the order of the terms is fixed: a
-    // balance's first term is assigned rather than added to zero (the same value).
-    double sj[3][3], sr[3];
-    // does the cell take well terms (then its rows are finished by k_bo_addends)?
-    bool finish = false;
-    {
-        int lo = 0, hi = nacell;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            const int v = __ldg(acell + mid);
-            if (v < a) lo = mid + 1;
-            else hi = mid;
-        }
-        finish = lo < nacell && __ldg(acell + lo) == a;
-    }
-    const double s = finish ? 1.0 : dt / __ldg(pv0 + a);
-    // accumulation (acc - accOld) / dt
-#pragma unroll
-    for (int p = 0; p < 3; ++p) {
-        D3 acc = ld3(rec, N, 10 + p, a);
-        acc.v = acc.v - __ldg(accOld + size_t(a) * 3 + p);
-        sr[p] = acc.v * invDt;
-        sj[p][0] = acc.d0 * invDt;
-        sj[p][1] = acc.d1 * invDt;
-        sj[p][2] = acc.d2 * invDt;
-    }
-    const int r0 = a * nv;
-    int rowp[3];
-#pragma unroll
-    for (int p = 0; p < 3; ++p) rowp[p] = __ldg(Jrow + r0 + m.eq[p]);
-    const int nblk = __ldg(blkStart + a + 1) - __ldg(blkStart + a);
-    const int e1 = __ldg(adjStart + a + 1);
-    for (int q = __ldg(adjStart + a); q < e1; ++q) {
-        const int cn = __ldg(adjConn + q);
-        const bool first = __ldg(connA + cn) == a;            // the connection's first cell: its fluxes as stored
-        const unsigned fl = __ldg(flag + cn);
-        double nbk[3][3];   // the neighbour's block of this connection
-        // add one flux term to balance `bal`; `lead`: the connection's first term of that balance in nbk
-        auto add = [&](int bal, bool lead, double v, const double* own, const double* nb) {
-            sr[bal] += v;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                sj[bal][k] += own[k];
-                nbk[bal][k] = lead ? nb[k] : nbk[bal][k] + nb[k];
+                                                       const int* __restrict__ adjSide, const int* __restrict__ adjPos,
+                                                       const double* __restrict__ trans, const double* __restrict__ dDepth,
+                                                       const int* __restrict__ blkStart, const int* __restrict__ selfPos,
+                                                       const int* __restrict__ Jrow, const int* __restrict__ acell, int nacell,
+                                                       double* __restrict__ J, double* __restrict__ R) {
+    __shared__ double sm[kCellWords];
+    const int a0 = blockIdx.x * kCellThreads, a1 = min(na, a0 + kCellThreads);
+    const int j0 = __ldg(Jrow + a0 * nv), j1 = __ldg(Jrow + a1 * nv);
+    const bool staged = j1 - j0 <= kCellWords;
+    double* const out = staged ? sm : J + j0;                 // row words from j0 on
+    const int a = a0 + threadIdx.x;
+    if (a < na) {
+        const size_t N = size_t(na), NC = size_t(nconn);
+        // Accumulators per phase balance (the equation row of phase p is m.eq[p]): the cell's own block and residual.
+        // The model has all three phases and dissolved gas (checked at creation), so the order of the terms is fixed: a
+        // balance's first term is assigned rather than added to zero (the same value).
+        double sj[3][3], sr[3];
+        // does the cell take well terms (then its rows are finished by k_bo_addends)?
+        bool finish = false;
+        {
+            int lo = 0, hi = nacell;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                const int v = __ldg(acell + mid);
+                if (v < a) lo = mid + 1;
+                else hi = mid;
             }
+            finish = lo < nacell && __ldg(acell + lo) == a;
+        }
+        const bool ga = __ldg(gen + a) != 0;
+        const double s = finish ? 1.0 : dt / __ldg(pv0 + a);
+        // accumulation (acc - accOld) / dt
+        auto accum = [&](int p, D3 acc) {
+            sr[p] = (acc.v - __ldg(accOld + size_t(a) * 3 + p)) * invDt;
+            sj[p][0] = acc.d0 * invDt;
+            sj[p][1] = acc.d1 * invDt;
+            sj[p][2] = acc.d2 * invDt;
         };
-        auto stored = [&](int kind, int bal, bool lead) {
-            double w[7];
-#pragma unroll
-            for (int j = 0; j < 7; ++j) w[j] = __ldg(flux + (7 * kind + j) * NC + cn);
-            if (first) add(bal, lead, w[0], w + 1, w + 4);
-            else {
-                const double own[3] = {-w[4], -w[5], -w[6]}, nb[3] = {-w[1], -w[2], -w[3]};
-                add(bal, lead, -w[0], own, nb);
+        accum(PW, ldfield<10>(rec, N, a, ga));
+        accum(PO, ldfield<11>(rec, N, a, ga));
+        accum(PG, ldfield<12>(rec, N, a, ga));
+        const int r0 = a * nv;
+        int rowp[3];
+    #pragma unroll
+        for (int p = 0; p < 3; ++p) rowp[p] = __ldg(Jrow + r0 + m.eq[p]) - j0;
+        const int nblk = __ldg(blkStart + a + 1) - __ldg(blkStart + a);
+        const int e1 = __ldg(adjStart + a + 1);
+        const int q0 = __ldg(adjStart + a);
+        int next = q0 < e1 ? __ldg(adjSide + q0) : 0;
+        for (int q = q0; q < e1; ++q) {
+            const int cn = next >> 1;
+            const bool first = next & 1;                          // the connection's first cell: its fluxes as stored
+            if (q + 1 < e1) next = __ldg(adjSide + q + 1);
+            const unsigned fl = __ldg(flag + cn);
+            double nbk[3][3];   // the neighbour's block of this connection
+    #pragma unroll
+            for (int p = 0; p < 3; ++p) nbk[p][0] = nbk[p][1] = nbk[p][2] = 0.0;
+            // add one flux term to balance `bal`; `lead`: the connection's first term of that balance in nbk
+            auto add = [&](int bal, bool lead, double v, const double* own, const double* nb) {
+                sr[bal] += v;
+    #pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    sj[bal][k] += own[k];
+                    nbk[bal][k] = lead ? nb[k] : nbk[bal][k] + nb[k];
+                }
+            };
+            const long long neg = first ? 0 : (long long)0x8000000000000000ULL;
+            auto stored = [&](auto kindTag, int bal, bool lead) {
+                constexpr int kind = decltype(kindTag)::value;
+                auto w = [&](int j) { return __longlong_as_double(__double_as_longlong(__ldg(flux + (7 * kind + j) * NC + cn)) ^ neg); };
+                const int o = first ? 1 : 4, n = first ? 4 : 1;
+                sr[bal] += w(0);
+    #pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    if (!flux_slot(kind, k)) continue;
+                    sj[bal][k] += w(o + k);
+                    nbk[bal][k] = lead ? w(n + k) : nbk[bal][k] + w(n + k);
+                }
+            };
+            // a zero (or not finite) potential difference, a general cell: the cell forms the phase's terms itself
+            auto formed = [&](auto pTag) {
+                constexpr int p = decltype(pTag)::value;
+                const int b = __ldg(adjNbr + q);
+                const bool gb = __ldg(gen + b) != 0;
+                const double dD = first ? __ldg(dDepth + cn) : -__ldg(dDepth + cn);
+                const double tr = __ldg(trans + cn);
+                const Dphi d = dphi_of(ldfield<p>(rec, N, a, ga), ldfield<p>(rec, N, b, gb), ldfield<6 + p>(rec, N, a, ga),
+                                       ldfield<6 + p>(rec, N, b, gb), m.gravity * dD);
+                const bool upA = d.v >= 0;
+                const int up = upA ? a : b;
+                const bool gu = upA ? ga : gb;
+                const Flux F = flux_of(ldfield<3 + p>(rec, N, up, gu), upA, d, tr);
+                add(p, p != PG, F.v, F.fa, F.fb);
+                if constexpr (p == PO) {
+                    const Flux Fd = flux_of(ldfield<9>(rec, N, up, gu), upA, d, tr);
+                    add(PG, true, Fd.v, Fd.fa, Fd.fb);
+                }
+            };
+            using I0 = std::integral_constant<int, 0>;
+            using I1 = std::integral_constant<int, 1>;
+            using I2 = std::integral_constant<int, 2>;
+            using I3 = std::integral_constant<int, 3>;
+            if (!(fl & 1u)) stored(I0(), PW, true);
+            else formed(I0());
+            if (!(fl & 2u)) {
+                stored(I1(), PO, true);
+                stored(I2(), PG, true);
+            } else {
+                formed(I1());
             }
-        };
-#pragma unroll
-        for (int p = 0; p < 3; ++p) {
-            if (!((fl >> p) & 1u)) {
-                stored(p == PG ? 3 : p, p, p != PG);
-                if (p == PO) stored(2, PG, true);
-                continue;
-            }
-            // a zero (or undefined) potential difference: the cell forms the phase's terms itself
-            const int b = __ldg(adjNbr + q);
-            const double dD = first ? __ldg(dDepth + cn) : -__ldg(dDepth + cn);
-            const double tr = __ldg(trans + cn);
-            const Dphi d = dphi_of(rec, N, p, b, ld3(rec, N, p, a), ld3(rec, N, 6 + p, a), m.gravity * dD);
-            const bool upA = d.v >= 0;
-            const int up = upA ? a : b;
-            const Flux F = flux_of(ld3(rec, N, 3 + p, up), upA, d, tr);
-            add(p, p != PG, F.v, F.fa, F.fb);
-            if (p == PO) {
-                const Flux Fd = flux_of(ld3(rec, N, 9, up), upA, d, tr);
-                add(PG, true, Fd.v, Fd.fa, Fd.fb);
+            if (!(fl & 4u)) stored(I3(), PG, false);
+            else formed(I2());
+            const int pos = __ldg(adjPos + q);
+    #pragma unroll
+            for (int p = 0; p < 3; ++p) {
+                double* row = out + rowp[p] + pos * 3;
+                row[0] = nbk[p][0] * s;
+                row[m.iSw] = nbk[p][1] * s;
+                row[m.iX] = nbk[p][2] * s;
             }
         }
-        const int pos = __ldg(adjPos + q);
-#pragma unroll
+        const int sp = __ldg(selfPos + a);
+    #pragma unroll
         for (int p = 0; p < 3; ++p) {
-            double* row = J + rowp[p] + pos * 3;
-            row[0] = nbk[p][0] * s;
-            row[1] = nbk[p][1] * s;
-            row[2] = nbk[p][2] * s;
+            const int e = m.eq[p];
+            double* row = out + rowp[p];
+            row[sp * 3 + 0] = sj[p][0] * s;
+            row[sp * 3 + m.iSw] = sj[p][1] * s;
+            row[sp * 3 + m.iX] = sj[p][2] * s;
+            const int re = __ldg(Jrow + r0 + e + 1) - j0;
+            for (int k = rowp[p] + nblk * 3; k < re; ++k) out[k] = 0.0;   // well columns: the caller's terms only
+            R[r0 + e] = sr[p] * s;
         }
     }
-    const int sp = __ldg(selfPos + a);
-#pragma unroll
-    for (int p = 0; p < 3; ++p) {
-        const int e = m.eq[p];
-        double* row = J + rowp[p];
-        row[sp * 3 + 0] = sj[p][0] * s;
-        row[sp * 3 + 1] = sj[p][1] * s;
-        row[sp * 3 + 2] = sj[p][2] * s;
-        const int re = __ldg(Jrow + r0 + e + 1);
-        for (int k = rowp[p] + nblk * 3; k < re; ++k) J[k] = 0.0;   // well columns: the caller's terms only
-        R[r0 + e] = sr[p] * s;
-    }
+    if (!staged) return;
+    __syncthreads();
+    for (int k = threadIdx.x; k < j1 - j0; k += kCellThreads) J[j0 + k] = sm[k];
 }
 
 // Rows that take well terms: the caller's addends in their order, then (cell rows) the row scaling dt / PV. Entry i of
@@ -566,14 +809,15 @@ struct rsg_bo_assembler {
     double* tab = nullptr;
     Tab* utab = nullptr;
     double* pv0 = nullptr;
-    int *adjStart = nullptr, *adjNbr = nullptr, *adjConn = nullptr, *adjPos = nullptr, *connA = nullptr;
+    int *adjStart = nullptr, *adjNbr = nullptr, *adjSide = nullptr, *adjPos = nullptr, *connA = nullptr;
     double *trans = nullptr, *dDepth = nullptr;
     int *blkStart = nullptr, *selfPos = nullptr, *Jrow = nullptr;
     double* rec = nullptr;
     int* connB = nullptr;
     int nconn = 0;
     double* flux = nullptr;          // kFluxWords per connection (k_bo_conn)
-    unsigned char* flag = nullptr;   // per connection: phases whose potential difference is zero
+    unsigned char* flag = nullptr;   // per connection: phases its cells form themselves
+    unsigned char* gen = nullptr;    // per cell: 1 = its record holds full dual numbers
     // well addend lists: packed on the host, one upload per assembly into a device buffer grown on demand
     std::vector<char> stage;
     char* dstage = nullptr;
@@ -770,7 +1014,15 @@ extern "C" int rsg_bo_create(rsg_bo_assembler** out, const rsg_bo_grid* g, const
     }
     if (m.pbOfRs.n < 1) { delete h; return fail(RSG_EINVAL, "rsg_bo_create: live oil needs the pb(Rs) table"); }
 
+    m.plain = 1;
+    for (size_t i = 0; i < tb.size(); ++i) m.plain = m.plain && std::isfinite(tb[i]);   // (an order key that reads as one not finite: general)
+    for (double v : {m.pw_ref, m.pw_cw, m.pw_cwv, m.inv_bw, m.inv_bwvisc, m.rock_ref, m.rock_cr, m.rho_oil, m.rho_water, m.rho_gfac, m.swco})
+        m.plain = m.plain && std::isfinite(v);
     std::vector<double> trans(g->conn_trans, g->conn_trans + nconn), dd(g->conn_ddepth, g->conn_ddepth + nconn);
+    // 2 connection + (the cell is its first); every connection is named twice, so the indexes stay below 2^30
+    std::vector<int> adjSide(static_cast<size_t>(nadj));
+    for (int a = 0; a < na; ++a)
+        for (int q = adjStart[a]; q < adjStart[a + 1]; ++q) adjSide[size_t(q)] = 2 * adjConn[size_t(q)] + (connA[size_t(adjConn[size_t(q)])] == a);
     std::vector<double> pv(g->pore_vol, g->pore_vol + na);
     cudaStream_t st = h->own;
     int rc = RSG_OK;
@@ -780,14 +1032,18 @@ extern "C" int rsg_bo_create(rsg_bo_assembler** out, const rsg_bo_grid* g, const
         if (*d) h->owned.push_back(*d);
     };
     up(&h->tab, tb); up(&h->utab, ut); up(&h->pv0, pv);
-    up(&h->adjStart, adjStart); up(&h->adjNbr, adjNbr); up(&h->adjConn, adjConn); up(&h->adjPos, adjPos);
+    up(&h->adjStart, adjStart); up(&h->adjNbr, adjNbr); up(&h->adjSide, adjSide); up(&h->adjPos, adjPos);
     up(&h->connA, connA); up(&h->connB, connB); up(&h->trans, trans); up(&h->dDepth, dd);
     h->nconn = int(nconn);
     up(&h->blkStart, blkStart); up(&h->selfPos, selfPos); up(&h->Jrow, JrowH);
     if (rc == RSG_OK) {
         e = cudaMallocAsync(reinterpret_cast<void**>(&h->rec), size_t(kRecWords) * size_t(na) * sizeof(double), st);
+        if (e == cudaSuccess) {
+            h->owned.push_back(h->rec);
+            e = cudaMallocAsync(reinterpret_cast<void**>(&h->gen), size_t(na), st);
+            if (e == cudaSuccess) h->owned.push_back(h->gen);
+        }
         if (e != cudaSuccess) rc = fail(RSG_ENOMEM, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
-        else h->owned.push_back(h->rec);
     }
     if (rc == RSG_OK && nconn > 0) {
         e = cudaMallocAsync(reinterpret_cast<void**>(&h->flux), size_t(kFluxWords) * size_t(nconn) * sizeof(double), st);
@@ -897,13 +1153,13 @@ extern "C" int rsg_bo_assemble(rsg_bo_assembler* h, const double* d_p, const dou
     }
     const int* dIds = reinterpret_cast<const int*>(D + oId);
     const int grid = (na + kThreads - 1) / kThreads;
-    k_bo_props<<<grid, kThreads, 0, st>>>(na, h->m, h->tab, h->utab, h->pv0, d_p, d_sw, d_x, d_state, h->rec);
+    k_bo_props<<<grid, kThreads, 0, st>>>(na, h->m, h->tab, h->utab, h->pv0, d_p, d_sw, d_x, d_state, h->rec, h->gen);
     if (h->nconn > 0)
-        k_bo_conn<<<(h->nconn + kThreads - 1) / kThreads, kThreads, 0, st>>>(h->nconn, na, h->m, h->rec, h->connA, h->connB, h->trans,
+        k_bo_conn<<<(h->nconn + kThreads - 1) / kThreads, kThreads, 0, st>>>(h->nconn, na, h->m, h->rec, h->gen, h->connA, h->connB, h->trans,
                                                                          h->dDepth, h->flux, h->flag);
-    k_bo_cells<<<grid, kThreads, 0, st>>>(na, nv, h->nconn, h->m, dt, h->rec, h->flux, h->flag, d_acc_old, h->pv0, h->adjStart, h->adjNbr,
-                                          h->adjConn, h->adjPos,
-                                          h->connA, h->trans, h->dDepth, h->blkStart, h->selfPos, h->Jrow, dIds, ncell, d_J, d_R);
+    k_bo_cells<<<(na + kCellThreads - 1) / kCellThreads, kCellThreads, 0, st>>>(
+        na, nv, h->nconn, h->m, dt, 1.0 / dt, h->rec, h->gen, h->flux, h->flag, d_acc_old, h->pv0, h->adjStart, h->adjNbr, h->adjSide, h->adjPos,
+        h->trans, h->dDepth, h->blkStart, h->selfPos, h->Jrow, dIds, ncell, d_J, d_R);
     h->launches += h->nconn > 0 ? 3 : 2;
     if (nac > 0) {
         k_bo_addends<<<(nac + 127) / 128, 128, 0, st>>>(na, nv, nrows, dt, dIds, nac, reinterpret_cast<const int*>(D + oAB),
