@@ -888,6 +888,38 @@ int build_dev_amg(rsg_solver* h, const std::vector<SysAmg>& H) {
             const AmgLevel& A = H[size_t(s)].lv[size_t(l)];
             for (int e = 0; e < d.nnz; ++e) gci[size_t(d.entOff + e)] = d.rowOff + A.ci[size_t(e)];
         }
+    // slabs of the large colours: a slab is as wide as its longest row in the slab
+    const size_t nslab = (cdesc.size() + 31) / 32;
+    std::vector<int> slabOff(nslab + 1, 0), slabCol, slabSrc;
+    {
+        std::vector<char> big(cdesc.size(), 0);
+        for (int l = 0; l < maxL; ++l)
+            if (G.colTail[size_t(l)] > 0)
+                std::fill(big.begin() + G.colBeg[size_t(l)][0], big.begin() + G.colBeg[size_t(l)][size_t(G.colTail[size_t(l)])], char(1));
+        auto kept = [&](size_t i) { return std::min(cdesc[i].z - cdesc[i].y - 1, kSlabEntries); };
+        for (size_t i = 0; i < cdesc.size(); ++i)
+            if (big[i]) slabOff[i / 32 + 1] = std::max(slabOff[i / 32 + 1], 1 + kept(i));
+        std::partial_sum(slabOff.begin(), slabOff.end(), slabOff.begin());
+        slabCol.assign(size_t(slabOff[nslab]) * 32, kSlabPad);
+        slabSrc.assign(size_t(slabOff[nslab]) * 32, -1);
+        constexpr int kBit = int(0x80000000u);
+        for (size_t i = 0; i < cdesc.size(); ++i) {
+            if (!big[i]) continue;
+            const int4 d = cdesc[i];
+            size_t q = size_t(slabOff[i / 32]) * 32 + i % 32;
+            slabCol[q] = d.x | (d.z - d.y - 1 > kSlabEntries ? kBit : 0);
+            slabSrc[q] = d.w;
+            for (int p = d.y, left = kept(i); left > 0; ++p) {
+                if (p == d.w) continue;
+                q += 32;
+                slabCol[q] = gci[size_t(p)] | (wave[size_t(gci[size_t(p)])] > wave[size_t(d.x)] ? kBit : 0);
+                slabSrc[q] = p;
+                --left;
+            }
+        }
+        G.slabWords = slabCol.size();
+        if (slabCol.empty()) { slabCol.push_back(kSlabPad); slabSrc.push_back(-1); }
+    }
     // pointer arrays are prefix sums over the level-major order: fill gaps (levels absent for some systems)
     for (size_t e = 1; e < apPtr.size(); ++e) apPtr[e] = std::max(apPtr[e], apPtr[e - 1]);
     for (size_t e = 1; e < acPtr.size(); ++e) acPtr[e] = std::max(acPtr[e], acPtr[e - 1]);
@@ -902,6 +934,8 @@ int build_dev_amg(rsg_solver* h, const std::vector<SysAmg>& H) {
         (rc = upload(M, &G.diagGlob, dgG, st)) || (rc = upload(M, &G.luPerm, luPerm, st)) ||
         (rc = upload(M, &G.slotSrc, slotSrc, st)) || (rc = upload(M, &G.slotCol, slotCol, st)) || (rc = upload(M, &G.gsRows, gsRows, st)) ||
         (rc = upload(M, reinterpret_cast<int**>(&G.rowMeta), meta, st)) || (rc = upload(M, &G.rowLv, rowLv, st)) || (rc = upload(M, &G.cdesc, cdesc, st)) || (rc = upload(M, &G.gci, gci, st)) ||
+        (rc = upload(M, &G.slabOff, slabOff, st)) || (rc = upload(M, &G.slabCol, slabCol, st)) || (rc = upload(M, &G.slabSrc, slabSrc, st)) ||
+        (rc = dalloc(M, &G.slabVal, slabCol.size())) ||
         (rc = upload(M, &G.wave, wave, st)) || (rc = dalloc(M, &G.gsFlag, size_t(std::max(rows, 1)))) ||
         (rc = dalloc(M, &G.gsWord, 2 * size_t(std::max(rows, 1)))) ||
         (rc = dalloc(M, &G.gsCtr, 4 * size_t(std::max(maxL, 1)))) || (rc = dalloc(M, &G.coarse64, size_t(std::max(nsys, 1)))))
@@ -1016,7 +1050,11 @@ int setup_cpr(rsg_solver* h, const double* acc) {
         return RSG_OK;
     }
     launch_amg_coarse_lu(G, h->opt.precision != RSG_FP64, st);
-    if (h->opt.precision != RSG_FP64) launch_amg_round(G, st);
+    if (h->opt.precision != RSG_FP64) {
+        launch_amg_round(G, st);
+        launch_amg_slabs(G, st);
+        h->launches += G.slabWords ? 1 : 0;
+    }
     if (h->cta) {                                              // row slots of the thread-block application
         launch_amg_slots(G, h->opt.precision != RSG_FP64, st);
         launch_cpr_sp(D, h->val, G, h->opt.precision != RSG_FP64, st);

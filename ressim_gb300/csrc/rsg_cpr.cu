@@ -410,6 +410,14 @@ __global__ void k_round(size_t n, const double* __restrict__ a, float* b) {
     for (size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x; q < n; q += size_t(gridDim.x) * blockDim.x) b[q] = float(a[q]);
 }
 
+// values of the multicolour slabs (a padding word is not read)
+__global__ void k_amg_slabs(size_t n, const int* __restrict__ src, const float* __restrict__ val, float* slab) {
+    for (size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x; q < n; q += size_t(gridDim.x) * blockDim.x) {
+        const int p = __ldg(src + q);
+        slab[q] = p >= 0 ? __ldg(val + p) : 0.0f;
+    }
+}
+
 }  // namespace
 
 void launch_gather_acc(const DevPlan& P, const double* accOrig, double* accLev, cudaStream_t st) {
@@ -530,6 +538,9 @@ void launch_amg_coarse_lu(const DevAmg& G, bool fp32, cudaStream_t st) {
 }
 void launch_amg_round(const DevAmg& G, cudaStream_t st) {
     k_round<<<grid_for(size_t(G.totEnt)), 256, 0, st>>>(size_t(G.totEnt), G.val, G.valf);
+}
+void launch_amg_slabs(const DevAmg& G, cudaStream_t st) {
+    if (G.slabWords) k_amg_slabs<<<grid_for(G.slabWords), 256, 0, st>>>(G.slabWords, G.slabSrc, G.valf, G.slabVal);
 }
 void launch_amg_slots(const DevAmg& G, bool fp32, cudaStream_t st) {
     k_amg_slots<<<grid_for(size_t(G.totSlots) + size_t(G.totRows)), 256, 0, st>>>(G.totSlots, G.totRows, G.slotSrc, G.diagGlob, G.val,

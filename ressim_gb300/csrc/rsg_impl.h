@@ -229,6 +229,12 @@ struct DevAmg {
     // cells that the well Schur fill creates) and are swept together by one sync-free pass.
     int4* cdesc = nullptr;
     int* gci = nullptr;                // global column of every entry (rowOff + local column)
+    // the large colours' rows once more in slabs of 32 rows of cdesc, word u of every row together (rsg_sweep_cta.cu): word 0 the
+    // row (bit 31: it has entries beyond the slab) and its diagonal, then up to kSlabEntries columns (bit 31: a later colour's) and
+    // values; slab g at words 32 slabOff[g] ..
+    int *slabOff = nullptr, *slabCol = nullptr, *slabSrc = nullptr;
+    float* slabVal = nullptr;
+    size_t slabWords = 0;
     std::vector<std::vector<int>> colBeg;
     std::vector<int> colTail;
     std::vector<int> gsBlocks;         // host: persistent grid of the sync-free Gauss-Seidel sweeps of each level
@@ -251,6 +257,9 @@ void launch_gather_acc(const DevPlan& P, const double* accOrig, double* accLev, 
 void launch_amg_refresh(const DevAmg& G, cudaStream_t st);           // Galerkin values of levels >= 1, diagonal fix
 void launch_amg_coarse_lu(const DevAmg& G, bool fp32, cudaStream_t st);     // fp32: the LU in FP32 (luf), else FP64 (lu)
 void launch_amg_round(const DevAmg& G, cudaStream_t st);             // valf = float(val), luf = float(lu)
+constexpr int kSlabEntries = 12;       // off-diagonal entries of a row in its slab; a longer row takes the others from valf
+constexpr int kSlabPad = 0x7fffffff;   // no entry
+void launch_amg_slabs(const DevAmg& G, cudaStream_t st);             // slabVal from valf
 void launch_amg_slots(const DevAmg& G, bool fp32, cudaStream_t st);  // V-cycle row slots from val
 // pressure columns of S in the slot order of the factors (second stage of the CPR application)
 void launch_cpr_sp(const DevPlan& P, const double* val, const DevAmg& G, bool fp32, cudaStream_t st);

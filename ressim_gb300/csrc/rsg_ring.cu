@@ -18,7 +18,7 @@
 //
 // Measured against the sweeps with register lookahead and per-thread staging (rsg_sweep_cta.cu), both sweeps of one
 // application: all FP32, 11,200 rows alone 178 -> 113 us, 1,600 rows 84 -> 43 us, 64 systems of 8,000-14,400 rows
-// 250 -> 234 us (the largest vector leaves the ring 50 KB: one to two steps ahead); FP64, 1,600 rows 232 -> 127 us. What is
+// 250 -> 157 us (the largest vector leaves the ring 50 KB: one to two steps ahead); FP64, 1,600 rows 232 -> 127 us. What is
 // left of a step (0.6 us at 130 rows) is the shared-memory traffic of its records, written once and read once, and the
 // barrier. FP64 vectors of more than about 6,000 rows do not fit and stay with the other sweeps.
 //
@@ -38,8 +38,12 @@ namespace {
 constexpr int kRingWriters = 64;           // writer threads; beside them the consumers and one producer warp
 constexpr int kRingFlight = 16;            // steps in flight at most (mbarriers of the ring)
 constexpr uint32_t kRingHeader = kRingFlight * 32 + 16;   // full and empty mbarriers, step infos, input mbarrier (+ pad)
+// steps between a step's prefetch into L2 and its copy: where the vector leaves the ring room for one wide step only, a copy's
+// latency is on the chain (64 systems of 8,000-14,400 rows, 187 MB of factors an application: 169 -> 157 us)
+constexpr int kRingPrefetch = 6;
 constexpr size_t kRingReserve = 1024;      // shared memory the runtime keeps per block
 // rows of one step at most (a wider level is several steps): one per consumer thread (FP32), or ten per warp (FP64)
+// (FP32 steps of 128 rows would let two fit a short ring: 157 -> 168 us, alone 99 -> 115 us, by the added barriers)
 constexpr int kRingRows32 = 256, kRingRows64 = 120;
 template <class TV> __host__ __device__ constexpr int ring_rows() { return sizeof(TV) == 8 ? kRingRows64 : kRingRows32; }
 template <class TV> __host__ __device__ constexpr int ring_max_threads() { return (sizeof(TV) == 8 ? 384 : 256) + kRingWriters + 32; }
@@ -151,7 +155,17 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
         }
         ByteRing R{smemBytes - uint32_t(ring - sm)};
         int oldest = 0;                                      // steps oldest .. next - 1 hold ring bytes
+        auto prefetch = [&](int step) {
+            if (step >= S) return;
+            const int4 d = desc[step];
+            const bool f = step < nl;
+            const uint32_t n = uint32_t(d.y) & 0xffffu;
+            bulk_prefetch((f ? A.L : A.UD) + size_t(d.x) * (f ? LREC : UREC), n * uint32_t((f ? LREC : UREC) * sizeof(TF)));
+            bulk_prefetch((f ? A.Lslot : A.Uslot) + d.x, 16 * n);
+        };
+        for (int step = 1; step < kRingPrefetch; ++step) prefetch(step);
         for (int next = 0; next < S; ++next) {
+            prefetch(next + kRingPrefetch);
             const int4 d = desc[next];
             const bool f = next < nl;
             const uint32_t n = uint32_t(d.y) & 0xffffu;

@@ -47,6 +47,10 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                  "l"(reinterpret_cast<unsigned long long>(src)), "r"(bytes), "r"(bar)
                  : "memory");
 }
+// the same bytes into L2 only, without waiting
+__device__ __forceinline__ void bulk_prefetch(const void* src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<unsigned long long>(src)), "r"(bytes) : "memory");
+}
 // Byte ring: allocations in order, freed in order; an allocation is contiguous (it wraps to the start when the end is too
 // short). head == tail only when empty.
 struct ByteRing {

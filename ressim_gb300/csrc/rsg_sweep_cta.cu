@@ -1483,55 +1483,93 @@ __global__ void __launch_bounds__(kGridThreads) k_gs_grid(int q0, int q1, int ma
     gs_grid_body<TA, FWD, ZERO, POS>(q0, q1, maxL, phase, rowLv, lv, gsRows, wave, rp, ci, val, diag, b, x, words, totRows, ctr, ks, err);
 }
 
-// Multicolour Gauss-Seidel (FP32 forms) on the colour-major row descriptors {row, first entry, end, diagonal}:
-// the rows of a colour are independent. ZERO: pre-smoothing from x = 0 (the terms of later colours vanish and are
-// not read).
-template <class TA, bool ZERO>
-__device__ __forceinline__ void gs_colour_row(const int4 d, const int* __restrict__ gci, const TA* __restrict__ val,
-                                              const int* __restrict__ wave, const TA* b, TA* x) {
-    const int wi = ZERO ? __ldg(wave + d.x) : 0;
-    TA s = b[d.x];
+// Multicolour Gauss-Seidel (FP32 forms): the rows of a colour are independent, one thread per row. ZERO: pre-smoothing from
+// x = 0 (1: the terms of later colours vanish and are not taken; 2: the first colour, which has no others).
+// Colours alternate along the rows, so reading the rows where they lie in the matrix costs a 32-byte sector for every few entries
+// and a separate line per thread: such a pass over 352,000 rows was bound by its L1 wavefronts (17-20 us, the values 3 us of
+// HBM time). The slabs hold word u of 32 rows together. 64 systems, 742,384 rows, two colours: a post-smoothing pass 17.3 -> 12.5
+// us, the first colour's pre-smoothing pass 18.7 -> 6.3 us. (Issuing the first chunk's loads beside the row's own words costs
+// registers and with them resident blocks: 15.5 us.) What is left is the chain of its four loads.
+template <class TA>
+struct GsSlabs {
+    const int *off, *col;
+    const TA* val;
+    const int4* cdesc;
+    const int *gci, *wave;
+    const TA* all;
+};
+template <class TA, int ZERO>
+__device__ __forceinline__ TA gs_colour_row(const GsSlabs<TA>& W, int i, int w, size_t q, int n, TA s, const TA* x) {
     // entries in chunks whose loads are all issued before the terms are taken (in entry order): a row costs two
     // dependent loads per chunk, not per entry
-    constexpr int CH = 8;
-    for (int p0 = d.y; p0 < d.z; p0 += CH) {
-        int j[CH];
+    constexpr int CH = 6;
+    for (int u0 = 0; u0 < n; u0 += CH) {
+        int c[CH];
         TA a[CH], xv[CH];
-        bool use[CH];
 #pragma unroll
         for (int u = 0; u < CH; ++u) {
-            const int p = p0 + u;
-            use[u] = p < d.z && p != d.w;
-            j[u] = use[u] ? __ldg(gci + p) : 0;
-            a[u] = use[u] ? __ldg(val + p) : TA(0);
+            const size_t at = q + size_t(u0 + u + 1) * 32;
+            c[u] = u0 + u < n ? __ldg(W.col + at) : kSlabPad;
+            a[u] = u0 + u < n ? __ldg(W.val + at) : TA(0);
+            if (ZERO && c[u] < 0) c[u] = kSlabPad;           // x_j still zero
+            c[u] &= 0x7fffffff;
         }
 #pragma unroll
-        for (int u = 0; u < CH; ++u) {
-            if (ZERO && use[u] && __ldg(wave + j[u]) > wi) use[u] = false;   // x_j still zero: the term is not taken
-            xv[u] = use[u] ? x[j[u]] : TA(0);
-        }
+        for (int u = 0; u < CH; ++u) xv[u] = c[u] != kSlabPad ? x[c[u]] : TA(0);
 #pragma unroll
         for (int u = 0; u < CH; ++u)
-            if (use[u]) s = asub(s, amul(a[u], xv[u]));
+            if (c[u] != kSlabPad) s = asub(s, amul(a[u], xv[u]));
     }
-    x[d.x] = adiv(s, __ldg(val + d.w));
+    if (w < 0) {                                             // the row's entries beyond the slab
+        const int4 d = __ldg(W.cdesc + i);
+        const int wi = ZERO ? __ldg(W.wave + d.x) : 0;
+        constexpr int CT = 8;
+        for (int p0 = d.y + kSlabEntries + (d.w - d.y <= kSlabEntries ? 1 : 0); p0 < d.z; p0 += CT) {
+            int j[CT];
+            TA a[CT], xv[CT];
+            bool use[CT];
+#pragma unroll
+            for (int u = 0; u < CT; ++u) {
+                use[u] = p0 + u < d.z && p0 + u != d.w;
+                j[u] = use[u] ? __ldg(W.gci + p0 + u) : 0;
+                a[u] = use[u] ? __ldg(W.all + p0 + u) : TA(0);
+            }
+#pragma unroll
+            for (int u = 0; u < CT; ++u) {
+                if (ZERO && use[u] && __ldg(W.wave + j[u]) > wi) use[u] = false;
+                xv[u] = use[u] ? x[j[u]] : TA(0);
+            }
+#pragma unroll
+            for (int u = 0; u < CT; ++u)
+                if (use[u]) s = asub(s, amul(a[u], xv[u]));
+        }
+    }
+    return s;
 }
-// one large colour: a parallel pass over the descriptors [i0, i1)
-template <class TA, bool ZERO>
-__device__ __forceinline__ void gs_colour_body(int i0, int i1, int maxL, const int4* __restrict__ cdesc, const int* __restrict__ gci,
-                                                   const TA* __restrict__ val, const int* __restrict__ wave, const int* __restrict__ rowLv,
-                                                   const TA* b, TA* x, const KScal* ks) {
-    for (int i = i0 + int(blockIdx.x * blockDim.x + threadIdx.x); i < i1; i += int(gridDim.x * blockDim.x)) {
-        const int4 d = __ldg(cdesc + i);
-        if (ks && ks[__ldg(rowLv + d.x) / maxL].status != ST_RUNNING) continue;
-        gs_colour_row<TA, ZERO>(d, gci, val, wave, b, x);
+// one large colour: the rows [i0, i1) of the colour-major order
+template <class TA, int ZERO>
+__device__ __forceinline__ void gs_colour_body(int i0, int i1, int maxL, const GsSlabs<TA>& W, const int* __restrict__ rowLv, const TA* b,
+                                               TA* x, const KScal* ks) {
+    for (int i = (i0 & ~31) + int(blockIdx.x * blockDim.x + threadIdx.x); i < i1; i += int(gridDim.x * blockDim.x)) {
+        if (i < i0) continue;
+        const int o = __ldg(W.off + i / 32), n = __ldg(W.off + i / 32 + 1) - o - 1;
+        const size_t q = size_t(o) * 32 + size_t(i & 31);
+        const int w = __ldg(W.col + q), row = w & 0x7fffffff;
+        if (ks && ks[__ldg(rowLv + row) / maxL].status != ST_RUNNING) continue;
+        const TA d = __ldg(W.val + q);
+        TA s = b[row];
+        if (ZERO != 2) s = gs_colour_row<TA, ZERO>(W, i, w, q, n, s, x);
+        x[row] = adiv(s, d);
     }
 }
-template <class TA, bool ZERO>
-__global__ void __launch_bounds__(256) k_gs_colour(int i0, int i1, int maxL, const int4* __restrict__ cdesc, const int* __restrict__ gci,
-                                                   const TA* __restrict__ val, const int* __restrict__ wave, const int* __restrict__ rowLv,
-                                                   const TA* b, TA* x, const KScal* ks) {
-    gs_colour_body<TA, ZERO>(i0, i1, maxL, cdesc, gci, val, wave, rowLv, b, x, ks);
+template <class TA, int ZERO>
+__global__ void __launch_bounds__(256) k_gs_colour(int i0, int i1, int maxL, GsSlabs<TA> W, const int* __restrict__ rowLv, const TA* b, TA* x,
+                                                   const KScal* ks) {
+    gs_colour_body<TA, ZERO>(i0, i1, maxL, W, rowLv, b, x, ks);
+}
+template <class TA>
+GsSlabs<TA> gs_slabs(const DevAmg& G, const TA* val) {       // (the schedules of double values are not multicolour)
+    return GsSlabs<TA>{G.slabOff, G.slabCol, reinterpret_cast<const TA*>(G.slabVal), G.cdesc, G.gci, G.wave, val};
 }
 // The small colours (from colour `tail` on) of a level in one sync-free pass. Their rows are the long rows of the
 // well cliques, so a warp takes one row: rows are claimed in colour order (forward ascending, backward
@@ -1862,6 +1900,7 @@ struct VcArgs {
     const AmgSysLv* lv;
     const int4* cdesc;
     const TA* val;
+    GsSlabs<TA> slabs;
     int* gsFlag;
     unsigned long long* gsWord;
     unsigned* gsCtr;
@@ -1908,8 +1947,9 @@ __global__ void __launch_bounds__(256, 4) k_vcycle(const VPhase* __restrict__ ph
             else gcpr_in_body<IN_PLAIN, TA, TT, TT>(A.n, A.rowSys, A.r, A.pv, A.v, A.C.w, A.T, A.C.b, ks);
             break;
         case VP_COLOUR:
-            if (f.c) gs_colour_body<TA, true>(f.a, f.b, A.maxL, A.cdesc, A.gci, A.val, A.wave, A.rowLv, A.C.b, A.C.x, ks);
-            else gs_colour_body<TA, false>(f.a, f.b, A.maxL, A.cdesc, A.gci, A.val, A.wave, A.rowLv, A.C.b, A.C.x, ks);
+            if (f.c == 2) gs_colour_body<TA, 2>(f.a, f.b, A.maxL, A.slabs, A.rowLv, A.C.b, A.C.x, ks);
+            else if (f.c) gs_colour_body<TA, 1>(f.a, f.b, A.maxL, A.slabs, A.rowLv, A.C.b, A.C.x, ks);
+            else gs_colour_body<TA, 0>(f.a, f.b, A.maxL, A.slabs, A.rowLv, A.C.b, A.C.x, ks);
             break;
         case VP_TAIL: {
             unsigned* ctr = A.gsCtr + 4 * f.d;
@@ -2077,7 +2117,7 @@ int cpr_grid(const DevPlan& P, const PrecDev& M, const DevAmg& G, const CprArgs<
     if (M.split && M.vform == 1 && G.nPhases > 0) {
         // the whole pass sequence (input .. t) as the phases of one cooperative launch, then the BILU0 stage
         VcArgs<TA, TT> A{C, n, P.nsys, G.maxL, G.totRows, P.rowSys, P.sysRow0, r, v, pv, Tsplit, G.rowLv, G.gsRows, G.wave, G.rp, G.ci,
-                         G.diag, G.gci, G.agg, G.lv, G.cdesc, val, G.gsFlag, G.gsWord, G.gsCtr, P.Lslot, P.Uslot, P.LovCol, P.UovCol,
+                         G.diag, G.gci, G.agg, G.lv, G.cdesc, val, gs_slabs(G, val), G.gsFlag, G.gsWord, G.gsCtr, P.Lslot, P.Uslot, P.LovCol, P.UovCol,
                          G.coarseChunks};
         cudaMemsetAsync(G.vbar, 0, sizeof(unsigned), st);
         if (G.posOrder) launch_vcycle<TA, TT, true>(G, A, mode, ks, err, st);
@@ -2103,12 +2143,11 @@ int cpr_grid(const DevPlan& P, const PrecDev& M, const DevAmg& G, const CprArgs<
             const int nc = int(cb.size()) - 1, tail = G.colTail[size_t(l)];
             auto big = [&](int c) {
                 const int i0 = cb[size_t(c)], i1 = cb[size_t(c) + 1];
-                if (zero)
-                    k_gs_colour<TA, true><<<grid_for(i1 - i0, 256), 256, 0, st>>>(i0, i1, G.maxL, G.cdesc, G.gci, val, G.wave, G.rowLv, C.b,
-                                                                                 C.x, ks);
-                else
-                    k_gs_colour<TA, false><<<grid_for(i1 - i0, 256), 256, 0, st>>>(i0, i1, G.maxL, G.cdesc, G.gci, val, G.wave, G.rowLv,
-                                                                                  C.b, C.x, ks);
+                const GsSlabs<TA> W = gs_slabs(G, val);
+                const int g = grid_for(i1 - (i0 & ~31), 256);
+                if (zero && c == 0) k_gs_colour<TA, 2><<<g, 256, 0, st>>>(i0, i1, G.maxL, W, G.rowLv, C.b, C.x, ks);
+                else if (zero) k_gs_colour<TA, 1><<<g, 256, 0, st>>>(i0, i1, G.maxL, W, G.rowLv, C.b, C.x, ks);
+                else k_gs_colour<TA, 0><<<g, 256, 0, st>>>(i0, i1, G.maxL, W, G.rowLv, C.b, C.x, ks);
                 ++launches;
             };
             auto small = [&]() {
@@ -2210,7 +2249,7 @@ void vcycle_phases(const DevAmg& G, std::vector<VPhase>& out) {
         const std::vector<int>& cb = G.colBeg[size_t(l)];
         if (cb.size() > 1) {                                  // multicolour: large colours one phase each, the tail in one
             const int nc = int(cb.size()) - 1, tail = G.colTail[size_t(l)];
-            auto big = [&](int c) { out.push_back(VPhase{VP_COLOUR, cb[size_t(c)], cb[size_t(c) + 1], zero ? 1 : 0, 0, 0, 0, 0}); };
+            auto big = [&](int c) { out.push_back(VPhase{VP_COLOUR, cb[size_t(c)], cb[size_t(c) + 1], zero ? (c == 0 ? 2 : 1) : 0, 0, 0, 0, 0}); };
             auto small = [&]() {
                 if (tail < nc) out.push_back(VPhase{VP_TAIL, cb[size_t(tail)], cb[size_t(nc)], tail, l, fwd ? 1 : 0, zero ? 1 : 0, 0});
             };

@@ -89,3 +89,22 @@ def test_batch_of_uneven_systems(precision):
         d.set_batch(mats)
         d.setup()
         assert np.array_equal(d.precond_apply(r), np.concatenate(alone))
+
+
+@pytest.mark.parametrize("precision", ["mixed", "mixed_f32"])
+@pytest.mark.parametrize("form", [1, 2, 3])
+def test_multicolour_slabs_match_the_block_kernel(precision, form):
+    """The large colours' rows in slabs of 32 (a remainder, colours that do not start on a slab, a batch; rows longer than a
+    slab's: cliques of 20 rows, which hold one row of each large colour) give the pre- and post-smoothing of the one-block
+    application, which reads the rows where they lie: bit for bit."""
+    from ressim_gb300.solver import DeviceSolver
+    cliques = [(a, b) for g in range(3) for a in range(100 + 999 * g, 120 + 999 * g) for b in range(a + 1, 120 + 999 * g)]
+    mats = [system(61 * 45 * 2 + k, box(61, 45, 2) + cliques + [(61 * 45 * 2 - 1, 61 * 45 * 2)] * k, seed=5 + k) for k in (0, 1)]
+    r = np.random.default_rng(4).standard_normal(sum(3 * A.n for A in mats))
+    z = []
+    for opt in (dict(sweep="cta"), dict(sweep="split", vcycle_form=form)):
+        with DeviceSolver(precond="cpr", precision=precision, **opt) as d:
+            d.set_batch(mats)
+            d.setup()
+            z.append(d.precond_apply(r))
+    assert np.isfinite(z[0]).all() and np.array_equal(z[0], z[1])
