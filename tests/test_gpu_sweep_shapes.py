@@ -108,3 +108,25 @@ def test_multicolour_slabs_match_the_block_kernel(precision, form):
             d.setup()
             z.append(d.precond_apply(r))
     assert np.isfinite(z[0]).all() and np.array_equal(z[0], z[1])
+
+
+@pytest.mark.parametrize("name", ["star", "arrow", "clique", "two_colours", "long_rows", "slab"])
+def test_grid_sweeps_long_rows(name, oracle):
+    """The grid-wide sweeps at rows around the length from which a whole warp takes a row, and of one and several rounds of 32
+    entries, alone, side by side and dependent on each other within a claim: FP64 and mixed bit for bit the oracle's (and the
+    solve, whose input is fused, converges)."""
+    from ressim_gb300.solver import DeviceSolver
+    long_rows = [(k, 200 + j) for k in range(60) for j in range(5 + k)] + [(k, k + 1) for k in range(60)] + [(a, b) for a in range(300, 340) for b in range(a + 1, 340)]
+    n, pairs = SHAPES.get(name, (345, long_rows))
+    A = system(n, pairs, seed=9)
+    r = np.random.default_rng(7).standard_normal(3 * n)
+    ref = {"fp64": lambda: oracle.bilu0_apply(A, oracle.bilu0_factor(A)[0], r), "mixed": lambda: oracle.bilu0_apply_fd(A, oracle.bilu0_factor_lean(A)[0], r)}
+    for precision in ("fp64", "mixed", "mixed_f32"):
+        with DeviceSolver(precond="bilu0", precision=precision, sweep="grid") as d:
+            d.set_matrix(A)
+            d.setup()
+            z = d.precond_apply(r)
+            x, res = d.solve(r, tol=1e-8, maxit=100)
+            assert res.converged
+        if precision in ref:
+            assert np.array_equal(z, ref[precision]())
