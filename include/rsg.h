@@ -64,10 +64,11 @@ typedef struct rsg_options {
     int device;             /* CUDA device ordinal */
     size_t mem_budget;      /* bytes this handle may hold on the device (0 = no limit) */
     int sweep;              /* BILU0 sweep scheduling: 0 auto, 1 one thread block per system (level barriers,
-                               shared-memory vector), 2 grid-wide sync-free (per-row flags), 3 split CPR: the
-                               V-cycle's passes grid-wide over all systems, the BILU0 sweeps one thread block per
-                               system (same results as 1). Auto takes 3 for CPR on a batch, 1 for a single system and
-                               for BILU0 where the thread-block sweeps apply, else 2 */
+                               shared-memory vector; CPR: the one-kernel application), 2 grid-wide sync-free, 3 split
+                               CPR: the V-cycle's passes grid-wide over all systems, then the BILU0 sweeps (same results
+                               as 1). Auto takes the split form for CPR and, for the BILU0 sweeps, one thread block per
+                               system where the vector fits one SM and does not bind there (FP32; FP64 up to 2,000
+                               rows), else the grid-wide ones */
     int fma;                /* 1 (default): the SpMV accumulates with fused multiply-adds (half the FP64
                                instructions; results within rounding of the reference); 0: the reference's separately
                                rounded products and sums, bit for bit (engine/src/bsr.cpp:109-117) */
@@ -80,7 +81,8 @@ typedef struct rsg_options {
                                one cooperative kernel (grid barriers between them); 2 = every pass grid-wide, one launch
                                per pass; 3 = the finest level's passes grid-wide, the coarser levels one thread block per
                                system in one launch; 0 = tuned (default 3) */
-    int cpr2_threads;       /* split CPR: threads per system of the BILU0 stage, 128, 256 or 512; 0 = tuned (default 256) */
+    int cpr2_threads;       /* split CPR: threads per system of the BILU0 stage, 128, 256 or 512; 0 = the stage
+                               that auto chooses (sweep = 3: tuned among all of them) */
 } rsg_options;
 
 typedef struct rsg_stats {
@@ -233,7 +235,7 @@ int rsg_spmv_dot_noalloc(int n, int nb, const int* d_rowPtr, const int* d_col, c
 /* Statistics of the last setup / solve. */
 int rsg_get_stats(rsg_solver* h, rsg_stats* st);
 
-/* The launch shapes in use after rsg_setup and how they were chosen, as text ("vcycle_form=3 cpr2_threads=256
+/* The launch shapes in use after rsg_setup and how they were chosen, as text ("vcycle_form=3 bilu0=ring
  * source=tuned ..." with the timed candidates), written NUL-terminated into buf (at most len bytes). No counterpart in
  * the reference, whose device kernels have fixed 64-thread groups (app/src/gpu_compute.cpp:57-80). */
 int rsg_tuning(rsg_solver* h, char* buf, int len);

@@ -12,36 +12,6 @@ __device__ __forceinline__ double dm(double a, double b) { return __dmul_rn(a, b
 __device__ __forceinline__ double da(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double ds(double a, double b) { return __dsub_rn(a, b); }
 
-// c = a b   (engine/src/bsr.cpp:26-32: row accumulator, k outer, j inner)
-__device__ __forceinline__ void gemm3(const double* a, const double* b, double* c) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        double r0 = 0, r1 = 0, r2 = 0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const double f = a[i * 3 + k];
-            r0 = da(r0, dm(f, b[k * 3 + 0]));
-            r1 = da(r1, dm(f, b[k * 3 + 1]));
-            r2 = da(r2, dm(f, b[k * 3 + 2]));
-        }
-        c[i * 3 + 0] = r0; c[i * 3 + 1] = r1; c[i * 3 + 2] = r2;
-    }
-}
-// c -= a b  (engine/src/bsr.cpp:33-39)
-__device__ __forceinline__ void gemm3_sub(const double* a, const double* b, double* c) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        double r0 = 0, r1 = 0, r2 = 0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const double f = a[i * 3 + k];
-            r0 = da(r0, dm(f, b[k * 3 + 0]));
-            r1 = da(r1, dm(f, b[k * 3 + 1]));
-            r2 = da(r2, dm(f, b[k * 3 + 2]));
-        }
-        c[i * 3 + 0] = ds(c[i * 3 + 0], r0); c[i * 3 + 1] = ds(c[i * 3 + 1], r1); c[i * 3 + 2] = ds(c[i * 3 + 2], r2);
-    }
-}
 // one row of a 3x3 block times a 3-vector, accumulated from zero left to right
 __device__ __forceinline__ double dot3(const double* a, const double* x) {
     return da(da(dm(a[0], x[0]), dm(a[1], x[1])), dm(a[2], x[2]));
@@ -106,10 +76,6 @@ __device__ int invert_pivot3(double* d) {
     return 1;
 }
 
-__device__ __forceinline__ void load9(const double* p, double* a) {
-#pragma unroll
-    for (int e = 0; e < 9; ++e) a[e] = p[e];
-}
 __device__ __forceinline__ void store9(double* p, const double* a) {
 #pragma unroll
     for (int e = 0; e < 9; ++e) p[e] = a[e];

@@ -1,5 +1,6 @@
 // Thread-block-per-system BILU0 and CPR application: exact natural-order ILU(0) sweeps and the CPR V-cycle for
-// systems that fit one SM.
+// systems that fit one SM, and the passes of the split CPR application. (The BILU0 sweeps of this file run where a launch
+// shape is asked for; otherwise those of rsg_ring.cu and rsg_kernels.cu, which give the same bits sooner.)
 //
 // One thread block owns one system of the (block-diagonal) batch and walks its forward levels with a block
 // barrier between levels, then the same levels in reverse for the backward sweep (valid for the structurally
