@@ -290,8 +290,7 @@ int check_device_errors(rsg_solver* h) {
         if (h->S.yw) cudaMemsetAsync(h->S.yw, 0xff, 2 * size_t(h->plan.n) * NB * sizeof(unsigned long long), h->stream);
         cudaMemsetAsync(h->S.ctr, 0, sizeof(unsigned) * 4, h->stream);
         cudaMemsetAsync(h->R.done, 0, sizeof(unsigned), h->stream);
-        if (h->amg.gsFlag) {
-            cudaMemsetAsync(h->amg.gsFlag, 0, size_t(std::max(h->amg.totRows, 1)) * sizeof(int), h->stream);
+        if (h->amg.gsWord) {
             cudaMemsetAsync(h->amg.gsWord, 0xff, 2 * size_t(std::max(h->amg.totRows, 1)) * sizeof(unsigned long long), h->stream);
             cudaMemsetAsync(h->amg.gsCtr, 0, 4 * size_t(std::max(h->amg.maxL, 1)) * sizeof(unsigned), h->stream);
         }
@@ -936,7 +935,7 @@ int build_dev_amg(rsg_solver* h, const std::vector<SysAmg>& H) {
         (rc = upload(M, reinterpret_cast<int**>(&G.rowMeta), meta, st)) || (rc = upload(M, &G.rowLv, rowLv, st)) || (rc = upload(M, &G.cdesc, cdesc, st)) || (rc = upload(M, &G.gci, gci, st)) ||
         (rc = upload(M, &G.slabOff, slabOff, st)) || (rc = upload(M, &G.slabCol, slabCol, st)) || (rc = upload(M, &G.slabSrc, slabSrc, st)) ||
         (rc = dalloc(M, &G.slabVal, slabCol.size())) ||
-        (rc = upload(M, &G.wave, wave, st)) || (rc = dalloc(M, &G.gsFlag, size_t(std::max(rows, 1)))) ||
+        (rc = upload(M, &G.wave, wave, st)) ||
         (rc = dalloc(M, &G.gsWord, 2 * size_t(std::max(rows, 1)))) ||
         (rc = dalloc(M, &G.gsCtr, 4 * size_t(std::max(maxL, 1)))) || (rc = dalloc(M, &G.coarse64, size_t(std::max(nsys, 1)))))
         return rc;
@@ -955,7 +954,6 @@ int build_dev_amg(rsg_solver* h, const std::vector<SysAmg>& H) {
             (rc = upload(M, &G.dcWorkOff, woff, st)))
             return rc;
     }
-    RSG_CUDA(cudaMemsetAsync(G.gsFlag, 0, size_t(std::max(rows, 1)) * sizeof(int), st));
     RSG_CUDA(cudaMemsetAsync(G.gsWord, 0xff, 2 * size_t(std::max(rows, 1)) * sizeof(unsigned long long), st));
     RSG_CUDA(cudaMemsetAsync(G.gsCtr, 0, 4 * size_t(std::max(maxL, 1)) * sizeof(unsigned), st));
     {

@@ -207,7 +207,7 @@ struct DevAmg {
     float *spf = nullptr, *spLovf = nullptr, *spUovf = nullptr;
     // grid-wide V-cycle (systems too large for one SM): per AMG row its (system, level) descriptor index s*maxL+l and
     // its wave (forward GS level, or colour: adjacent rows of an earlier wave are updated before it in a forward
-    // sweep), sync-free sweep words, flags of the small colours' pass and claim counters (per level and phase -- 0: the
+    // sweep), sync-free sweep words and claim counters (per level and phase -- 0: the
     // smoothing sweeps, 1: the GS solve of a coarsest level without dense LU: forward, backward)
     int* coarse64 = nullptr;           // FP32 forms, per system: 1 = coarsest level solved in FP64 (LU), the FP32 inverse too inexact
     // the GPU-shaped float CPR-AMG (RSG_PREC_CPR_DEVICE): float inverse diagonal of every AMG row, float block-Jacobi
@@ -219,8 +219,7 @@ struct DevAmg {
     size_t* dcWorkOff = nullptr;
     int* rowLv = nullptr;
     int* wave = nullptr;
-    int* gsFlag = nullptr;             // totRows: the small colours' pass
-    unsigned long long* gsWord = nullptr;   // 2 x totRows: forward and backward values of the sync-free sweeps
+    unsigned long long* gsWord = nullptr;   // 2 x totRows: forward and backward values of the sync-free sweeps and of the small colours' pass
     unsigned* gsCtr = nullptr;         // maxL x 4
     std::vector<int> coarseGsLevels;   // host: levels that are some system's coarsest without a dense LU
     // multicolour schedule (FP32 forms), grid-wide: per level the rows of every system that smooths it, colour by

@@ -1574,89 +1574,97 @@ GsSlabs<TA> gs_slabs(const DevAmg& G, const TA* val) {       // (the schedules o
 }
 // The small colours (from colour `tail` on) of a level in one sync-free pass. Their rows are the long rows of the
 // well cliques, so a warp takes one row: rows are claimed in colour order (forward ascending, backward
-// descending), the lanes split the row's entries, poll together the flags of its neighbours of an earlier colour
-// inside the tail (forward; a later one backward) until the whole warp sees them set, then take the terms in entry
-// order. The large colours are done before (forward) or after (backward) by their own passes, so
-// their values are final or old as the multicolour order wants. Flags: 1 after the forward pass, 0 after the
-// backward one; bounded waits (ERR_TIMEOUT).
+// descending), the lanes split the row's entries, poll together the words of its neighbours of an earlier colour
+// inside the tail (forward; a later one backward; values that are their own flags, as in gs_grid_body), then every lane
+// takes the terms in entry order from shared memory, one rounding after another as the thread-per-row passes and the
+// thread-block sweeps do, so a row's value does not depend on which pass took its colour. A term not taken is 0 * 0, which
+// leaves s as it is. The large colours are done before (forward) or after (backward) by their own passes, so their values
+// are final or old as the multicolour order wants. The rows of a clique are a chain: a trip through L2 and a multiply-subtract
+// an entry each. Against flags, with a fence and a second load a row, and the terms broadcast by two shuffles each: 277,000 rows
+// with five 42-layer wells 66 / 56 -> 23 / 21 us (forward / backward, mean of four levels), 64 systems 20 / 18 -> 9 us.
 template <class TA, bool FWD, bool ZERO>
 __device__ __forceinline__ void gs_tail_body(int i0, int i1, int tail, int maxL, const int4* __restrict__ cdesc,
                                                           const int* __restrict__ gci, const TA* __restrict__ val,
                                                           const int* __restrict__ wave, const int* __restrict__ rowLv, const TA* b, TA* x,
-                                                          int* flag, unsigned* ctr, const KScal* ks, int* err) {
+                                                          unsigned long long* words, int totRows, unsigned* ctr, const KScal* ks, int* err) {
+    using U = typename Word<TA>::type;
+    __shared__ TA sh[8][2][32];                               // per warp: factors and values of 32 entries
+    U* wf = reinterpret_cast<U*>(words);
+    U* wb = reinterpret_cast<U*>(words + totRows);
+    U* out = FWD ? wf : wb;
+    U* clear = FWD ? wb : wf;
     if (blockIdx.x == 0 && threadIdx.x == 0) ctr[FWD ? 1 : 0] = 0u;   // the opposite direction's counter, for its next pass
     const int n = i1 - i0, lane = int(threadIdx.x & 31);
-    const int want = FWD ? 1 : 0;
+    TA(*my)[32] = sh[threadIdx.x >> 5];
     for (;;) {
-        unsigned got = 0;
-        if (lane == 0) got = atomicAdd(ctr + (FWD ? 0 : 1), 1u);
-        const int idx = int(__shfl_sync(0xffffffffu, got, 0));
+        const int idx = warp_claim(ctr + (FWD ? 0 : 1), 1);
         if (idx >= n) break;
         const int4 d = __ldg(cdesc + (FWD ? i0 + idx : i1 - 1 - idx));
-        const bool run = !ks || ks[__ldg(rowLv + d.x) / maxL].status == ST_RUNNING;
-        if (run) {
-            const int wi = __ldg(wave + d.x);
-            // this lane's entries: up to four polled at once per round (longer rows: the rest in later passes)
-            for (int p0 = d.y; p0 < d.z; p0 += 128) {
-                int k[4];
-                unsigned pending = 0;
+        if (ks && ks[__ldg(rowLv + d.x) / maxL].status != ST_RUNNING) continue;
+        const int wi = __ldg(wave + d.x);
+        const TA dv = __ldg(val + d.w);
+        TA s = b[d.x];
+        constexpr int CH = 2;                                 // entries of a lane per round
+        for (int p0 = d.y; p0 < d.z; p0 += 32 * CH) {
+            int k[CH];
+            TA a[CH], xv[CH];
+            unsigned pending = 0;
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int p = p0 + lane + 32 * u;
-                    k[u] = -1;
-                    if (p < d.z && p != d.w) {
-                        const int j = __ldg(gci + p);
-                        const int w = __ldg(wave + j);
-                        if (FWD ? (w < wi && w >= tail) : w > wi) { k[u] = j; pending |= 1u << u; }
-                    }
-                }
-                unsigned ns = 0;
-                for (unsigned it = 0;; ++it) {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (((pending >> u) & 1u) && ld_relaxed(flag + k[u]) == want) pending &= ~(1u << u);
-                    if (!__any_sync(0xffffffffu, pending != 0)) break;
-                    if (it >= 64) {
-                        __nanosleep(ns);
-                        ns = ns < 32 ? 32 : (ns < 256 ? 2 * ns : 256);
-                        if (it >= 64 + kSpinLimit) { if (pending) atomicOr(err, ERR_TIMEOUT); break; }
-                        if ((it & 255u) == 255u && *(volatile int*)err != 0) break;
-                    }
-                }
-            }
-            fence_acquire();
-            // s = b - sum a_p x_p in entry order, one rounding after another as the thread-per-row passes and the
-            // thread-block sweeps do (the lanes load a chunk's terms, every lane runs the chain on the broadcasts),
-            // so a row's value does not depend on which pass took its colour
-            TA s = b[d.x];
-            for (int p0 = d.y; p0 < d.z; p0 += 32) {
-                const int p = p0 + lane;
-                TA a = TA(0), xv = TA(0);
-                bool use = false;
+            for (int u = 0; u < CH; ++u) {
+                const int p = p0 + lane + 32 * u;
+                a[u] = xv[u] = TA(0);
+                k[u] = 0;
                 if (p < d.z && p != d.w) {
-                    const int j = __ldg(gci + p);
-                    use = !(ZERO && __ldg(wave + j) > wi);              // x_j still zero: the term is not taken
-                    if (use) { a = __ldg(val + p); xv = x[j]; }
-                }
-                const unsigned m = __ballot_sync(0xffffffffu, use);
-                const int cnt = min(32, d.z - p0);
-                for (int u = 0; u < cnt; ++u) {
-                    const TA au = __shfl_sync(0xffffffffu, a, u), xu = __shfl_sync(0xffffffffu, xv, u);
-                    if ((m >> u) & 1u) s = asub(s, amul(au, xu));
+                    const int j = __ldg(gci + p), w = __ldg(wave + j);
+                    if (FWD ? (w < wi && w >= tail) : w > wi) { k[u] = j; pending |= 1u << u; a[u] = __ldg(val + p); }
+                    else if (!(ZERO && w > wi)) { a[u] = __ldg(val + p); xv[u] = x[j]; }   // (x_j still zero: not taken)
                 }
             }
-            if (lane == 0) x[d.x] = adiv(s, __ldg(val + d.w));
+            unsigned ns = 0;
+            for (unsigned it = 0;; ++it) {
+#pragma unroll
+                for (int u = 0; u < CH; ++u)
+                    if ((pending >> u) & 1u) {
+                        const U got = ld_word(out + k[u]);
+                        if (got != Word<TA>::empty) { xv[u] = Word<TA>::value(got); pending &= ~(1u << u); }
+                    }
+                if (!__any_sync(0xffffffffu, pending != 0)) break;
+                if (it >= 64) {
+                    __nanosleep(ns);
+                    ns = ns < 32 ? 32 : (ns < 256 ? 2 * ns : 256);
+                    bool stop = (it & 255u) == 255u && *(volatile int*)err != 0;
+                    if (it >= 64 + kSpinLimit) { if (pending) atomicOr(err, ERR_TIMEOUT); stop = true; }
+                    if (__any_sync(0xffffffffu, stop)) break;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < CH; ++u) {
+                const int cnt = min(32, d.z - p0 - 32 * u);
+                if (cnt <= 0) break;
+                my[0][lane] = a[u];
+                my[1][lane] = xv[u];
+                __syncwarp();
+                for (int e = 0; e < cnt; e += 8) {
+#pragma unroll
+                    for (int f = 0; f < 8; ++f) s = asub(s, amul(my[0][e + f], my[1][e + f]));
+                }
+                __syncwarp();
+            }
         }
-        __syncwarp();
-        if (lane == 0) st_release(flag + d.x, want);
+        if (lane == 0) {
+            const TA xn = adiv(s, dv);
+            st_word(out + d.x, Word<TA>::make(xn));
+            x[d.x] = xn;
+            clear[d.x] = Word<TA>::empty;
+        }
     }
 }
 template <class TA, bool FWD, bool ZERO>
 __global__ void __launch_bounds__(kGridThreads) k_gs_tail(int i0, int i1, int tail, int maxL, const int4* __restrict__ cdesc,
                                                           const int* __restrict__ gci, const TA* __restrict__ val,
                                                           const int* __restrict__ wave, const int* __restrict__ rowLv, const TA* b, TA* x,
-                                                          int* flag, unsigned* ctr, const KScal* ks, int* err) {
-    gs_tail_body<TA, FWD, ZERO>(i0, i1, tail, maxL, cdesc, gci, val, wave, rowLv, b, x, flag, ctr, ks, err);
+                                                          unsigned long long* words, int totRows, unsigned* ctr, const KScal* ks, int* err) {
+    gs_tail_body<TA, FWD, ZERO>(i0, i1, tail, maxL, cdesc, gci, val, wave, rowLv, b, x, words, totRows, ctr, ks, err);
 }
 
 // r = b - A x on the rows [q0, q1) of one level of every system (engine/src/amg.cpp:321-322: the row sum from
@@ -1902,7 +1910,6 @@ struct VcArgs {
     const int4* cdesc;
     const TA* val;
     GsSlabs<TA> slabs;
-    int* gsFlag;
     unsigned long long* gsWord;
     unsigned* gsCtr;
     const int4 *Lslot, *Uslot;
@@ -1955,11 +1962,11 @@ __global__ void __launch_bounds__(256, 4) k_vcycle(const VPhase* __restrict__ ph
         case VP_TAIL: {
             unsigned* ctr = A.gsCtr + 4 * f.d;
             if (f.e && f.f)
-                gs_tail_body<TA, true, true>(f.a, f.b, f.c, A.maxL, A.cdesc, A.gci, A.val, A.wave, A.rowLv, A.C.b, A.C.x, A.gsFlag, ctr, ks, err);
+                gs_tail_body<TA, true, true>(f.a, f.b, f.c, A.maxL, A.cdesc, A.gci, A.val, A.wave, A.rowLv, A.C.b, A.C.x, A.gsWord, A.totRows, ctr, ks, err);
             else if (f.e)
-                gs_tail_body<TA, true, false>(f.a, f.b, f.c, A.maxL, A.cdesc, A.gci, A.val, A.wave, A.rowLv, A.C.b, A.C.x, A.gsFlag, ctr, ks, err);
+                gs_tail_body<TA, true, false>(f.a, f.b, f.c, A.maxL, A.cdesc, A.gci, A.val, A.wave, A.rowLv, A.C.b, A.C.x, A.gsWord, A.totRows, ctr, ks, err);
             else
-                gs_tail_body<TA, false, false>(f.a, f.b, f.c, A.maxL, A.cdesc, A.gci, A.val, A.wave, A.rowLv, A.C.b, A.C.x, A.gsFlag, ctr, ks,
+                gs_tail_body<TA, false, false>(f.a, f.b, f.c, A.maxL, A.cdesc, A.gci, A.val, A.wave, A.rowLv, A.C.b, A.C.x, A.gsWord, A.totRows, ctr, ks,
                                                err);
             break;
         }
@@ -2118,7 +2125,7 @@ int cpr_grid(const DevPlan& P, const PrecDev& M, const DevAmg& G, const CprArgs<
     if (M.split && M.vform == 1 && G.nPhases > 0) {
         // the whole pass sequence (input .. t) as the phases of one cooperative launch, then the BILU0 stage
         VcArgs<TA, TT> A{C, n, P.nsys, G.maxL, G.totRows, P.rowSys, P.sysRow0, r, v, pv, Tsplit, G.rowLv, G.gsRows, G.wave, G.rp, G.ci,
-                         G.diag, G.gci, G.agg, G.lv, G.cdesc, val, gs_slabs(G, val), G.gsFlag, G.gsWord, G.gsCtr, P.Lslot, P.Uslot, P.LovCol, P.UovCol,
+                         G.diag, G.gci, G.agg, G.lv, G.cdesc, val, gs_slabs(G, val), G.gsWord, G.gsCtr, P.Lslot, P.Uslot, P.LovCol, P.UovCol,
                          G.coarseChunks};
         cudaMemsetAsync(G.vbar, 0, sizeof(unsigned), st);
         if (G.posOrder) launch_vcycle<TA, TT, true>(G, A, mode, ks, err, st);
@@ -2155,17 +2162,16 @@ int cpr_grid(const DevPlan& P, const PrecDev& M, const DevAmg& G, const CprArgs<
                 if (tail >= nc) return;
                 const int i0 = cb[size_t(tail)], i1 = cb[size_t(nc)];
                 const int g = std::max(1, std::min(G.gsBlocks[size_t(l)], (i1 - i0 + kGridThreads / 32 - 1) / (kGridThreads / 32)));
-                int* flag = G.gsFlag;                               // phase-0 flags: unused otherwise on multicolour levels
                 unsigned* ctr = G.gsCtr + 4 * l;
                 if (fwd && zero)
                     k_gs_tail<TA, true, true><<<g, kGridThreads, 0, st>>>(i0, i1, tail, G.maxL, G.cdesc, G.gci, val, G.wave, G.rowLv, C.b,
-                                                                          C.x, flag, ctr, ks, err);
+                                                                          C.x, G.gsWord, G.totRows, ctr, ks, err);
                 else if (fwd)
                     k_gs_tail<TA, true, false><<<g, kGridThreads, 0, st>>>(i0, i1, tail, G.maxL, G.cdesc, G.gci, val, G.wave, G.rowLv, C.b,
-                                                                           C.x, flag, ctr, ks, err);
+                                                                           C.x, G.gsWord, G.totRows, ctr, ks, err);
                 else
                     k_gs_tail<TA, false, false><<<g, kGridThreads, 0, st>>>(i0, i1, tail, G.maxL, G.cdesc, G.gci, val, G.wave, G.rowLv,
-                                                                            C.b, C.x, flag, ctr, ks, err);
+                                                                            C.b, C.x, G.gsWord, G.totRows, ctr, ks, err);
                 ++launches;
             };
             if (fwd) {

@@ -130,3 +130,22 @@ def test_grid_sweeps_long_rows(name, oracle):
             assert res.converged
         if precision in ref:
             assert np.array_equal(z, ref[precision]())
+
+
+@pytest.mark.parametrize("form", [1, 3])
+@pytest.mark.parametrize("size", [31, 65, 150])
+def test_small_colours_match_the_block_kernel(size, form):
+    """Cliques whose rows take one, two and three rounds of the small colours' pass (64 entries a round), one system after
+    another in a batch and over two applications: bit for bit the one-block application's."""
+    from ressim_gb300.solver import DeviceSolver
+    clique = [(a, b) for a in range(50, 50 + size) for b in range(a + 1, 50 + size)]
+    mats = [system(31 * 22 * 2 + k, box(31, 22, 2) + clique + [(31 * 22 * 2 - 1, 31 * 22 * 2)] * k, seed=11 + k) for k in (0, 1)]
+    r = np.random.default_rng(8).standard_normal(sum(3 * A.n for A in mats))
+    z = []
+    for opt in (dict(sweep="cta"), dict(sweep="split", vcycle_form=form)):
+        with DeviceSolver(precond="cpr", precision="mixed_f32", **opt) as d:
+            d.set_batch(mats)
+            d.setup()
+            z.append(d.precond_apply(r))
+            assert np.array_equal(d.precond_apply(r), z[-1])
+    assert np.isfinite(z[0]).all() and np.array_equal(z[0], z[1])
