@@ -709,15 +709,37 @@ __global__ void k_gather_blocks(int nnzb, const int* __restrict__ src, const dou
     for (size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x; q < total; q += size_t(gridDim.x) * blockDim.x)
         b[q] = __ldg(a + size_t(__ldg(src + q / 9)) * 9 + q % 9);
 }
-__global__ void k_gather_vec(int n, const int* __restrict__ perm, const double* __restrict__ orig, double* lev) {
-    const size_t total = size_t(n) * 3;
-    for (size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x; q < total; q += size_t(gridDim.x) * blockDim.x)
-        lev[q] = __ldg(orig + size_t(__ldg(perm + q / 3)) * 3 + q % 3);
+// Four words a thread and round, their loads issued together: a word is two dependent loads (742,384 rows: gather 9.9 -> 9.4 us,
+// scatter 9-10 us either way; a product with both 121.7 -> 120.4 us; 40 MB, 6 us of HBM time).
+template <bool GATHER>
+__device__ __forceinline__ void permute_vec(int n, const int* __restrict__ perm, const double* __restrict__ from, double* to) {
+    const size_t total = size_t(n) * 3, step = size_t(gridDim.x) * blockDim.x;
+    constexpr int U = 4;
+    for (size_t q0 = size_t(blockIdx.x) * blockDim.x + threadIdx.x; q0 < total; q0 += U * step) {
+        size_t at[U];
+        double v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const size_t q = q0 + u * step;
+            const unsigned row = q < total ? unsigned(q / 3) : 0u;
+            at[u] = size_t(__ldg(perm + row)) * 3 + size_t(q - size_t(row) * 3);
+            if (!GATHER && q < total) v[u] = __ldg(from + q);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (GATHER && q0 + u * step < total) v[u] = __ldg(from + at[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const size_t q = q0 + u * step;
+            if (q < total) to[GATHER ? q : at[u]] = v[u];
+        }
+    }
 }
-__global__ void k_scatter_vec(int n, const int* __restrict__ perm, const double* __restrict__ lev, double* orig) {
-    const size_t total = size_t(n) * 3;
-    for (size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x; q < total; q += size_t(gridDim.x) * blockDim.x)
-        orig[size_t(__ldg(perm + q / 3)) * 3 + q % 3] = __ldg(lev + q);
+__global__ void __launch_bounds__(256) k_gather_vec(int n, const int* __restrict__ perm, const double* __restrict__ orig, double* lev) {
+    permute_vec<true>(n, perm, orig, lev);
+}
+__global__ void __launch_bounds__(256) k_scatter_vec(int n, const int* __restrict__ perm, const double* __restrict__ lev, double* orig) {
+    permute_vec<false>(n, perm, lev, orig);
 }
 
 int g_sm_count = 0;
