@@ -40,8 +40,9 @@ constexpr int kSweepThreads = 128;
 // lanes: the row lives in shared memory, nine lanes form the block L_ik, 27 lanes update three target blocks at a time
 // (one element each, the reference's operations in its order), six lanes hold the columns of [D | I] in the inversion, and
 // the blocks of the next entry are on their way while one is eliminated. A thread per row paid every block's loads and
-// arithmetic one after another: 180,000 rows with four 30-layer wells 28 ms, 277,000 rows with five 42-layer wells (lean)
-// 115 ms, 1,600 rows 1.16 ms.
+// arithmetic one after another: 180,000 rows with four 30-layer wells 28 -> 3.4 ms, 277,000 rows with five 42-layer wells
+// (lean) 115 -> 11.9 ms, 11,200 rows 2.82 -> 0.57 ms; FP32, a block per system before, 11,200 rows 2.4 -> 0.47 ms, 64 systems
+// 3.29 -> 2.95 ms.
 constexpr int kFacRow = 40;                  // blocks of a row in shared memory; longer rows work in global memory
 __device__ __forceinline__ double fmul(double a, double b) { return dm(a, b); }
 __device__ __forceinline__ double fadd(double a, double b) { return da(a, b); }
