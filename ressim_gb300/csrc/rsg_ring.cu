@@ -286,6 +286,7 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
         if (R.k >= 0)
             ring_row_load(R, reinterpret_cast<const TF*>(ring + d.x), reinterpret_cast<const int4*>(ring + d.y), t0, e, step < nl);
         R.held = (d.z & 512) != 0;
+        __syncwarp();                                        // (the arrival releases the reads of all lanes, not of lane 0 alone)
         if (!R.held && lane == 0) mbar_arrive(empty + 8 * (step % kRingFlight));
     };
     auto body = [&](Row& R, Row& N, int step) {

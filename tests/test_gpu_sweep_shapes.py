@@ -149,3 +149,29 @@ def test_small_colours_match_the_block_kernel(size, form):
             z.append(d.precond_apply(r))
             assert np.array_equal(d.precond_apply(r), z[-1])
     assert np.isfinite(z[0]).all() and np.array_equal(z[0], z[1])
+
+
+def test_ring_steps_keep_their_records_until_every_lane_has_read_them(oracle):
+    """A step's bytes in the ring are given back only when all lanes of a warp have read theirs: steps whose warps are partly
+    filled and mix rows with and without overflow entries, many more steps than the ring holds, more systems than SMs, applied
+    again and again -- the oracle's bits every time (FP32: the fixed-thread-count kernel's)."""
+    from ressim_gb300.solver import DeviceSolver
+    mats = []
+    for k in range(170):
+        m = 90 + k % 7                                                     # a band with long rows here and there: levels of a few rows
+        pairs = [(i, i + d) for i in range(m) for d in (1, 9, 10) if i + d < m] + [(i, i + 5 + j) for i in range(k % 3, m, 11) for j in range(9) if i + 5 + j < m]
+        mats.append(system(m, pairs, seed=k))
+    r = np.random.default_rng(12).standard_normal(sum(3 * A.n for A in mats))
+    off = np.concatenate([[0], np.cumsum([3 * A.n for A in mats])])
+    z = {}
+    for precision, threads in (("fp64", 0), ("mixed_f32", 0), ("mixed_f32", 256)):
+        with DeviceSolver(precond="bilu0", precision=precision, sweep="cta", cpr2_threads=threads) as d:
+            d.set_batch(mats)
+            d.setup()
+            z[precision, threads] = d.precond_apply(r)
+            for _ in range(20 if not threads else 0):
+                assert np.array_equal(d.precond_apply(r), z[precision, threads])
+    for s, A in enumerate(mats):
+        b = r[off[s]:off[s + 1]]
+        assert np.array_equal(z["fp64", 0][off[s]:off[s + 1]], oracle.bilu0_apply(A, oracle.bilu0_factor(A)[0], b))
+    assert np.array_equal(z["mixed_f32", 0], z["mixed_f32", 256])
