@@ -69,7 +69,7 @@ __device__ __forceinline__ int ov_col(const TF* e) {
 // diagonal; three lanes per row: one block row of each)
 template <class TF, int LPR>
 struct RingRow {
-    int k, ov;                             // row (system; -1: none), offset of the overflow entries in the ring
+    int k, ov;                             // row (system; -1: none), offset of its overflow entries in the ring (-1: none)
     bool held;                             // the step has overflow lists: its ring bytes are read until its end
     int4 c;
     TF a[LPR == 3 ? 9 : 28], D[LPR == 3 ? 3 : 9];
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
     const int d0 = __ldg(A.stepOff + s), S = __ldg(A.stepOff + s + 1) - d0, nl = S / 2;
     const int x0 = XP ? __ldg(&lv[s * maxL].rowOff) : 0;
     // a step in the ring: {record offset, slot column offset, first row (system) << 10 | has overflow entries << 9 | rows,
-    // offset of overflow entry 0}
+    // offset of its first overflow entry}
     int4* info = reinterpret_cast<int4*>(sm + kRingFlight * 16);
     int4* desc = reinterpret_cast<int4*>(sm + kRingHeader);
     // the vector, placed so that it is as far from a 16-byte boundary as its input in global memory (bulk copy)
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
                 R.free_oldest(oldest < next ? uint32_t(info[oldest % kRingFlight].x) : 0);
             }
             info[next % kRingFlight] = make_int4(int(at), int(at + rec), ((d.x - row0) << 10) | (ov ? 512 : 0) | int(n),
-                                                 int(at + rec + 16 * n + xp) - d.z * int(ov_words<TF>() * sizeof(TF)));
+                                                 int(at + rec + 16 * n + xp));
             const uint32_t bar = full + 8 * (next % kRingFlight);
             mbar_expect_tx(bar, bytes);
             uint32_t dst = ringA + at;
@@ -281,10 +281,11 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
         await(step);
         const int4 d = info[step % kRingFlight];
         R.k = mine && !dead && t0 < (d.z & 511) ? (d.z >> 10) + t0 : -1;
-        R.ov = d.w;
+        R.ov = -1;
         R.c.w = -1;
         if (R.k >= 0)
             ring_row_load(R, reinterpret_cast<const TF*>(ring + d.x), reinterpret_cast<const int4*>(ring + d.y), t0, e, step < nl);
+        if (R.c.w >= 0) R.ov = int(ring_entry(uint32_t(d.w), R.c.w, desc[step].z, ov_words<TF>() * uint32_t(sizeof(TF))));
         R.held = (d.z & 512) != 0;
         __syncwarp();                                        // (the arrival releases the reads of all lanes, not of lane 0 alone)
         if (!R.held && lane == 0) mbar_arrive(empty + 8 * (step % kRingFlight));
@@ -318,9 +319,9 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
                     yi[f] = cj >= 0 ? u : yi[f];
                 }
             }
-            if (R.c.w >= 0) {
+            if (R.ov >= 0) {
                 constexpr int OW = int(ov_words<TF>());
-                for (const TF* o = reinterpret_cast<const TF*>(ring + R.ov + R.c.w * OW * int(sizeof(TF)));; o += OW) {
+                for (const TF* o = reinterpret_cast<const TF*>(ring + R.ov);; o += OW) {
                     const int cj = ov_col(o);
                     if (cj < 0) break;
                     const TV w[3] = {y[3 * cj], y[3 * cj + 1], y[3 * cj + 2]};

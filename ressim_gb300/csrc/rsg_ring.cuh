@@ -51,6 +51,11 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 __device__ __forceinline__ void bulk_prefetch(const void* src, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<unsigned long long>(src)), "r"(bytes) : "memory");
 }
+// Ring offset of entry `entry` of a batch-wide list of which a step holds the part from `first` on, at offset `base`. The
+// difference is taken before it is scaled: entry numbers of a whole batch times their bytes do not fit 32 bits.
+__host__ __device__ constexpr uint32_t ring_entry(uint32_t base, int entry, int first, uint32_t entryBytes) {
+    return base + uint32_t(entry - first) * entryBytes;
+}
 // Byte ring: allocations in order, freed in order; an allocation is contiguous (it wraps to the start when the end is too
 // short). head == tail only when empty.
 struct ByteRing {

@@ -32,6 +32,28 @@ def test_library_builds_and_exports_every_declared_symbol():
     assert set(_lib.EXPORTS) <= syms
 
 
+def test_ring_overflow_offsets_of_large_batches(tmp_path):
+    """Offsets of a step's overflow entries in the ring stay exact where entry number times entry size passes 2^31 and 2^32
+    (host evaluation of the function the kernel uses; signed overflow traps)."""
+    import subprocess
+    from ressim_gb300 import _build
+    src = tmp_path / "t.cu"
+    src.write_text("""#include "rsg_ring.cuh"
+#include <climits>
+int main() {
+    for (uint32_t bytes : {48u, 80u})
+        for (int first : {0, 7, 26843545, 44739242, 53687091, INT_MAX - 70000})
+            for (int k : {0, 1, 700, 65534})
+                if (rsg::ring_entry(1024u, first + k, first, bytes) != 1024u + uint32_t(k) * bytes) return 1;
+    return 0;
+}
+""")
+    nvcc = _build._nvcc()
+    subprocess.run([nvcc, *_build.ARCH, "-std=c++17", "-I" + _build.CSRC, "-I" + _build.INCLUDE, "-Xcompiler", "-ftrapv", "-cudart", "static",
+                    "-o", str(tmp_path / "t"), str(src)], check=True, capture_output=True)
+    assert subprocess.run([str(tmp_path / "t")]).returncode == 0
+
+
 def test_create_without_gpu_fails_cleanly():
     from conftest import gpu_available
     if gpu_available():
