@@ -120,8 +120,9 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
     const int row0 = __ldg(A.sysRow0 + s), ns = __ldg(A.sysRow0 + s + 1) - row0;
     const int d0 = __ldg(A.stepOff + s), S = __ldg(A.stepOff + s + 1) - d0, nl = S / 2;
     const int x0 = XP ? __ldg(&lv[s * maxL].rowOff) : 0;
-    // a step in the ring: {record offset, slot column offset, first row (system) << 10 | has overflow entries << 9 | rows,
-    // offset of its first overflow entry}
+    // a step in the ring: offsets of {its records, its slot columns, its corrections, its first overflow entry}. What steers the
+    // warps -- rows and whether there are overflow lists -- is in desc, which does not change: after a wait that ran out `info` may
+    // be another step's, and the lanes must not part
     int4* info = reinterpret_cast<int4*>(sm + kRingFlight * 16);
     int4* desc = reinterpret_cast<int4*>(sm + kRingHeader);
     // the vector, placed so that it is as far from a 16-byte boundary as its input in global memory (bulk copy)
@@ -185,8 +186,7 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
                 ++oldest;
                 R.free_oldest(oldest < next ? uint32_t(info[oldest % kRingFlight].x) : 0);
             }
-            info[next % kRingFlight] = make_int4(int(at), int(at + rec), ((d.x - row0) << 10) | (ov ? 512 : 0) | int(n),
-                                                 int(at + rec + 16 * n + xp));
+            info[next % kRingFlight] = make_int4(int(at), int(at + rec), int(at + rec + 16 * n), int(at + rec + 16 * n + xp));
             const uint32_t bar = full + 8 * (next % kRingFlight);
             mbar_expect_tx(bar, bytes);
             uint32_t dst = ringA + at;
@@ -217,24 +217,28 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
             }
         };
         for (int step = 0; step <= S; ++step) {
-            int4 d = make_int4(0, 0, 0, 0);
+            int m = 0, j0 = 0;
             TX xn[RPT];
             if (step >= nl && step < S) {
                 await(step);
-                if (!dead) d = info[step % kRingFlight];
+                if (!dead) {
+                    const int4 d = desc[step];
+                    m = d.y & 0xffff;
+                    j0 = d.x - row0;
+                }
                 if (XP) {
-                    const uint64_t xa = reinterpret_cast<uint64_t>(x) + uint64_t(x0 + (d.z >> 10)) * sizeof(TX);
-                    const TX* xs = reinterpret_cast<const TX*>(ring + d.y + 16 * (d.z & 511) + (xa & 15));
+                    const uint64_t xa = reinterpret_cast<uint64_t>(x) + uint64_t(x0 + j0) * sizeof(TX);
+                    const TX* xs = reinterpret_cast<const TX*>(ring + (dead ? 0 : info[step % kRingFlight].z) + (xa & 15));
 #pragma unroll
-                    for (int q = 0; q < RPT; ++q) xn[q] = w + q * kRingWriters < (d.z & 511) ? xs[w + q * kRingWriters] : TX(0);
+                    for (int q = 0; q < RPT; ++q) xn[q] = w + q * kRingWriters < m ? xs[w + q * kRingWriters] : TX(0);
                 }
             }
             __syncwarp();
             if (lane == 0 && step < S) mbar_arrive(empty + 8 * (step % kRingFlight));
             step_end();                                      // the step before is final
             store();
-            n = d.z & 511;
-            k0 = d.z >> 10;
+            n = m;
+            k0 = j0;
             if (XP) {
 #pragma unroll
                 for (int q = 0; q < RPT; ++q) xp[q] = xn[q];
@@ -278,15 +282,16 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
     const bool mine = LPR == 1 || lane < 30;
     using Row = RingRow<TF, LPR>;
     auto fetch = [&](Row& R, int step) {
+        const int4 t = desc[step];
         await(step);
         const int4 d = info[step % kRingFlight];
-        R.k = mine && !dead && t0 < (d.z & 511) ? (d.z >> 10) + t0 : -1;
+        R.k = mine && !dead && t0 < (t.y & 0xffff) ? t.x - row0 + t0 : -1;
         R.ov = -1;
         R.c.w = -1;
         if (R.k >= 0)
             ring_row_load(R, reinterpret_cast<const TF*>(ring + d.x), reinterpret_cast<const int4*>(ring + d.y), t0, e, step < nl);
-        if (R.c.w >= 0) R.ov = int(ring_entry(uint32_t(d.w), R.c.w, desc[step].z, ov_words<TF>() * uint32_t(sizeof(TF))));
-        R.held = (d.z & 512) != 0;
+        if (R.c.w >= 0) R.ov = int(ring_entry(uint32_t(d.w), R.c.w, t.z, ov_words<TF>() * uint32_t(sizeof(TF))));
+        R.held = uint32_t(t.y) >> 16 != 0;                   // (the same in every lane)
         __syncwarp();                                        // (the arrival releases the reads of all lanes, not of lane 0 alone)
         if (!R.held && lane == 0) mbar_arrive(empty + 8 * (step % kRingFlight));
     };
