@@ -155,7 +155,8 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
             if (mid) bulk_load(smem_addr(y) + mid0, reinterpret_cast<const unsigned char*>(T) + inByte + mid0, mid, inBar);
         }
         ByteRing R{smemBytes - uint32_t(ring - sm)};
-        int oldest = 0;                                      // steps oldest .. next - 1 hold ring bytes
+        int oldest = 0, next = 0;                            // steps oldest .. next - 1 hold ring bytes
+        auto landed = [&](int step, bool& late) { mbar_wait(full + 8 * (step % kRingFlight), (step / kRingFlight) & 1, late, err); };
         auto prefetch = [&](int step) {
             if (step >= S) return;
             const int4 d = desc[step];
@@ -165,7 +166,7 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
             bulk_prefetch((f ? A.Lslot : A.Uslot) + d.x, 16 * n);
         };
         for (int step = 1; step < kRingPrefetch; ++step) prefetch(step);
-        for (int next = 0; next < S; ++next) {
+        for (; next < S; ++next) {
             prefetch(next + kRingPrefetch);
             const int4 d = desc[next];
             const bool f = next < nl;
@@ -182,10 +183,12 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
             uint32_t at = 0;
             while (next - oldest >= kRingFlight || !R.alloc(bytes, at)) {
                 mbar_wait(empty + 8 * (oldest % kRingFlight), (oldest / kRingFlight) & 1, dead, err);
-                if (dead) return;                            // (the steps not issued are skipped by whoever waits for them)
+                landed(oldest, dead);                        // (a reader whose wait ran out gives the bytes back unread)
+                if (dead) break;                             // (the steps not issued are skipped by whoever waits for them)
                 ++oldest;
                 R.free_oldest(oldest < next ? uint32_t(info[oldest % kRingFlight].x) : 0);
             }
+            if (dead) break;
             info[next % kRingFlight] = make_int4(int(at), int(at + rec), int(at + rec + 16 * n), int(at + rec + 16 * n + xp));
             const uint32_t bar = full + 8 * (next % kRingFlight);
             mbar_expect_tx(bar, bytes);
@@ -197,6 +200,10 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
             if (xp) bulk_load(dst, reinterpret_cast<const void*>(xa), xp, bar);
             if (ov) bulk_load(dst + xp, (f ? A.Lov : A.Uov) + size_t(d.z) * ov_words<TF>(), ov, bar);
         }
+        // the block's shared memory is not given up before its copies have landed, whoever stopped waiting for them
+        bool late = false;
+        for (; oldest < next; ++oldest) landed(oldest, late);
+        if (IN == 0) mbar_wait(inBar, 0, late, err);
         return;
     }
     if (tid >= nc) {                                         // ---- writers
