@@ -69,7 +69,7 @@ __device__ __forceinline__ int ov_col(const TF* e) {
 // diagonal; three lanes per row: one block row of each)
 template <class TF, int LPR>
 struct RingRow {
-    int k, ov;                             // row (system; -1: none), offset of its overflow entries in the ring (-1: none)
+    int k, ov;                             // row (system; -1: none), offset of the step's overflow entries in the ring
     bool held;                             // the step has overflow lists: its ring bytes are read until its end
     int4 c;
     TF a[LPR == 3 ? 9 : 28], D[LPR == 3 ? 3 : 9];
@@ -120,9 +120,8 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
     const int row0 = __ldg(A.sysRow0 + s), ns = __ldg(A.sysRow0 + s + 1) - row0;
     const int d0 = __ldg(A.stepOff + s), S = __ldg(A.stepOff + s + 1) - d0, nl = S / 2;
     const int x0 = XP ? __ldg(&lv[s * maxL].rowOff) : 0;
-    // a step in the ring: offsets of {its records, its slot columns, its corrections, its first overflow entry}. What steers the
-    // warps -- rows and whether there are overflow lists -- is in desc, which does not change: after a wait that ran out `info` may
-    // be another step's, and the lanes must not part
+    // a step in the ring: {record offset, slot column offset, first row (system) << 10 | has overflow entries << 9 | rows,
+    // offset of its first overflow entry}
     int4* info = reinterpret_cast<int4*>(sm + kRingFlight * 16);
     int4* desc = reinterpret_cast<int4*>(sm + kRingHeader);
     // the vector, placed so that it is as far from a 16-byte boundary as its input in global memory (bulk copy)
@@ -142,10 +141,10 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    bool dead = false;
+    int dead = 0;                                            // 1 + the step whose wait ran out
     const int lane = tid & 31;
     auto step_end = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(nc + kRingWriters) : "memory"); };
-    auto await = [&](int step) { mbar_wait(full + 8 * (step % kRingFlight), (step / kRingFlight) & 1, dead, err); };
+    auto await = [&](int step) { mbar_wait(full + 8 * (step % kRingFlight), (step / kRingFlight) & 1, dead, err, step + 1); };
     if (tid >= nc + kRingWriters) {                          // ---- producer: one thread
         if (lane) return;
         if (IN == 0) {                                       // the 16-byte aligned middle of the input
@@ -155,8 +154,7 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
             if (mid) bulk_load(smem_addr(y) + mid0, reinterpret_cast<const unsigned char*>(T) + inByte + mid0, mid, inBar);
         }
         ByteRing R{smemBytes - uint32_t(ring - sm)};
-        int oldest = 0, next = 0;                            // steps oldest .. next - 1 hold ring bytes
-        auto landed = [&](int step, bool& late) { mbar_wait(full + 8 * (step % kRingFlight), (step / kRingFlight) & 1, late, err); };
+        int oldest = 0;                                      // steps oldest .. next - 1 hold ring bytes
         auto prefetch = [&](int step) {
             if (step >= S) return;
             const int4 d = desc[step];
@@ -166,7 +164,7 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
             bulk_prefetch((f ? A.Lslot : A.Uslot) + d.x, 16 * n);
         };
         for (int step = 1; step < kRingPrefetch; ++step) prefetch(step);
-        for (; next < S; ++next) {
+        for (int next = 0; next < S; ++next) {
             prefetch(next + kRingPrefetch);
             const int4 d = desc[next];
             const bool f = next < nl;
@@ -183,13 +181,12 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
             uint32_t at = 0;
             while (next - oldest >= kRingFlight || !R.alloc(bytes, at)) {
                 mbar_wait(empty + 8 * (oldest % kRingFlight), (oldest / kRingFlight) & 1, dead, err);
-                landed(oldest, dead);                        // (a reader whose wait ran out gives the bytes back unread)
-                if (dead) break;                             // (the steps not issued are skipped by whoever waits for them)
+                if (dead) return;                            // (the steps not issued are skipped by whoever waits for them)
                 ++oldest;
                 R.free_oldest(oldest < next ? uint32_t(info[oldest % kRingFlight].x) : 0);
             }
-            if (dead) break;
-            info[next % kRingFlight] = make_int4(int(at), int(at + rec), int(at + rec + 16 * n), int(at + rec + 16 * n + xp));
+            info[next % kRingFlight] = make_int4(int(at), int(at + rec), ((d.x - row0) << 10) | (ov ? 512 : 0) | int(n),
+                                                 int(at + rec + 16 * n + xp));
             const uint32_t bar = full + 8 * (next % kRingFlight);
             mbar_expect_tx(bar, bytes);
             uint32_t dst = ringA + at;
@@ -200,10 +197,6 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
             if (xp) bulk_load(dst, reinterpret_cast<const void*>(xa), xp, bar);
             if (ov) bulk_load(dst + xp, (f ? A.Lov : A.Uov) + size_t(d.z) * ov_words<TF>(), ov, bar);
         }
-        // the block's shared memory is not given up before its copies have landed, whoever stopped waiting for them
-        bool late = false;
-        for (; oldest < next; ++oldest) landed(oldest, late);
-        if (IN == 0) mbar_wait(inBar, 0, late, err);
         return;
     }
     if (tid >= nc) {                                         // ---- writers
@@ -224,28 +217,24 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
             }
         };
         for (int step = 0; step <= S; ++step) {
-            int m = 0, j0 = 0;
+            int4 d = make_int4(0, 0, 0, 0);
             TX xn[RPT];
             if (step >= nl && step < S) {
                 await(step);
-                if (!dead) {
-                    const int4 d = desc[step];
-                    m = d.y & 0xffff;
-                    j0 = d.x - row0;
-                }
+                if (!dead) d = info[step % kRingFlight];
                 if (XP) {
-                    const uint64_t xa = reinterpret_cast<uint64_t>(x) + uint64_t(x0 + j0) * sizeof(TX);
-                    const TX* xs = reinterpret_cast<const TX*>(ring + (dead ? 0 : info[step % kRingFlight].z) + (xa & 15));
+                    const uint64_t xa = reinterpret_cast<uint64_t>(x) + uint64_t(x0 + (d.z >> 10)) * sizeof(TX);
+                    const TX* xs = reinterpret_cast<const TX*>(ring + d.y + 16 * (d.z & 511) + (xa & 15));
 #pragma unroll
-                    for (int q = 0; q < RPT; ++q) xn[q] = w + q * kRingWriters < m ? xs[w + q * kRingWriters] : TX(0);
+                    for (int q = 0; q < RPT; ++q) xn[q] = w + q * kRingWriters < (d.z & 511) ? xs[w + q * kRingWriters] : TX(0);
                 }
             }
             __syncwarp();
             if (lane == 0 && step < S) mbar_arrive(empty + 8 * (step % kRingFlight));
             step_end();                                      // the step before is final
             store();
-            n = m;
-            k0 = j0;
+            n = d.z & 511;
+            k0 = d.z >> 10;
             if (XP) {
 #pragma unroll
                 for (int q = 0; q < RPT; ++q) xp[q] = xn[q];
@@ -288,19 +277,26 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
     const int rw = LPR == 3 ? lane / 3 : lane, e = LPR == 3 ? lane % 3 : 0, t0 = (tid >> 5) * RPW + rw;
     const bool mine = LPR == 1 || lane < 30;
     using Row = RingRow<TF, LPR>;
+    int gate = lane;                                         // 0: gives the warp's bytes back
     auto fetch = [&](Row& R, int step) {
-        const int4 t = desc[step];
         await(step);
-        const int4 d = info[step % kRingFlight];
-        R.k = mine && !dead && t0 < (t.y & 0xffff) ? t.x - row0 + t0 : -1;
-        R.ov = -1;
+        int4 d = info[step % kRingFlight];
+        // After a wait that ran out `info` may be another step's: no rows, and whether the step has lists (which decides the warp
+        // synchronisations that follow) from the step table, as the other lanes see it. The bytes are not given back then:
+        // the producer would reuse them under a copy. (Checks outside this branch -- a vote, `&& !dead` at the arrivals, the
+        // producer waiting for the copies -- cost 0.5 to 2 % of a sweep.)
+        if (dead) {
+            gate = 32;
+            d.z = uint32_t(desc[step].y) >> 16 ? 512 : 0;
+        }
+        R.k = mine && t0 < (d.z & 511) ? (d.z >> 10) + t0 : -1;
+        R.ov = d.w;
         R.c.w = -1;
         if (R.k >= 0)
             ring_row_load(R, reinterpret_cast<const TF*>(ring + d.x), reinterpret_cast<const int4*>(ring + d.y), t0, e, step < nl);
-        if (R.c.w >= 0) R.ov = int(ring_entry(uint32_t(d.w), R.c.w, t.z, ov_words<TF>() * uint32_t(sizeof(TF))));
-        R.held = uint32_t(t.y) >> 16 != 0;                   // (the same in every lane)
+        R.held = (d.z & 512) != 0;
         __syncwarp();                                        // (the arrival releases the reads of all lanes, not of lane 0 alone)
-        if (!R.held && lane == 0) mbar_arrive(empty + 8 * (step % kRingFlight));
+        if (!R.held && gate == 0) mbar_arrive(empty + 8 * (step % kRingFlight));
     };
     auto body = [&](Row& R, Row& N, int step) {
         const bool fwd = step < nl;
@@ -331,9 +327,10 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
                     yi[f] = cj >= 0 ? u : yi[f];
                 }
             }
-            if (R.ov >= 0) {
+            if (R.c.w >= 0) {
                 constexpr int OW = int(ov_words<TF>());
-                for (const TF* o = reinterpret_cast<const TF*>(ring + R.ov);; o += OW) {
+                const uint32_t at = ring_entry(uint32_t(R.ov), R.c.w, desc[step].z, uint32_t(OW * sizeof(TF)));
+                for (const TF* o = reinterpret_cast<const TF*>(ring + at);; o += OW) {
                     const int cj = ov_col(o);
                     if (cj < 0) break;
                     const TV w[3] = {y[3 * cj], y[3 * cj + 1], y[3 * cj + 2]};
@@ -361,7 +358,7 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
         }
         if (held) {
             __syncwarp();
-            if (lane == 0) mbar_arrive(empty + 8 * (step % kRingFlight));
+            if (gate == 0) mbar_arrive(empty + 8 * (step % kRingFlight));
             if (step + 1 < S) fetch(N, step + 1);
         }
     };
@@ -372,6 +369,11 @@ __global__ void __launch_bounds__(ring_max_threads<TV>(), 1) k_ring(RingArgs<TF>
         if (step + 1 < S) body(Q, P, step + 1);
     }
     step_end();                                              // (the writers store the last step)
+    if (dead) {                                              // the block ends after the copies in flight have landed (in order, to the first not issued)
+        int late = 0;
+        if (IN == 0) mbar_wait(inBar, 0, late, err);
+        for (int step = dead - 1; step < S && !late; ++step) mbar_wait(full + 8 * (step % kRingFlight), (step / kRingFlight) & 1, late, err);
+    }
 }
 
 // factors (level-space CSR block order) -> row-major slot records and overflow entries

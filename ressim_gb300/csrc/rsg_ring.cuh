@@ -32,13 +32,13 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 // of the hardware's choosing, so the limit is in clocks). `dead`: an earlier wait of this thread ran out -- the later ones
 // are not waited for, so that the kernel ends.
 constexpr long long kBarClocks = 2000000000ll;
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, bool& dead, int* err) {
+__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, int& dead, int* err, int tag = 1) {
     if (dead || mbar_try(bar, parity)) return;
     const long long t0 = clock64();
     do {
         if (mbar_try(bar, parity)) return;
     } while (clock64() - t0 < kBarClocks);
-    dead = true;
+    dead = tag;
     atomicOr(err, ERR_TIMEOUT);
 }
 // bytes (a multiple of 16) from global memory to shared memory, both 16-byte aligned; completes on the mbarrier
