@@ -132,8 +132,9 @@ __global__ void __launch_bounds__(kSweepThreads) k_factor(int n, int chunk, cons
                     if (it >= 64) {
                         __nanosleep(ns);
                         ns = ns < 32 ? 32 : (ns < 256 ? 2 * ns : 256);
-                        if (it >= 64 + kSpinLimit) { if (pending) atomicOr(err, ERR_TIMEOUT); break; }
-                        if ((it & 255u) == 255u && *(volatile int*)err != 0) break;
+                        bool stop = (it & 255u) == 255u && *(volatile int*)err != 0;
+                        if (it >= 64 + kSpinLimit) { if (pending) atomicOr(err, ERR_TIMEOUT); stop = true; }
+                        if (__any_sync(all, stop)) break;     // (the lanes leave together: they may read *err differently)
                     }
                 }
             }
