@@ -190,8 +190,7 @@ __device__ __noinline__ void dense_lu(const DenseCols<T>& D, int* piv) {
 // cluster launch of a dense factorisation: kDenseCluster blocks per system
 template <class K, class... A>
 void launch_dense(K kernel, int nsys, unsigned smem, cudaStream_t st, A... args) {
-    // (the static shared memory counts too: the opt-in is taken from 24 KB on)
-    if (smem > 24 * 1024) raise_smem_limit(reinterpret_cast<const void*>(kernel), int(std::max(smem, 48u * 1024 + 16)));
+    raise_smem_limit(reinterpret_cast<const void*>(kernel), int(smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(nsys * kDenseCluster));
     cfg.blockDim = dim3(kDenseThreads);

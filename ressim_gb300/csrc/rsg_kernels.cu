@@ -869,18 +869,23 @@ void spmv(const DevPlan& P, const double* val, const double* x, double* y, const
 }
 
 // The dynamic shared-memory opt-in of a kernel is one process-wide value per device: handles on several threads
-// (serving slots) with plans of different sizes only ever raise it, under one lock.
+// (serving slots) with plans of different sizes only ever raise it, under one lock. Without it a launch may have 48 KB of
+// static and dynamic shared memory together (the static part of every kernel here is below 32 KB).
 void raise_smem_limit(const void* fn, int bytes) {
-    if (bytes <= 48 * 1024) return;
+    if (bytes <= 16 * 1024) return;
     static std::mutex mu;
     static std::map<std::pair<int, const void*>, int> lim;
     int dev = 0;
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lk(mu);
-    int& cur = lim[{dev, fn}];
-    if (bytes > cur) {
+    const auto [it, first] = lim.try_emplace({dev, fn}, 0);
+    if (first) {
+        cudaFuncAttributes a{};
+        if (cudaFuncGetAttributes(&a, fn) == cudaSuccess) it->second = std::max(0, 48 * 1024 - int(a.sharedSizeBytes));
+    }
+    if (bytes > it->second) {
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        cur = bytes;
+        it->second = bytes;
     }
 }
 

@@ -1,0 +1,86 @@
+"""Device memory that runs out, and what a set-up reserves: a handle whose budget ends anywhere between its first array and its
+last returns RSG_ENOMEM, and again when the call is repeated, never a solve on part of its arrays; a solve that
+escalates to FP64 sweep vectors allocates nothing."""
+import numpy as np
+import pytest
+
+from test_gpu_sweep_shapes import box, system
+
+pytestmark = pytest.mark.gpu
+
+ENOMEM, ESTATE = -3, -4
+
+
+def code(call):
+    from ressim_gb300._lib import RsgError
+    try:
+        call()
+        return 0
+    except RsgError as e:
+        return e.code
+
+
+FORMS = [dict(precond="bilu0", precision="fp64"), dict(precond="bilu0", precision="mixed"), dict(precond="bilu0", precision="mixed_f32"),
+         dict(precond="cpr", precision="fp64"), dict(precond="cpr", precision="mixed_f32"), dict(precond="cpr", precision="mixed_f32", sweep="split"),
+         dict(precond="cpr", precision="mixed_f32", sweep="cta"), dict(precond="cpr", precision="mixed", sweep="grid"),
+         dict(precond="cpr", precision="mixed_f32", krylov="gmres", restart=10), dict(precond="cpr_device", precision="fp64")]
+
+
+@pytest.mark.parametrize("form", FORMS, ids=lambda f: "-".join(str(v) for v in f.values()))
+def test_budget_that_runs_out(form):
+    from ressim_gb300.solver import DeviceSolver
+    A = system(27 * 17 * 5, box(27, 17, 5), seed=2)                        # 2,295 rows: FP32 on the ring, FP64 vectors grid-wide
+    b = np.random.default_rng(3).standard_normal(3 * A.n)
+    with DeviceSolver(**form) as d:
+        d.set_matrix(A)
+        plan = d.stats().device_bytes
+        d.setup()
+        ready = d.stats().device_bytes
+        ref = d.solve(b, 1e-8, 60)[0]
+        full = d.stats().device_bytes
+    assert plan < ready <= full
+    budgets = sorted({*np.linspace(plan, ready, 40).astype(int).tolist(), *np.linspace(ready, full, 8).astype(int).tolist(), ready - 1, full - 1, full})
+    seen = set()
+    for budget in budgets:
+        with DeviceSolver(**form, mem_budget=budget) as d:
+            d.set_matrix(A)
+            for _ in range(2):
+                rc = code(d.setup)
+                seen.add(rc)
+                if rc:
+                    assert rc == ENOMEM
+                    assert code(lambda: d.solve(b, 1e-8, 60)) == ESTATE
+            if rc == 0:
+                rcs = [code(lambda: d.solve(b, 1e-8, 60)) for _ in range(2)]
+                assert rcs in ([0, 0], [ENOMEM, ENOMEM])
+                assert budget < full or rcs == [0, 0]
+                if not rcs[0]:
+                    assert np.array_equal(d.solve(b, 1e-8, 60)[0], ref)
+    assert seen == {0, ENOMEM}
+
+
+@pytest.mark.parametrize("precond", ["bilu0", "cpr"])
+@pytest.mark.parametrize("sweep", ["auto", "grid", "split", "cta"])
+@pytest.mark.parametrize("shape", [(9, 7, 5), (27, 17, 5), (33, 40, 10)])
+def test_escalation_takes_no_memory(precond, sweep, shape):
+    """Systems below and beyond the length to which FP64 vectors run on the ring, cut off after two iterations: the second
+    attempt with FP64 sweep vectors runs within what the set-up held."""
+    from ressim_gb300.solver import DeviceSolver
+    if precond == "bilu0" and sweep == "split":
+        pytest.skip("a form of CPR")
+    nx, ny, nz = shape
+    A = system(nx * ny * nz, box(nx, ny, nz), seed=4)
+    b = np.random.default_rng(5).standard_normal(3 * A.n)
+    opt = dict(precond=precond, precision="mixed_f32", sweep=sweep)
+    with DeviceSolver(**opt) as d:
+        d.set_matrix(A)
+        d.setup()
+        held = d.stats().device_bytes
+    with DeviceSolver(**opt, mem_budget=held) as d:
+        d.set_matrix(A)
+        d.setup()
+        for _ in range(2):
+            d.setup()
+            x, res = d.solve(b, tol=1e-13, maxit=2)
+            assert not res.converged and d.stats().escalated_systems == 1 and np.isfinite(x).all()
+            assert d.stats().device_bytes == held

@@ -175,3 +175,46 @@ def test_ring_steps_keep_their_records_until_every_lane_has_read_them(oracle):
         b = r[off[s]:off[s + 1]]
         assert np.array_equal(z["fp64", 0][off[s]:off[s + 1]], oracle.bilu0_apply(A, oracle.bilu0_factor(A)[0], b))
     assert np.array_equal(z["mixed_f32", 0], z["mixed_f32", 256])
+
+
+@pytest.mark.parametrize("n", [1880, 1925, 1960, 2000, 2047, 2048, 2049, 2200, 2295, 2340])
+def test_shared_memory_around_the_default_limit(n, oracle):
+    """Systems whose vectors need just under 48 KB of dynamic shared memory, beside the kernels' static part: the one-block
+    sweeps (24 n and 12 n bytes), the split form's stage with its staging buffers, the coarse V-cycle's vectors."""
+    from ressim_gb300.solver import DeviceSolver
+    for m, precision in ((n, "fp64"), (2 * n, "mixed_f32"), (n, "mixed_f32")):
+        nx = 40
+        pairs = [(i, i + 1) for i in range(m - 1) if (i + 1) % nx] + [(i, i + nx) for i in range(m - nx)]
+        A = system(m, pairs, seed=6)
+        r = np.random.default_rng(6).standard_normal(3 * m)
+        z = []
+        for opt in (dict(precond="bilu0", sweep="cta", cpr2_threads=256), dict(precond="bilu0", sweep="cta")):   # (the latter: the ring)
+            with DeviceSolver(precision=precision, **opt) as d:
+                d.set_matrix(A)
+                d.setup()
+                z.append(d.precond_apply(r))
+        assert np.array_equal(z[0], z[1])
+        z = []
+        for opt in [dict(sweep="cta"), dict(sweep="auto")] + [dict(sweep="split", autotune=False, vcycle_form=3, cpr2_threads=t) for t in (128, 256, 512)]:
+            with DeviceSolver(precond="cpr", precision=precision, **opt) as d:
+                d.set_matrix(A)
+                d.setup()
+                z.append(d.precond_apply(r))
+        assert np.isfinite(z[0]).all() and all(np.array_equal(z[0], v) for v in z[1:])
+
+
+@pytest.mark.parametrize("cells", [9900, 10300, 10600, 10900, 11200, 11500])
+def test_coarse_levels_around_the_default_limit(cells):
+    """The same for the levels below the finest of one system, kept in shared memory by the split form (24 bytes a row)."""
+    from ressim_gb300.solver import DeviceSolver
+    ny = cells // 100
+    A = system(20 * ny * 5, box(20, ny, 5), seed=8)
+    r = np.random.default_rng(8).standard_normal(3 * A.n)
+    z = []
+    for form in (3, 2):
+        with DeviceSolver(precond="cpr", vcycle_form=form) as d:
+            d.set_matrix(A)
+            d.setup()
+            z.append(d.precond_apply(r))
+            assert 1700 < d.amg_level_sizes()[0][1:].sum() < 2300
+    assert np.isfinite(z[0]).all() and np.array_equal(z[0], z[1])
