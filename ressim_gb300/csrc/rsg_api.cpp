@@ -73,6 +73,15 @@ struct DevMem {
         blocks.clear();
         bytes = 0;
     }
+    // everything allocated after the first `keep` blocks goes back: arrays that are used together are allocated into locals and
+    // taken over when the last one is there, so that a call after RSG_ENOMEM finds none of them instead of a part
+    int undo(size_t keep, int rc) {
+        for (; blocks.size() > keep; blocks.pop_back()) {
+            cudaFreeAsync(blocks.back().first, st);
+            bytes -= blocks.back().second;
+        }
+        return rc;
+    }
 };
 
 template <class T>
@@ -582,68 +591,76 @@ int do_set_jacobian(rsg_solver* h, int nsys, int nv, const int* nrows, const int
     return RSG_OK;
 }
 
-template <class T>
-int alloc_split(rsg_solver* h, SplitFactors<T>& F) {
+// records of the thread-block sweeps (component-major or ring), all of them or none
+template <class F>
+int alloc_records(rsg_solver* h, F& out, size_t ovWords) {
+    DevMem& M = h->pmem;
+    const size_t keep = M.blocks.size();
+    F f;
     int rc;
-    if ((rc = dalloc(h->pmem, &F.L, size_t(h->dp.n) * LREC)) || (rc = dalloc(h->pmem, &F.UD, size_t(h->dp.n) * UREC)) ||
-        (rc = dalloc(h->pmem, &F.Lov, size_t(h->dp.nLov) * NB2)) || (rc = dalloc(h->pmem, &F.Uov, size_t(h->dp.nUov) * NB2)))
-        return rc;
+    if ((rc = dalloc(M, &f.L, size_t(h->dp.n) * LREC)) || (rc = dalloc(M, &f.UD, size_t(h->dp.n) * UREC)) ||
+        (rc = dalloc(M, &f.Lov, size_t(h->dp.nLov) * ovWords)) || (rc = dalloc(M, &f.Uov, size_t(h->dp.nUov) * ovWords)))
+        return M.undo(keep, rc);
+    out = f;
     return RSG_OK;
 }
-
-template <class T>
-int alloc_ring(rsg_solver* h, RingFactors<T>& F) {
-    const size_t ow = ring_ov_words(sizeof(T) == 4);
+// what the BILU0 stage of a factor kind reads besides the factors, allocated once
+int reserve_stage(rsg_solver* h, int kind) {
+    if (kind == 2) return RSG_OK;
     int rc;
-    if ((rc = dalloc(h->pmem, &F.L, size_t(h->dp.n) * LREC)) || (rc = dalloc(h->pmem, &F.UD, size_t(h->dp.n) * UREC)) ||
-        (rc = dalloc(h->pmem, &F.Lov, size_t(h->dp.nLov) * ow)) || (rc = dalloc(h->pmem, &F.Uov, size_t(h->dp.nUov) * ow)))
-        return rc;
-    return RSG_OK;
+    switch (ilu_stage(h, kind)) {
+    case STAGE_GRID: {                             // the sweeps' word vectors, all words empty
+        if (h->S.yw) return RSG_OK;
+        const size_t words = 2 * size_t(h->plan.n) * NB;
+        unsigned long long* yw = nullptr;
+        if ((rc = dalloc(h->pmem, &yw, words))) return rc;
+        h->S.yw = yw;
+        RSG_CUDA(cudaMemsetAsync(yw, 0xff, words * sizeof(unsigned long long), h->stream));
+        return RSG_OK;
+    }
+    case STAGE_RING:
+        if (kind == 0) return h->r64.L ? RSG_OK : alloc_records(h, h->r64, ring_ov_words(false));
+        return h->r32.L ? RSG_OK : alloc_records(h, h->r32, ring_ov_words(true));
+    default:
+        if (kind == 0) return h->s64.L ? RSG_OK : alloc_records(h, h->s64, NB2);
+        return h->s32.L ? RSG_OK : alloc_records(h, h->s32, NB2);
+    }
 }
 // the thread-block sweeps' records of the current factors, in the layout of the sweeps that will read them
 int pack_factors(rsg_solver* h) {
     const int kind = prec_kind(h), stage = ilu_stage(h, kind);
-    int rc;
-    if (stage == STAGE_GRID) {                     // the CSR factors themselves; the sweeps' word vectors, all words empty
-        if (h->S.yw) return RSG_OK;
-        const size_t words = 2 * size_t(h->plan.n) * NB;
-        if ((rc = dalloc(h->pmem, &h->S.yw, words))) return rc;
-        RSG_CUDA(cudaMemsetAsync(h->S.yw, 0xff, words * sizeof(unsigned long long), h->stream));
-        return RSG_OK;
-    }
+    const int rc = reserve_stage(h, kind);
+    if (rc || stage == STAGE_GRID) return rc;      // (the grid-wide sweeps read the CSR factors themselves)
     if (kind == 0) {
-        if (stage == STAGE_RING) {
-            if (!h->r64.L && (rc = alloc_ring(h, h->r64))) return rc;
-            launch_ring_pack(h->dp, h->lu, h->r64, h->stream);
-        } else {
-            if (!h->s64.L && (rc = alloc_split(h, h->s64))) return rc;
-            launch_pack_f64(h->dp, h->lu, h->s64, h->stream);
-        }
-    } else if (stage == STAGE_RING) {
-        if (!h->r32.L && (rc = alloc_ring(h, h->r32))) return rc;
-        launch_ring_pack(h->dp, h->luf, h->r32, h->stream);
+        if (stage == STAGE_RING) launch_ring_pack(h->dp, h->lu, h->r64, h->stream);
+        else launch_pack_f64(h->dp, h->lu, h->s64, h->stream);
     } else {
-        if (!h->s32.L && (rc = alloc_split(h, h->s32))) return rc;
-        launch_pack_f32(h->dp, h->luf, h->s32, h->stream);
+        if (stage == STAGE_RING) launch_ring_pack(h->dp, h->luf, h->r32, h->stream);
+        else launch_pack_f32(h->dp, h->luf, h->s32, h->stream);
     }
     h->launches += 1;
     return RSG_OK;
 }
 
+// factors, and the storage of every BILU0 stage the solves can reach: the precision form's with FP64 sweep vectors too (a
+// solve that escalates allocates nothing)
 int ensure_precond_storage(rsg_solver* h) {
     const size_t E = size_t(h->plan.nnzb) * NB2;
     int rc;
     if (h->opt.precond == RSG_PREC_CPR_DEVICE) return RSG_OK;    // its arrays live with the hierarchy
     if (h->opt.precond == RSG_PREC_JACOBI) {
         if (!h->dinv && (rc = dalloc(h->pmem, &h->dinv, size_t(h->plan.n) * NB2))) return rc;
-    } else if (h->opt.precision == RSG_MIXED || h->opt.precision == RSG_MIXED_F32) {
+        return RSG_OK;
+    }
+    if (h->opt.precision == RSG_MIXED || h->opt.precision == RSG_MIXED_F32) {
         if (!h->luf && (rc = dalloc(h->pmem, &h->luf, E))) return rc;
         if (!h->work && (rc = dalloc(h->pmem, &h->work, E))) return rc;
         if (h->opt.precision == RSG_MIXED_F32 && !h->V.y32 && (rc = dalloc(h->pmem, &h->V.y32, size_t(h->plan.n) * NB))) return rc;
     } else {
         if (!h->lu && (rc = dalloc(h->pmem, &h->lu, E))) return rc;
     }
-    return RSG_OK;
+    if ((rc = reserve_stage(h, prec_kind(h)))) return rc;
+    return h->opt.precision == RSG_MIXED_F32 ? reserve_stage(h, 1) : RSG_OK;
 }
 
 // Gauss-Seidel schedule of one AMG level: the reference's natural-order sweep as forward levels of its lower
@@ -994,9 +1011,16 @@ int setup_cpr(rsg_solver* h, const double* acc) {
     int rc;
     DevAmg& G = h->amg;
     if (!G.w) {
-        if ((rc = dalloc(h->pmem, &G.w, size_t(P.n) * 3)) || (rc = dalloc(h->pmem, &G.T, size_t(P.n) * 3)) ||
-            (rc = dalloc(h->pmem, &G.acc, size_t(P.n) * 9)) || (rc = dalloc(h->pmem, &h->d_nfb, 1)))
-            return rc;
+        const size_t keep = h->pmem.blocks.size();
+        double *w = nullptr, *T = nullptr, *ac = nullptr;
+        int* nfb = nullptr;
+        if ((rc = dalloc(h->pmem, &w, size_t(P.n) * 3)) || (rc = dalloc(h->pmem, &T, size_t(P.n) * 3)) || (rc = dalloc(h->pmem, &ac, size_t(P.n) * 9)) ||
+            (rc = dalloc(h->pmem, &nfb, 1)))
+            return h->pmem.undo(keep, rc);
+        G.w = w;
+        G.T = T;
+        G.acc = ac;
+        h->d_nfb = nfb;
     }
     const double* accLev = nullptr;
     if (acc) {   // caller's blocks in the original row order, staged through val0 (free after the value gather)
@@ -1036,7 +1060,12 @@ int setup_cpr(rsg_solver* h, const double* acc) {
         for (auto& th : pool) th.join();
         for (int s = 0; s < P.nsys; ++s)
             if (!ok[size_t(s)]) return fail(RSG_EINVAL, "AMG set-up of system " + std::to_string(s) + ": " + errs[size_t(s)]);
-        if ((rc = build_dev_amg(h, H))) return rc;
+        const size_t keep = h->pmem.blocks.size();
+        const DevAmg before = G;
+        if ((rc = build_dev_amg(h, H))) {
+            G = before;
+            return h->pmem.undo(keep, rc);
+        }
         h->haveAmg = true;
     }
     launch_cpr_pressure(D, h->val, G.w, G.val, st);          // level 0 of every system = the block pattern
@@ -1213,6 +1242,7 @@ int do_setup(rsg_solver* h, const double* acc) {
         if (rc == RSG_OK) gen_stats(h->gen, &h->st);
         return rc;
     }
+    h->haveSetup = false;                            // until this set-up has ended: it overwrites what the one before left
     h->escalated = false;
     h->st.escalated_systems = 0;
     const bool amgPrec = h->opt.precond == RSG_PREC_CPR || h->opt.precond == RSG_PREC_CPR_DEVICE;
@@ -1248,8 +1278,10 @@ int do_setup(rsg_solver* h, const double* acc) {
     h->st.setup_ms = ms;
     h->st.regularised_blocks = h->h_pin[2];
     h->st.amg_levels = amgPrec ? h->amgLevels : 0;
+    // (the tuner may have chosen another BILU0 stage: then the storage of that one)
+    if ((rc = tune_shapes(h)) || (h->opt.precision == RSG_MIXED_F32 && h->luf && (rc = reserve_stage(h, 1)))) return rc;
     h->haveSetup = true;
-    return tune_shapes(h);
+    return RSG_OK;
 }
 
 // what a captured graph depends on besides its iteration count: the preconditioner's kind and launch shapes
@@ -1307,13 +1339,14 @@ int run_bicgstab(rsg_solver* h, double tol, int maxIt, bool onlyFailed = false) 
 int ensure_gmres(rsg_solver* h) {
     if (h->gm.V) return RSG_OK;
     const int m = h->opt.restart > 0 ? h->opt.restart : 40;
-    const size_t N = size_t(h->plan.n) * NB;
-    GmState& G = h->gm;
+    const size_t N = size_t(h->plan.n) * NB, keep = h->pmem.blocks.size();
+    GmState G;
     int rc;
     if ((rc = dalloc(h->pmem, &G.V, N * size_t(m + 1))) || (rc = dalloc(h->pmem, &G.Z, N * size_t(m))) || (rc = dalloc(h->pmem, &G.w, N)) ||
         (rc = dalloc(h->pmem, &G.H, gm_stride(m) * size_t(h->plan.nsys))) || (rc = dalloc(h->pmem, &G.inner, 2)))
-        return rc;
+        return h->pmem.undo(keep, rc);
     G.m = m;
+    h->gm = G;
     h->gmExec.assign(size_t(m) + 2, nullptr);
     return RSG_OK;
 }
@@ -1403,9 +1436,12 @@ int escalate(rsg_solver* h, double tol, int maxIt, bool gmres = false) {
         launch_factor_lean(h->dp, h->val, h->luf, h->work, h->S, h->epoch, h->d_nreg, h->d_err, h->stream);
         h->launches += 1;
         h->escalated = true;                       // the FP32 factors with FP64 sweep vectors
-        const int rc = pack_factors(h);
-        if (rc) return rc;
-        RSG_CUDA(cudaGetLastError());
+        int rc = pack_factors(h);
+        if (!rc && cudaGetLastError() != cudaSuccess) rc = fail(RSG_ECUDA, "escalation: launch failed");
+        if (rc) {                                  // the factors are overwritten and nothing reads the new ones: set up again
+            h->escalated = h->haveSetup = false;
+            return rc;
+        }
     }
     h->escalated = true;
     h->st.escalated_systems = failed;
@@ -1447,8 +1483,14 @@ int do_solve_device(rsg_solver* h, const double* d_b, double* d_x, double tol, i
             for (const KScal& k : k0) failed |= k.status != ST_CONV;
             if (failed) {
                 const size_t N = size_t(h->plan.n) * NB;
-                if (!h->xPrev && ((rc = dalloc(h->pmem, &h->xPrev, N)) || (rc = dalloc(h->pmem, &h->ksPrev, size_t(h->plan.nsys)))))
-                    return rc;
+                if (!h->xPrev) {
+                    const size_t keep = h->pmem.blocks.size();
+                    decltype(h->xPrev) x = nullptr;
+                    decltype(h->ksPrev) k = nullptr;
+                    if ((rc = dalloc(h->pmem, &x, N)) || (rc = dalloc(h->pmem, &k, size_t(h->plan.nsys)))) return h->pmem.undo(keep, rc);
+                    h->xPrev = x;
+                    h->ksPrev = k;
+                }
                 RSG_CUDA(cudaMemcpyAsync(h->xPrev, h->V.x, N * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
                 RSG_CUDA(cudaMemcpyAsync(h->ksPrev, h->ks, sizeof(KScal) * size_t(h->plan.nsys), cudaMemcpyDeviceToDevice, h->stream));
                 if ((rc = run_gmres(h, tol, maxIt, true))) return rc;
@@ -1505,9 +1547,16 @@ int do_solve_refined(rsg_solver* h, const double* d_b, double* d_x, double tol, 
     const size_t N = size_t(h->plan.n) * NB;
     const int ns = h->plan.nsys;
     int rc;
-    if (!h->refB && ((rc = dalloc(h->pmem, &h->refB, N)) || (rc = dalloc(h->pmem, &h->refX, N)) || (rc = dalloc(h->pmem, &h->refR, N)) ||
-                     (rc = dalloc(h->pmem, &h->refRel, size_t(ns)))))
-        return rc;
+    if (!h->refB) {
+        const size_t keep = h->pmem.blocks.size();
+        double *b = nullptr, *x = nullptr, *r = nullptr, *rel = nullptr;
+        if ((rc = dalloc(h->pmem, &b, N)) || (rc = dalloc(h->pmem, &x, N)) || (rc = dalloc(h->pmem, &r, N)) || (rc = dalloc(h->pmem, &rel, size_t(ns))))
+            return h->pmem.undo(keep, rc);
+        h->refB = b;
+        h->refX = x;
+        h->refR = r;
+        h->refRel = rel;
+    }
     RSG_CUDA(cudaEventRecord(h->ev0, h->stream));
     launch_gather_vec(h->dp, d_b, h->refB, h->stream);
     RSG_CUDA(cudaMemsetAsync(h->refX, 0, N * sizeof(double), h->stream));

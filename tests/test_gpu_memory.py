@@ -81,6 +81,7 @@ def test_escalation_takes_no_memory(precond, sweep, shape):
         d.setup()
         for _ in range(2):
             d.setup()
+            before = d.stats().device_bytes                                # (at most `held`: shapes tuned before are not tuned again)
             x, res = d.solve(b, tol=1e-13, maxit=2)
             assert not res.converged and d.stats().escalated_systems == 1 and np.isfinite(x).all()
-            assert d.stats().device_bytes == held
+            assert d.stats().device_bytes == before <= held
