@@ -53,7 +53,10 @@ struct DevMem {
         if (n == 0) n = 16;
         if (budget && bytes + n > budget) return fail(RSG_ENOMEM, "device memory budget exhausted");
         cudaError_t e = cudaMallocAsync(p, n, st);
-        if (e != cudaSuccess) return fail(RSG_ENOMEM, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
+        if (e != cudaSuccess) {
+            cudaGetLastError();                              // (reported here; not by the next launch's check)
+            return fail(RSG_ENOMEM, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
+        }
         blocks.push_back({*p, n});
         bytes += n;
         return RSG_OK;
@@ -569,6 +572,7 @@ int do_set_jacobian(rsg_solver* h, int nsys, int nv, const int* nrows, const int
         std::vector<const int*> rpS(static_cast<size_t>(nsys)), ciS(static_cast<size_t>(nsys));
         for (int s = 0; s < nsys; ++s) { rpS[size_t(s)] = W.srp[size_t(s)].data(); ciS[size_t(s)] = W.sci[size_t(s)].data(); }
         if ((rc = set_batch_pattern(h, nsys, nS.data(), rpS.data(), ciS.data(), nnzbs))) return rc;
+        h->wsValues = false;                                 // until its arrays are there again
         h->wsVal.release_all();
         WsDev& D = h->wsd;
         DevMem& M = h->wsVal;

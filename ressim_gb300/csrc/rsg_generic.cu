@@ -658,9 +658,14 @@ namespace {
 template <class T>
 int galloc(GenEngine& g, std::vector<void*>& list, size_t& bytes, T** p, size_t count) {
     const size_t by = std::max<size_t>(count, 1) * sizeof(T);
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(p), by, g.st);
-    if (e != cudaSuccess) return gfail(RSG_ENOMEM, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
-    list.push_back(*p);
+    void* q = nullptr;
+    cudaError_t e = cudaMallocAsync(&q, by, g.st);
+    if (e != cudaSuccess) {
+        cudaGetLastError();                                  // (reported here; not by the next launch's check)
+        return gfail(RSG_ENOMEM, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
+    }
+    *p = static_cast<T*>(q);
+    list.push_back(q);
     bytes += by;
     return RSG_OK;
 }
@@ -874,7 +879,7 @@ void refresh_amg(GenEngine& g) {
 int ensure_krylov(GenEngine& g, bool gmres, int m) {
     const size_t N = size_t(g.n) * g.nb;
     int rc;
-    if (!g.vx) {
+    if (!g.vb) {                                 // (the last of them)
         double** vs[] = {&g.vx, &g.vr, &g.vrh, &g.vp, &g.vv, &g.vs, &g.vt, &g.vph, &g.vsh, &g.vb};
         for (double** v : vs)
             if ((rc = galloc(g, g.pat, g.bytesPat, v, N))) return rc;
@@ -1066,14 +1071,15 @@ int gen_set_matrix(GenEngine* gp, const rsg_options& o, int n, int nb, const int
     const int nnzb = rowPtr[n];
     const bool same = g.haveMatrix && g.n == n && g.nb == nb && g.nnzb == nnzb && std::equal(rowPtr, rowPtr + n + 1, g.rp0.begin()) &&
                       std::equal(col, col + nnzb, g.ci0.begin());
-    if (!g.part) {
+    if (!g.hpin) {                                          // (each by itself: an earlier call may have failed between them)
         int rc;
-        if ((rc = galloc(g, g.pat, g.bytesPat, &g.part, kDotBlocks))) return rc;
-        g.pat.pop_back();                                   // kept across patterns (freed by gen_destroy)
-        if ((rc = galloc(g, g.pat, g.bytesPat, &g.dotOut, 1))) return rc;
-        g.pat.pop_back();
-        if ((rc = galloc(g, g.pat, g.bytesPat, &g.dCnt, 2))) return rc;
-        g.pat.pop_back();
+        auto keep = [&](auto** p, size_t count) {           // kept across patterns (freed by gen_destroy)
+            if (*p) return RSG_OK;
+            const int r = galloc(g, g.pat, g.bytesPat, p, count);
+            if (r == RSG_OK) g.pat.pop_back();
+            return r;
+        };
+        if ((rc = keep(&g.part, kDotBlocks)) || (rc = keep(&g.dotOut, 1)) || (rc = keep(&g.dCnt, 2))) return rc;
         GEN_CUDA(cudaMallocHost(reinterpret_cast<void**>(&g.hpin), 4 * sizeof(double)));
     }
     if (!same) {
@@ -1226,7 +1232,7 @@ int gen_solve_device(GenEngine* gp, const rsg_options& o, const double* d_b, dou
 
 namespace {
 int ensure_staging(GenEngine& g) {
-    if (g.stIn) return RSG_OK;
+    if (g.stOut) return RSG_OK;                // (the last of them)
     const size_t N = size_t(g.n) * g.nb;
     int rc;
     if ((rc = galloc(g, g.pat, g.bytesPat, &g.stIn, N)) || (rc = galloc(g, g.pat, g.bytesPat, &g.stOut, N))) return rc;
