@@ -213,6 +213,34 @@ int upload(DevMem& M, T** d, const std::vector<T>& v, cudaStream_t st, size_t pa
     return RSG_OK;
 }
 
+// How the BILU0 stage of a factor kind (0 FP64, 1 FP32 factors with FP64 vectors, 3 all FP32) runs on systems with a
+// thread-block plan:
+// * on the ring where its vector and steps fit one SM and the arithmetic does not bind it there: all FP32, and FP64 vectors up
+//   to kRingRows64 rows;
+// * else by the grid-wide sweeps, whatever the size: FP64 vectors on one SM are bound by its FP64 pipe;
+// * by the kernels on the component-major records only where the options fix the launch shape (the one-kernel CPR
+//   application, a BILU0 stage of a given thread count) or the tuner, asked for the split form, found them faster.
+// Measured: both sweeps alone, FP64, ring / grid-wide: 1,600 rows 127 / 157 us, 3,300 rows 320 / 205 us, 9,800 rows
+// 724 (component-major) / 387 us; a CPR application, FP64, component-major / grid-wide: 11,200 rows 1.89 / 1.47 ms, 64 systems
+// of 8,000-14,400 rows 4.45 / 3.87 ms; FP32 factors with FP64 vectors: 1.13 / 0.51 and 1.72 / 1.00 ms; all FP32, 25,000 rows
+// (no ring): 0.56 / 0.45 ms.
+constexpr int kRingRows64 = 2000;
+enum { STAGE_CTA = 0, STAGE_RING = 1, STAGE_GRID = 2 };
+// whether a BILU0 stage on the component-major records, or on the ring with vectors of this type, can come up for these options
+bool cta_stage_possible(const rsg_solver* h) { return h->cta && (h->opt.cpr2_threads != 0 || h->opt.sweep == 1 || h->opt.sweep == 3); }
+bool ring_wanted(const rsg_solver* h, bool vec32) {
+    if (h->opt.precond == RSG_PREC_JACOBI || h->opt.precond == RSG_PREC_CPR_DEVICE || h->opt.cpr2_threads != 0) return false;
+    if (h->opt.precond == RSG_PREC_CPR && h->opt.sweep == 1) return false;
+    return vec32 ? h->opt.precision == RSG_MIXED_F32 : h->plan.maxSysRows <= kRingRows64 || h->opt.sweep == 1;
+}
+int ilu_stage(const rsg_solver* h, int kind) {
+    if (!h->cta || kind == 2) return STAGE_GRID;
+    if (h->opt.cpr2_threads != 0 || !h->tune.stage) return STAGE_CTA;
+    if (h->opt.precond == RSG_PREC_CPR && h->opt.sweep == 1) return STAGE_CTA;
+    const bool fits = ring_fits(h->ring[kind == 3 ? 1 : 0], kind != 0, kind == 3);
+    if (fits && (kind == 3 || h->plan.maxSysRows <= kRingRows64 || h->opt.sweep == 1)) return STAGE_RING;
+    return h->opt.sweep == 1 ? STAGE_CTA : STAGE_GRID;
+}
 int alloc_plan(rsg_solver* h) {
     HostPlan& P = h->plan;
     DevMem& M = h->pmem;
@@ -220,6 +248,8 @@ int alloc_plan(rsg_solver* h) {
     DevPlan& D = h->dp;
     cudaStream_t st = h->stream;
     D.n = P.n; D.nnzb = P.nnzb; D.nsys = P.nsys; D.ntiles = int(P.tileSys.size());
+    D.maxSysRows = P.maxSysRows;
+    h->cta = h->opt.sweep != 2 && cta_sweep_supported(D, P);
     int rc;
     if ((rc = upload(M, &D.rowPtr, P.rowPtr, st)) || (rc = upload(M, &D.col, P.col, st)) || (rc = upload(M, &D.diag, P.diag, st)) ||
         (rc = upload(M, &D.ford, P.ford, st)) || (rc = upload(M, &D.bord, P.bord, st)) || (rc = upload(M, &D.elimPtr, P.elimPtr, st)) ||
@@ -227,13 +257,15 @@ int alloc_plan(rsg_solver* h) {
         (rc = upload(M, &D.tileRow0, P.tileRow0, st)) || (rc = upload(M, &D.tileSys, P.tileSys, st)) ||
         (rc = upload(M, &D.sysTile0, P.sysTile0, st)) || (rc = upload(M, &D.sysRow0, P.sysRow0, st)) ||
         (rc = upload(M, &D.perm, P.perm, st)) || (rc = upload(M, &D.valSrc, P.valSrc, st)) ||
-        (rc = upload(M, &D.lvlStart, P.lvlStart, st)) || (rc = upload(M, &D.sysLvl0, P.sysLvl0, st)) ||
+        (rc = upload(M, &D.lvlStart, P.lvlStart, st)) || (rc = upload(M, &D.sysLvl0, P.sysLvl0, st)))
+        return rc;
+    if (h->cta && (                              // the thread-block sweeps' slots
         (rc = upload(M, reinterpret_cast<int**>(&D.Lslot), P.Lslot, st)) || (rc = upload(M, &D.LslotSrc, P.LslotSrc, st)) ||
         (rc = upload(M, &D.LovCol, P.LovCol, st)) || (rc = upload(M, &D.LovSrc, P.LovSrc, st)) ||
         (rc = upload(M, reinterpret_cast<int**>(&D.Uslot), P.Uslot, st)) || (rc = upload(M, &D.UslotSrc, P.UslotSrc, st)) ||
-        (rc = upload(M, &D.UovCol, P.UovCol, st)) || (rc = upload(M, &D.UovSrc, P.UovSrc, st)) || (rc = upload(M, &D.Dsrc, P.Dsrc, st)))
+        (rc = upload(M, &D.UovCol, P.UovCol, st)) || (rc = upload(M, &D.UovSrc, P.UovSrc, st)) || (rc = upload(M, &D.Dsrc, P.Dsrc, st))))
         return rc;
-    {   // (first row, rows) of every row's forward level: the component-major layout of the sweep records
+    if (cta_stage_possible(h)) {   // (first row, rows) of every row's forward level: the component-major layout of the sweep records
         std::vector<int> rl(size_t(P.n) * 2, 0);
         for (int sy = 0; sy < P.nsys; ++sy)
             for (int q = P.sysLvl0[size_t(sy)]; q + 1 < P.sysLvl0[size_t(sy) + 1]; ++q)
@@ -246,29 +278,28 @@ int alloc_plan(rsg_solver* h) {
     D.spmvFma = h->opt.fma != 0;
     D.nLov = int(P.LovCol.size());
     D.nUov = int(P.UovCol.size());
-    D.maxSysRows = P.maxSysRows;
     {
         int maxLv = 1;
         for (int s = 0; s < P.nsys; ++s) maxLv = std::max(maxLv, P.sysLvl0[size_t(s) + 1] - P.sysLvl0[size_t(s)] - 1);
         D.avgLevelRows = double(P.n) / double(std::max(1, P.nlevF));
         D.sweepBlocks = sweep_blocks_for(double(P.n) / double(maxLv), h->opt.sweep_inflight);
     }
-    h->cta = h->opt.sweep != 2 && cta_sweep_supported(D, P);
     if ((h->opt.sweep == 1 || h->opt.sweep == 3) && !h->cta)
         return fail(RSG_EINVAL, "thread-block sweeps need a structurally symmetric pattern of <= 32768 block rows per system");
     // CPR on the thread-block path: for a batch, the V-cycle's passes grid-wide (all systems at once, the whole
     // GPU's loads in flight); a single system keeps the one-kernel form (one launch per application instead of a
     // launch per pass). Both give the same results bit for bit, so a system's result does not depend on its batch.
     h->splitCpr = h->cta && (h->opt.sweep == 3 || (h->opt.sweep == 0 && P.nsys > 1));
-    for (int v32 = 0; v32 < 2 && h->cta; ++v32) {
+    for (int v32 = 0; v32 < 2 && h->cta; ++v32) {           // the steps of the ring sweeps, where ilu_stage can ask for them
+        if (!ring_wanted(h, v32 != 0)) continue;
         RingHost H;
         ring_steps(P, v32 != 0, H);
-        if (H.ok) {
-            RingDev& R = h->ring[v32];
-            if ((rc = upload(M, &R.desc, H.desc, st)) || (rc = upload(M, &R.stepOff, H.stepOff, st))) return rc;
-            R.maxSteps = H.maxSteps; R.maxRows = H.maxRows; R.maxWidth = H.maxWidth;
-            R.maxStage32 = H.maxStage32; R.maxStage64 = H.maxStage64;
-        }
+        RingDev R;
+        R.maxSteps = H.maxSteps; R.maxRows = H.maxRows; R.maxWidth = H.maxWidth;
+        R.maxStage32 = H.maxStage32; R.maxStage64 = H.maxStage64;
+        if (!H.ok || !ring_fits(R, h->opt.precision != RSG_FP64, v32 != 0)) continue;
+        if ((rc = upload(M, &R.desc, H.desc, st)) || (rc = upload(M, &R.stepOff, H.stepOff, st))) return rc;
+        h->ring[v32] = R;
     }
     const size_t N = size_t(P.n) * NB, E = size_t(P.nnzb) * NB2;
     if ((rc = dalloc(M, &h->val, E)) || (rc = dalloc(M, &h->val0, E)) || (rc = dalloc(M, &h->b, N)) || (rc = dalloc(M, &h->xout, N)) ||
@@ -303,7 +334,7 @@ int check_device_errors(rsg_solver* h) {
         cudaMemsetAsync(h->S.ctr, 0, sizeof(unsigned) * 4, h->stream);
         cudaMemsetAsync(h->R.done, 0, sizeof(unsigned), h->stream);
         if (h->amg.gsWord) {
-            cudaMemsetAsync(h->amg.gsWord, 0xff, 2 * size_t(std::max(h->amg.totRows, 1)) * sizeof(unsigned long long), h->stream);
+            cudaMemsetAsync(h->amg.gsWord, 0xff, h->amg.gsWordBytes, h->stream);
             cudaMemsetAsync(h->amg.gsCtr, 0, 4 * size_t(std::max(h->amg.maxL, 1)) * sizeof(unsigned), h->stream);
         }
         cudaStreamSynchronize(h->stream);
@@ -320,27 +351,6 @@ int precond_launches(const PrecDev& M) {
     return (M.cpr || M.cta || M.kind == 2) && !M.gridIlu ? 1 : 2;
 }
 
-// How the BILU0 stage of a factor kind (0 FP64, 1 FP32 factors with FP64 vectors, 3 all FP32) runs on systems with a
-// thread-block plan:
-// * on the ring where its vector and steps fit one SM and the arithmetic does not bind it there: all FP32, and FP64 vectors up
-//   to kRingRows64 rows;
-// * else by the grid-wide sweeps, whatever the size: FP64 vectors on one SM are bound by its FP64 pipe;
-// * by the kernels on the component-major records only where the options fix the launch shape (the one-kernel CPR
-//   application, a BILU0 stage of a given thread count) or the tuner, asked for the split form, found them faster.
-// Measured: both sweeps alone, FP64, ring / grid-wide: 1,600 rows 127 / 157 us, 3,300 rows 320 / 205 us, 9,800 rows
-// 724 (component-major) / 387 us; a CPR application, FP64, component-major / grid-wide: 11,200 rows 1.89 / 1.47 ms, 64 systems
-// of 8,000-14,400 rows 4.45 / 3.87 ms; FP32 factors with FP64 vectors: 1.13 / 0.51 and 1.72 / 1.00 ms; all FP32, 25,000 rows
-// (no ring): 0.56 / 0.45 ms.
-constexpr int kRingRows64 = 2000;
-enum { STAGE_CTA = 0, STAGE_RING = 1, STAGE_GRID = 2 };
-int ilu_stage(const rsg_solver* h, int kind) {
-    if (!h->cta || kind == 2) return STAGE_GRID;
-    if (h->opt.cpr2_threads != 0 || !h->tune.stage) return STAGE_CTA;
-    if (h->opt.precond == RSG_PREC_CPR && h->opt.sweep == 1) return STAGE_CTA;
-    const bool fits = ring_fits(h->ring[kind == 3 ? 1 : 0], kind != 0, kind == 3);
-    if (fits && (kind == 3 || h->plan.maxSysRows <= kRingRows64 || h->opt.sweep == 1)) return STAGE_RING;
-    return h->opt.sweep == 1 ? STAGE_CTA : STAGE_GRID;
-}
 int prec_kind(const rsg_solver* h) {
     if (h->opt.precond == RSG_PREC_JACOBI) return 2;
     if (h->opt.precision == RSG_MIXED) return 1;
@@ -658,8 +668,8 @@ int ensure_precond_storage(rsg_solver* h) {
     }
     if (h->opt.precision == RSG_MIXED || h->opt.precision == RSG_MIXED_F32) {
         if (!h->luf && (rc = dalloc(h->pmem, &h->luf, E))) return rc;
-        if (!h->work && (rc = dalloc(h->pmem, &h->work, E))) return rc;
-        if (h->opt.precision == RSG_MIXED_F32 && !h->V.y32 && (rc = dalloc(h->pmem, &h->V.y32, size_t(h->plan.n) * NB))) return rc;
+        if (h->plan.maxRowBlocks > kFacRow && !h->work && (rc = dalloc(h->pmem, &h->work, E))) return rc;
+        if (h->opt.precision == RSG_MIXED_F32 && cta_stage_possible(h) && !h->V.y32 && (rc = dalloc(h->pmem, &h->V.y32, size_t(h->plan.n) * NB))) return rc;
     } else {
         if (!h->lu && (rc = dalloc(h->pmem, &h->lu, E))) return rc;
     }
@@ -712,6 +722,8 @@ int build_dev_amg(rsg_solver* h, const std::vector<SysAmg>& H) {
     for (const auto& s : H) maxL = std::max(maxL, int(s.lv.size()));
     G.nsys = nsys;
     G.maxL = maxL;
+    // which of the arrays this form reads
+    const bool devcpr = h->opt.precond == RSG_PREC_CPR_DEVICE, f32 = h->opt.precision != RSG_FP64, slotted = h->cta && !devcpr;
     std::vector<AmgSysLv> lv(size_t(nsys) * maxL);
     const bool mc = h->opt.precision != RSG_FP64;
     std::vector<std::vector<int>> schRows(size_t(nsys) * maxL), schStart(size_t(nsys) * maxL);
@@ -913,7 +925,7 @@ int build_dev_amg(rsg_solver* h, const std::vector<SysAmg>& H) {
     std::vector<int> slabOff(nslab + 1, 0), slabCol, slabSrc;
     {
         std::vector<char> big(cdesc.size(), 0);
-        for (int l = 0; l < maxL; ++l)
+        for (int l = 0; l < maxL && !devcpr; ++l)
             if (G.colTail[size_t(l)] > 0)
                 std::fill(big.begin() + G.colBeg[size_t(l)][0], big.begin() + G.colBeg[size_t(l)][size_t(G.colTail[size_t(l)])], char(1));
         auto kept = [&](size_t i) { return std::min(cdesc[i].z - cdesc[i].y - 1, kSlabEntries); };
@@ -952,12 +964,10 @@ int build_dev_amg(rsg_solver* h, const std::vector<SysAmg>& H) {
         (rc = upload(M, &G.memPtr, memPtr, st)) || (rc = upload(M, &G.mem, mem, st)) || (rc = upload(M, &G.apPtr, apPtr, st)) ||
         (rc = upload(M, &G.apSrc, apSrc, st)) || (rc = upload(M, &G.acPtr, acPtr, st)) || (rc = upload(M, &G.acSrc, acSrc, st)) ||
         (rc = upload(M, &G.diagGlob, dgG, st)) || (rc = upload(M, &G.luPerm, luPerm, st)) ||
-        (rc = upload(M, &G.slotSrc, slotSrc, st)) || (rc = upload(M, &G.slotCol, slotCol, st)) || (rc = upload(M, &G.gsRows, gsRows, st)) ||
-        (rc = upload(M, reinterpret_cast<int**>(&G.rowMeta), meta, st)) || (rc = upload(M, &G.rowLv, rowLv, st)) || (rc = upload(M, &G.cdesc, cdesc, st)) || (rc = upload(M, &G.gci, gci, st)) ||
+        (rc = upload(M, &G.gsRows, gsRows, st)) || (rc = upload(M, &G.rowLv, rowLv, st)) || (rc = upload(M, &G.cdesc, cdesc, st)) || (rc = upload(M, &G.gci, gci, st)) ||
         (rc = upload(M, &G.slabOff, slabOff, st)) || (rc = upload(M, &G.slabCol, slabCol, st)) || (rc = upload(M, &G.slabSrc, slabSrc, st)) ||
         (rc = dalloc(M, &G.slabVal, slabCol.size())) ||
         (rc = upload(M, &G.wave, wave, st)) ||
-        (rc = dalloc(M, &G.gsWord, 2 * size_t(std::max(rows, 1)))) ||
         (rc = dalloc(M, &G.gsCtr, 4 * size_t(std::max(maxL, 1)))) || (rc = dalloc(M, &G.coarse64, size_t(std::max(nsys, 1)))))
         return rc;
     RSG_CUDA(cudaMemsetAsync(G.coarse64, 0, size_t(std::max(nsys, 1)) * sizeof(int), st));
@@ -975,24 +985,37 @@ int build_dev_amg(rsg_solver* h, const std::vector<SysAmg>& H) {
             (rc = upload(M, &G.dcWorkOff, woff, st)))
             return rc;
     }
-    RSG_CUDA(cudaMemsetAsync(G.gsWord, 0xff, 2 * size_t(std::max(rows, 1)) * sizeof(unsigned long long), st));
+    if (!devcpr) {
+        G.gsWordBytes = 2 * size_t(std::max(rows, 1)) * (f32 ? sizeof(float) : sizeof(double));
+        if ((rc = dalloc(M, &G.gsWord, (G.gsWordBytes + 7) / 8))) return rc;
+        RSG_CUDA(cudaMemsetAsync(G.gsWord, 0xff, G.gsWordBytes, st));
+    }
     RSG_CUDA(cudaMemsetAsync(G.gsCtr, 0, 4 * size_t(std::max(maxL, 1)) * sizeof(unsigned), st));
     {
         const size_t S = size_t(std::max(slots, 1)), R = size_t(std::max(rows, 1)), n = size_t(h->plan.n);
         const size_t nLo = size_t(h->dp.nLov) * 3, nUo = size_t(h->dp.nUov) * 3;
-        if ((rc = dalloc(M, &G.slotVal, S)) || (rc = dalloc(M, &G.slotValf, S)) || (rc = dalloc(M, &G.diagVal, R)) ||
-            (rc = dalloc(M, &G.diagValf, R)) || (rc = dalloc(M, &G.cin, size_t(std::max(lurows, 1)))) ||
-            (rc = dalloc(M, &G.sp, n * SPREC)) || (rc = dalloc(M, &G.spf, n * SPREC)) || (rc = dalloc(M, &G.spLov, nLo)) ||
-            (rc = dalloc(M, &G.spLovf, nLo)) || (rc = dalloc(M, &G.spUov, nUo)) || (rc = dalloc(M, &G.spUovf, nUo)))
+        if ((rc = dalloc(M, &G.cin, size_t(std::max(lurows, 1))))) return rc;
+        if (slotted && ((rc = upload(M, &G.slotSrc, slotSrc, st)) || (rc = upload(M, &G.slotCol, slotCol, st)) ||
+                        (rc = upload(M, reinterpret_cast<int**>(&G.rowMeta), meta, st))))
+            return rc;
+        if (slotted && f32 &&
+            ((rc = dalloc(M, &G.slotValf, S)) || (rc = dalloc(M, &G.diagValf, R)) || (rc = dalloc(M, &G.spf, n * SPREC)) ||
+             (rc = dalloc(M, &G.spLovf, nLo)) || (rc = dalloc(M, &G.spUovf, nUo))))
+            return rc;
+        if (slotted && !f32 &&
+            ((rc = dalloc(M, &G.slotVal, S)) || (rc = dalloc(M, &G.diagVal, R)) || (rc = dalloc(M, &G.sp, n * SPREC)) ||
+             (rc = dalloc(M, &G.spLov, nLo)) || (rc = dalloc(M, &G.spUov, nUo))))
             return rc;
     }
     RSG_CUDA(cudaMemcpyAsync(G.lv, lv.data(), lv.size() * sizeof(AmgSysLv), cudaMemcpyHostToDevice, st));
-    if ((rc = dalloc(M, &G.val, size_t(ents) + OV_CHUNK - 1)) || (rc = dalloc(M, &G.valf, size_t(ents) + OV_CHUNK - 1)) || (rc = dalloc(M, &G.apVal, size_t(std::max(aps, 1)))) ||
-        (rc = dalloc(M, &G.lu, size_t(std::max(lus, 1)))) || (rc = dalloc(M, &G.luf, size_t(std::max(lus, 1)))) ||
-        (rc = dalloc(M, &G.invf, size_t(std::max(lus, 1)))) ||
-        (rc = dalloc(M, &G.piv, size_t(std::max(lurows, 1)))) || (rc = dalloc(M, &G.x, size_t(rows) + 2)) || (rc = dalloc(M, &G.b, size_t(rows))) ||
-        (rc = dalloc(M, &G.r, size_t(rows))) || (rc = dalloc(M, &G.xf, size_t(rows) + 4)) || (rc = dalloc(M, &G.bf, size_t(rows))) ||
-        (rc = dalloc(M, &G.rf, size_t(rows))))
+    if ((rc = dalloc(M, &G.val, size_t(ents) + OV_CHUNK - 1)) || (rc = dalloc(M, &G.apVal, size_t(std::max(aps, 1)))) ||
+        (rc = dalloc(M, &G.lu, size_t(std::max(lus, 1)))) || (rc = dalloc(M, &G.piv, size_t(std::max(lurows, 1)))) ||
+        (rc = dalloc(M, &G.x, size_t(rows) + 2)) || (rc = dalloc(M, &G.b, size_t(rows))) || (rc = dalloc(M, &G.r, size_t(rows))))
+        return rc;
+    if ((f32 || devcpr) &&
+        ((rc = dalloc(M, &G.valf, size_t(ents) + OV_CHUNK - 1)) || (rc = dalloc(M, &G.luf, size_t(std::max(lus, 1)))) ||
+         (rc = dalloc(M, &G.invf, size_t(std::max(lus, 1)))) || (rc = dalloc(M, &G.xf, size_t(rows) + 4)) || (rc = dalloc(M, &G.bf, size_t(rows))) ||
+         (rc = dalloc(M, &G.rf, size_t(rows)))))
         return rc;
     // the fused V-cycle's phase table and barrier counter (the split CPR form)
     {
@@ -1144,6 +1167,21 @@ bool fused_capturable(rsg_solver* h, const double* d_r, double* d_z) {
     return ok;
 }
 
+// the records of BILU0 stages other than the present shape's go back (one set at a time; the word vectors stay)
+void drop_records(rsg_solver* h) {
+    auto drop = [&](auto& f) {
+        for (void* p : {(void*)f.L, (void*)f.UD, (void*)f.Lov, (void*)f.Uov}) h->pmem.release(p);
+        f = {};
+    };
+    bool cta = false, ring = false;
+    for (int kind : {prec_kind(h), h->opt.precision == RSG_MIXED_F32 ? 1 : prec_kind(h)}) {
+        cta = cta || ilu_stage(h, kind) == STAGE_CTA;
+        ring = ring || ilu_stage(h, kind) == STAGE_RING;
+    }
+    if (!cta) { drop(h->s64); drop(h->s32); }
+    if (!ring) { drop(h->r64); drop(h->r32); }
+}
+
 int tune_shapes(rsg_solver* h) {
     rsg_solver::Tune t;
     const bool cprCta = h->opt.precond == RSG_PREC_CPR && h->cta && h->haveAmg;
@@ -1167,9 +1205,13 @@ int tune_shapes(rsg_solver* h) {
     // a shape is taken: the records its BILU0 stage reads are packed if they are not yet
     auto take = [&](const rsg_solver::Tune& c) {
         const bool repack = own && c.stage != packed;
-        packed = c.stage;
         h->tune = c;
-        return repack ? pack_factors(h) : RSG_OK;
+        if (!repack) return int(RSG_OK);
+        packed = -1;
+        drop_records(h);
+        const int rc = pack_factors(h);
+        if (rc == RSG_OK) packed = c.stage;
+        return rc;
     };
     if (!split) { t.desc = "no split CPR: fixed shapes"; h->tune = t; return RSG_OK; }
     if (!h->opt.autotune || (!free_form && !free_thr)) {

@@ -354,13 +354,13 @@ __global__ void k_amg_slots(int totSlots, int totRows, const int* __restrict__ s
         if (q < totSlots) {
             const int src = __ldg(slotSrc + q);
             const double v = src >= 0 ? val[src] : 0.0;
-            slotVal[q] = v;
             if (slotValf) slotValf[q] = float(v);
+            else slotVal[q] = v;
         } else {
             const int g = q - totSlots;
             const double v = val[__ldg(diagGlob + g)];
-            diagVal[g] = v;
             if (diagValf) diagValf[g] = float(v);
+            else diagVal[g] = v;
         }
     }
 }

@@ -46,6 +46,7 @@ constexpr int SLOTS = 3;              // factor block slots per row and triangle
 constexpr int LREC = 28;              // factor values per row record of L: SLOTS blocks + 1 pad (16-byte multiple)
 constexpr int UREC = 36;              // per row record of U and D: SLOTS blocks + the inverted diagonal block
 constexpr int SPREC = 24;             // CPR pressure columns of S per row: (SLOTS + 1 + SLOTS) blocks x 3 + 3 pad
+constexpr int kFacRow = 40;           // factorisation: blocks of a row kept in shared memory; longer rows work in global memory
 constexpr int OV_CHUNK = 4;           // overflow entries a sweep reads at once (the lists are padded to allow it)
 
 // Krylov status per system (device int)
@@ -102,6 +103,7 @@ struct HostPlan {
     std::vector<int> Uslot, UslotSrc, UovCol, UovSrc;
     std::vector<int> Dsrc;               // diagonal (U_ii^-1) block of row k
     int maxSysRows = 0;
+    int maxRowBlocks = 0;                // blocks of the longest row
 };
 
 struct PrecDev;
@@ -219,7 +221,9 @@ struct DevAmg {
     size_t* dcWorkOff = nullptr;
     int* rowLv = nullptr;
     int* wave = nullptr;
-    unsigned long long* gsWord = nullptr;   // 2 x totRows: forward and backward values of the sync-free sweeps and of the small colours' pass
+    unsigned long long* gsWord = nullptr;   // 2 x totRows words of the V-cycle's type: forward and backward values of the sync-free sweeps
+                                            // and of the small colours' pass
+    size_t gsWordBytes = 0;
     unsigned* gsCtr = nullptr;         // maxL x 4
     std::vector<int> coarseGsLevels;   // host: levels that are some system's coarsest without a dense LU
     // multicolour schedule (FP32 forms), grid-wide: per level the rows of every system that smooths it, colour by
@@ -385,7 +389,7 @@ struct RingHost {
 struct RingDev {
     int4* desc = nullptr;
     int* stepOff = nullptr;
-    int maxSteps = 0, maxRows = 0, maxWidth = 0;
+    int maxSteps = 0, maxRows = 0, maxWidth = 0;   // (maxSteps 0: no steps)
     size_t maxStage32 = 0, maxStage64 = 0;
 };
 

@@ -43,7 +43,6 @@ constexpr int kSweepThreads = 128;
 // arithmetic one after another: 180,000 rows with four 30-layer wells 28 -> 3.4 ms, 277,000 rows with five 42-layer wells
 // (lean) 115 -> 11.9 ms, 11,200 rows 2.82 -> 0.57 ms; FP32, a block per system before, 11,200 rows 2.4 -> 0.47 ms, 64 systems
 // 3.29 -> 2.95 ms.
-constexpr int kFacRow = 40;                  // blocks of a row in shared memory; longer rows work in global memory
 __device__ __forceinline__ double fmul(double a, double b) { return dm(a, b); }
 __device__ __forceinline__ double fadd(double a, double b) { return da(a, b); }
 __device__ __forceinline__ double fsub(double a, double b) { return ds(a, b); }

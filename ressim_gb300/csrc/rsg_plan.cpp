@@ -136,6 +136,8 @@ bool build_plan(HostPlan& P, int nsys, const std::vector<int>& sysRow0, const st
     P.lvlStart.clear();
     P.sysLvl0.assign(size_t(nsys) + 1, 0);
     P.maxSysRows = 0;
+    P.maxRowBlocks = 0;
+    for (int i = 0; i < n; ++i) P.maxRowBlocks = std::max(P.maxRowBlocks, rowPtr0[size_t(i) + 1] - rowPtr0[size_t(i)]);
     std::vector<int> levNew(size_t(n), 0);
     for (int s = 0; s < nsys; ++s) {
         const int r0 = sysRow0[size_t(s)], r1 = sysRow0[size_t(s) + 1];

@@ -427,7 +427,7 @@ size_t ring_smem(const RingDev& R, size_t sizeTF, size_t sizeTV) {
     const size_t fixed = kRingHeader + size_t(R.maxSteps) * sizeof(int4) + ((size_t(R.maxRows) * 3 * sizeTV + 31) & ~size_t(15));
     const size_t stage = (sizeTF == 4 ? R.maxStage32 : R.maxStage64) + 32;
     const size_t cap = smem_cap();
-    if (!R.desc || fixed + stage > cap) return 0;
+    if (R.maxSteps == 0 || fixed + stage > cap) return 0;
     return std::min(cap, fixed + std::max(stage, kRingWant));
 }
 

@@ -1397,7 +1397,7 @@ __device__ __forceinline__ void gs_grid_body(int q0, int q1, int maxL, int phase
                                                           int totRows, unsigned* ctr, const KScal* ks, int* err) {
     using U = typename Word<TA>::type;
     U* wf = reinterpret_cast<U*>(words);
-    U* wb = reinterpret_cast<U*>(words + totRows);
+    U* wb = wf + totRows;
     const U* in = FWD ? wf : wb;
     U* out = FWD ? wf : wb;
     U* clear = FWD ? wb : wf;
@@ -1590,7 +1590,7 @@ __device__ __forceinline__ void gs_tail_body(int i0, int i1, int tail, int maxL,
     using U = typename Word<TA>::type;
     __shared__ TA sh[8][2][32];                               // per warp: factors and values of 32 entries
     U* wf = reinterpret_cast<U*>(words);
-    U* wb = reinterpret_cast<U*>(words + totRows);
+    U* wb = wf + totRows;
     U* out = FWD ? wf : wb;
     U* clear = FWD ? wb : wf;
     if (blockIdx.x == 0 && threadIdx.x == 0) ctr[FWD ? 1 : 0] = 0u;   // the opposite direction's counter, for its next pass

@@ -85,3 +85,34 @@ def test_escalation_takes_no_memory(precond, sweep, shape):
             x, res = d.solve(b, tol=1e-13, maxit=2)
             assert not res.converged and d.stats().escalated_systems == 1 and np.isfinite(x).all()
             assert d.stats().device_bytes == before <= held
+
+
+# what a handle held after a solve before the sweeps by value words, the ring and the slabs: a budget that was just enough
+# for it still is (system, preconditioner, precision, sweep, Krylov method, bytes)
+BUDGETS = [("box315", "bilu0", "fp64", "auto", "bicgstab", 729168), ("box315", "bilu0", "mixed_f32", "auto", "bicgstab", 728952),
+           ("box315", "cpr", "fp64", "auto", "bicgstab", 2578728), ("box315", "cpr", "mixed_f32", "auto", "bicgstab", 2578444),
+           ("box13k", "bilu0", "fp64", "auto", "bicgstab", 32368308), ("box13k", "bilu0", "fp64", "auto", "gmres", 39339124),
+           ("box13k", "bilu0", "fp64", "grid", "bicgstab", 25609876), ("box13k", "bilu0", "mixed_f32", "auto", "bicgstab", 32643108),
+           ("box13k", "bilu0", "mixed_f32", "auto", "gmres", 39613924), ("box13k", "bilu0", "mixed_f32", "grid", "bicgstab", 29263876),
+           ("box13k", "cpr", "fp64", "auto", "bicgstab", 47553864), ("box13k", "cpr", "fp64", "auto", "gmres", 54524680),
+           ("box13k", "cpr", "fp64", "grid", "bicgstab", 40795432), ("box13k", "cpr", "fp64", "split", "bicgstab", 47553864),
+           ("box13k", "cpr", "mixed_f32", "auto", "bicgstab", 48073480), ("box13k", "cpr", "mixed_f32", "auto", "gmres", 55044296),
+           ("box13k", "cpr", "mixed_f32", "grid", "bicgstab", 44694248), ("box13k", "cpr", "mixed_f32", "split", "bicgstab", 48073480),
+           ("box13k", "cpr_device", "fp64", "auto", "bicgstab", 35943664), ("box13k", "cpr_device", "fp64", "auto", "gmres", 42914480),
+           ("box13k", "cpr_device", "mixed_f32", "auto", "bicgstab", 36188480), ("box13k", "cpr_device", "mixed_f32", "auto", "gmres", 43159296),
+           ("box2295c", "cpr", "fp64", "auto", "bicgstab", 11848668), ("box2295c", "cpr", "fp64", "grid", "bicgstab", 10427460),
+           ("box2295c", "cpr", "mixed_f32", "auto", "bicgstab", 11907448), ("box2295c", "cpr", "mixed_f32", "grid", "bicgstab", 11196844)]
+CLIQUE = [(a, b) for a in range(50, 110) for b in range(a + 1, 110)]
+
+
+@pytest.mark.parametrize("case", BUDGETS, ids=lambda c: "-".join(c[:5]))
+def test_budgets_that_were_enough(case):
+    from ressim_gb300.solver import DeviceSolver
+    name, precond, precision, sweep, krylov, budget = case
+    n, pairs = {"box315": (315, box(9, 7, 5)), "box13k": (13200, box(33, 40, 10)), "box2295c": (2295, box(27, 17, 5) + CLIQUE)}[name]
+    A = system(n, pairs, seed=1)
+    with DeviceSolver(precond=precond, precision=precision, sweep=sweep, krylov=krylov, restart=10, mem_budget=budget) as d:
+        d.set_matrix(A)
+        d.setup()
+        d.solve(np.ones(3 * n), 1e-6, 2)
+        assert d.stats().device_bytes <= budget
