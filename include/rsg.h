@@ -73,7 +73,7 @@ typedef struct rsg_options {
                                instructions; results within rounding of the reference); 0: the reference's separately
                                rounded products and sums, bit for bit (engine/src/bsr.cpp:109-117) */
     int sweep_inflight;     /* sync-free grid sweeps (BILU0, factorisation, Gauss-Seidel): levels in flight, which sizes
-                               the persistent grid; 0 = auto (the full grid) */
+                               each pass's persistent grid by the rows its warps take; 0 = auto (the full grid) */
     int autotune;           /* 1 (default): the launch shapes left at 0 below are chosen by timing the candidates on the
                                system at its first set-up (cached per pattern for the life of the process); 0: their
                                defaults. Every shape gives the same results bit for bit. */

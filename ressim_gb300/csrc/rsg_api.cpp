@@ -282,7 +282,8 @@ int alloc_plan(rsg_solver* h) {
         int maxLv = 1;
         for (int s = 0; s < P.nsys; ++s) maxLv = std::max(maxLv, P.sysLvl0[size_t(s) + 1] - P.sysLvl0[size_t(s)] - 1);
         D.avgLevelRows = double(P.n) / double(std::max(1, P.nlevF));
-        D.sweepBlocks = sweep_blocks_for(double(P.n) / double(maxLv), h->opt.sweep_inflight);
+        D.sweepBlocks = sweep_blocks_for(double(P.n) / double(maxLv), h->opt.sweep_inflight, kSweepRows);
+        D.factorBlocks = sweep_blocks_for(double(P.n) / double(maxLv), h->opt.sweep_inflight, 1);
     }
     if ((h->opt.sweep == 1 || h->opt.sweep == 3) && !h->cta)
         return fail(RSG_EINVAL, "thread-block sweeps need a structurally symmetric pattern of <= 32768 block rows per system");
@@ -875,7 +876,7 @@ int build_dev_amg(rsg_solver* h, const std::vector<SysAmg>& H) {
         int maxNl = 1;
         for (int s = 0; s < nsys; ++s)
             if (l < int(H[size_t(s)].lv.size())) maxNl = std::max(maxNl, lv[size_t(s) * maxL + l].nl);
-        G.gsBlocks[size_t(l)] = sweep_blocks_for(double(G.levelRowBeg[size_t(l) + 1] - G.levelRowBeg[size_t(l)]) / maxNl, h->opt.sweep_inflight);
+        G.gsBlocks[size_t(l)] = sweep_blocks_for(double(G.levelRowBeg[size_t(l) + 1] - G.levelRowBeg[size_t(l)]) / maxNl, h->opt.sweep_inflight, kGsRows);
     }
     // colour-major rows of every level that is smoothed (multicolour schedule only): colour c of every system, then
     // c + 1; colours from colTail on (all of them small) are swept together by one sync-free pass

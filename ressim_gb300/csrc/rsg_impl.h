@@ -46,6 +46,8 @@ constexpr int SLOTS = 3;              // factor block slots per row and triangle
 constexpr int LREC = 28;              // factor values per row record of L: SLOTS blocks + 1 pad (16-byte multiple)
 constexpr int UREC = 36;              // per row record of U and D: SLOTS blocks + the inverted diagonal block
 constexpr int SPREC = 24;             // CPR pressure columns of S per row: (SLOTS + 1 + SLOTS) blocks x 3 + 3 pad
+constexpr int kSweepRows = 10;        // grid-wide BILU0 sweeps: rows of a warp (three lanes each)
+constexpr int kGsRows = 32;           // grid-wide Gauss-Seidel sweeps: rows of a warp (a lane each)
 constexpr int kFacRow = 40;           // factorisation: blocks of a row kept in shared memory; longer rows work in global memory
 constexpr int OV_CHUNK = 4;           // overflow entries a sweep reads at once (the lists are padded to allow it)
 
@@ -252,7 +254,7 @@ struct DevAmg {
 // phase table of the fused V-cycle for a built hierarchy (empty when the fused kernel does not apply)
 void vcycle_phases(const DevAmg& G, std::vector<VPhase>& out);
 // blocks of 4 warps for a sync-free sweep that keeps `inflight` of its levels (avgRows rows each) in flight
-int sweep_blocks_for(double avgRows, int inflight);
+int sweep_blocks_for(double avgRows, int inflight, int rowsPerWarp);
 // CPR set-up kernels (rsg_cpr.cu)
 void launch_cpr_weights(const DevPlan& P, const double* val, const double* accLev, double* w, int* nfallback, cudaStream_t st);
 void launch_cpr_pressure(const DevPlan& P, const double* val, const double* w, double* ap, cudaStream_t st);
@@ -358,7 +360,8 @@ struct DevPlan {
     int2* rowLevel = nullptr;         // level-space row -> (first row of its forward level, rows of that level)
     int nLov = 0, nUov = 0, maxSysRows = 0;
     double avgLevelRows = 0;          // rows of a forward level of the whole batch, on average
-    int sweepBlocks = 0;              // persistent grid of the sync-free sweeps (0: sized from n)
+    int sweepBlocks = 0;              // persistent grid of the sync-free sweeps
+    int factorBlocks = 0;             // and of the factorisation
     bool spmvFma = true;              // SpMV with fused multiply-adds (else the reference's rounding, bitwise)
 };
 

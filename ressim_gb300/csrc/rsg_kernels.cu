@@ -251,7 +251,6 @@ __device__ __forceinline__ bool sys_running(const KScal* ks, const int* rowSys, 
 // TF: factor storage, TV: vector and arithmetic -- (double, double), (float, double): FP64 explicitly rounded, the
 // reference's sweeps; (float, float): BILU0f (engine/src/bsr.cpp:1100-1121).
 // IN_PUPDATE: in = p = r + beta (p - omega v) (p stored); IN_SUPDATE: in = s = r - alpha v (s stored in pv)
-constexpr int kSweepRows = 10;               // rows of a warp
 
 // yi -= sum_p (row e of B_p) . y_col(p) over the entries [p0, p1) of a row, in order, four entries at a time
 template <class TF, class TV>
@@ -748,29 +747,17 @@ int stream_grid(size_t total) {
     const size_t g = (total + 255) / 256, cap = size_t(device_sm_count()) * 16;
     return int(g < cap ? (g > 0 ? g : 1) : cap);
 }
-int sweep_grid(int n) {
-    const int sms = device_sm_count();
-    // enough warps for several levels in flight, at most 8 blocks of 4 warps per SM
-    const int warps = (n + 31) / 32;
-    int blocks = (warps + 3) / 4;
-    const int maxb = sms * 8;
-    if (blocks > maxb) blocks = maxb;
-    if (blocks < 1) blocks = 1;
-    return blocks;
-}
-
-// the plan's grid when it was sized from the level widths, else one from n
-int sweep_blocks(const DevPlan& P) { return P.sweepBlocks > 0 ? P.sweepBlocks : sweep_grid(P.n); }
-
 }  // namespace
 
-// Warps that poll flags of levels far ahead of the sweep front only add memory traffic to the critical path:
-// keep about `inflight` levels' rows in flight (a warp per 32 rows), at most 8 blocks of 4 warps per SM.
-int sweep_blocks_for(double avgRows, int inflight) {
-    if (inflight <= 0) return 8 * device_sm_count();              // auto: the full grid (measured no slower)
-    const double warps = double(inflight) * avgRows / 32.0;
-    const long long blocks = (long long)((warps + 3.0) / 4.0);
+// Persistent grid of a sync-free pass whose warps claim rowsPerWarp rows each: `inflight` levels of avgRows rows in flight (a
+// warp far ahead of the front only polls), at most 8 blocks of 4 warps per SM, which is what auto takes. CPR application, grid-wide,
+// auto / 32 / 8 / 2 levels: 180,000 rows FP64 3.85 / 3.75 / 3.77 / 4.24 ms, 277,000 rows FP32 1.26 / 1.28 / 1.53 / 2.73 ms, 11,200 rows
+// FP64 1.24 / 1.22 / 1.26 / 1.28 ms; factorisation 4.9, 13.5 and 2.07 ms, the same from two levels on.
+int sweep_blocks_for(double avgRows, int inflight, int rowsPerWarp) {
     const long long cap = 8LL * device_sm_count();
+    if (inflight <= 0) return int(cap);
+    const double warps = double(inflight) * avgRows / double(rowsPerWarp);
+    const long long blocks = (long long)((warps + 3.0) / 4.0);
     return int(blocks < 1 ? 1 : (blocks < cap ? blocks : cap));
 }
 
@@ -800,7 +787,7 @@ template <class W, class F>
 static void launch_factor_t(const DevPlan& P, const double* val, F* lu, W* work, SweepState& S, int epoch, int* nreg, int* err,
                             cudaStream_t st) {
     cudaMemsetAsync(S.ctr + 2, 0, sizeof(unsigned), st);
-    const int blocks = std::max(1, std::min(8 * device_sm_count(), (P.n + 3) / 4));
+    const int blocks = std::max(1, std::min(P.factorBlocks, (P.n + 3) / 4));
     const int chunk = std::max(1, std::min(8, int(P.avgLevelRows / double(blocks * (kSweepThreads / 32)))));
     k_factor<W, F><<<blocks, kSweepThreads, 0, st>>>(P.n, chunk, P.rowPtr, P.col, P.diag, P.ford, P.elimPtr, P.elimT, P.elimQ, val, lu, work,
                                                     S.flagL, epoch, S.ctr + 2, nreg, err);
@@ -822,7 +809,7 @@ template <class TF, class TV, class TI, class TX>
 static void launch_sweeps(const DevPlan& P, const TF* lu, int mode, const TI* r, double* pv, const double* v, double* z, const TX* xp,
                           const KScal* ks, SweepState& S, int* err, cudaStream_t st) {
     using U = typename Word<TV>::type;
-    const int g = std::min(sweep_blocks(P), std::max(1, (P.n + 4 * kSweepRows - 1) / (4 * kSweepRows)));
+    const int g = std::min(P.sweepBlocks, std::max(1, (P.n + 4 * kSweepRows - 1) / (4 * kSweepRows)));
     U* yf = reinterpret_cast<U*>(S.yw);
     U* yb = reinterpret_cast<U*>(S.yw + size_t(P.n) * 3);
     auto fwd = [&](auto tag) {

@@ -218,3 +218,19 @@ def test_coarse_levels_around_the_default_limit(cells):
             z.append(d.precond_apply(r))
             assert 1700 < d.amg_level_sizes()[0][1:].sum() < 2300
     assert np.isfinite(z[0]).all() and np.array_equal(z[0], z[1])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "mixed_f32"])
+def test_levels_in_flight_do_not_change_results(precision):
+    """Persistent grids from one block on (sweep_inflight) give the factors and the application of the full one, bit for bit."""
+    from ressim_gb300.solver import DeviceSolver
+    A = system(33 * 40 * 3, box(33, 40, 3), seed=9)
+    r = np.random.default_rng(9).standard_normal(3 * A.n)
+    out = []
+    for inflight in (0, 1, 2, 8):
+        with DeviceSolver(precond="cpr", precision=precision, sweep="grid", sweep_inflight=inflight) as d:
+            d.set_matrix(A)
+            d.setup()
+            out.append((d.factors(A.nnzb), d.precond_apply(r)))
+    for f, z in out[1:]:
+        assert np.array_equal(f, out[0][0]) and np.array_equal(z, out[0][1])

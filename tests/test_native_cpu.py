@@ -353,3 +353,20 @@ def test_synthetic_assembly_model_is_the_engines_layout():
     with pytest.raises(_lib.RsgError) as e:
         BlackOilAssembler(z)
     assert e.value.code == _lib.RSG_ECUDA, e.value
+
+
+def test_levels_in_flight_by_the_rows_of_a_warp():
+    """sweep_inflight: the persistent grid holds that many levels, whatever a warp takes (10 rows in the BILU0 sweeps, 32 in
+    Gauss-Seidel, one in the factorisation); 0 is the full grid, the limit of every other value."""
+    from ressim_gb300 import _lib
+    f = _lib.load()._ZN3rsg16sweep_blocks_forEdii
+    f.argtypes, f.restype = [C.c_double, C.c_int, C.c_int], C.c_int
+    full = f(1000.0, 0, 10)
+    assert full % 8 == 0 and full >= 8                                     # 8 blocks of 4 warps per SM
+    for rows in (1, 10, 32):
+        for level in (3.0, 7.0, 25.0):
+            for n in (1, 2, 4):
+                want = max(1, min(full, int((n * level / rows + 3) // 4)))
+                assert f(level, n, rows) == want
+                assert want == full or 4 * want * rows >= n * level - 3 * rows
+        assert f(1e9, 1, rows) == full
