@@ -108,15 +108,15 @@ __device__ __forceinline__ bool coarse_level(const AmgSysLv* __restrict__ lv, in
 }
 
 // dense LU with partial pivoting of every system's coarsest level in its natural numbering
-// (engine/src/amg.cpp:273-295; rsg_dense.cuh), one cluster of blocks per system. T = double (reference arithmetic) or float (the
+// (engine/src/amg.cpp:273-295; rsg_dense.cuh), a cluster of blocks or one block per system. T = double (reference arithmetic) or float (the
 // FP32 hierarchy of the precision forms: same algorithm, float operations).
-template <class T>
-__global__ void __launch_bounds__(kDenseThreads) k_coarse_lu(int maxL, const AmgSysLv* __restrict__ lv, const int* __restrict__ rp,
+template <class T, int CL, int NT>
+__global__ void __launch_bounds__(NT) k_coarse_lu(int maxL, const AmgSysLv* __restrict__ lv, const int* __restrict__ rp,
                                                              const int* __restrict__ ci, const double* __restrict__ val,
                                                              const int* __restrict__ luPerm, T* luAll, int* pivAll, int* cinAll,
                                                              int skipUpTo, const int* only, unsigned smemBytes) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    const int s = int(blockIdx.x) / kDenseCluster, tid = int(threadIdx.x), nt = int(blockDim.x), rank = cluster_rank();
+    const int s = int(blockIdx.x) / CL, tid = int(threadIdx.x), nt = int(blockDim.x), rank = cluster_rank<CL>();
     if (only && !only[s]) return;                                 // only the systems flagged (FP64 coarse solve); whole clusters
     AmgSysLv L;
     if (!coarse_level(lv, maxL, s, L) || L.n <= skipUpTo) return;   // skipUpTo: levels inverted in shared memory
@@ -124,9 +124,9 @@ __global__ void __launch_bounds__(kDenseThreads) k_coarse_lu(int maxL, const Amg
     T* lu = luAll + L.luOff;
     int* piv = pivAll + L.luRowOff;
     const int* nat = luPerm + L.luRowOff;
-    const DenseCols<T> D = dense_place(m, rank, smemBytes, smraw, lu);
+    const auto D = dense_place<T, CL>(m, rank, smemBytes, smraw, lu);
     dense_fill(D, rp + L.rpOff, ci + L.entOff, val + L.entOff, nat);
-    dense_lu(D, piv);
+    dense_lu<NT>(D, piv);
     dense_out(D, lu);
     if (rank) return;
     __syncthreads();                                              // (piv: written by this block)
@@ -513,6 +513,24 @@ __global__ void __launch_bounds__(256) k_coarse_check(int maxL, const AmgSysLv* 
     }
 }
 
+// The cluster shortens the chain of one matrix's steps but holds eight blocks for it, so it pays while all matrices run at once: up
+// to about two blocks (FP64) or seven (FP32, beyond 224 rows) per SM; and a matrix of 128 rows is too small for it. Whole CPR
+// set-ups, cluster / one block (/ one block a system with a barrier for every part of a step, as it was): FP64, 1 system
+// of 225 rows 1.74 / 3.01 (4.95) ms, 32 of 225 2.18 / 3.06 (5.20), 48 of 225 4.09 / 3.06 (5.21), 300 of 225 18.1 / 5.6 (7.9), 300 of 100
+// 6.36 / 1.09 (1.34), 1,000 of 27 4.82 / 0.46 (0.44); FP32, 64 of 300 3.47 / 4.98 (29), 300 of 300 11.6 / 10.7 (54).
+template <int CL, int NT, class T>
+static void coarse_lu_cl(const DevAmg& G, T* lu, int skipUpTo, const int* only, cudaStream_t st) {
+    const unsigned sm = dense_lu_smem<T, CL>(G.maxCoarse);
+    launch_dense<CL, NT>(k_coarse_lu<T, CL, NT>, G.nsys, sm, st, G.maxL, (const AmgSysLv*)G.lv, (const int*)G.rp, (const int*)G.ci,
+                         (const double*)G.val, (const int*)G.luPerm, lu, G.piv, G.cin, skipUpTo, only, sm);
+}
+template <class T>
+static void coarse_lu(const DevAmg& G, T* lu, int skipUpTo, const int* only, cudaStream_t st) {
+    const long long blocks = (long long)G.nsys * kDenseCluster, sms = device_sm_count();
+    if (G.maxCoarse > 128 && blocks <= (sizeof(T) == 8 ? 2 : 7) * sms) coarse_lu_cl<kDenseCluster, kDenseThreads>(G, lu, skipUpTo, only, st);
+    else if (G.maxCoarse > 128 || G.nsys <= sms) coarse_lu_cl<1, 256>(G, lu, skipUpTo, only, st);
+    else coarse_lu_cl<1, 128>(G, lu, skipUpTo, only, st);             // (small and many: 1,000 of 100 rows 3.54 -> 3.00 ms)
+}
 void launch_amg_coarse_lu(const DevAmg& G, bool fp32, cudaStream_t st) {
     if (G.totLu <= 0) return;
     if (fp32) {
@@ -520,10 +538,9 @@ void launch_amg_coarse_lu(const DevAmg& G, bool fp32, cudaStream_t st) {
         raise_smem_limit(reinterpret_cast<const void*>(k_coarse_gj), smem);
         k_coarse_gj<<<G.nsys, kGjThreads, smem, st>>>(G.maxL, G.lv, G.rp, G.ci, G.val, G.luPerm, G.invf);
         if (G.maxCoarse > kInvSmemRows) {                        // levels too large for shared memory: LU, then columns
-            const unsigned sl = dense_lu_smem<float>(G.maxCoarse), si = unsigned(size_t(G.maxCoarse) * (kInvCols + 2) * sizeof(float));
+            const unsigned si = unsigned(size_t(G.maxCoarse) * (kInvCols + 2) * sizeof(float));
             raise_smem_limit(reinterpret_cast<const void*>(k_coarse_inv), int(si));
-            launch_dense(k_coarse_lu<float>, G.nsys, sl, st, G.maxL, (const AmgSysLv*)G.lv, (const int*)G.rp, (const int*)G.ci,
-                         (const double*)G.val, (const int*)G.luPerm, G.luf, G.piv, G.cin, kInvSmemRows, (const int*)nullptr, sl);
+            coarse_lu(G, G.luf, kInvSmemRows, nullptr, st);
             k_coarse_inv<<<dim3(unsigned((G.maxCoarse + kInvCols - 1) / kInvCols), unsigned(G.nsys)), 256, si, st>>>(
                 G.maxL, G.lv, G.cin, G.luf, G.invf, kInvSmemRows, si);
         }
@@ -532,9 +549,7 @@ void launch_amg_coarse_lu(const DevAmg& G, bool fp32, cudaStream_t st) {
         // only for the systems that need it
         k_coarse_check<<<G.nsys, 256, 0, st>>>(G.maxL, G.lv, G.rp, G.ci, G.val, G.luPerm, G.invf, G.x, G.b, G.coarse64);
     }
-    const unsigned sm = dense_lu_smem<double>(G.maxCoarse);
-    launch_dense(k_coarse_lu<double>, G.nsys, sm, st, G.maxL, (const AmgSysLv*)G.lv, (const int*)G.rp, (const int*)G.ci, (const double*)G.val,
-                 (const int*)G.luPerm, G.lu, G.piv, G.cin, 0, (const int*)(fp32 ? G.coarse64 : nullptr), sm);
+    coarse_lu(G, G.lu, 0, fp32 ? G.coarse64 : nullptr, st);
 }
 void launch_amg_round(const DevAmg& G, cudaStream_t st) {
     k_round<<<grid_for(size_t(G.totEnt)), 256, 0, st>>>(size_t(G.totEnt), G.val, G.valf);

@@ -436,10 +436,10 @@ __global__ void __launch_bounds__(kDenseThreads) k_gen_coarse_lu(int m, const in
                                                                  const double* __restrict__ v, const int* __restrict__ perm, double* lu,
                                                                  int* piv, unsigned smemBytes) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    const int rank = cluster_rank();
-    const DenseCols<double> D = dense_place(m, rank, smemBytes, smraw, lu);
+    const int rank = cluster_rank<kDenseCluster>();
+    const auto D = dense_place<double, kDenseCluster>(m, rank, smemBytes, smraw, lu);
     dense_fill(D, rp, ci, v, perm);
-    dense_lu(D, piv);
+    dense_lu<kDenseThreads>(D, piv);
     dense_out(D, lu);
 }
 
@@ -869,8 +869,8 @@ void refresh_amg(GenEngine& g) {
     }
     GenLevel& Lc = g.lv.back();
     if (Lc.dense) {
-        const unsigned sm = dense_lu_smem<double>(Lc.n);
-        launch_dense(k_gen_coarse_lu, 1, sm, g.st, Lc.n, (const int*)Lc.rp, (const int*)Lc.ci, (const double*)Lc.v, (const int*)Lc.perm, Lc.lu,
+        const unsigned sm = dense_lu_smem<double, kDenseCluster>(Lc.n);
+        launch_dense<kDenseCluster, kDenseThreads>(k_gen_coarse_lu, 1, sm, g.st, Lc.n, (const int*)Lc.rp, (const int*)Lc.ci, (const double*)Lc.v, (const int*)Lc.perm, Lc.lu,
                      Lc.piv, sm);
         ++g.launches;
     }
