@@ -68,7 +68,7 @@ typedef struct rsg_options {
                                CPR: the V-cycle's passes grid-wide over all systems, then the BILU0 sweeps (same results
                                as 1). Auto takes the split form for CPR and, for the BILU0 sweeps, one thread block per
                                system where the vector fits one SM and does not bind there (FP32; FP64 up to 2,000
-                               rows), else the grid-wide ones */
+                               rows, longer in large batches), else the grid-wide ones */
     int fma;                /* 1 (default): the SpMV accumulates with fused multiply-adds (half the FP64
                                instructions; results within rounding of the reference); 0: the reference's separately
                                rounded products and sums, bit for bit (engine/src/bsr.cpp:109-117) */

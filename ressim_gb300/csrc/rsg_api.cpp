@@ -216,7 +216,7 @@ int upload(DevMem& M, T** d, const std::vector<T>& v, cudaStream_t st, size_t pa
 // How the BILU0 stage of a factor kind (0 FP64, 1 FP32 factors with FP64 vectors, 3 all FP32) runs on systems with a
 // thread-block plan:
 // * on the ring where its vector and steps fit one SM and the arithmetic does not bind it there: all FP32, and FP64 vectors up
-//   to kRingRows64 rows;
+//   to kRingRows64 rows, or longer ones in batches (ring_pays);
 // * else by the grid-wide sweeps, whatever the size: FP64 vectors on one SM are bound by its FP64 pipe;
 // * by the kernels on the component-major records only where the options fix the launch shape (the one-kernel CPR
 //   application, a BILU0 stage of a given thread count) or the tuner, asked for the split form, found them faster.
@@ -225,20 +225,29 @@ int upload(DevMem& M, T** d, const std::vector<T>& v, cudaStream_t st, size_t pa
 // of 8,000-14,400 rows 4.45 / 3.87 ms; FP32 factors with FP64 vectors: 1.13 / 0.51 and 1.72 / 1.00 ms; all FP32, 25,000 rows
 // (no ring): 0.56 / 0.45 ms.
 constexpr int kRingRows64 = 2000;
+// Longer systems in batches: the grid-wide sweeps of many systems are bound by the GPU's FP64 throughput (0.65 ns a row and
+// application), a ring by its system's chain (FP64 40 us + 56 ns a row, FP32 factors 55 us + 72 ns; one system per SM at a time).
+// Ring / grid-wide, both sweeps, FP64: 152 systems of 2,500 rows 186 / 297 us, 300 of 3,300 478 / 656 us, 152 of 6,000 376 / 616 us,
+// but 200 of 1,000 and one of 2,100 245 / 185 us; FP32 factors: 300 of 3,300 614 / 666 us, 152 of 6,000 491 / 624 us.
+bool ring_pays(const HostPlan& P, bool factors32) {
+    const double waves = double((P.nsys + device_sm_count() - 1) / device_sm_count());
+    return waves * (factors32 ? 55.0 + 0.072 * P.maxSysRows : 40.0 + 0.056 * P.maxSysRows) < 0.65e-3 * P.n;
+}
 enum { STAGE_CTA = 0, STAGE_RING = 1, STAGE_GRID = 2 };
 // whether a BILU0 stage on the component-major records, or on the ring with vectors of this type, can come up for these options
 bool cta_stage_possible(const rsg_solver* h) { return h->cta && (h->opt.cpr2_threads != 0 || h->opt.sweep == 1 || h->opt.sweep == 3); }
 bool ring_wanted(const rsg_solver* h, bool vec32) {
     if (h->opt.precond == RSG_PREC_JACOBI || h->opt.precond == RSG_PREC_CPR_DEVICE || h->opt.cpr2_threads != 0) return false;
     if (h->opt.precond == RSG_PREC_CPR && h->opt.sweep == 1) return false;
-    return vec32 ? h->opt.precision == RSG_MIXED_F32 : h->plan.maxSysRows <= kRingRows64 || h->opt.sweep == 1;
+    if (vec32) return h->opt.precision == RSG_MIXED_F32;
+    return h->plan.maxSysRows <= kRingRows64 || h->opt.sweep == 1 || ring_pays(h->plan, h->opt.precision != RSG_FP64);
 }
 int ilu_stage(const rsg_solver* h, int kind) {
     if (!h->cta || kind == 2) return STAGE_GRID;
     if (h->opt.cpr2_threads != 0 || !h->tune.stage) return STAGE_CTA;
     if (h->opt.precond == RSG_PREC_CPR && h->opt.sweep == 1) return STAGE_CTA;
     const bool fits = ring_fits(h->ring[kind == 3 ? 1 : 0], kind != 0, kind == 3);
-    if (fits && (kind == 3 || h->plan.maxSysRows <= kRingRows64 || h->opt.sweep == 1)) return STAGE_RING;
+    if (fits && (kind == 3 || h->plan.maxSysRows <= kRingRows64 || h->opt.sweep == 1 || ring_pays(h->plan, kind != 0))) return STAGE_RING;
     return h->opt.sweep == 1 ? STAGE_CTA : STAGE_GRID;
 }
 int alloc_plan(rsg_solver* h) {

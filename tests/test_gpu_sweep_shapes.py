@@ -234,3 +234,32 @@ def test_levels_in_flight_do_not_change_results(precision):
             out.append((d.factors(A.nnzb), d.precond_apply(r)))
     for f, z in out[1:]:
         assert np.array_equal(f, out[0][0]) and np.array_equal(z, out[0][1])
+
+
+@pytest.mark.parametrize("precond", ["bilu0", "cpr"])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_large_batches_of_fp64_vectors(precision, precond, oracle):
+    """FP64 vectors of more than 2,000 rows go through the ring in large batches and over the whole GPU in small ones: the
+    same bits, and the oracle's."""
+    from ressim_gb300.solver import DeviceSolver
+    kinds = [system(2600 + k, box(20, 13, 10) + [(2599, 2600)] * (k > 0), seed=k) for k in (0, 1)]
+    r = np.random.default_rng(3).standard_normal(3 * 150 * 2601)
+    z = {}
+    # (a CPR application with the sweeps of one block per system: sweep="grid" forms the second stage's input in another order)
+    for copies, sweep, threads in ((150, "auto", 0), (150, "grid", 0) if precond == "bilu0" else (150, "split", 256), (3, "auto", 0)):
+        mats = [kinds[k % 2] for k in range(copies)]
+        N = sum(3 * A.n for A in mats)
+        with DeviceSolver(precond=precond, precision=precision, sweep=sweep, cpr2_threads=threads) as d:
+            d.set_batch(mats)
+            d.setup()
+            if precond == "cpr" and sweep == "auto":
+                assert ("bilu0=ring" if copies == 150 else "bilu0=grid") in d.tuning()
+            z[copies, sweep == "auto"] = d.precond_apply(r[:N])
+    z = {(150, "auto"): z[150, True], (150, "other"): z[150, False], (3, "auto"): z[3, True]}
+    N3 = z[3, "auto"].size
+    assert np.array_equal(z[150, "auto"], z[150, "other"]) and np.array_equal(z[150, "auto"][:N3], z[3, "auto"])
+    if precond == "bilu0":
+        A = kinds[0]
+        f, _ = (oracle.bilu0_factor if precision == "fp64" else oracle.bilu0_factor_lean)(A)
+        ref = (oracle.bilu0_apply if precision == "fp64" else oracle.bilu0_apply_fd)(A, f, r[:3 * A.n])
+        assert np.array_equal(z[150, "auto"][:3 * A.n], ref)
