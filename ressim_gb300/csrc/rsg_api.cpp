@@ -306,7 +306,7 @@ int alloc_plan(rsg_solver* h) {
         ring_steps(P, v32 != 0, H);
         RingDev R;
         R.maxSteps = H.maxSteps; R.maxRows = H.maxRows; R.maxWidth = H.maxWidth;
-        R.maxStage32 = H.maxStage32; R.maxStage64 = H.maxStage64;
+        R.maxStage32 = H.maxStage32; R.maxStage64 = H.maxStage64; R.maxBytes32 = H.maxBytes32; R.maxBytes64 = H.maxBytes64;
         if (!H.ok || !ring_fits(R, h->opt.precision != RSG_FP64, v32 != 0)) continue;
         if ((rc = upload(M, &R.desc, H.desc, st)) || (rc = upload(M, &R.stepOff, H.stepOff, st))) return rc;
         h->ring[v32] = R;
@@ -772,7 +772,7 @@ int build_dev_amg(rsg_solver* h, const std::vector<SysAmg>& H) {
             if (l + 1 == int(H[size_t(s)].lv.size())) {
                 d.coarse = 1;
                 d.dense = H[size_t(s)].coarseDense ? 1 : 0;
-                if (d.dense) { d.luOff = lus; d.luRowOff = lurows; lus += A.n * A.n; lurows += A.n; G.maxCoarse = std::max(G.maxCoarse, A.n); }
+                if (d.dense) { d.luOff = lus; d.luRowOff = lurows; lus += A.n * A.n; lurows += A.n; G.maxCoarse = std::max(G.maxCoarse, A.n); G.coarseLarge += A.n > kInvSmemRows; }
             }
         }
     }

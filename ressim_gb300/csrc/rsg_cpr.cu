@@ -151,7 +151,6 @@ __global__ void __launch_bounds__(NT) k_coarse_lu(int maxL, const AmgSysLv* __re
 // column by column (a row's terms come in the same ascending order as row by row); backward a row's terms are taken in
 // ascending order too, which starts with the value just found, so one warp runs the chain while the others stage the
 // factors' next row. 277 rows: one thread per column in global memory took 7.2 ms.
-constexpr int kInvSmemRows = 224;
 constexpr int kInvCols = 32;
 __global__ void __launch_bounds__(256) k_coarse_inv(int maxL, const AmgSysLv* __restrict__ lv, const int* __restrict__ cinAll,
                                                     const float* __restrict__ luAll, float* invAll, int skipUpTo, unsigned smemBytes) {
@@ -526,7 +525,8 @@ static void coarse_lu_cl(const DevAmg& G, T* lu, int skipUpTo, const int* only, 
 }
 template <class T>
 static void coarse_lu(const DevAmg& G, T* lu, int skipUpTo, const int* only, cudaStream_t st) {
-    const long long blocks = (long long)G.nsys * kDenseCluster, sms = device_sm_count();
+    // (systems that are left out end at once)
+    const long long blocks = (long long)(skipUpTo ? G.coarseLarge : G.nsys) * kDenseCluster, sms = device_sm_count();
     if (G.maxCoarse > 128 && blocks <= (sizeof(T) == 8 ? 2 : 7) * sms) coarse_lu_cl<kDenseCluster, kDenseThreads>(G, lu, skipUpTo, only, st);
     else if (G.maxCoarse > 128 || G.nsys <= sms) coarse_lu_cl<1, 256>(G, lu, skipUpTo, only, st);
     else coarse_lu_cl<1, 128>(G, lu, skipUpTo, only, st);             // (small and many: 1,000 of 100 rows 3.54 -> 3.00 ms)

@@ -227,6 +227,7 @@ struct DevAmg {
                                             // and of the small colours' pass
     size_t gsWordBytes = 0;
     unsigned* gsCtr = nullptr;         // maxL x 4
+    int coarseLarge = 0;               // host: systems with a dense coarsest level beyond kInvSmemRows rows
     std::vector<int> coarseGsLevels;   // host: levels that are some system's coarsest without a dense LU
     // multicolour schedule (FP32 forms), grid-wide: per level the rows of every system that smooths it, colour by
     // colour, as {row, first entry, end of entries, diagonal entry} (global indices); colour c of level l at
@@ -262,6 +263,7 @@ void launch_gather_acc(const DevPlan& P, const double* accOrig, double* accLev, 
 void launch_amg_refresh(const DevAmg& G, cudaStream_t st);           // Galerkin values of levels >= 1, diagonal fix
 void launch_amg_coarse_lu(const DevAmg& G, bool fp32, cudaStream_t st);     // fp32: the LU in FP32 (luf), else FP64 (lu)
 void launch_amg_round(const DevAmg& G, cudaStream_t st);             // valf = float(val), luf = float(lu)
+constexpr int kInvSmemRows = 224;      // FP32 forms: dense coarsest levels inverted in shared memory (larger ones by LU)
 constexpr int kSlabEntries = 12;       // off-diagonal entries of a row in its slab; a longer row takes the others from valf
 constexpr int kSlabPad = 0x7fffffff;   // no entry
 void launch_amg_slabs(const DevAmg& G, cudaStream_t st);             // slabVal from valf
@@ -387,13 +389,14 @@ struct RingHost {
     std::vector<int> stepOff;
     int maxSteps = 0, maxRows = 0, maxWidth = 0;
     size_t maxStage32 = 0, maxStage64 = 0;      // largest step in the ring (bytes), by factor type
+    size_t maxBytes32 = 0, maxBytes64 = 0;      // all steps of a system, at most
     bool ok = false;
 };
 struct RingDev {
     int4* desc = nullptr;
     int* stepOff = nullptr;
     int maxSteps = 0, maxRows = 0, maxWidth = 0;   // (maxSteps 0: no steps)
-    size_t maxStage32 = 0, maxStage64 = 0;
+    size_t maxStage32 = 0, maxStage64 = 0, maxBytes32 = 0, maxBytes64 = 0;
 };
 
 struct SweepState {                   // sync-free sweep flags and claim counters
