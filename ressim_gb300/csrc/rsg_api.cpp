@@ -290,6 +290,7 @@ int alloc_plan(rsg_solver* h) {
     {
         int maxLv = 1;
         for (int s = 0; s < P.nsys; ++s) maxLv = std::max(maxLv, P.sysLvl0[size_t(s) + 1] - P.sysLvl0[size_t(s)] - 1);
+        D.maxRowBlocks = P.maxRowBlocks;
         D.avgLevelRows = double(P.n) / double(std::max(1, P.nlevF));
         D.sweepBlocks = sweep_blocks_for(double(P.n) / double(maxLv), h->opt.sweep_inflight, kSweepRows);
         D.factorBlocks = sweep_blocks_for(double(P.n) / double(maxLv), h->opt.sweep_inflight, 1);

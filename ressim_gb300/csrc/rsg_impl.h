@@ -361,6 +361,7 @@ struct DevPlan {
     int* Dsrc = nullptr;
     int2* rowLevel = nullptr;         // level-space row -> (first row of its forward level, rows of that level)
     int nLov = 0, nUov = 0, maxSysRows = 0;
+    int maxRowBlocks = 0;             // blocks of the longest row
     double avgLevelRows = 0;          // rows of a forward level of the whole batch, on average
     int sweepBlocks = 0;              // persistent grid of the sync-free sweeps
     int factorBlocks = 0;             // and of the factorisation

@@ -231,6 +231,87 @@ __global__ void __launch_bounds__(kSweepThreads) k_factor(int n, int chunk, cons
     }
 }
 
+// The same elimination by a thread per row, for levels so wide that a warp per row is bound by its FP64 instructions (the
+// inversion of a row's pivot block costs a warp what it costs 32 rows here): rows of at most kLaneRow blocks, held in local
+// memory. The line is at 70 rows of a level per SM, 30 where the elimination is FP32 and the inversion most of the FP64 work; a warp
+// per row / a thread per row (/ the former kernels), FP64: 152 systems of 2,500 rows (7,900 rows a level) 2.28 / 2.69 (2.60) ms,
+// 300 of 1,000 (10,700) 1.79 / 1.57 (1.61), 300 of 3,300 (22,000) 5.90 / 4.25 (4.22); FP32 factors of FP64 rows: 7.26 / 5.31 (5.52);
+// FP32: 64 of 2,500 (3,300) 0.73 / 0.90 (0.87), 300 of 400 (5,500) 0.53 / 0.46 (0.54), 300 of 3,300 4.17 / 1.51 (2.22).
+constexpr int kLaneRow = 8;
+template <class W, class F>
+__global__ void __launch_bounds__(kSweepThreads) k_factor_lanes(int n, const int* __restrict__ rowPtr, const int* __restrict__ col,
+                                                                const int* __restrict__ diag, const int* __restrict__ ford,
+                                                                const int* __restrict__ elimPtr, const int* __restrict__ elimT,
+                                                                const int* __restrict__ elimQ, const double* __restrict__ val, F* lu,
+                                                                int* flagL, int epoch, unsigned* ctr, int* nreg, int* err) {
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+        __syncwarp();
+        const int base = warp_claim(ctr);
+        if (base >= n) break;
+        if (base + lane >= n) continue;
+        const int i = __ldg(ford + base + lane);
+        const int r0 = __ldg(rowPtr + i), r1 = __ldg(rowPtr + i + 1), d = __ldg(diag + i);
+        W row[kLaneRow * 9];
+        for (int e = 0; e < 9 * (r1 - r0); ++e) row[e] = W(F(__ldg(val + size_t(r0) * 9 + e)));
+        for (int p0 = r0; p0 < d; p0 += 4) {                  // wait for the rows before it (bounded), four polled together
+            int k[4];
+            unsigned pending = 0, ns = 0;
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                k[v] = p0 + v < d ? __ldg(col + p0 + v) : -1;
+                if (k[v] >= 0) pending |= 1u << v;
+            }
+            for (unsigned it = 0; pending; ++it) {
+#pragma unroll
+                for (int v = 0; v < 4; ++v)
+                    if (((pending >> v) & 1u) && ld_relaxed(flagL + k[v]) == epoch) pending &= ~(1u << v);
+                if (!pending || !poll_again(it, ns, err)) break;
+            }
+        }
+        fence_acquire();
+        for (int p = r0; p < d; ++p) {
+            const int k = __ldg(col + p), q0 = __ldg(elimPtr + p), q1 = __ldg(elimPtr + p + 1);
+            const F* u = lu + size_t(__ldg(diag + k)) * 9;
+            W U[9], L[9];
+            W* a = row + size_t(p - r0) * 9;
+#pragma unroll
+            for (int e = 0; e < 9; ++e) U[e] = W(u[e]);
+#pragma unroll
+            for (int e = 0; e < 9; ++e) {                     // L_ik = A_ik U_kk^-1
+                W l = W(0);
+#pragma unroll
+                for (int m = 0; m < 3; ++m) l = fadd(l, fmul(a[3 * (e / 3) + m], U[3 * m + e % 3]));
+                L[e] = l;
+            }
+#pragma unroll
+            for (int e = 0; e < 9; ++e) a[e] = L[e];
+            for (int q = q0; q < q1; ++q) {                   // A_it -= L_ik U_kq
+                const F* f = lu + size_t(__ldg(elimQ + q)) * 9;
+                W* t = row + size_t(__ldg(elimT + q) - r0) * 9;
+#pragma unroll
+                for (int e = 0; e < 9; ++e) U[e] = W(f[e]);
+#pragma unroll
+                for (int e = 0; e < 9; ++e) {
+                    W s = W(0);
+#pragma unroll
+                    for (int m = 0; m < 3; ++m) s = fadd(s, fmul(L[3 * (e / 3) + m], U[3 * m + e % 3]));
+                    t[e] = fsub(t[e], s);
+                }
+            }
+        }
+        double B[9];
+        W* D = row + size_t(d - r0) * 9;
+#pragma unroll
+        for (int e = 0; e < 9; ++e) B[e] = double(D[e]);
+        if (invert_pivot3(B)) atomicAdd(nreg, 1);
+#pragma unroll
+        for (int e = 0; e < 9; ++e) D[e] = W(B[e]);
+        for (int e = 0; e < 9 * (r1 - r0); ++e) lu[size_t(r0) * 9 + e] = F(row[e]);
+        st_release(flagL + i, epoch);
+    }
+}
+
 // ------------------------------------------------------------------ sweeps
 // Input modes of the forward sweep (fusions of the BiCGSTAB vector updates, engine/src/linsolve.cpp:172-186):
 enum { IN_PLAIN = 0, IN_PUPDATE = 1, IN_SUPDATE = 2 };
@@ -787,6 +868,12 @@ template <class W, class F>
 static void launch_factor_t(const DevPlan& P, const double* val, F* lu, W* work, SweepState& S, int epoch, int* nreg, int* err,
                             cudaStream_t st) {
     cudaMemsetAsync(S.ctr + 2, 0, sizeof(unsigned), st);
+    if (P.maxRowBlocks <= kLaneRow && P.avgLevelRows >= (sizeof(W) == 8 ? 70.0 : 30.0) * device_sm_count()) {
+        const int g = std::max(1, std::min(8 * device_sm_count(), (P.n + kSweepThreads - 1) / kSweepThreads));
+        k_factor_lanes<W, F><<<g, kSweepThreads, 0, st>>>(P.n, P.rowPtr, P.col, P.diag, P.ford, P.elimPtr, P.elimT, P.elimQ, val, lu, S.flagL, epoch,
+                                                         S.ctr + 2, nreg, err);
+        return;
+    }
     const int blocks = std::max(1, std::min(P.factorBlocks, (P.n + 3) / 4));
     const int chunk = std::max(1, std::min(8, int(P.avgLevelRows / double(blocks * (kSweepThreads / 32)))));
     k_factor<W, F><<<blocks, kSweepThreads, 0, st>>>(P.n, chunk, P.rowPtr, P.col, P.diag, P.ford, P.elimPtr, P.elimT, P.elimQ, val, lu, work,

@@ -263,3 +263,23 @@ def test_large_batches_of_fp64_vectors(precision, precond, oracle):
         f, _ = (oracle.bilu0_factor if precision == "fp64" else oracle.bilu0_factor_lean)(A)
         ref = (oracle.bilu0_apply if precision == "fp64" else oracle.bilu0_apply_fd)(A, f, r[:3 * A.n])
         assert np.array_equal(z[150, "auto"][:3 * A.n], ref)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "mixed_f32"])
+def test_factors_of_wide_levels(precision, oracle):
+    """Batches whose levels are wide enough for a thread per row, with a singular pivot block in one kind of system and a claim
+    that ends in the middle: the oracle's factors bit for bit, and its count of regularised blocks."""
+    from ressim_gb300.solver import DeviceSolver
+    kinds = [system(100 + k, box(5, 5, 4) + [(99, 100)] * k, seed=k) for k in (0, 1)] + [system(100, box(5, 5, 4), seed=7)]
+    v = kinds[2].val.reshape(-1, 9)
+    v[0] = 0.0                                                             # block (0, 0): nothing is eliminated from it
+    copies = 1303
+    mats = [kinds[k % 3] for k in range(copies)]
+    with DeviceSolver(precond="bilu0", precision=precision) as d:
+        d.set_batch(mats)
+        d.setup()
+        f = d.factors(sum(A.nnzb for A in mats))
+        reg = d.stats().regularised_blocks
+    ref = [{"fp64": oracle.bilu0_factor, "mixed": oracle.bilu0_factor_lean, "mixed_f32": oracle.bilu0_factor_f32}[precision](A) for A in kinds]
+    assert reg == sum(ref[k % 3][1] for k in range(copies)) >= copies // 3
+    assert np.array_equal(f, np.concatenate([ref[k % 3][0].reshape(-1) for k in range(copies)]).reshape(f.shape))
