@@ -315,7 +315,7 @@ int rsg_server_load(rsg_server* s, int* queued, int* running, size_t* bytes_in_u
  * into device memory in the engine's scalar Jacobian layout, so that a Newton step uploads the state (about 50 bytes
  * per cell) instead of the matrix (about 500 bytes per cell) and hands the result to rsg_set_jacobian_device.
  * Replaces Simulator::evalAll / evalCell (engine/src/simulator.cpp:2133-2276, 2429-2459), the cell loop of
- * Simulator::assemble (:2500-2686) and its row scaling dt / PV (:3010-3032), bit for bit, for the standard black-oil
+ * Simulator::assemble (:2500-2686) and its row scaling dt / PV (:3010-3032), bit for bit up to the sign of zeros, for the standard black-oil
  * model: water (PVTW), live oil (saturated nodes + undersaturated ratio tables), dry gas, rock compressibility,
  * unscaled SWOF / SGOF tables, the ECLIPSE default three-phase oil kr, gravity, one PVT and one saturation region.
  * Other model options are rejected with RSG_EINVAL. The wells remain the caller's (the engine's well loop,

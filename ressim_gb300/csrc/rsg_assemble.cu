@@ -13,7 +13,8 @@
 // terms come in as addends to entries of J and R, applied after the reservoir terms and before the row scaling, in
 // the caller's order -- the order in which the engine adds them. Every addition, product and quotient is the
 // reference's, in the reference's order (this file is compiled without contraction into fused multiply-adds), so the
-// Jacobian and residual are the engine's bit for bit.
+// Jacobian and residual are the engine's bit for bit, up to the sign of zeros (terms that are structurally zero are left out:
+// -0 + 0 is not formed).
 //
 // Three kernels per assembly (four with well terms): k_bo_props evaluates every cell's properties with their
 // derivatives, one thread per cell (13 dual numbers, stored component-major so that neighbouring threads read

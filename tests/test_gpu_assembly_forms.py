@@ -43,3 +43,41 @@ def test_short_and_full_forms_match_oracle(slots, eq, gravity, no_oil):
         J, R = asm.assemble(*args)
     assert np.array_equal(J, Jo), np.flatnonzero(J != Jo)[:10]
     assert np.array_equal(R, Ro), np.flatnonzero(R != Ro)[:10]
+
+
+@pytest.mark.parametrize("slots,eq", [((1, 2), (0, 1, 2)), ((2, 1), (2, 0, 1))])
+@pytest.mark.parametrize("gravity", [0.0, 1.0 / 144.0])
+@pytest.mark.parametrize("general", ["sw", "x", "both", "tables"])
+def test_general_cells_among_plain_ones_match_oracle(slots, eq, gravity, general):
+    """Cells that take the full form although everything stays finite: saturations just above 2^256 (single cells among plain
+    ones, neighbours of each other and of no-oil cells), and a model whose tables hold a value that is not finite and that no
+    cell reaches, which makes every cell general."""
+    pytest.importorskip("torch")
+    from oracle import Oracle
+    from ressim_gb300.assembly import BlackOilAssembler
+    z = dict(np.load(os.path.join(GOLDEN, "waterflood_asm.npz"), allow_pickle=False))
+    z["vars"] = np.array([*slots, *eq], dtype=z["vars"].dtype)
+    z["gravity"] = np.array([gravity])
+    na = int(z["na"][0])
+    rng = np.random.default_rng(11)
+    p = rng.uniform(500.0, 6000.0, na)
+    sw = rng.uniform(0.2, 0.8, na)
+    state = rng.integers(0, 2, na).astype(np.uint8)
+    x = np.where(state == 1, rng.uniform(0.0, 0.2, na), rng.uniform(0.0, 1.2, na))
+    acc = rng.standard_normal(3 * na)
+    wide = np.array([7, 8, 60, 61, 200, na - 1])
+    if general in ("sw", "both"):
+        sw[wide[::2]] = 2.0 ** 256 * np.array([1.0, -1.5, 1.25])
+    if general in ("x", "both"):
+        state[wide[1::2]] = 1
+        x[wide[1::2]] = 2.0 ** 256 * np.array([1.0, -1.25, 1.5])
+        state[wide[1] + 1] = 2
+    if general == "tables":
+        z["deadB_x"], z["deadB_y"] = np.array([0.0, 1.0]), np.array([np.inf, 1.0])   # (live oil does not read the dead-oil tables)
+    args = (p, sw, x, state, acc, 3.0)
+    Jo, Ro = Oracle().bo_assemble(z, *args)
+    assert np.isfinite(Jo).all() and np.isfinite(Ro).all()
+    with BlackOilAssembler(z) as asm:
+        J, R = asm.assemble(*args)
+    assert np.array_equal(J, Jo), np.flatnonzero(J != Jo)[:10]
+    assert np.array_equal(R, Ro), np.flatnonzero(R != Ro)[:10]
