@@ -297,9 +297,9 @@ int alloc_plan(rsg_solver* h) {
     }
     if ((h->opt.sweep == 1 || h->opt.sweep == 3) && !h->cta)
         return fail(RSG_EINVAL, "thread-block sweeps need a structurally symmetric pattern of <= 32768 block rows per system");
-    // CPR on the thread-block path: for a batch, the V-cycle's passes grid-wide (all systems at once, the whole
-    // GPU's loads in flight); a single system keeps the one-kernel form (one launch per application instead of a
-    // launch per pass). Both give the same results bit for bit, so a system's result does not depend on its batch.
+    // CPR on the thread-block path: the V-cycle's passes grid-wide (all systems at once, the whole GPU's loads in flight); a
+    // single system keeps the one-kernel form only until its first set-up has chosen its shapes (tune_shapes). Both give
+    // the same results bit for bit, so a system's result does not depend on its batch.
     h->splitCpr = h->cta && (h->opt.sweep == 3 || (h->opt.sweep == 0 && P.nsys > 1));
     for (int v32 = 0; v32 < 2 && h->cta; ++v32) {           // the steps of the ring sweeps, where ilu_stage can ask for them
         if (!ring_wanted(h, v32 != 0)) continue;

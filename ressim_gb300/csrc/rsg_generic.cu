@@ -1162,8 +1162,10 @@ int gen_setup(GenEngine* gp, const rsg_options& o, const double* acc) {
     }
     GEN_CUDA(cudaMemcpyAsync(g.LU, g.S, size_t(g.nnzb) * b2 * sizeof(double), cudaMemcpyDeviceToDevice, g.st));
     const int nlf = int(g.fStart.size()) - 1;
-    // levels of a few rows: every level in one block of four warps; wider ones spread their rows over the GPU, a launch each
-    // (960 rows of 8 x 8 blocks in 31 levels: 9.9 ms in one block)
+    // levels of up to eight rows on average: every level in one block of four warps; wider ones spread their rows over the GPU, a
+    // launch each. BILU0 set-ups, all in one block / by this rule: 960 rows of 8 x 8 blocks in 31 levels 9.3 / 1.4 ms, 512 of 5 x 5 in 22
+    // 3.3 / 0.84, 240 of 16 x 16 in 19 8.0 / 2.4, 1,800 of 4 x 4 in 60 8.3 / 1.3 ms; narrow ones in one block either way: 240 of 4 x 4
+    // in 62 1.0 ms, a chain of 400 5.2 ms
     if (g.n <= 4 * kWarpsPerBlock * nlf / 2) {
         k_gen_factor_cta<<<1, kWarpsPerBlock * 32, 0, g.st>>>(nlf, g.fLvl, g.fOrd, g.nb, g.rp, g.ci, g.dg, g.LU, g.dCnt);
         ++g.launches;

@@ -791,11 +791,11 @@ __global__ void k_gather_blocks(int nnzb, const int* __restrict__ src, const dou
         b[q] = __ldg(a + size_t(__ldg(src + q / 9)) * 9 + q % 9);
 }
 // Four words a thread and round, their loads issued together: a word is two dependent loads (742,384 rows: gather 9.9 -> 9.4 us,
-// scatter 9-10 us either way; a product with both 121.7 -> 120.4 us; 40 MB, 6 us of HBM time).
-template <bool GATHER>
+// scatter 9-10 us either way; a product with both 121.7 -> 120.4 us; 40 MB, 6 us of HBM time). A vector that the grid covers in
+// one round takes a word a thread (80,000 rows: a product 24.6 us, with four 25.8).
+template <bool GATHER, int U>
 __device__ __forceinline__ void permute_vec(int n, const int* __restrict__ perm, const double* __restrict__ from, double* to) {
     const size_t total = size_t(n) * 3, step = size_t(gridDim.x) * blockDim.x;
-    constexpr int U = 4;
     for (size_t q0 = size_t(blockIdx.x) * blockDim.x + threadIdx.x; q0 < total; q0 += U * step) {
         size_t at[U];
         double v[U];
@@ -816,11 +816,13 @@ __device__ __forceinline__ void permute_vec(int n, const int* __restrict__ perm,
         }
     }
 }
+template <int U>
 __global__ void __launch_bounds__(256) k_gather_vec(int n, const int* __restrict__ perm, const double* __restrict__ orig, double* lev) {
-    permute_vec<true>(n, perm, orig, lev);
+    permute_vec<true, U>(n, perm, orig, lev);
 }
+template <int U>
 __global__ void __launch_bounds__(256) k_scatter_vec(int n, const int* __restrict__ perm, const double* __restrict__ lev, double* orig) {
-    permute_vec<false>(n, perm, lev, orig);
+    permute_vec<false, U>(n, perm, lev, orig);
 }
 
 int g_sm_count = 0;
@@ -856,10 +858,14 @@ void launch_gather_blocks(const DevPlan& P, const double* src, double* dst, cuda
     k_gather_blocks<<<stream_grid(size_t(P.nnzb) * 9), 256, 0, st>>>(P.nnzb, P.valSrc, src, dst);
 }
 void launch_gather_vec(const DevPlan& P, const double* orig, double* lev, cudaStream_t st) {
-    k_gather_vec<<<stream_grid(size_t(P.n) * 3), 256, 0, st>>>(P.n, P.perm, orig, lev);
+    const int g = stream_grid(size_t(P.n) * 3);
+    if (size_t(g) * 256 >= size_t(P.n) * 3) k_gather_vec<1><<<g, 256, 0, st>>>(P.n, P.perm, orig, lev);
+    else k_gather_vec<4><<<g, 256, 0, st>>>(P.n, P.perm, orig, lev);
 }
 void launch_scatter_vec(const DevPlan& P, const double* lev, double* orig, cudaStream_t st) {
-    k_scatter_vec<<<stream_grid(size_t(P.n) * 3), 256, 0, st>>>(P.n, P.perm, lev, orig);
+    const int g = stream_grid(size_t(P.n) * 3);
+    if (size_t(g) * 256 >= size_t(P.n) * 3) k_scatter_vec<1><<<g, 256, 0, st>>>(P.n, P.perm, lev, orig);
+    else k_scatter_vec<4><<<g, 256, 0, st>>>(P.n, P.perm, lev, orig);
 }
 
 // a row per warp in a persistent grid; several rows per claim only where a level (of the whole batch) has more rows than the

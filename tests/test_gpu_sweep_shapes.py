@@ -283,3 +283,26 @@ def test_factors_of_wide_levels(precision, oracle):
     ref = [{"fp64": oracle.bilu0_factor, "mixed": oracle.bilu0_factor_lean, "mixed_f32": oracle.bilu0_factor_f32}[precision](A) for A in kinds]
     assert reg == sum(ref[k % 3][1] for k in range(copies)) >= copies // 3
     assert np.array_equal(f, np.concatenate([ref[k % 3][0].reshape(-1) for k in range(copies)]).reshape(f.shape))
+
+
+@pytest.mark.parametrize("n", [1, 85, 86, 207530, 207531, 300001])
+def test_product_on_the_callers_vectors(n):
+    """The permutations into and out of level space at one word a thread, at the line where the grid no longer covers the vector
+    in one round (207,531 rows on 152 SMs) and beyond it with a remainder: a diagonal system's product, exact."""
+    from ressim_gb300.solver import DeviceSolver
+    from ressim_gb300.bsr import BSR
+    rng = np.random.default_rng(n)
+    val = np.zeros((n, 3, 3))
+    val[:, np.arange(3), np.arange(3)] = rng.standard_normal((n, 3))
+    order = rng.permutation(n)                                             # couplings that reverse the row order within levels
+    x = rng.standard_normal((n, 3))
+    pairs = [] if n < 1000 else [(int(min(a, b)), int(max(a, b))) for a, b in zip(order[:500], order[500:1000]) if a != b]
+    rows = np.concatenate([np.arange(n), [p[0] for p in pairs], [p[1] for p in pairs]]).astype(np.int64)
+    cols = np.concatenate([np.arange(n), [p[1] for p in pairs], [p[0] for p in pairs]]).astype(np.int64)
+    o = np.lexsort((cols, rows))
+    v = np.concatenate([val, np.zeros((2 * len(pairs), 3, 3))])[o]
+    A = BSR(n, 3, np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=n))]).astype(np.int32), cols[o].astype(np.int32), v.reshape(-1))
+    with DeviceSolver(precond="bilu0") as d:
+        d.set_matrix(A)
+        y = d.spmv(x.reshape(-1))
+    assert np.array_equal(y, (val[:, np.arange(3), np.arange(3)] * x).reshape(-1))
