@@ -162,6 +162,9 @@ int rsg_set_batch(rsg_solver* h, int nsys, int nb, const int* n, const int* cons
 /* Preconditioner set-up on the device: BILU0 factorisation (and, for CPR, the pressure matrix, the AMG
  * hierarchy and its refresh). acc: optional accumulation blocks (n*nb*nb per system, concatenated) for
  * true-IMPES weights, or NULL for quasi-IMPES (Jacobian diagonal block).
+ * It reserves what its solves reach, the precision form's second attempt with FP64 sweep vectors included; GMRES takes
+ * its basis at the first solve. A set-up that fails (RSG_ENOMEM: the budget) leaves the handle without one: solves
+ * return RSG_ESTATE until a set-up succeeds.
  * Replaces: BILU0::factor (engine/src/bsr.cpp:347-435), BlockCPR::setup (engine/src/bsr.cpp:993-1059). */
 int rsg_setup(rsg_solver* h, const double* acc);
 
